@@ -22,7 +22,7 @@
 // kernel (one CTA per tile, persistent, CTA pairs) per plan.
 #include "common.cuh"
 #include "g2stream.cuh"
-#include "gemm_f64.cuh"
+#include "oz_gemm.cuh"
 #include "tc_gemm.cuh"
 
 #include <algorithm>
@@ -77,6 +77,10 @@ struct LadderPlan {
   DBuf<int32_t> d_by_star, d_star_ptr, d_klo;
   DBuf<double> d_wlo, d_whi, d_g2, d_wq, d_wf, d_R, d_B, d_Bt, d_X, d_Cp, d_Cm;
   long Ktot = 0;
+  // FP64 paths: the products' work buffers, and the digit planes of KK, G̃ and (per chunk, as B̃) B̃
+  OzWork oz;
+  OzPlanes ozKK, ozGt;
+  std::vector<OzPlanes> ozBt;
   double Bt_T = std::numeric_limits<double>::quiet_NaN();  // temperature B̃ was built for
   // GEMM paths: rows (j, q, c0, ri) with j padded to nwp (a multiple of 32), K = (ν, b, i') with ν
   // padded to nmp (a multiple of 16)
@@ -1644,6 +1648,7 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
     EPSP_LAUNCHED(ctx);
     P->d_B.alloc(ctx, size_t(ns * maxnf * ni * 2));
     P->d_Bt.alloc(ctx, size_t(P->Ktot * 6 * ni));
+    P->ozBt.resize(P->chunks.size());
     P->d_X.alloc(ctx, size_t(16 * nw * ns * 3 * maxnip));
     P->d_Cp.alloc(ctx, size_t(16 * nw * 6 * ni));
     P->d_Cm.alloc(ctx, size_t(16 * nw * 6 * ni));
@@ -1712,6 +1717,7 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
     if (!tc_path(P->path)) P->d_D.alloc(ctx, size_t(M * N));  // the tensor-core paths keep D as split-K parts
     if (P->path == EPSP_PATH_GEMM_FP64) {
       P->d_Af.alloc(ctx, size_t(M * P->Kx));
+      oz_split(ctx, P->d_Gt.p, P->Kx, N, P->Kx, true, oz_tile_n(N), P->ozGt);
     } else {
       plog.mark("g2 streamed, G~ built");
       // mode tables: for node j, mode ν and sign s, the two shift tables (m_ν, m_ν + 1) with the
@@ -1856,6 +1862,8 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
   } else {
     P->d_Y.alloc(ctx, size_t(nw * 48 * ni));
     P->d_KY.alloc(ctx, size_t(nw * 48 * ni));
+    oz_split(ctx, P->d_KK.p, nw, nw, nw, false, kOzBoxM, P->ozKK);
+    EPSP_CUDA(cudaStreamSynchronize(s));
     P->d_Gm.alloc(ctx, size_t(nw * 4 * ni));
     P->d_Gp.alloc(ctx, size_t(nw * 4 * ni));
   }
@@ -1924,6 +1932,8 @@ static void build_Bt(LadderPlan* P, double T) {
     star_sum_kernel<<<div_up(size_t(total), 256), 256, 0, s>>>(P->d_B.p, P->d_R.p, P->d_by_star.p, P->d_star_ptr.p, c.i0, nip,
                                                                c.f0, nfc, int(ns), int(ni), P->Ktot, c.k_off, P->d_Bt.p);
     EPSP_LAUNCHED(ctx);
+    oz_split(ctx, P->d_Bt.p + c.k_off, P->Ktot, 6 * ni, ns * 3 * nip, true, oz_tile_n(6 * ni),
+             P->ozBt[size_t(&c - P->chunks.data())]);
   }
   P->Bt_T = T;
 }
@@ -1967,15 +1977,15 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
                                                                             P->d_X.p);
         EPSP_LAUNCHED(ctx);
         long pg = prof_begin(ctx, "ladder_gemm");
-        gemm_f64(ctx, false, int(nrow), int(ncol), int(kc), 1.0, P->d_X.p, nrow, P->d_Bt.p + c.k_off, P->Ktot, 1.0,
-                 sg == 0 ? P->d_Cp.p : P->d_Cm.p, nrow);
+        oz_gemm(ctx, P->oz, nrow, ncol, kc, P->d_X.p, nrow, nullptr, P->d_Bt.p + c.k_off, P->Ktot,
+                &P->ozBt[size_t(&c - P->chunks.data())], 1.0, sg == 0 ? P->d_Cp.p : P->d_Cm.p, nrow);
         prof_end(ctx, pg);
       }
     }
     const long ny = nw * 48 * ni;
     y_direct_kernel<<<div_up(size_t(ny), 256), 256, 0, s>>>(P->d_Cp.p, P->d_Cm.p, ny, P->d_Y.p);
     EPSP_LAUNCHED(ctx);
-    gemm_f64(ctx, false, int(nw), int(48 * ni), int(nw), 1.0, P->d_KK.p, nw, P->d_Y.p, nw, 0.0, P->d_KY.p, nw);
+    oz_gemm(ctx, P->oz, nw, 48 * ni, nw, P->d_KK.p, nw, &P->ozKK, P->d_Y.p, nw, nullptr, 0.0, P->d_KY.p, nw);
     finish_direct_kernel<<<div_up(size_t(nw * 6 * ni), 256), 256, 0, s>>>(P->d_Cp.p, P->d_Cm.p, P->d_KY.p, P->d_Gm.p, P->d_Gp.p,
                                                                           int(nw), int(ni), LJ);
     EPSP_LAUNCHED(ctx);
@@ -1991,12 +2001,12 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, px);
   long pg = prof_begin(ctx, "ladder_gemm");
-  gemm_f64(ctx, false, int(M), int(N), int(P->Kx), 1.0, P->d_Af.p, M, P->d_Gt.p, P->Kx, 0.0, P->d_D.p, M);
+  oz_gemm(ctx, P->oz, M, N, P->Kx, P->d_Af.p, M, nullptr, P->d_Gt.p, P->Kx, &P->ozGt, 0.0, P->d_D.p, M);
   prof_end(ctx, pg);
   const long ny = nw * 8 * N;
   y_gemm_kernel<<<div_up(size_t(ny), 256), 256, 0, s>>>(P->d_D.p, int(nw), int(nwp), N, P->d_Y.p);
   EPSP_LAUNCHED(ctx);
-  gemm_f64(ctx, false, int(nw), int(8 * N), int(nw), 1.0, P->d_KK.p, nw, P->d_Y.p, nw, 0.0, P->d_KY.p, nw);
+  oz_gemm(ctx, P->oz, nw, 8 * N, nw, P->d_KK.p, nw, &P->ozKK, P->d_Y.p, nw, nullptr, 0.0, P->d_KY.p, nw);
   finish_gemm_kernel<double><<<dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, s>>>(
       P->d_D.p, M, 1, 0, P->d_KY.p, 1, 0, P->d_Gm.p, P->d_Gp.p, nullptr, int(nw), int(nwp), int(ni), LJ, X);
   EPSP_LAUNCHED(ctx);
@@ -2051,7 +2061,10 @@ static void apply_L(LadderPlan* P, const float2* J, float2* LJ, const float2* X 
 }
 
 static void check_tc_err(LadderPlan* P) {
-  if (!tc_path(P->path)) return;
+  if (!tc_path(P->path)) {
+    oz_check(P->ctx, P->oz);
+    return;
+  }
   int e = 0;
   P->d_err.download(&e, 1, P->ctx->stream);
   EPSP_CUDA(cudaStreamSynchronize(P->ctx->stream));
@@ -2297,7 +2310,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
                                                P->g_sn.p, P->g_z.p, P->g_st.p, P->g_inv.p);
           EPSP_LAUNCHED(ctx);
           P->g_st.download(&gs, 1, s);
-          if (tc) P->d_err.download(&werr, 1, s);
+          (tc ? P->d_err : P->oz.err).download(&werr, 1, s);
           if (inner == 1) {
             EPSP_CUDA(cudaMemcpyAsync(Yb.data(), Ybuf.p, size_t(ny) * sizeof(cplx), cudaMemcpyDeviceToHost, s));
             if (warm && !needJ)
@@ -2312,7 +2325,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
           prof_end(ctx, pbl);
           EPSP_CUDA(cudaStreamSynchronize(s));
           if (werr) {
-            P->d_err.zero(s);
+            (tc ? P->d_err : P->oz.err).zero(s);
             fail(EPSP_EDEVICE_TIMEOUT, "a tensor-core GEMM wait ran out (bounded device wait)");
           }
           if (inner == 1) {

@@ -11,7 +11,6 @@
 #include "common.cuh"
 #include "fp_pair.cuh"
 #include "g2stream.cuh"
-#include "gemm_f64.cuh"
 #include "scgd0.cuh"
 #include "warmstart.cuh"
 
@@ -1067,12 +1066,17 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
     P->d_Fe.alloc(ctx, size_t(P->nw * nm));
     if (P->path == EPSP_PATH_GEMM_FP64) {
       P->d_Kt.alloc(ctx, size_t(P->nw * nm * P->nc));
+      oz_split(ctx, P->d_G.p, nm * P->nc, ni, nm * P->nc, true, oz_tile_n(ni), P->ozG);
     } else {
       tc_setup(P);
     }
     EPSP_CUDA(cudaStreamSynchronize(s));
   } else {
     fail(EPSP_EINVAL, "unknown path");
+  }
+  if (P->path != EPSP_PATH_GEMM_BF16) {
+    oz_split(ctx, P->d_KK.p, P->nw, P->nw, P->nw, false, kOzBoxM, P->ozKK);
+    EPSP_CUDA(cudaStreamSynchronize(s));
   }
   plog.mark("cells, tensor-core operands");
   // iteration buffers
@@ -1125,7 +1129,7 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
     prof_end(ctx, pk);
     long pg = prof_begin(ctx, "fm_gemm");
     // ImΣ[ω, i] += Σ_k K_t[ω, k] G[k, i]
-    gemm_f64(ctx, false, int(nw), int(ni), int(nk), 1.0, P->d_Kt.p, nw, P->d_G.p, nk, 1.0, d_ImS, nw);
+    oz_gemm(ctx, P->oz, nw, ni, nk, P->d_Kt.p, nw, nullptr, P->d_G.p, nk, &P->ozG, 1.0, d_ImS, nw);
     prof_end(ctx, pg);
     return;
   }
@@ -1284,12 +1288,13 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
           P->d_ImS.zero(s);
           scgd0_imsigma(P, Sin_b.p + slab * a, mu[size_t(iT)], occ->Tlist[iT], P->d_ImS.p);
           long pk = prof_begin(ctx, "kk");
-          gemm_f64(ctx, false, int(nw), int(ni), int(nw), 1.0, P->d_KK.p, nw, P->d_ImS.p, nw, 0.0, P->d_ReS.p, nw);
+          oz_gemm(ctx, P->oz, nw, ni, nw, P->d_KK.p, nw, &P->ozKK, P->d_ImS.p, nw, nullptr, 0.0, P->d_ReS.p, nw);
           assemble_kernel<<<eb, 256, 0, s>>>(P->d_ReS.p, P->d_ImS.p, Snew.p + slab * iT, slab);
           EPSP_LAUNCHED(ctx);
           prof_end(ctx, pk);
         }
       }
+      if (!f32_spec) EPSP_CUDA(cudaMemcpyAsync(d_tcerr, P->oz.err.p, sizeof(int), cudaMemcpyDeviceToDevice, s));
       if (P->nmult > 0 && !f32_spec) {
         multiplet_kernel<<<dim3(div_up(size_t(nw * P->nmult), 256), unsigned(nA)), 256, 0, s>>>(
             Snew.p, int(nw), slab, d_slots.p, P->d_mptr.p, P->d_midx.p, P->nmult);
@@ -1372,11 +1377,12 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
     }
     EPSP_CUDA(cudaMemcpyAsync(h_pack, d_pack.p, npack * sizeof(double), cudaMemcpyDeviceToHost, s));
     EPSP_CUDA(cudaStreamSynchronize(s));
-    if (P->path == EPSP_PATH_GEMM_BF16) {
+    {
       int tcerr = 0;
       std::memcpy(&tcerr, &h_pack[size_t(4 * nT)], sizeof(int));
       if (tcerr) {
-        EPSP_CUDA(cudaMemsetAsync(tc_err_ptr(P), 0, sizeof(int), s));  // the plan's next run starts clean
+        int* flag = P->path == EPSP_PATH_GEMM_BF16 ? tc_err_ptr(P) : P->oz.err.p;
+        EPSP_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));  // the plan's next run starts clean
         fail(EPSP_EDEVICE_TIMEOUT, "a tensor-core GEMM wait ran out (bounded device wait)");
       }
     }
@@ -1521,6 +1527,7 @@ epsp_status epsp_scgd0_imsigma(epsp_scgd0_plan* plan, const double* sigma_in, do
     P->d_Sin.upload(reinterpret_cast<const double2*>(sigma_in), n, s);
     P->d_ImS.upload(imsigma, n, s);
     scgd0_imsigma(P, P->d_Sin.p, mu, T, P->d_ImS.p);
+    oz_check(P->ctx, P->oz);
     P->d_ImS.download(imsigma, n, s);
     EPSP_CUDA(cudaStreamSynchronize(s));
   });

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "oz_gemm.cuh"
 
 #include <memory>
 
@@ -37,6 +38,9 @@ struct Scgd0Plan {
   int64_t nf_chunk = 1;
   DBuf<double> d_g2t, d_wqt, d_eps_f, d_w_f;
   DBuf<int32_t> d_f_to_i;
+  // FP64 paths: the products' work buffers, and the digit planes of the operands that do not change
+  OzWork oz;
+  OzPlanes ozKK, ozG;
   // GEMM paths
   bool star_reduced = false;
   long nc = 0;

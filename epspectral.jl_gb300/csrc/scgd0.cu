@@ -166,6 +166,149 @@ __global__ void __launch_bounds__(kFmTile) fm_direct_kernel(
   if (iw < nw) imsigma[iw + long(nw) * i] += acc;
 }
 
+// The same sum with the FP64 operations of a term cut from about 160 to 27: FP64 instructions issue at
+// 1/64 of the FP32 and integer rate here and bound the kernel (the term-by-term kernel above ran at that
+// limit, on 30 of 152 SMs at 126 nodes and 30 states).
+//  * Interpolation: Σ(x) = Σ_j + (x - ω_j) Σ'_j from a table per column, 4 doubles per cell: ω_j - ReΣ_j,
+//    ImΣ_j, 1 - ReΣ'_j, ImΣ'_j (fm_cell_kernel), so that Re z = (U_j - ε) + (x - ω_j) E_j and Im Σ cost one
+//    operation each beside x - ω_j; the flat continuation is an entry before and after the grid. The
+//    cell is found without FP64: an FP32 bucket, lowered by a guard above its error, then two comparisons
+//    on the values' ordered integers.
+//  * Occupations: with E = exp((ω - μ)/T), e = exp(ωq/T): n + f(x_a - μ) = (1 + n)(1 + E)/(1 + E e) and
+//    n + 1 - f(x_e - μ) = n (1 + E)/(1 + E/e) (detailed balance; no difference is taken), so a term
+//    needs no exponential, and 1 + E leaves the sum. For E > 1 both sides are divided by E (p + q e with
+//    (p, q) = (1/E, 1) in place of (1, E)). E and e carry the rounding of their arguments as a factor.
+//  * One reciprocal per term: N_a/D_a + N_e/D_e = (N_a D_e + N_e D_a)/(D_a D_e), from an FP32 seed of the
+//    mantissa (the exponent by integers) and one third-order Newton step (2^-23 -> 2^-69). A denominator that is
+//    0, not finite or subnormal takes the plain formula.
+// The sum over (ν, f) is split over blockIdx.z (partials summed in order by fm_add_kernel) until the SMs
+// have work. Needs T > 0 with ωq/T <= 300 (e^300 squared times the denominators stays in range),
+// ω_acoustic > 0 and a guard below half a bucket; other calls run the kernel above.
+// Measured (126 nodes, 30 states, 5 modes x 375 inner states; and 401, 33, 1 x 64): 9.88 -> 0.433 ms,
+// 0.355 -> 0.074 ms: about 36 operations' time a term with the staging, of the 27 it issues.
+struct FmPair {
+  double g1, g0, e, ie, wq, eps;  // w_f g2 (1 + n), w_f g2 n, exp(±ωq/T), ωq, ε
+};
+
+// Cell table of every column: entry j + 1 holds cell j, entry 0 the flat part below the grid.
+__global__ void fm_cell_kernel(const double* __restrict__ ws, int nw, const double2* __restrict__ Sin, long ncol,
+                               double4* __restrict__ tab) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= (nw + 1l) * ncol) return;
+  const int j = int(k % (nw + 1)) - 1;
+  const double2* col = Sin + long(nw) * (k / (nw + 1));
+  const int b = max(j, 0);
+  const double2 lo = col[b];
+  double4 o;
+  o.x = ws[b] - lo.x;
+  o.y = lo.y;
+  o.z = 1.0;
+  o.w = 0.0;
+  if (j >= 0 && j < nw - 1) {
+    const double inv = 1.0 / (ws[j + 1] - ws[j]);
+    o.z = 1.0 - (col[j + 1].x - lo.x) * inv;
+    o.w = (col[j + 1].y - lo.y) * inv;
+  }
+  tab[k] = o;
+}
+
+// A double as an integer of the same order.
+__host__ __device__ __forceinline__ long long ordered(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+
+__device__ __forceinline__ double recip_seeded(double d) {
+  const int hi = __double2hiint(d), lo = __double2loint(d);
+  const float m = __uint_as_float(0x3f800000u | ((uint32_t(hi) & 0xfffffu) << 3) | (uint32_t(lo) >> 29));
+  float s;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(m));  // in (1/2, 1]
+  const uint32_t b = __float_as_uint(s);
+  const int ex = int(b >> 23) + (1023 - 127) - (((hi >> 20) & 0x7ff) - 1023);
+  const double r = __hiloint2double(int((uint32_t(ex) << 20) | ((b >> 3) & 0xfffffu)), int(b << 29));
+  const double h = fma(-d, r, 1.0);
+  return fma(r, fma(h, h, h), r);
+}
+
+constexpr int kFmFastTile = 128;  // staged (ν, f) pairs
+
+__global__ void __launch_bounds__(128) fm_direct_fast_kernel(
+    const double* __restrict__ ws, int nw, const long long* __restrict__ wkey, const int32_t* __restrict__ jtab, int ntab,
+    float x0f, float inv_hf, float guard, const double4* __restrict__ tab, const double* __restrict__ g2t,
+    const double* __restrict__ wqt, long nvf, const double* __restrict__ eps_f, const double* __restrict__ w_f,
+    const int32_t* __restrict__ f_to_i, int nm, long vf0, long vf1, long per, double mu, double T, double w_ac,
+    double* __restrict__ part) {
+  __shared__ FmPair sp[kFmFastTile];
+  __shared__ int s_col[kFmFastTile];
+  const int i = blockIdx.y;
+  const int iw = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool in = iw < nw;
+  const double w = in ? ws[iw] : ws[0];
+  const float wf = float(w);
+  // exp(v / T), the rounding of v / T put back as a factor
+  auto ex = [&](double v) {
+    const double a = v / T, E = exp(a);
+    return E > 0.0 && E < INFINITY ? fma(E, fma(-a, T, v) / T, E) : E;
+  };
+  const bool below = w <= mu;
+  const double Ew = ex(below ? w - mu : mu - w);  // E, or 1/E above μ
+  const double p = below ? 1.0 : Ew, q = below ? Ew : 1.0;
+  const long t_end = min(vf1, vf0 + per * (long(blockIdx.z) + 1));
+  double acc = 0.0;
+  for (long t0 = vf0 + per * long(blockIdx.z); t0 < t_end; t0 += kFmFastTile) {
+    const int nt = int(min(long(kFmFastTile), t_end - t0));
+    __syncthreads();
+    for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+      const long vf = t0 + k, f = vf / nm;
+      const double wq = wqt[vf + nvf * i];
+      s_col[k] = wq < w_ac ? -1 : f_to_i[f];
+      if (!(wq < w_ac)) {
+        const double g = w_f[f] * g2t[vf + nvf * i], nq = occ_boson_d(wq, T);
+        sp[k] = FmPair{g * (nq + 1.0), g * nq, ex(wq), ex(-wq), wq, eps_f[f]};
+      }
+    }
+    __syncthreads();
+    if (!in) continue;
+    // the cell of x (as cell + 1: the table's entry) and x - ω_cell
+    auto cell = [&](double x, float xf, int& e) -> double {
+      const float v = fminf(fmaxf((xf - x0f) * inv_hf - guard, 0.f), float(ntab - 1));
+      const int c = jtab[int(v)];
+      const long long kx = ordered(__double_as_longlong(x));
+      e = c + (kx >= wkey[c] ? 1 : 0) + (kx >= wkey[c + 1] ? 1 : 0);
+      return x - ws[max(e - 1, 0)];
+    };
+#pragma unroll 2
+    for (int k = 0; k < nt; ++k) {
+      if (s_col[k] < 0) continue;
+      const FmPair P = sp[k];
+      const double4* col = tab + (nw + 1l) * s_col[k];
+      const float wqf = float(P.wq);
+      int ea, ee;
+      const double da = cell(w + P.wq, wf + wqf, ea), de = cell(w - P.wq, wf - wqf, ee);
+      const double4 A = col[ea], B = col[ee];
+      const double zar = fma(da, A.z, A.x - P.eps), sia = fma(da, A.w, A.y);
+      const double zer = fma(de, B.z, B.x - P.eps), sie = fma(de, B.w, B.y);
+      const double dna = fma(zar, zar, sia * sia), dne = fma(zer, zer, sie * sie);
+      const double oa = fma(q, P.e, p), oe = fma(q, P.ie, p);
+      const double Da = dna * oa, De = dne * oe;
+      const double Na = P.g1 * sia, Ne = P.g0 * sie;
+      const double D = Da * De;
+      const int E = (__double2hiint(D) >> 20) & 0x7ff;
+      if (E > 0 && E < 0x7f0)
+        acc = fma(fma(Na, De, Ne * Da), recip_seeded(D), acc);
+      else
+        acc += Na / dna / oa + Ne / dne / oe;
+    }
+  }
+  if (in) part[iw + long(nw) * (i + long(gridDim.y) * blockIdx.z)] = acc * (p + q);
+}
+
+// ImΣ += Σ_s part[s] in ascending s.
+__global__ void fm_add_kernel(const double* __restrict__ part, long n, int splits, double* __restrict__ imsigma) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  double v = 0.0;
+  for (int s = 0; s < splits; ++s) v += part[k + n * s];
+  imsigma[k] += v;
+}
+
 // The occupation factors of the recast sum, per (ω, ν): F_abs = n_ν + f(ω + ω_ν - μ) and
 // F_emi = n_ν + 1 - f(ω - ω_ν - μ) (the two brackets of src/scgd0_kernel.jl:37-38); 0 for a mode
 // below ω_acoustic.
@@ -950,7 +1093,27 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
     P->d_eps_f = to_device(ctx, m->eps_f, size_t(nf));
     P->d_w_f = to_device(ctx, m->w_f, size_t(nf));
     P->d_f_to_i = to_device(ctx, m->f_to_i, size_t(nf));
-    EPSP_CUDA(cudaStreamSynchronize(s));
+    {  // fm_direct_fast_kernel: the nodes as ordered integers (one above all values after them), the largest ωq, and the
+       // FP32 bucket's guard: x, x - x0 and the product round by 2^-24 of at most 9 max|ω| + 5 max ωq, over h, in all
+      std::vector<long long> key(size_t(P->nw) + 1);
+      double big = 0;
+      for (long j = 0; j < P->nw; ++j) {
+        long long b;
+        std::memcpy(&b, &P->ws.nodes[size_t(j)], 8);
+        key[size_t(j)] = ordered(b);
+        big = std::max(big, std::fabs(P->ws.nodes[size_t(j)]));
+      }
+      key[size_t(P->nw)] = std::numeric_limits<long long>::max();
+      P->d_wkey = to_device(ctx, key);
+      for (int64_t k = 0; k < nm * m->nq; ++k) {
+        if (!std::isfinite(m->omega_ph[k])) P->wq_max = std::numeric_limits<double>::infinity();
+        P->wq_max = std::max(P->wq_max, m->omega_ph[k]);
+      }
+      const double guard = (12 * (big + std::min(P->wq_max, 1e30)) * P->ct.inv_h + 8) * 0x1p-24;
+      P->fm_guard = float(guard);
+      P->fm_fast = P->w_ac > 0 && guard < 0.4;
+      EPSP_CUDA(cudaStreamSynchronize(s));  // key is a local
+    }
   } else if (P->path == EPSP_PATH_GEMM_BF16 && [&] {
                std::vector<double> w;
                return !dispersionless(m, w);
@@ -1100,13 +1263,39 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
   const long nm = P->nm, ni = P->ni, nf = P->nf, nw = P->nw;
   if (P->path == EPSP_PATH_DIRECT_FP64) {
     const long nvf = nm * nf;
-    dim3 grid(div_up(size_t(nw), kFmTile), unsigned(ni));
+    const bool fast = P->fm_fast && T > 1.4901161193847656e-08 && P->wq_max <= 300.0 * T;
+    // warps of 32 nodes a block, 4 or fewer where that leaves fewer idle (a block stages its pairs itself)
+    const long nwarp = div_up(size_t(nw), 32);
+    int wpb = 4;
+    for (int k = 3; k >= 2; --k)
+      if (div_up(size_t(nwarp), size_t(k)) * k < div_up(size_t(nwarp), size_t(wpb)) * wpb) wpb = k;
+    const dim3 tiles(fast ? div_up(size_t(nwarp), size_t(wpb)) : div_up(size_t(nw), kFmTile), unsigned(ni));
+    if (fast) {
+      const long n = (nw + 1) * ni;
+      ensure(P->w_fmtab, ctx, size_t(n));
+      fm_cell_kernel<<<div_up(size_t(n), 128), 128, 0, s>>>(P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
+      EPSP_LAUNCHED(ctx);
+    }
     for (long f0 = 0; f0 < nf; f0 += P->nf_chunk) {
       long f1 = std::min(nf, f0 + P->nf_chunk);
       long pi = prof_begin(ctx, "fan_migdal");
-      fm_direct_kernel<<<grid, kFmTile, 0, s>>>(P->d_ws.p, int(nw), P->ct, d_Sin, P->d_g2t.p, P->d_wqt.p, nvf,
-                                                P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm), nm * f0, nm * f1, mu, T,
-                                                P->w_ac, d_ImS);
+      if (fast) {
+        // splits of the (ν, f) range: 32 warps a multiprocessor, 32 pairs a split at least
+        const long len = nm * (f1 - f0), want = 32l * ctx->sm_count / (long(tiles.x) * ni * wpb) + 1;
+        const long per = std::max<long>(32, (len + want - 1) / want);
+        const int splits = int((len + per - 1) / per);
+        ensure(P->w_fmpart, ctx, size_t(nw * ni * splits));
+        fm_direct_fast_kernel<<<dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0, s>>>(
+            P->d_ws.p, int(nw), P->d_wkey.p, P->d_jtab.p, int(P->d_jtab.n), float(P->ct.x0), float(P->ct.inv_h),
+            P->fm_guard, P->w_fmtab.p, P->d_g2t.p, P->d_wqt.p, nvf, P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm),
+            nm * f0, nm * f1, per, mu, T, P->w_ac, P->w_fmpart.p);
+        EPSP_LAUNCHED(ctx);
+        fm_add_kernel<<<div_up(size_t(nw * ni), 128), 128, 0, s>>>(P->w_fmpart.p, nw * ni, splits, d_ImS);
+      } else {
+        fm_direct_kernel<<<tiles, kFmTile, 0, s>>>(P->d_ws.p, int(nw), P->ct, d_Sin, P->d_g2t.p, P->d_wqt.p, nvf,
+                                                   P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm), nm * f0, nm * f1, mu,
+                                                   T, P->w_ac, d_ImS);
+      }
       EPSP_LAUNCHED(ctx);
       prof_end(ctx, pi);
     }

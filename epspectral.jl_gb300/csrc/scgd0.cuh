@@ -38,6 +38,13 @@ struct Scgd0Plan {
   int64_t nf_chunk = 1;
   DBuf<double> d_g2t, d_wqt, d_eps_f, d_w_f;
   DBuf<int32_t> d_f_to_i;
+  // ... fm_direct_fast_kernel's node keys, cell table and partial sums; whether the grid allows it
+  DBuf<long long> d_wkey;
+  DBuf<double4> w_fmtab;
+  DBuf<double> w_fmpart;
+  double wq_max = 0;
+  float fm_guard = 0.f;
+  bool fm_fast = false;
   // FP64 paths: the products' work buffers, and the digit planes of the operands that do not change
   OzWork oz;
   OzPlanes ozKK, ozG;

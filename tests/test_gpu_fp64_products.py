@@ -78,3 +78,30 @@ def test_not_finite_values_go_where_the_sums_take_them(api, oracle):
     assert np.array_equal(np.isnan(got), np.isnan(ref))
     fin = ~np.isnan(ref)
     assert rel(got[fin], ref[fin]) <= 4e-12
+
+
+# ---- the term-by-term FP64 sum (DIRECT_FP64) ----
+# The same terms as the oracle's, to a few roundings each (2^-53 of |x| <= 1.3 against |z| >= 0.05: 3e-15), all of one
+# sign: the sum's own gate of 1e-13 (the Fan-Migdal test of the reference's kernel) holds at every size.
+@pytest.mark.parametrize("nw,ni,nm,nf,T,mu", [
+    (2, 1, 1, 1, 0.03, 0.07), (33, 2, 1, 31, 0.03, -2.0), (127, 3, 2, 16, 0.03, 2.0), (129, 5, 3, 11, 0.003, 0.07),
+    (65, 7, 4, 75, 8.4e-4, 0.0), (65, 7, 4, 75, 5e-4, 0.0), (40, 3, 2, 9, 0.0, 0.07), (97, 33, 5, 101, 0.5, 0.3)])
+@pytest.mark.parametrize("graded", [False, True])
+def test_direct_sum_matches_oracle(api, oracle, nw, ni, nm, nf, T, mu, graded):
+    from test_oracle_scgd0 import per_pair_setup
+    off = np.arange(nw) if not graded else np.cumsum(1 + 4 * (np.abs(np.arange(nw) - nw // 2) > nw // 4))
+    g = FrequencyGrid(-1.0, 2.0 / (off[-1] - off[0]), off - off[0])
+    wq = 0.05 + 0.2 * np.abs(R.pseudorandom(nm, ni, nf, seed=10))
+    g2 = np.abs(R.pseudorandom(nm, ni, nf, seed=9))
+    if ni > 2:
+        wq[0, 1, :], g2[0, 1, :] = 0.0, np.inf  # below the acoustic cutoff: never read
+    s = per_pair_setup(g, g2, wq, 0.8 * R.pseudorandom(nf, seed=11),
+                       np.array([(5 * (f + 1)) % ni for f in range(nf)], dtype=np.int32), np.full(nf, 1.0 / nf))
+    S = _sigma(nw, ni)
+    ref = oracle.imsigma(s, S, mu, T, np.zeros((nw, ni)), omega_acoustic=1e-3)
+    for tile in (None, 7):
+        plan = api.Scgd0Plan(s, path="direct_fp64", omega_acoustic=1e-3, gpu_tile=tile)
+        got = plan.imsigma(S, mu, T, np.zeros((nw, ni)))
+        assert np.all(np.isfinite(got)) and rel(got, ref) <= 1e-13
+        assert np.array_equal(plan.imsigma(S, mu, T, np.zeros((nw, ni))), got)
+        plan.close()

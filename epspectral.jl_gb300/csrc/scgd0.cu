@@ -1420,6 +1420,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
     const long cap0 = tc_capacity(P);
     tc_reserve(P, nT);
     grown |= tc_capacity(P) != cap0;
+    tc_disp_choose(P, occ->Tlist, nT);
   }
   if (grown) ++P->w_gen;
   std::vector<TParams> h_tp(static_cast<size_t>(nT));
@@ -1429,10 +1430,11 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   bool use_graph = P->path == EPSP_PATH_GEMM_BF16;
   for (const char* nm : kBodyProfiles)
     if (ctx->prof_name == nm) use_graph = false;
-  // a replayed graph bakes in the buffers, nT, fix_mu, the spin degeneracy and the active count
+  // a replayed graph bakes in the buffers, nT, fix_mu, the spin degeneracy, the active count and the choice of the
+  // dispersive kernel
   auto graph_key = [&](int nA) {
     return std::array<long, 6>{long(nA), long(nT), long(fix_mu), P->w_gen,
-                               long(std::llround(occ->spin_degeneracy * 1e6)), long(P->path)};
+                               long(std::llround(occ->spin_degeneracy * 1e6)), long(P->path) + 16 * long(P->fd_fast)};
   };
   for (int32_t iter = 1; iter <= maxiter; ++iter) {
     auto t0 = std::chrono::steady_clock::now();

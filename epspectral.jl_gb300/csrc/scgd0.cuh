@@ -57,6 +57,7 @@ struct Scgd0Plan {
   // w_f g2 [ν f, i] (FP32), ωph, the pair table and its indices, ε_f, f_to_i, the nodes
   // as float pairs with their neighbouring cells' inverse widths, the bucket table's origin and scale
   bool disp = false;
+  bool fd_fast = false;  // this call's temperatures allow fm_disp_fast_kernel
   long nk_i = 0, ntab = 0;
   float x0f = 0.f, inv_hf = 0.f;
   DBuf<float> d_gwf;
@@ -98,6 +99,7 @@ struct Scgd0Plan {
 void tc_setup(Scgd0Plan* P);
 // The FP32 term-by-term Fan-Migdal sum's tables for a model with dispersive modes (before tc_setup).
 void tc_setup_dispersive(Scgd0Plan* P, const epsp_model* m);
+void tc_disp_choose(Scgd0Plan* P, const double* Tlist, long nT);
 void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS);
 void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, double* d_ImS);
 // The g2 upload of the term-by-term sums: g2 [nm, ni, nf] of any dtype to [nm nf, ni] FP64 (scgd0.cu).

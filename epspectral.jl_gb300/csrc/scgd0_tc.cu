@@ -13,6 +13,7 @@
 #include "tc_gemm.cuh"
 
 #include <algorithm>
+#include <limits>
 
 namespace epsp {
 
@@ -43,6 +44,10 @@ struct Scgd0Plan::Tc {
   DBuf<float2> xf, ef;
   DBuf<float> tf, Ff;
   DBuf<float4> Sf;
+  // dispersive modes: cell records and Im slopes of every column and slot, partial sums of the splits
+  DBuf<float4> fdrec;
+  DBuf<float> fddim;
+  DBuf<double> fdpart;
   // 1 for modes below the acoustic cutoff (left out of the sum)
   DBuf<uint8_t> skip;
   // batched iteration: capacity in temperatures, ImΣ of every slot
@@ -355,6 +360,165 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
   }
 }
 
+// The same sum in about 70 instructions a term (issue slots bound it; fm_disp_f32_kernel above takes about 180), for
+// temperatures above ωq / 40:
+//  * cells with slopes: record (side, c) of a column describes the cell above (side 1) or below (side 0) node c
+//    from that node: ω_c - ReΣ_c as a float pair, 1 - ReΣ', ImΣ_c, ImΣ', so that Re z = (U_hi - ε_hi) +
+//    ((U_lo - ε_lo) + (x - ω_c)(1 - ReΣ')): the first difference is exact where Re z is small against its parts, and
+//    outside the grid the record's slopes are 0 (fd_cell_kernel). No weight, no boundary test.
+//  * n + f(x_a - μ) = (1 + n)(1 + E)/(1 + E e) and n + 1 - f(x_e - μ) = n (1 + E)/(1 + E/e), E = exp((ω - μ)/T),
+//    e = exp(ωq/T): one FMA a side, the bracket's reciprocal shared with 1/|z|², and 1 + E outside the sum
+//    (both sides over E above μ, so that every factor stays below e^40).
+// The records of one side are contiguous over the nodes (four wavefronts of L1 a load); the bucket table is 16-bit
+// in shared memory. Grid (nω / 256, ni, slots x splits): the (ν, f) range is split, in whole tiles, until the
+// last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
+// 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
+// Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 -> 3.25 ms;
+// the L1 data pipe is then 92 % busy (about 24 wavefronts a term and warp, half records, half shared memory) and
+// the issue slots 71 %.
+constexpr float kFdMaxArg = 40.f;
+
+__device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v / T's rounding put back
+  const float a = v / T, E = expf(a);
+  return fmaf(E, fmaf(-a, T, v) / T, E);
+}
+
+__global__ void fd_cell_kernel(const float4* __restrict__ Sf, const float4* __restrict__ wtab, const double* __restrict__ ws,
+                               int nw, long n, float4* __restrict__ rec, float* __restrict__ dim) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;  // node and column, all slots
+  if (k >= n) return;
+  const int j = int(k % nw);
+  const float4 s = Sf[k], wj = wtab[j];
+  const float2 u = split_df(ws[j] - (double(s.x) + double(s.y)));
+  const long col = 2 * (k - j) + j;  // records [side][nω] of the column
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    const bool out = side ? j == nw - 1 : j == 0;
+    const float4 o = out ? s : Sf[side ? k + 1 : k - 1];
+    const float inv = out ? 0.f : side ? wj.z : -wj.w;
+    const float dre = ((o.x - s.x) + (o.y - s.y)) * inv, di = (o.z - s.z) * inv;
+    rec[col + long(nw) * side] = make_float4(u.x, u.y, 1.f - dre, s.z);
+    dim[col + long(nw) * side] = di;
+  }
+}
+
+template <bool kSmemTab>
+__global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
+    int nw, long slab, const float4* __restrict__ rec_all, const float* __restrict__ dim_all,
+    const float4* __restrict__ wtab_g, const int32_t* __restrict__ jtab_g, float x0, float inv_h, int ntab,
+    const float* __restrict__ gw, const double* __restrict__ wph, const int32_t* __restrict__ iq_kk,
+    const int32_t* __restrict__ iks_i, const int32_t* __restrict__ iks_f, long nk_i, const double* __restrict__ eps_f,
+    const int32_t* __restrict__ f_to_i, int nm, long nvf, long per, int nsplit, double w_ac, const int* __restrict__ slots,
+    const TParams* __restrict__ tp, double* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char fd_tab[];  // kSmemTab: nodes [nw] float2, then the buckets (16 bits)
+  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε and ωq as float pairs}, the column
+  __shared__ float4 s_a[kFdTile], s_e[kFdTile];
+  __shared__ int s_c[kFdTile];
+  float2* sw = reinterpret_cast<float2*>(fd_tab);
+  uint16_t* sj = reinterpret_cast<uint16_t*>(fd_tab + sizeof(float2) * size_t(nw));
+  if constexpr (kSmemTab) {
+    for (int k = threadIdx.x; k < nw; k += kFdTile) sw[k] = make_float2(wtab_g[k].x, wtab_g[k].y);
+    for (int k = threadIdx.x; k < ntab; k += kFdTile) sj[k] = uint16_t(jtab_g[k]);
+  }
+  const int i = blockIdx.y, a = blockIdx.z / nsplit, sp = blockIdx.z % nsplit;
+  const int iw = blockIdx.x * kFdTile + threadIdx.x;
+  const TParams tq = tp[slots[a]];
+  const float T = float(tq.T);
+  const float4* rec = rec_all + 2 * slab * a;
+  const float* dim = dim_all + 2 * slab * a;
+  const float4 wn = wtab_g[min(iw, nw - 1)];
+  const float2 w = make_float2(wn.x, wn.y), mu = split_df(tq.mu);
+  const float wm = (w.x - mu.x) + (w.y - mu.y);
+  const float Ew = exp_comp(-fabsf(wm), T);  // E, or 1/E above μ
+  const float p = wm <= 0.f ? 1.f : Ew, q = wm <= 0.f ? Ew : 1.f;
+  // the bucket floor((x - x0) / h) by an FP32 addition (1.5 2^23: the integer lands in the mantissa): an
+  // off-by-one bucket at a bucket's edge picks the neighbouring cell, continuous there
+  const float bk1 = fmaf(-x0, inv_h, -0.5f), bmax = float(ntab - 1);
+  const int ki = iks_i[i];
+  auto side = [&](float wh, float wl, float2 e, int col, float o, float g, float& run) {
+    const float v = fminf(fmaxf(fmaf(w.x + wh, inv_h, bk1), 0.f), bmax);
+    const int b = __float_as_int(v + 12582912.f) - 0x4B400000;
+    int c;
+    float2 wc;
+    if constexpr (kSmemTab) {
+      c = sj[b];
+      wc = sw[c];
+    } else {
+      c = jtab_g[b];
+      const float4 t = wtab_g[c];
+      wc = make_float2(t.x, t.y);
+    }
+    const float dx = ((w.x - wc.x) + wh) + ((w.y - wc.y) + wl);
+    const int at = col + c + (dx < 0.f ? 0 : nw);
+    const float4 r = rec[at];
+    const float zr = (r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
+    const float si = fmaf(dx, dim[at], r.w);
+    const float d = fmaf(zr, zr, si * si) * o;
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
+    run = fmaf(g * si, inv, run);
+  };
+  double acc = 0.0;
+  const long t_end = min(nvf, per * (sp + 1l));
+  for (long t0 = per * sp; t0 < t_end; t0 += kFdTile) {
+    const long vf = t0 + threadIdx.x;
+    __syncthreads();  // the previous tile's readers are done (and, first, the tables are staged)
+    // below ω_acoustic no term: zero coupling, and ε = -1e25, so that |z|² overflows and the reciprocal is 0
+    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, 0.f, 0.f);
+    int sc = 0;
+    if (vf < t_end) {
+      const int nu = int(vf % nm);
+      const long f = vf / nm;
+      const double wq = wph[nu + long(nm) * iq_kk[ki + nk_i * long(iks_f[f])]];
+      if (!(wq < w_ac)) {
+        const float2 ep = split_df(eps_f[f]), wp = split_df(wq);
+        const float n = occ_boson_f(wp.x, T), g = gw[vf + nvf * i];
+        sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp.x, T), exp_comp(-wp.x, T));
+        se = make_float4(ep.x, ep.y, wp.x, wp.y);
+        sc = 2 * nw * f_to_i[f];
+      }
+    }
+    s_a[threadIdx.x] = sa;
+    s_e[threadIdx.x] = se;
+    s_c[threadIdx.x] = sc;
+    __syncthreads();
+    float run0 = 0.f, run1 = 0.f;
+    const int nt = int(min(long(kFdTile), t_end - t0));
+#pragma unroll 2
+    for (int k = 0; k < nt; ++k) {
+      const float4 A = s_a[k], Q = s_e[k];
+      const int col = s_c[k];
+      const float2 e = make_float2(Q.x, Q.y);
+      side(Q.z, Q.w, e, col, fmaf(q, A.z, p), A.x, run0);
+      side(-Q.z, -Q.w, e, col, fmaf(q, A.w, p), A.y, run1);
+    }
+    acc += double(run0) + double(run1);
+  }
+  if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc * double(p + q);
+}
+
+// ImΣ of slot a = the sum of its partials in order: into ImS_b and the Kramers-Kronig operand, or added to add_out.
+__global__ void fd_finish_kernel(const double* __restrict__ part, int nw, long slab, int nsplit, double* __restrict__ ImS_b,
+                                 __nv_bfloat16* __restrict__ Im0, __nv_bfloat16* __restrict__ Im1,
+                                 __nv_bfloat16* __restrict__ Im2, long Kp2, double* __restrict__ add_out) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= slab) return;
+  const long a = blockIdx.y;
+  double v = 0.0;
+  for (int s = 0; s < nsplit; ++s) v += part[k + slab * (a * nsplit + s)];
+  if (!ImS_b) {
+    add_out[k] += v;
+    return;
+  }
+  ImS_b[slab * a + k] = v;
+  __nv_bfloat16 p[3];
+  split_bf16_n(float(v), 3, p);
+  const long o = (slab / nw * a + k / nw) * Kp2 + k % nw;
+  Im0[o] = p[0];
+  Im1[o] = p[1];
+  Im2[o] = p[2];
+}
+
 // The node table of fm_disp_f32_kernel: node j as (hi, lo, 1 / (w[j+1] - w[j]), 1 / (w[j] - w[j-1]))
 // (0 past the ends).
 __global__ void fd_node_table_kernel(const double* __restrict__ ws, int nw, float4* __restrict__ out) {
@@ -633,7 +797,17 @@ static void check_err(Scgd0Plan* P) {
   }
 }
 
-// fm_disp_f32_kernel over nA slots (Σ_in in T->Sf): into ImS_b and the Kramers-Kronig operand, or
+// Splits of the (ν, f) range for nA slots: about 40 blocks a multiprocessor (four are resident, so the last wave is a
+// tenth of the time), eight tiles of pairs a split at least (a block's tables and tail).
+static int fd_splits(const Scgd0Plan* P, long nA) {
+  const long tiles = div_up(size_t(P->nm * P->nf), kFdTile);
+  const long blocks = long(div_up(size_t(P->nw), kFdTile)) * P->ni * nA;
+  const long want = std::max<long>(1, (40l * P->ctx->sm_count + blocks - 1) / blocks);
+  const long n = std::min(want, std::max<long>(1, tiles / 8));
+  return int(div_up(size_t(tiles), div_up(size_t(tiles), size_t(n))));  // no empty split
+}
+
+// The Fan-Migdal sum term by term over nA slots (Σ_in in T->Sf): into ImS_b and the Kramers-Kronig operand, or
 // added into add_out (one slot).
 static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, double* ImS_b,
                            double* add_out) {
@@ -641,6 +815,36 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
   auto* T = P->tc.get();
   const long nw = P->nw, ni = P->ni;
   // the grid nodes and the bucket table in shared memory when they fit 96 KB
+  if (P->fd_fast) {
+    const long slab = nw * ni, n = slab * nA, nvf = P->nm * P->nf;
+    ensure(T->fdrec, ctx, size_t(2 * n));
+    ensure(T->fddim, ctx, size_t(2 * n));
+    fd_cell_kernel<<<div_up(size_t(n), 256), 256, 0, ctx->stream>>>(T->Sf.p, P->d_wtab.p, P->d_ws.p, int(nw), n, T->fdrec.p,
+                                                                    T->fddim.p);
+    EPSP_LAUNCHED(ctx);
+    const size_t tab = sizeof(float2) * size_t(nw) + 2 * size_t(P->ntab);
+    const bool smem = tab <= (size_t(96) << 10) && nw <= 65535;
+    const int nsplit = fd_splits(P, nA);
+    const long per = (div_up(size_t(nvf), kFdTile) + nsplit - 1) / nsplit * kFdTile;
+    ensure(T->fdpart, ctx, size_t(n) * size_t(nsplit));
+    const dim3 grid(div_up(size_t(nw), kFdTile), unsigned(ni), unsigned(nA * nsplit));
+    auto go = [&](auto kern, size_t bytes) {
+      EPSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+      kern<<<grid, kFdTile, bytes, ctx->stream>>>(int(nw), slab, T->fdrec.p, T->fddim.p, P->d_wtab.p, P->d_jtab.p, P->x0f,
+                                                  P->inv_hf, int(P->ntab), P->d_gwf.p, P->d_wph.p, P->d_iq.p, P->d_iksi.p,
+                                                  P->d_iksf.p, P->nk_i, P->d_epsf.p, P->d_fti.p, int(P->nm), nvf, per,
+                                                  nsplit, P->w_ac, d_slots, d_tp, T->fdpart.p);
+    };
+    if (smem)
+      go(fm_disp_fast_kernel<true>, tab);
+    else
+      go(fm_disp_fast_kernel<false>, size_t(0));
+    EPSP_LAUNCHED(ctx);
+    fd_finish_kernel<<<dim3(div_up(size_t(slab), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
+        T->fdpart.p, int(nw), slab, nsplit, ImS_b, T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2, add_out);
+    EPSP_LAUNCHED(ctx);
+    return;
+  }
   const size_t tab = sizeof(float4) * size_t(nw) + sizeof(int32_t) * size_t(P->ntab);
   const bool smem = tab <= (size_t(96) << 10);
   const dim3 grid(div_up(size_t(nw), kFdTile), unsigned(ni), unsigned(nA));
@@ -662,6 +866,23 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
   EPSP_LAUNCHED(ctx);
 }
 
+// Whether the temperatures of a call allow fm_disp_fast_kernel (every exp(ωq/T) within e^40; ω_acoustic above 0,
+// so that n(ωq) is finite). Reserves its buffers for nT slots, so that none is allocated while a graph is captured.
+void tc_disp_choose(Scgd0Plan* P, const double* Tlist, long nT) {
+  if (!P->disp) return;
+  P->fd_fast = P->w_ac > 0 && 2 * P->nw * P->ni < (1l << 31);  // (32-bit record offsets)
+  for (long t = 0; t < nT; ++t) P->fd_fast = P->fd_fast && Tlist[t] > 1.4901161193847656e-08 && P->wq_max <= kFdMaxArg * Tlist[t];
+  if (!P->fd_fast) return;
+  auto* T = P->tc.get();
+  const size_t n = size_t(P->nw * P->ni) * size_t(nT);
+  bool grown = ensure(T->fdrec, P->ctx, 2 * n);
+  grown |= ensure(T->fddim, P->ctx, 2 * n);
+  size_t part = 0;
+  for (long a = 1; a <= nT; ++a) part = std::max(part, size_t(P->nw * P->ni) * size_t(a) * size_t(fd_splits(P, a)));
+  grown |= ensure(T->fdpart, P->ctx, part);
+  if (grown) ++P->w_gen;
+}
+
 // One Fan-Migdal sum at (μ, T) for a model with dispersive modes, added into d_ImS.
 void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, double* d_ImS) {
   Ctx* ctx = P->ctx;
@@ -670,6 +891,7 @@ void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, do
   const long nw = P->nw, ni = P->ni;
   sigma_f32_kernel<<<div_up(size_t(nw * ni), 256), 256, 0, s>>>(d_Sin, nw * ni, T_->Sf.p);
   EPSP_LAUNCHED(ctx);
+  tc_disp_choose(P, &T, 1);
   TParams q{};
   q.T = T;
   q.mu = mu;
@@ -701,6 +923,8 @@ void tc_setup_dispersive(Scgd0Plan* P, const epsp_model* m) {
     EPSP_LAUNCHED(ctx);
     EPSP_CUDA(cudaStreamSynchronize(s));
   }
+  for (int64_t k = 0; k < nm * m->nq; ++k)
+    P->wq_max = std::isfinite(m->omega_ph[k]) ? std::max(P->wq_max, m->omega_ph[k]) : std::numeric_limits<double>::infinity();
   P->d_wph = to_device(ctx, m->omega_ph, size_t(nm * m->nq));
   P->d_iq = to_device(ctx, m->iq_kk, size_t(m->nk_i * m->nk_f));
   P->d_iksi = to_device(ctx, m->iks_i, size_t(ni));

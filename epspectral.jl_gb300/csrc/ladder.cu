@@ -89,6 +89,7 @@ struct LadderPlan {
   // tensor-core paths: the contraction Z = Jr Bz (M = 16 nwp rows (ri, c0, p, c12), N = nm 3ni
   // columns (ν, a, i), K = 3ni pairs (b, i') padded to Kzp), then D from Z by zgather_kernel
   long Mz = 0, Nz = 0, Kz = 0, Kzp = 0;
+  DBuf<double4> d_xtab;          // GEMM_FP64: the same tables for xgen_f64_kernel
   DBuf<float> d_ztab;            // [nm, 2, nwp][4] the weights of p0, p0 + 1, p0 + 2 (tent weights folded in), p0
                                  // (integer bits): the three nodes a mode's two shift tables read
   DBuf<int32_t> d_zwin;          // [node ranges, nm][2] zgather_kernel's staging windows (float4 chunks)
@@ -99,8 +100,7 @@ struct LadderPlan {
   TcOperand opKK{}, opY{};
   int bn2 = 128, splits2 = 1;
   DBuf<double> d_Gt, d_Af, d_D;   // G̃ [Kx, 3ni]; A (FP64) [24nω, Kx]; D [24nω, 3ni]
-  DBuf<int32_t> d_mnu;
-  DBuf<double> d_rnu, d_nnu;
+  DBuf<double> d_nnu;
   DBuf<__nv_bfloat16> d_Jh, d_Jl, d_Bzh, d_Bzl;  // GEMM_BF16: Jr and Bz as BF16 hi/lo rows of Kzp
   DBuf<float> d_Jt, d_Bzt;                        // GEMM_TF32: the same as TF32-rounded FP32
   DBuf<float> d_Z, d_Dz;  // Z (split-K partials, zsplit_cap of them at most) [Mz, Nz]; D [24 nwp, 3ni]
@@ -569,58 +569,51 @@ __global__ void coupling_rot_chunk_kernel(const T* __restrict__ g2c, const doubl
   }
 }
 
-// One element of the A operand: row (j, q, c0, ri), column k = (ν, b, i'). The shifted vertex of
-// sign s at shift m, node j: wlo J[klo] + whi J[klo + 1]; the mode value
-// X±_ν = (1 - r_ν) S_{m_ν} + r_ν S_{m_ν + 1}; the combination q folds the channel algebra:
+// The FP64 A operand, column-major [24 nwp, Kx]: row (j, q, c0, ri), column k = (ν, b, i'). The mode value of
+// sign s at node j, X±_ν = (1 - r_ν) S_{m_ν} + r_ν S_{m_ν + 1} of the shifted vertices, is three taps of J
+// (xtab [nm][2][nwp]: their weights and, as integer bits, the first node); the combination q folds the channel
+// algebra:
 //   q = 0, 2 : (X+ - X-)/2 of c12 = 11, 22        (the Kramers-Kronig argument)
 //   q = 1, 3 : -(1/2 + n_ν)(X+ + X-) of c12 = 11, 22
 //   q = 4    : n_ν X+ + (1 + n_ν) X- of c12 = 21
 //   q = 5    : (1 + n_ν) X+ + n_ν X- of c12 = 12
-__device__ __forceinline__ double xgen_value(const double2* __restrict__ J, const int32_t* __restrict__ klo,
-                                             const double* __restrict__ wlo, const double* __restrict__ whi, int nw,
-                                             int ns, int j, int q, int c0, int ri, int m, double r, double n, int b,
-                                             long ip) {
-  const int c12 = (q < 2) ? 0 : (q < 4 ? 3 : (q == 4 ? 1 : 2));
-  double xs[2];
-  for (int s = 0; s < 2; ++s) {
-    double acc = 0;
-    for (int dm = 0; dm < 2; ++dm) {
-      const int mm = m + dm;
-      const double wgt = dm == 0 ? 1 - r : r;
-      if (wgt == 0.0 || mm >= ns) continue;
-      const long t = j + long(nw) * (mm + long(ns) * s);
-      const int kl = klo[t];
-      const double2 z0 = J[jidx(nw, kl, c12, b, c0, ip)], z1 = J[jidx(nw, kl + 1, c12, b, c0, ip)];
-      const double zz = ri == 0 ? wlo[t] * z0.x + whi[t] * z1.x : wlo[t] * z0.y + whi[t] * z1.y;
-      acc += wgt * zz;
+// Thread (j, c0, k) forms all twelve rows: 72 FP64 operations, which bound the kernel (six an element; one
+// thread per element took about 18 and eight 16-byte loads: 647 us for 7680 x 2880, here 240). Rows j >= nω
+// and the columns of padding modes stay zero from the set-up. Grid (nω / 128, 3 ni, 2 nm).
+__global__ void __launch_bounds__(128) xgen_f64_kernel(const double2* __restrict__ J, const double4* __restrict__ xtab,
+                                                       const double* __restrict__ nnu, int nw, int nwp, int nm, int nmp,
+                                                       double* __restrict__ A) {
+  const int j = blockIdx.x * 128 + threadIdx.x;
+  if (j >= nw) return;
+  const int b = blockIdx.y % 3, nu = blockIdx.z / 2, c0 = blockIdx.z % 2;
+  const long ip = blockIdx.y / 3;
+  const double n = nnu[nu];
+  const double4 t[2] = {xtab[(2l * nu) * nwp + j], xtab[(2l * nu + 1) * nwp + j]};
+  const int p[2] = {int(__double_as_longlong(t[0].w)), int(__double_as_longlong(t[1].w))};
+  double* out = A + j + 24l * nwp * (nu + long(nmp) * blockIdx.y) + 6l * nwp * c0;
+#pragma unroll
+  for (int c12 = 0; c12 < 4; ++c12) {
+    const double2* col = J + jidx(nw, 0, c12, b, c0, ip);
+    double2 x[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const double2 z0 = col[p[s]], z1 = col[p[s] + 1], z2 = col[min(p[s] + 2, nw - 1)];  // (its weight there is 0)
+      x[s].x = fma(t[s].z, z2.x, fma(t[s].y, z1.x, t[s].x * z0.x));
+      x[s].y = fma(t[s].z, z2.y, fma(t[s].y, z1.y, t[s].x * z0.y));
     }
-    xs[s] = acc;
+    if (c12 == 0 || c12 == 3) {
+      const long q = c12 == 0 ? 0 : 2;
+      out[nwp * q] = (x[0].x - x[1].x) * 0.5;
+      out[nwp * (q + 12)] = (x[0].y - x[1].y) * 0.5;
+      out[nwp * (q + 1)] = -(0.5 + n) * (x[0].x + x[1].x);
+      out[nwp * (q + 13)] = -(0.5 + n) * (x[0].y + x[1].y);
+    } else {
+      const long q = c12 == 1 ? 4 : 5;
+      const double fp = c12 == 1 ? n : 1 + n, fm = c12 == 1 ? 1 + n : n;
+      out[nwp * q] = fma(fm, x[1].x, fp * x[0].x);
+      out[nwp * (q + 12)] = fma(fm, x[1].y, fp * x[0].y);
+    }
   }
-  switch (q) {
-    case 0:
-    case 2: return (xs[0] - xs[1]) / 2;
-    case 1:
-    case 3: return -(0.5 + n) * (xs[0] + xs[1]);
-    case 4: return n * xs[0] + (1 + n) * xs[1];
-    default: return (1 + n) * xs[0] + n * xs[1];
-  }
-}
-
-// FP64 A operand, column-major [24 nwp, Kx] (rows j >= nω and modes ν >= nm are zero).
-__global__ void xgen_f64_kernel(const double2* __restrict__ J, const int32_t* __restrict__ klo, const double* __restrict__ wlo,
-                                const double* __restrict__ whi, const int32_t* __restrict__ mnu, const double* __restrict__ rnu,
-                                const double* __restrict__ nnu, int nw, int nwp, int ns, int nm, int nmp, int ni,
-                                double* __restrict__ A) {
-  const long nrow = 24l * nwp;
-  long idx = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= nrow * nmp * 3 * ni) return;
-  long row = idx % nrow, k = idx / nrow;
-  int j = int(row % nwp);
-  int rr = int(row / nwp);
-  int q = rr % 6, c0 = (rr / 6) % 2, ri = rr / 12;
-  int nu = int(k % nmp), b = int((k / nmp) % 3);
-  long ip = k / (3l * nmp);
-  A[idx] = (j < nw && nu < nm) ? xgen_value(J, klo, wlo, whi, nw, ns, j, q, c0, ri, mnu[nu], rnu[nu], nnu[nu], b, ip) : 0.0;
 }
 
 // ---- the tensor-core contraction, interpolation after the product ----
@@ -1674,8 +1667,6 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
         P->r_nu[size_t(nu)] = 0;
       }
     }
-    P->d_mnu = to_device(ctx, P->m_nu);
-    P->d_rnu = to_device(ctx, P->r_nu);
     P->d_nnu.alloc(ctx, size_t(nm));
     P->d_nnu_f.alloc(ctx, 16);
     auto d_wnu = to_device(ctx, P->wnu);
@@ -1715,58 +1706,78 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
     }
     const long M = 24 * P->nwp, N = 3 * ni;
     if (!tc_path(P->path)) P->d_D.alloc(ctx, size_t(M * N));  // the tensor-core paths keep D as split-K parts
+    // mode tables: for node j, mode ν and sign s, the two shift tables (m_ν, m_ν + 1) with the
+    // tent weights (1 - r_ν, r_ν) folded into their interpolation weights. The two tables'
+    // lower nodes differ by at most one (the grid's spacing is a multiple of its unit, the shift
+    // step), so their four taps lie on three consecutive nodes p0, p0 + 1, p0 + 2: three weights
+    // and the node per entry.
+    std::vector<int32_t> hk(size_t(P->nwp * nm * 2));
+    std::vector<double> hw(size_t(P->nwp * nm * 2 * 3), 0.0);
+    {
+      const long nwp = P->nwp;
+      const bool tc = tc_path(P->path);
+      std::vector<int32_t> klo(size_t(nw * ns * 2));
+      std::vector<double> wlo(klo.size()), whi(klo.size());
+      P->d_klo.download(klo.data(), klo.size(), s);
+      P->d_wlo.download(wlo.data(), wlo.size(), s);
+      P->d_whi.download(whi.data(), whi.size(), s);
+      EPSP_CUDA(cudaStreamSynchronize(s));
+      for (long j = 0; j < nwp; ++j)
+        for (long nu = 0; nu < nm; ++nu)
+          for (long sg = 0; sg < 2; ++sg) {
+            const size_t e = size_t((nu * 2 + sg) * nwp + j);  // [ν][s][j]: consecutive nodes adjacent
+            // zero weights; the taps j.. j + 2 stay inside the staged rows and pads
+            hk[e] = tc ? int32_t(j) : int32_t(std::min(j, std::max<long>(0, nw - 2)));
+            if (j >= nw || P->wnu[size_t(nu)] < P->w_ac) continue;
+            const long mm = P->m_nu[size_t(nu)];
+            const double r = P->r_nu[size_t(nu)];
+            const size_t t0 = size_t(j + nw * (mm + ns * sg));
+            long ka = klo[t0], kb = ka;
+            double tw[4] = {(1 - r) * wlo[t0], (1 - r) * whi[t0], 0.0, 0.0};
+            if (mm + 1 < ns && r != 0.0) {
+              const size_t t1 = size_t(j + nw * (mm + 1 + ns * sg));
+              kb = klo[t1];
+              tw[2] = r * wlo[t1];
+              tw[3] = r * whi[t1];
+            }
+            if (std::labs(kb - ka) > 1)
+              fail(EPSP_EUNSUPPORTED, "neighbouring shift tables more than one node apart (the grid spacing is below its unit)");
+            const long p0 = std::min(ka, kb);
+            double cw[3] = {0, 0, 0};
+            cw[ka - p0] += tw[0];
+            cw[ka + 1 - p0] += tw[1];
+            cw[kb - p0] += tw[2];
+            cw[kb + 1 - p0] += tw[3];
+            hk[e] = int32_t(p0);
+            for (int t = 0; t < 3; ++t) hw[3 * e + size_t(t)] = cw[t];
+          }
+    }
     if (P->path == EPSP_PATH_GEMM_FP64) {
+      std::vector<double4> x(hk.size());
+      for (size_t e = 0; e < hk.size(); ++e) {
+        const long long p0 = hk[e];
+        x[e].x = hw[3 * e];
+        x[e].y = hw[3 * e + 1];
+        x[e].z = hw[3 * e + 2];
+        std::memcpy(&x[e].w, &p0, 8);
+      }
+      P->d_xtab = to_device(ctx, x);
       P->d_Af.alloc(ctx, size_t(M * P->Kx));
+      P->d_Af.zero(s);  // rows j >= nω and the columns of padding modes stay zero
       oz_split(ctx, P->d_Gt.p, P->Kx, N, P->Kx, true, oz_tile_n(N), P->ozGt);
+      EPSP_CUDA(cudaStreamSynchronize(s));  // x is a local
     } else {
       plog.mark("g2 streamed, G~ built");
-      // mode tables: for node j, mode ν and sign s, the two shift tables (m_ν, m_ν + 1) with the
-      // tent weights (1 - r_ν, r_ν) folded into their interpolation weights (FP32). The two tables'
-      // lower nodes differ by at most one (the grid's spacing is a multiple of its unit, the shift
-      // step), so their four taps lie on three consecutive nodes p0, p0 + 1, p0 + 2: three weights
-      // and the node (as integer bits in the fourth slot) per entry.
       {
-        const long nwp = P->nwp;
-        std::vector<int32_t> hk(size_t(nwp * nm * 2));
-        std::vector<float> hw(size_t(nwp * nm * 2 * 4), 0.f);
-        std::vector<int32_t> klo(size_t(nw * ns * 2));
-        std::vector<double> wlo(klo.size()), whi(klo.size());
-        P->d_klo.download(klo.data(), klo.size(), s);
-        P->d_wlo.download(wlo.data(), wlo.size(), s);
-        P->d_whi.download(whi.data(), whi.size(), s);
-        EPSP_CUDA(cudaStreamSynchronize(s));
-        for (long j = 0; j < nwp; ++j)
-          for (long nu = 0; nu < nm; ++nu)
-            for (long sg = 0; sg < 2; ++sg) {
-              const size_t e = size_t((nu * 2 + sg) * nwp + j);  // [ν][s][j]: consecutive nodes adjacent
-              hk[e] = int32_t(j);  // zero weights; the taps j.. j + 2 stay inside the staged rows and pads
-              if (j >= nw || P->wnu[size_t(nu)] < P->w_ac) continue;
-              const long mm = P->m_nu[size_t(nu)];
-              const double r = P->r_nu[size_t(nu)];
-              const size_t t0 = size_t(j + nw * (mm + ns * sg));
-              long ka = klo[t0], kb = ka;
-              double tw[4] = {(1 - r) * wlo[t0], (1 - r) * whi[t0], 0.0, 0.0};
-              if (mm + 1 < ns && r != 0.0) {
-                const size_t t1 = size_t(j + nw * (mm + 1 + ns * sg));
-                kb = klo[t1];
-                tw[2] = r * wlo[t1];
-                tw[3] = r * whi[t1];
-              }
-              if (std::labs(kb - ka) > 1)
-                fail(EPSP_EUNSUPPORTED, "neighbouring shift tables more than one node apart (the grid spacing is below its unit)");
-              const long p0 = std::min(ka, kb);
-              double cw[3] = {0, 0, 0};
-              cw[ka - p0] += tw[0];
-              cw[ka + 1 - p0] += tw[1];
-              cw[kb - p0] += tw[2];
-              cw[kb + 1 - p0] += tw[3];
-              hk[e] = int32_t(p0);
-              for (int t = 0; t < 3; ++t) hw[4 * e + size_t(t)] = float(cw[t]);
-            }
-        for (size_t e = 0; e < hk.size(); ++e) std::memcpy(&hw[4 * e + 3], &hk[e], sizeof(int32_t));
-        P->d_ztab = to_device(ctx, hw);
+        std::vector<float> hf(4 * hk.size());
+        for (size_t e = 0; e < hk.size(); ++e) {
+          for (size_t t = 0; t < 3; ++t) hf[4 * e + t] = float(hw[3 * e + t]);
+          std::memcpy(&hf[4 * e + 3], &hk[e], sizeof(int32_t));
+        }
+        P->d_ztab = to_device(ctx, hf);
         P->zg = zgather_ranges(nw, 2);
-        P->d_zwin = to_device(ctx, zgather_windows(P->zg, hk, nw, nwp, nm));
+        P->d_zwin = to_device(ctx, zgather_windows(P->zg, hk, nw, P->nwp, nm));
+        EPSP_CUDA(cudaStreamSynchronize(s));  // hf is a local
       }
       P->Kp2 = (nw + 63) / 64 * 64;
       const bool tf = P->path == EPSP_PATH_GEMM_TF32;
@@ -1995,9 +2006,8 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   set_mode_occupations(P, T);
   const long nwp = P->nwp, M = 24 * nwp, N = 3 * ni;
   long px = prof_begin(ctx, "xgen");
-  xgen_f64_kernel<<<div_up(size_t(M * P->Kx), 256), 256, 0, s>>>(J, P->d_klo.p, P->d_wlo.p, P->d_whi.p, P->d_mnu.p, P->d_rnu.p,
-                                                                 P->d_nnu.p, int(nw), int(nwp), int(ns), int(P->nm),
-                                                                 int(P->nmp), int(ni), P->d_Af.p);
+  xgen_f64_kernel<<<dim3(div_up(size_t(nw), 128), unsigned(3 * ni), unsigned(2 * P->nm)), 128, 0, s>>>(
+      J, P->d_xtab.p, P->d_nnu.p, int(nw), int(nwp), int(P->nm), int(P->nmp), P->d_Af.p);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, px);
   long pg = prof_begin(ctx, "ladder_gemm");

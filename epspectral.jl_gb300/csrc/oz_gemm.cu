@@ -474,14 +474,27 @@ static void gemm_panel(Ctx* ctx, OzWork& W, const OzPlanes& A, long m0, long M, 
   sh.nseg = (chunks + kOzSegChunks - 1) / kOzSegChunks;
   sh.nkc = (chunks + sh.nseg - 1) / sh.nseg;
   sh.nseg = (chunks + sh.nkc - 1) / sh.nkc;
-  const long total = 43l * sh.nkc * sh.nseg * sh.nM * sh.nN;
-  sh.run = int(std::max<long>(1, std::min<long>(8l * sh.nkc, total / (4l * ctx->sm_count))));
-  sh.per_seg = 0;
+  // Chunks per item: the shortest critical path of whole rounds over the SMs, a chunk being 16 products at shared
+  // memory's rate and an item's end (registers to sums, pipeline drain) about four chunks; shared orders pay
+  // atomics, so ties go to longer runs.
   bool shared = false;
-  for (int d = 0; d < kOzOrders; ++d) {
-    const int n = (oz_pairs(d) * sh.nkc + sh.run - 1) / sh.run;
-    sh.per_seg += n;
-    shared |= n > 1;
+  long best = -1;
+  for (int run = 1; run <= 8 * sh.nkc; run += std::max(1, run / 16)) {
+    long per_seg = 0;
+    bool sh_ = false;
+    for (int d = 0; d < kOzOrders; ++d) {
+      const int n = (oz_pairs(d) * sh.nkc + run - 1) / run;
+      per_seg += n;
+      sh_ |= n > 1;
+    }
+    const long items = per_seg * sh.nseg * sh.nM * sh.nN;
+    const long cost = (items + ctx->sm_count - 1) / ctx->sm_count * (std::min(run, 8 * sh.nkc) + 4);
+    if (best < 0 || cost <= best) {
+      best = cost;
+      sh.run = run;
+      sh.per_seg = int(std::min<long>(per_seg, 1l << 30));
+      shared = sh_;
+    }
   }
   if (long(sh.nM) * sh.nN * sh.nseg * sh.per_seg > (1l << 30)) fail(EPSP_EINVAL, "sizes beyond the 32-bit tile grid");
   const size_t n = size_t(sh.nseg) * kOzOrders * size_t(sh.M) * size_t(sh.N);

@@ -229,11 +229,11 @@ __device__ __forceinline__ double recip_seeded(double d) {
 
 constexpr int kFmFastTile = 128;  // staged (ν, f) pairs
 
-__global__ void __launch_bounds__(128) fm_direct_fast_kernel(
+__global__ void __launch_bounds__(512) fm_direct_fast_kernel(
     const double* __restrict__ ws, int nw, const long long* __restrict__ wkey, const int32_t* __restrict__ jtab, int ntab,
     float x0f, float inv_hf, float guard, const double4* __restrict__ tab, const double* __restrict__ g2t,
     const double* __restrict__ wqt, long nvf, const double* __restrict__ eps_f, const double* __restrict__ w_f,
-    const int32_t* __restrict__ f_to_i, int nm, long vf0, long vf1, long per, double mu, double T, double w_ac,
+    const int32_t* __restrict__ f_to_i, int nm, long vf0, long vf1, long per, double mu, double T, double invT, double w_ac,
     double* __restrict__ part) {
   __shared__ FmPair sp[kFmFastTile];
   __shared__ int s_col[kFmFastTile];
@@ -242,13 +242,10 @@ __global__ void __launch_bounds__(128) fm_direct_fast_kernel(
   const bool in = iw < nw;
   const double w = in ? ws[iw] : ws[0];
   const float wf = float(w);
-  // exp(v / T), the rounding of v / T put back as a factor
-  auto ex = [&](double v) {
-    const double a = v / T, E = exp(a);
-    return E > 0.0 && E < INFINITY ? fma(E, fma(-a, T, v) / T, E) : E;
-  };
   const bool below = w <= mu;
-  const double Ew = ex(below ? w - mu : mu - w);  // E, or 1/E above μ
+  const double dv = below ? w - mu : mu - w;
+  // exp(v / T) with the rounding of v / T put back as a factor
+  const double av = dv * invT, E0 = exp(av), Ew = fma(E0, fma(-av, T, dv) * invT, E0);  // E, or 1/E above μ
   const double p = below ? 1.0 : Ew, q = below ? Ew : 1.0;
   const long t_end = min(vf1, vf0 + per * (long(blockIdx.z) + 1));
   double acc = 0.0;
@@ -260,8 +257,10 @@ __global__ void __launch_bounds__(128) fm_direct_fast_kernel(
       const double wq = wqt[vf + nvf * i];
       s_col[k] = wq < w_ac ? -1 : f_to_i[f];
       if (!(wq < w_ac)) {
-        const double g = w_f[f] * g2t[vf + nvf * i], nq = occ_boson_d(wq, T);
-        sp[k] = FmPair{g * (nq + 1.0), g * nq, ex(wq), ex(-wq), wq, eps_f[f]};
+        const double g = w_f[f] * g2t[vf + nvf * i];
+        const double a = wq * invT, m0 = expm1(a), m = fma(m0 + 1.0, fma(-a, T, wq) * invT, m0);  // exp(ωq/T) - 1
+        const double e = m + 1.0, nq = recip_seeded(m);
+        sp[k] = FmPair{g * (nq + 1.0), g * nq, e, recip_seeded(e), wq, eps_f[f]};
       }
     }
     __syncthreads();
@@ -300,13 +299,24 @@ __global__ void __launch_bounds__(128) fm_direct_fast_kernel(
   if (in) part[iw + long(nw) * (i + long(gridDim.y) * blockIdx.z)] = acc * (p + q);
 }
 
-// ImΣ += Σ_s part[s] in ascending s.
-__global__ void fm_add_kernel(const double* __restrict__ part, long n, int splits, double* __restrict__ imsigma) {
-  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+// ImΣ += Σ_s part[s]: 32 elements a block, eight runs of splits side by side, each in ascending s, added in order.
+__global__ void __launch_bounds__(256) fm_add_kernel(const double* __restrict__ part, long n, int splits,
+                                                     double* __restrict__ imsigma) {
+  __shared__ double sh[8][32];
+  const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
+  const long k = long(blockIdx.x) * 32 + lane;
+  const int per = (splits + 7) / 8;
   double v = 0.0;
-  for (int s = 0; s < splits; ++s) v += part[k + n * s];
-  imsigma[k] += v;
+  if (k < n)
+#pragma unroll 4
+    for (int s = g * per; s < min(splits, (g + 1) * per); ++s) v += part[k + n * s];
+  sh[g][lane] = v;
+  __syncthreads();
+  if (g == 0 && k < n) {
+#pragma unroll
+    for (int r = 1; r < 8; ++r) v += sh[r][lane];
+    imsigma[k] += v;
+  }
 }
 
 // The occupation factors of the recast sum, per (ω, ν): F_abs = n_ν + f(ω + ω_ν - μ) and
@@ -331,29 +341,33 @@ __global__ void occ_table_kernel(const double* __restrict__ ws, int nw, const do
 // The kernel tensor of the recast sum (dispersionless modes): K_t[ω, (ν, c)] =
 // Im G_c(ω + ω_ν) F_abs[ω, ν] + Im G_c(ω - ω_ν) F_emi[ω, ν], with Im G_c(x) = Im 1/(x - ε_c -
 // Σ_in,col(c)(x)), for the column set c (a star of inner states sharing ε and the representative's
-// Σ, or one inner state).
-__global__ void kbuild_f64_kernel(const double* __restrict__ ws, int nw, CellTableDev ct, const double2* __restrict__ Sin,
-                                  const double* __restrict__ wnu, int nm, const double* __restrict__ eps_c,
-                                  const int32_t* __restrict__ col_c, long nc, const double* __restrict__ Fa,
-                                  const double* __restrict__ Fe, double w_ac, double* __restrict__ Kt) {
+// Σ, or one inner state). Σ(x) from the columns' cell table (fm_cell_kernel) at the cells of ω ± ω_ν found at set-up
+// (cell_e: the table's entry, cell_dx: x less its node), and one reciprocal for both sides: 20 FP64 operations an
+// element, which bound the kernel, in place of about 90 with the search, two weights and two divisions
+// (501 nodes x 1575: 130 -> 32 us).
+__global__ void kbuild_f64_kernel(int nw, const double4* __restrict__ tab, const int32_t* __restrict__ cell_e,
+                                  const double* __restrict__ cell_dx, const double* __restrict__ wnu, int nm,
+                                  const double* __restrict__ eps_c, const int32_t* __restrict__ col_c,
+                                  const double* __restrict__ Fa, const double* __restrict__ Fe, double w_ac,
+                                  double* __restrict__ Kt) {
   const int iw = blockIdx.x * blockDim.x + threadIdx.x;
   const long kc = blockIdx.y;  // (ν, c) with ν fastest
   if (iw >= nw) return;
   const int nu = int(kc % nm);
   const long c = kc / nm;
-  double q = wnu[nu];
   double out = 0.0;
-  if (!(q < w_ac)) {
-    const double2* col = Sin + long(nw) * col_c[c];
-    double w = ws[iw], e = eps_c[c];
-    double xa = w + q, xe = w - q;
-    double2 sa = interp_grid_d(col, ct, xa);
-    double2 se = interp_grid_d(col, ct, xe);
-    double zar = xa - e - sa.x, zai = -sa.y;
-    double zer = xe - e - se.x, zei = -se.y;
-    double ga = -zai / (zar * zar + zai * zai);
-    double ge = -zei / (zer * zer + zei * zei);
-    out = ga * Fa[iw + long(nw) * nu] + ge * Fe[iw + long(nw) * nu];
+  if (!(wnu[nu] < w_ac)) {
+    const double4* col = tab + (nw + 1l) * col_c[c];
+    const long ka = iw + long(nw) * nu, ke = ka + long(nw) * nm;
+    const double4 A = col[cell_e[ka]], B = col[cell_e[ke]];
+    const double da = cell_dx[ka], de = cell_dx[ke], e = eps_c[c];
+    const double zar = fma(da, A.z, A.x - e), sia = fma(da, A.w, A.y);
+    const double zer = fma(de, B.z, B.x - e), sie = fma(de, B.w, B.y);
+    const double dna = fma(zar, zar, sia * sia), dne = fma(zer, zer, sie * sie);
+    const double Na = sia * Fa[ka], Ne = sie * Fe[ka];
+    const double D = dna * dne;
+    const int E = (__double2hiint(D) >> 20) & 0x7ff;
+    out = E > 0 && E < 0x7f0 ? fma(Na, dne, Ne * dna) * recip_seeded(D) : Na / dna + Ne / dne;
   }
   Kt[iw + long(nw) * kc] = out;
 }
@@ -1221,6 +1235,12 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
               ctt[k] = (x - w[size_t(j)]) / (w[size_t(j + 1)] - w[size_t(j)]);
             }
           }
+      if (P->path == EPSP_PATH_GEMM_FP64)  // the entry of the cell table, and x less its node (kbuild_f64_kernel)
+        for (size_t k = 0; k < cj.size(); ++k) {
+          const int32_t e = !(cx[k] > w[0]) ? 0 : cx[k] >= w[size_t(n - 1)] ? int32_t(n) : cj[k] + 1;
+          ctt[k] = cx[k] - w[size_t(std::max(e - 1, 0))];
+          cj[k] = e;
+        }
       P->d_cell_j = to_device(ctx, cj);
       P->d_cell_t = to_device(ctx, ctt);
       P->d_cell_x = to_device(ctx, cx);
@@ -1264,11 +1284,9 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
   if (P->path == EPSP_PATH_DIRECT_FP64) {
     const long nvf = nm * nf;
     const bool fast = P->fm_fast && T > 1.4901161193847656e-08 && P->wq_max <= 300.0 * T;
-    // warps of 32 nodes a block, 4 or fewer where that leaves fewer idle (a block stages its pairs itself)
+    // blocks of up to 16 warps of 32 nodes, as even as they come (a block stages its pairs: about 50 operations each)
     const long nwarp = div_up(size_t(nw), 32);
-    int wpb = 4;
-    for (int k = 3; k >= 2; --k)
-      if (div_up(size_t(nwarp), size_t(k)) * k < div_up(size_t(nwarp), size_t(wpb)) * wpb) wpb = k;
+    const int wpb = int(div_up(size_t(nwarp), div_up(size_t(nwarp), 16)));
     const dim3 tiles(fast ? div_up(size_t(nwarp), size_t(wpb)) : div_up(size_t(nw), kFmTile), unsigned(ni));
     if (fast) {
       const long n = (nw + 1) * ni;
@@ -1280,17 +1298,18 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
       long f1 = std::min(nf, f0 + P->nf_chunk);
       long pi = prof_begin(ctx, "fan_migdal");
       if (fast) {
-        // splits of the (ν, f) range: 32 warps a multiprocessor, 32 pairs a split at least
-        const long len = nm * (f1 - f0), want = 32l * ctx->sm_count / (long(tiles.x) * ni * wpb) + 1;
-        const long per = std::max<long>(32, (len + want - 1) / want);
+        // splits of the (ν, f) range: 64 warps a multiprocessor (the FP64 pipes take whole warps, so few of them share out
+        // unevenly), 8 pairs a split at least (a thread's own exponential is worth two), 64 splits at most
+        const long len = nm * (f1 - f0), want = std::min<long>(64, 64l * ctx->sm_count / (long(tiles.x) * ni * wpb) + 1);
+        const long per = std::max<long>(8, (len + want - 1) / want);
         const int splits = int((len + per - 1) / per);
         ensure(P->w_fmpart, ctx, size_t(nw * ni * splits));
         fm_direct_fast_kernel<<<dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0, s>>>(
             P->d_ws.p, int(nw), P->d_wkey.p, P->d_jtab.p, int(P->d_jtab.n), float(P->ct.x0), float(P->ct.inv_h),
             P->fm_guard, P->w_fmtab.p, P->d_g2t.p, P->d_wqt.p, nvf, P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm),
-            nm * f0, nm * f1, per, mu, T, P->w_ac, P->w_fmpart.p);
+            nm * f0, nm * f1, per, mu, T, 1.0 / T, P->w_ac, P->w_fmpart.p);
         EPSP_LAUNCHED(ctx);
-        fm_add_kernel<<<div_up(size_t(nw * ni), 128), 128, 0, s>>>(P->w_fmpart.p, nw * ni, splits, d_ImS);
+        fm_add_kernel<<<div_up(size_t(nw * ni), 32), 256, 0, s>>>(P->w_fmpart.p, nw * ni, splits, d_ImS);
       } else {
         fm_direct_kernel<<<tiles, kFmTile, 0, s>>>(P->d_ws.p, int(nw), P->ct, d_Sin, P->d_g2t.p, P->d_wqt.p, nvf,
                                                    P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm), nm * f0, nm * f1, mu,
@@ -1311,9 +1330,12 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
   const long nk = nm * P->nc;
   if (P->path == EPSP_PATH_GEMM_FP64) {
     long pk = prof_begin(ctx, "kbuild");
+    ensure(P->w_fmtab, ctx, size_t((nw + 1) * ni));
+    fm_cell_kernel<<<div_up(size_t((nw + 1) * ni), 128), 128, 0, s>>>(P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
+    EPSP_LAUNCHED(ctx);
     kbuild_f64_kernel<<<dim3(div_up(size_t(nw), 128), unsigned(nk)), 128, 0, s>>>(
-        P->d_ws.p, int(nw), P->ct, d_Sin, P->d_wnu.p, int(nm), P->d_epsc.p, P->d_colc.p, P->nc, P->d_Fa.p, P->d_Fe.p,
-        P->w_ac, P->d_Kt.p);
+        int(nw), P->w_fmtab.p, P->d_cell_j.p, P->d_cell_t.p, P->d_wnu.p, int(nm), P->d_epsc.p, P->d_colc.p, P->d_Fa.p,
+        P->d_Fe.p, P->w_ac, P->d_Kt.p);
     EPSP_LAUNCHED(ctx);
     prof_end(ctx, pk);
     long pg = prof_begin(ctx, "fm_gemm");

@@ -65,7 +65,8 @@ struct Scgd0Plan {
   DBuf<int32_t> d_iq, d_iksi, d_iksf, d_fti;
   DBuf<double> d_epsf;
   DBuf<float4> d_wtab;
-  // cells of ω ± ω_ν for every (ω, ν): [2][nω·nm] lower node, weight and point (absorption, emission)
+  // cells of ω ± ω_ν for every (ω, ν): [2][nω·nm] lower node, weight and point (absorption, emission); GEMM_FP64:
+  // the cell table's entry, the distance from its node, the point
   DBuf<int32_t> d_cell_j;
   DBuf<double> d_cell_t, d_cell_x;
   // tensor-core path state (scgd0_tc.cu)

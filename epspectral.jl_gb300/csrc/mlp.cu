@@ -6,8 +6,8 @@
 // BF16 by the products (BF16 weights, FP32 accumulation); biases FP32. The loss is the mean squared
 // error over the batch and the outputs; the optimiser is Adam. Every product of the training, of
 // the gradient and of the prediction runs on the tensor cores (tc_gemm_launch: tcgen05, TMA, TMEM)
-// with the FP32 activations and gradients split into three BF16 parts (six products, ~2^-24
-// relative, as FP32; the BF16 weights' second and third parts are zero), every reduction in fixed
+// with the FP32 activations and gradients split into three BF16 parts (~2^-24 relative, as FP32:
+// three products against the BF16 weights, six between two such operands), every reduction in fixed
 // order, so a training run is bitwise reproducible. The scGD0 hook's inference (forward_tc) splits
 // the activations into two parts.
 #include "common.cuh"
@@ -37,22 +37,56 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + expf(-
 //   kEmitCopy    src[m ld_src + j];
 //   kEmitBiasAct z = Σ_s part[s pstride + j + cols m] + bias[j] (a product's split-K slabs, summed in
 //                order), written to Zout[m cols + j] when given, then v = SiLU(z) if act, else z;
-//   kEmitActBack Σ_s part[s pstride + j + cols m] times SiLU'(Zin[m cols + j]).
+//   kEmitActBack Σ_s part[s pstride + j + cols m] times SiLU'(Zin[m cols + j]);
+//   kEmitGather  src[idx[m] ld_src + j], idx = B.perm + *B.cur B.batch (the minibatch's rows);
+//   kEmitLoss    inv_nd2 (z - Y[idx[m] cols + j]), z as in kEmitBiasAct (linear, written to Zout): the loss gradient.
 // v goes to out32[m cols + j] (FP32) and, as three BF16 parts, to rp[p rpart + m ldr + j] (rows)
 // and tp[p tpart + j ldt + m] (transposed, through shared memory; columns m in [rows, ldt) get
 // zeros, so that the padded K of a product over the rows adds nothing). Grid (cols / 32, M / 32)
 // with M = ldt when tp is given, else rows; 32 x 8 threads.
-enum { kEmitCopy = 0, kEmitBiasAct = 1, kEmitActBack = 2 };
+enum { kEmitCopy = 0, kEmitBiasAct = 1, kEmitActBack = 2, kEmitGather = 3, kEmitLoss = 4 };
+// A training step's minibatch: its rows are perm[*cur batch ..], its targets Y.
+struct Batch {
+  const int64_t* perm = nullptr;
+  const int* cur = nullptr;
+  long batch = 0;
+  const float* Y = nullptr;
+  float inv_nd2 = 0.f;
+};
 template <int MODE>
 __global__ void __launch_bounds__(256)
     emit_kernel(int rows, int cols, const float* __restrict__ src, long ld_src, const float* __restrict__ part, int splits,
                 long pstride, const float* __restrict__ bias, bool act, const float* __restrict__ Zin,
                 float* __restrict__ Zout, float* __restrict__ out32, __nv_bfloat16* __restrict__ rp, long ldr, long rpart,
-                __nv_bfloat16* __restrict__ tp, long ldt, long tpart) {
+                __nv_bfloat16* __restrict__ tp, long ldt, long tpart, const Batch B = Batch()) {
   __shared__ float tile[32][33];
+  const int64_t* idx = nullptr;
+  if constexpr (MODE == kEmitGather || MODE == kEmitLoss) idx = B.perm + *B.cur * B.batch;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int j0 = blockIdx.x * 32, m0 = blockIdx.y * 32;
   const int j = j0 + tx;
+  // the slabs of the thread's four elements, each in ascending order, all loads of a slab and several slabs in flight
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  if constexpr (MODE == kEmitBiasAct || MODE == kEmitActBack || MODE == kEmitLoss) {
+    const float* q[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) q[r] = part + min(j, cols - 1) + long(cols) * min(m0 + ty + 8 * r, rows - 1);
+    int sp = 0;
+    for (; sp + 4 <= splits; sp += 4) {
+      float x[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[u][r] = q[r][(sp + u) * pstride];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) sum[r] += x[u][r];
+    }
+    for (; sp < splits; ++sp)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sum[r] += q[r][sp * pstride];
+  }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int ml = ty + 8 * r, m = m0 + ml;
@@ -60,13 +94,19 @@ __global__ void __launch_bounds__(256)
     if (m < rows && j < cols) {
       if constexpr (MODE == kEmitCopy) {
         v = src[long(m) * ld_src + j];
+      } else if constexpr (MODE == kEmitGather) {
+        v = src[idx[m] * ld_src + j];
       } else {
-        float acc = 0.f;
-        for (int sp = 0; sp < splits; ++sp) acc += part[long(sp) * pstride + j + long(cols) * m];
+        const float acc = sum[r];
         if constexpr (MODE == kEmitBiasAct) {
           const float z = acc + bias[j];
           if (Zout) Zout[long(m) * cols + j] = z;
           v = act ? z * sigmoidf_(z) : z;
+        } else if constexpr (MODE == kEmitLoss) {
+          const float z = acc + bias[j];
+          Zout[long(m) * cols + j] = z;
+          const float e = z - B.Y[idx[m] * cols + j];
+          v = B.inv_nd2 * e;
         } else {
           const float z = Zin[long(m) * cols + j], sg = sigmoidf_(z);
           v = acc * (sg * (1.f + z * (1.f - sg)));
@@ -138,7 +178,42 @@ __global__ void sum_kernel(const float* __restrict__ x, long n, double* __restri
   if (threadIdx.x == 0) out[slot] = sh[0];
 }
 
-__global__ void step_kernel(int* t) { *t += 1; }
+// A training step's row losses (mse_kernel's, the targets gathered), and their sum into out[*cur], after which the
+// cursor and Adam's step count move on: every reader of this step's cursor has run, Adam reads the new count.
+__global__ void __launch_bounds__(256) row_loss_kernel(const float* __restrict__ P, int d, const Batch B,
+                                                       float* __restrict__ row_loss) {
+  __shared__ float sh[256];
+  const long m = blockIdx.x;
+  const float* Y = B.Y + B.perm[*B.cur * B.batch + m] * d;
+  float s = 0.f;
+  for (int j = threadIdx.x; j < d; j += 256) {
+    const float e = P[m * d + j] - Y[j];
+    s += e * e;
+  }
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int st = 128; st > 0; st >>= 1) {
+    if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) row_loss[m] = sh[0];
+}
+__global__ void loss_step_kernel(const float* __restrict__ x, long n, double* __restrict__ out, int* cur, int* step) {
+  __shared__ double sh[256];
+  double s = 0;
+  for (long k = threadIdx.x; k < n; k += 256) s += x[k];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int st = 128; st > 0; st >>= 1) {
+    if (threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    out[*cur] = sh[0];
+    *cur += 1;
+    *step += 1;
+  }
+}
 
 // BF16 copies of the weight element k = o d_in + i of W [d_out][d_in]: wbf[k], the tensor-core
 // products' rows wp[o ldp + i] and the transposed rows wt[i ldt + o].
@@ -152,37 +227,99 @@ __device__ __forceinline__ void store_wbf(long k, float w, int din, __nv_bfloat1
   wt[i * ldt + o] = h;
 }
 
-// Adam step t (read from the device, so a captured epoch replays with the right bias corrections)
-// on one parameter block; for a weight block (wbf given) writes the BF16 copies the products use.
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1, float* __restrict__ m2,
-                            long n, float lr, float b1, float b2, float eps, const int* __restrict__ t,
-                            __nv_bfloat16* __restrict__ wbf, int din, __nv_bfloat16* __restrict__ wp, long ldp,
-                            __nv_bfloat16* __restrict__ wt, long ldt) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const float c1 = 1.f - powf(b1, float(*t)), c2 = 1.f - powf(b2, float(*t));
-  const float gk = g[k];
-  const float a = b1 * m1[k] + (1.f - b1) * gk;
-  const float v = b2 * m2[k] + (1.f - b2) * gk * gk;
-  m1[k] = a;
-  m2[k] = v;
-  const float wn = w[k] - lr * (a / c1) / (sqrtf(v / c2) + eps);
-  w[k] = wn;
-  if (wbf) store_wbf(k, wn, din, wbf, wp, ldp, wt, ldt);
+// Adam step *t on every layer's weights in one launch, tiles of 32 x 32, the gradient summed from its product's
+// split-K slabs (element k = o d_in + i of slab z at z pstride + k, z ascending) as it is read; writes the BF16 copies
+// the products use, the transposed one through shared memory. (One launch a block of parameters with separate
+// slab sums took 12 launches a step and wrote the transposed weights 2 bytes at a time.)
+struct AdamLayer {
+  float *w, *m1, *m2;
+  const float* slab;
+  long pstride, ldp, ldt;
+  __nv_bfloat16 *wbf, *wp, *wt;
+  int splits, din, dout, tile0;  // the layer's first tile
+};
+struct AdamAll {
+  AdamLayer l[16];
+  int L;
+  float lr, b1, b2, eps;
+  const int* t;
+};
+// One parameter: the new moments stored, the new value returned.
+__device__ __forceinline__ float adam_one(float w, float gk, float* m1, float* m2, float lr, float b1, float b2, float eps,
+                                          float c1, float c2) {
+  const float a = b1 * *m1 + (1.f - b1) * gk;
+  const float v = b2 * *m2 + (1.f - b2) * gk * gk;
+  *m1 = a;
+  *m2 = v;
+  return w - lr * (a / c1) / (sqrtf(v / c2) + eps);
+}
+__global__ void __launch_bounds__(256) adam_weights_kernel(const __grid_constant__ AdamAll A) {
+  __shared__ __nv_bfloat16 tile[32][33];
+  __shared__ float sc[2];
+  int l = 0;
+  while (l + 1 < A.L && int(blockIdx.x) >= A.l[l + 1].tile0) ++l;
+  const AdamLayer& y = A.l[l];
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  if (threadIdx.x == 0) {
+    sc[0] = 1.f - powf(A.b1, float(*A.t));
+    sc[1] = 1.f - powf(A.b2, float(*A.t));
+  }
+  const int ti = (y.din + 31) / 32, tl = int(blockIdx.x) - y.tile0;
+  const int i0 = (tl % ti) * 32, o0 = (tl / ti) * 32;
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int o = o0 + ty + 8 * r, i = i0 + tx;
+    if (o >= y.dout || i >= y.din) continue;
+    const long k = long(o) * y.din + i;
+    float g = 0.f;
+#pragma unroll 4
+    for (int z = 0; z < y.splits; ++z) g += y.slab[z * y.pstride + k];
+    const float wn = adam_one(y.w[k], g, y.m1 + k, y.m2 + k, A.lr, A.b1, A.b2, A.eps, sc[0], sc[1]);
+    y.w[k] = wn;
+    const __nv_bfloat16 h = __float2bfloat16_rn(wn);
+    y.wbf[k] = h;
+    y.wp[o * y.ldp + i] = h;
+    tile[ty + 8 * r][tx] = h;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + ty + 8 * r, o = o0 + tx;
+    if (o < y.dout && i < y.din) y.wt[i * y.ldt + o] = tile[tx][ty + 8 * r];
+  }
+}
+// The biases of every layer: db[j] = Σ_m dZ[m][j] in ascending m (32 loads in flight), then their Adam step.
+struct BiasLayer {
+  const float* dz;
+  float *b, *m1, *m2;
+  int d, col0;
+};
+struct BiasAll {
+  BiasLayer l[16];
+  int L, cols;
+  long n;
+  float lr, b1, b2, eps;
+  const int* t;
+};
+__global__ void __launch_bounds__(32) adam_bias_kernel(const __grid_constant__ BiasAll A) {
+  const int c = blockIdx.x * 32 + threadIdx.x;
+  if (c >= A.cols) return;
+  int l = 0;
+  while (l + 1 < A.L && c >= A.l[l + 1].col0) ++l;
+  const BiasLayer& y = A.l[l];
+  const int j = c - y.col0;
+  float s = 0.f;
+#pragma unroll 32
+  for (long m = 0; m < A.n; ++m) s += y.dz[m * y.d + j];
+  const float c1 = 1.f - powf(A.b1, float(*A.t)), c2 = 1.f - powf(A.b2, float(*A.t));
+  y.b[j] = adam_one(y.b[j], s, y.m1 + j, y.m2 + j, A.lr, A.b1, A.b2, A.eps, c1, c2);
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ w, long n, int din, __nv_bfloat16* __restrict__ wbf,
                                __nv_bfloat16* __restrict__ wp, long ldp, __nv_bfloat16* __restrict__ wt, long ldt) {
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k < n) store_wbf(k, w[k], din, wbf, wp, ldp, wt, ldt);
-}
-
-// Gathers the rows idx[0..n) of X [N][d] into out [n][d].
-__global__ void gather_rows_kernel(const float* __restrict__ X, const int64_t* __restrict__ idx, long n, int d,
-                                   float* __restrict__ out) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n * d) return;
-  out[k] = X[idx[k / d] * d + k % d];
 }
 
 struct Mlp {
@@ -195,9 +332,10 @@ struct Mlp {
   DBuf<float> dA, dB, loss_rows, Yb;
   DBuf<int> d_err;                // the tensor-core products' bounded-wait flag
   DBuf<double> loss_sum;
-  DBuf<int> d_step;  // Adam's step counter
+  DBuf<int> d_step;  // Adam's step counter, and the training epoch's next minibatch
   long cap = 0;      // rows the activation buffers hold
   DBuf<float> dataX, dataY;
+  DBuf<int64_t> perm;  // the epoch's row order
   long ndata = 0;
   DBuf<float> x_mean, x_std, y_mean;  // feature standardisation for the in-iteration hook
   float y_scale = 1.f;
@@ -225,9 +363,19 @@ struct Mlp {
     long cap = 0, ldT = 0;
     std::vector<int> dp;
     std::vector<DBuf<__nv_bfloat16>> Wp, WT, Xs, XT, dZs, dZT;
-    DBuf<__nv_bfloat16> zero;  // the weights' second and third parts
     std::vector<TcOperand> opW, opWT, opXs, opXT, opdZs, opdZT;
     DBuf<float> part;
+    // a training step's FP32 dZ and gradient slabs of every layer, and the stream that runs beside the backward chain
+    std::vector<DBuf<float>> dz, slab;
+    struct Side {
+      cudaStream_t s = nullptr;
+      cudaEvent_t fork = nullptr, join = nullptr;
+      ~Side() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (s) cudaStreamDestroy(s);
+      }
+    } side;
   } tr;
 };
 
@@ -266,14 +414,13 @@ __global__ void correct_kernel(double2* __restrict__ S, int nw, const float* __r
   S[long(i) * nw + j] = v;
 }
 
-// A three-part operand over `parts` (three consecutive [rows][ld] BF16 blocks, or one block and
-// the shared zero block twice when zero is given), boxes of box_rows rows.
-static TcOperand three_part(const __nv_bfloat16* parts, const __nv_bfloat16* zero, long rows, long cols, long ld,
-                            int box_rows) {
+// An operand of ns = 3 parts (three consecutive [rows][ld] BF16 blocks) or, for the weights, of one; boxes of
+// box_rows rows.
+static TcOperand operand_parts(const __nv_bfloat16* parts, int ns, long rows, long cols, long ld, int box_rows) {
   TcOperand op;
-  op.ns = 3;
-  for (int p = 0; p < 3; ++p) {
-    const __nv_bfloat16* base = p == 0 ? parts : zero ? zero : parts + long(p) * rows * ld;
+  op.ns = ns;
+  for (int p = 0; p < ns; ++p) {
+    const __nv_bfloat16* base = parts + long(p) * rows * ld;
     op.m[p] = make_tmap_bf16(base, rows, cols, ld, box_rows);
     op.base[p] = base;
   }
@@ -291,23 +438,19 @@ static void train_weights_init(Mlp* P) {
   for (int l = 0; l <= L; ++l) T.dp[size_t(l)] = (P->dims[size_t(l)] + 7) / 8 * 8;
   T.Wp.resize(size_t(L));
   T.WT.resize(size_t(L));
-  size_t zmax = 0;
   for (int l = 0; l < L; ++l) {
     const long din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
     T.Wp[size_t(l)].alloc(P->ctx, size_t(dout * T.dp[size_t(l)]));
     T.WT[size_t(l)].alloc(P->ctx, size_t(din * T.dp[size_t(l + 1)]));
     T.Wp[size_t(l)].zero(P->ctx->stream);  // the padding columns stay zero
     T.WT[size_t(l)].zero(P->ctx->stream);
-    zmax = std::max(zmax, std::max(size_t(dout * T.dp[size_t(l)]), size_t(din * T.dp[size_t(l + 1)])));
   }
-  T.zero.alloc(P->ctx, zmax);
-  T.zero.zero(P->ctx->stream);
   T.opW.resize(size_t(L));
   T.opWT.resize(size_t(L));
   for (int l = 0; l < L; ++l) {
     const long din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
-    T.opW[size_t(l)] = three_part(T.Wp[size_t(l)].p, T.zero.p, dout, din, T.dp[size_t(l)], kTcBM);
-    T.opWT[size_t(l)] = three_part(T.WT[size_t(l)].p, T.zero.p, din, dout, T.dp[size_t(l + 1)], kTcBM);
+    T.opW[size_t(l)] = operand_parts(T.Wp[size_t(l)].p, 1, dout, din, T.dp[size_t(l)], kTcBM);
+    T.opWT[size_t(l)] = operand_parts(T.WT[size_t(l)].p, 1, din, dout, T.dp[size_t(l + 1)], kTcBM);
   }
 }
 
@@ -332,6 +475,7 @@ static void ensure_cap(Mlp* P, long n) {
   T.cap = n;
   T.ldT = (n + 7) / 8 * 8;
   for (auto* v : {&T.Xs, &T.XT, &T.dZs, &T.dZT}) v->resize(size_t(L));
+  for (auto* v : {&T.dz, &T.slab}) v->resize(size_t(L));
   for (auto* v : {&T.opXs, &T.opXT, &T.opdZs, &T.opdZT}) v->resize(size_t(L));
   const long sm = ctx->sm_count;
   auto tiles = [](long M, long N) { return ((M + 127) / 128) * ((N + 127) / 128); };
@@ -343,23 +487,28 @@ static void ensure_cap(Mlp* P, long n) {
     T.XT[size_t(l)].alloc(ctx, size_t(3 * din * T.ldT));
     T.dZs[size_t(l)].alloc(ctx, size_t(3 * n * dpo));
     T.dZT[size_t(l)].alloc(ctx, size_t(3 * dout * T.ldT));
-    T.opXs[size_t(l)] = three_part(T.Xs[size_t(l)].p, nullptr, n, din, dpi, 128);
-    T.opXT[size_t(l)] = three_part(T.XT[size_t(l)].p, nullptr, din, T.ldT, T.ldT, kTcBM);
-    T.opdZs[size_t(l)] = three_part(T.dZs[size_t(l)].p, nullptr, n, dout, dpo, 128);
-    T.opdZT[size_t(l)] = three_part(T.dZT[size_t(l)].p, nullptr, dout, T.ldT, T.ldT, 128);
+    T.opXs[size_t(l)] = operand_parts(T.Xs[size_t(l)].p, 3, n, din, dpi, 128);
+    T.opXT[size_t(l)] = operand_parts(T.XT[size_t(l)].p, 3, din, T.ldT, T.ldT, kTcBM);
+    T.opdZs[size_t(l)] = operand_parts(T.dZs[size_t(l)].p, 3, n, dout, dpo, 128);
+    T.opdZT[size_t(l)] = operand_parts(T.dZT[size_t(l)].p, 3, dout, T.ldT, T.ldT, 128);
+    T.dz[size_t(l)].alloc(ctx, size_t(n * dout));
+    const long tw = tiles(din, dout);
+    T.slab[size_t(l)].alloc(ctx, size_t(std::min<long>(16, (sm + tw - 1) / tw) * din * dout));
     for (const long t : {tiles(dout, n), tiles(din, dout), tiles(din, n)}) part = std::max(part, (sm + t) * 128 * 128);
   }
   T.part.alloc(ctx, size_t(part));
   P->cap = n;
 }
 
-// One three-part product into the split-K slabs T.part (out[s][m + ld_out n]); returns the splits.
-static int mlp_product(Mlp* P, const TcOperand& A, const TcOperand& B, int M, int N, int K, long ld_out) {
+// One three-part product into the split-K slabs `out` (T.part by default; out[s][m + ld_out n]); returns the splits.
+static int mlp_product(Mlp* P, const TcOperand& A, const TcOperand& B, int M, int N, int K, long ld_out,
+                       DBuf<float>* out = nullptr) {
+  if (!out) out = &P->tr.part;
   int bn = 0, sp = 0;
   tc_gemm_shape(P->ctx, M, N, K, 16, 3, &bn, &sp);
   if (bn != 128) fail(EPSP_EINVAL, "three-part products run with tiles of 128 columns");
-  if (size_t(sp) * size_t(M) * size_t(N) > P->tr.part.n) fail(EPSP_EINVAL, "split-K slabs exceed their buffer");
-  return tc_gemm_launch(P->ctx, A, B, M, N, K, P->tr.part.p, ld_out, long(M) * N, 16, P->d_err.p, "mlp");
+  if (size_t(sp) * size_t(M) * size_t(N) > out->n) fail(EPSP_EINVAL, "split-K slabs exceed their buffer");
+  return tc_gemm_launch(P->ctx, A, B, M, N, K, out->p, ld_out, long(M) * N, 16, P->d_err.p, "mlp");
 }
 
 static dim3 emit_grid(long cols, long rows) { return dim3(unsigned((cols + 31) / 32), unsigned((rows + 31) / 32)); }
@@ -571,24 +720,111 @@ static void forward_tc(Mlp* P, long n, int* d_err) {
   }
 }
 
-static void adam(Mlp* P, float lr) {
+// One training step on the minibatch of n rows at the cursor (B; the data set's inputs dataX): forward, backward, Adam.
+// The gradient products, the losses and the biases run on the side stream beside the backward chain, of which each
+// layer is one product and one epilogue: for four layers 17 launches in a row and 6 beside them, where the step was 41
+// in a row. Bound by the latency of those 17 (256 rows are 16 to 152 tiles of work). Measured with widths 2506, 256, 256,
+// 256, 2502: 238 -> 145 us a step of 256 rows, bitwise the same parameters.
+static void train_step(Mlp* P, long n, const Batch& B, float lr) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
+  Mlp::Train& T = P->tr;
+  auto& sd = T.side;
+  if (!sd.s) {
+    EPSP_CUDA(cudaStreamCreateWithFlags(&sd.s, cudaStreamNonBlocking));
+    EPSP_CUDA(cudaEventCreateWithFlags(&sd.fork, cudaEventDisableTiming));
+    EPSP_CUDA(cudaEventCreateWithFlags(&sd.join, cudaEventDisableTiming));
+  }
+  struct OnSide {  // launches through ctx go to the side stream while it lives, after what the main stream holds
+    Ctx* c;
+    cudaStream_t main;
+    OnSide(Ctx* c_, Mlp::Train::Side& d) : c(c_), main(c_->stream) {
+      EPSP_CUDA(cudaEventRecord(d.fork, main));
+      EPSP_CUDA(cudaStreamWaitEvent(d.s, d.fork, 0));
+      c->stream = d.s;
+    }
+    ~OnSide() { c->stream = main; }
+  };
+  const dim3 blk(32, 8);
+  const int L = P->L, d0 = P->dims[0], dl = P->dims.back();
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  step_kernel<<<1, 1, 0, s>>>(P->d_step.p);
+  emit_kernel<kEmitGather><<<emit_grid(d0, T.ldT), blk, 0, s>>>(
+      int(n), d0, P->dataX.p, d0, nullptr, 0, 0, nullptr, false, nullptr, nullptr, nullptr, T.Xs[0].p, T.dp[0],
+      long(T.cap) * T.dp[0], T.XT[0].p, T.ldT, long(d0) * T.ldT, B);
   EPSP_LAUNCHED(ctx);
-  for (int l = 0; l < P->L; ++l) {
-    const long nw = long(P->dims[size_t(l)]) * P->dims[size_t(l + 1)], nb = P->dims[size_t(l + 1)];
-    adam_kernel<<<div_up(size_t(nw), 256), 256, 0, s>>>(
-        P->W[size_t(l)].p, P->gW[size_t(l)].p, P->mW[size_t(l)].p, P->vW[size_t(l)].p, nw, lr, b1, b2, eps, P->d_step.p,
-        P->Wbf[size_t(l)].p, P->dims[size_t(l)], P->tr.Wp[size_t(l)].p, P->tr.dp[size_t(l)], P->tr.WT[size_t(l)].p,
-        P->tr.dp[size_t(l + 1)]);
-    EPSP_LAUNCHED(ctx);
-    adam_kernel<<<div_up(size_t(nb), 256), 256, 0, s>>>(P->b[size_t(l)].p, P->gb[size_t(l)].p, P->mb[size_t(l)].p,
-                                                        P->vb[size_t(l)].p, nb, lr, b1, b2, eps, P->d_step.p, nullptr, 1,
-                                                        nullptr, 0, nullptr, 0);
+  for (int l = 0; l < L; ++l) {
+    const int din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
+    const int sp = mlp_product(P, T.opW[size_t(l)], T.opXs[size_t(l)], dout, int(n), din, dout);
+    if (l + 1 < L)
+      emit_kernel<kEmitBiasAct><<<emit_grid(dout, T.ldT), blk, 0, s>>>(
+          int(n), dout, nullptr, 0, T.part.p, sp, long(dout) * n, P->b[size_t(l)].p, true, nullptr, P->Z[size_t(l)].p,
+          nullptr, T.Xs[size_t(l + 1)].p, T.dp[size_t(l + 1)], long(T.cap) * T.dp[size_t(l + 1)], T.XT[size_t(l + 1)].p,
+          T.ldT, long(dout) * T.ldT);
+    else  // the output and dZ of the last layer
+      emit_kernel<kEmitLoss><<<emit_grid(dout, T.ldT), blk, 0, s>>>(
+          int(n), dout, nullptr, 0, T.part.p, sp, long(dout) * n, P->b[size_t(l)].p, false, nullptr, P->X[size_t(L)].p,
+          T.dz[size_t(l)].p, T.dZs[size_t(l)].p, T.dp[size_t(L)], long(T.cap) * T.dp[size_t(L)], T.dZT[size_t(l)].p, T.ldT,
+          long(dl) * T.ldT, B);
     EPSP_LAUNCHED(ctx);
   }
+  AdamAll aw{};
+  BiasAll ab{};
+  aw.L = ab.L = L;
+  aw.lr = ab.lr = lr;
+  aw.b1 = ab.b1 = b1;
+  aw.b2 = ab.b2 = b2;
+  aw.eps = ab.eps = eps;
+  aw.t = ab.t = P->d_step.p;
+  ab.n = n;
+  // gW[o][i] = Σ_m dZ[m][o] X[m][i]: the product's slab element (i, o) at i + din o
+  auto weight_gradient = [&](int l) {
+    const int din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
+    aw.l[l].splits = mlp_product(P, T.opXT[size_t(l)], T.opdZT[size_t(l)], din, dout, int(n), din, &T.slab[size_t(l)]);
+  };
+  {
+    OnSide on(ctx, sd);
+    row_loss_kernel<<<unsigned(n), 256, 0, sd.s>>>(P->X[size_t(L)].p, dl, B, P->loss_rows.p);
+    EPSP_LAUNCHED(ctx);
+    loss_step_kernel<<<1, 256, 0, sd.s>>>(P->loss_rows.p, n, P->loss_sum.p, P->d_step.p + 1, P->d_step.p);
+    EPSP_LAUNCHED(ctx);
+    if (L > 1) weight_gradient(L - 1);
+  }
+  for (int l = L - 1; l >= 1; --l) {
+    // dX[m][i] = Σ_o dZ[m][o] W[o][i] (slab element (i, m) at i + din m), through SiLU of layer l - 1
+    const int din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
+    const int sx = mlp_product(P, T.opWT[size_t(l)], T.opdZs[size_t(l)], din, int(n), dout, din);
+    emit_kernel<kEmitActBack><<<emit_grid(din, T.ldT), blk, 0, s>>>(
+        int(n), din, nullptr, 0, T.part.p, sx, long(din) * n, nullptr, false, P->Z[size_t(l - 1)].p, nullptr,
+        T.dz[size_t(l - 1)].p, T.dZs[size_t(l - 1)].p, T.dp[size_t(l)], long(T.cap) * T.dp[size_t(l)],
+        T.dZT[size_t(l - 1)].p, T.ldT, long(din) * T.ldT);
+    EPSP_LAUNCHED(ctx);
+    if (l > 1) {
+      OnSide on(ctx, sd);
+      weight_gradient(l - 1);
+    }
+  }
+  {
+    OnSide on(ctx, sd);
+    for (int l = 0, c = 0; l < L; c += P->dims[size_t(++l)])
+      ab.l[l] = BiasLayer{T.dz[size_t(l)].p, P->b[size_t(l)].p, P->mb[size_t(l)].p, P->vb[size_t(l)].p, P->dims[size_t(l + 1)],
+                          c};
+    ab.cols = ab.l[L - 1].col0 + dl;
+    adam_bias_kernel<<<div_up(size_t(ab.cols), 32), 32, 0, sd.s>>>(ab);
+    EPSP_LAUNCHED(ctx);
+    EPSP_CUDA(cudaEventRecord(sd.join, sd.s));
+  }
+  weight_gradient(0);
+  EPSP_CUDA(cudaStreamWaitEvent(s, sd.join, 0));
+  int tiles = 0;
+  for (int l = 0; l < L; ++l) {
+    const int din = P->dims[size_t(l)], dout = P->dims[size_t(l + 1)];
+    aw.l[l] = AdamLayer{P->W[size_t(l)].p, P->mW[size_t(l)].p, P->vW[size_t(l)].p, T.slab[size_t(l)].p, long(din) * dout,
+                        T.dp[size_t(l)], T.dp[size_t(l + 1)], P->Wbf[size_t(l)].p, T.Wp[size_t(l)].p, T.WT[size_t(l)].p,
+                        aw.l[l].splits, din, dout, tiles};
+    tiles += ((din + 31) / 32) * ((dout + 31) / 32);
+  }
+  adam_weights_kernel<<<unsigned(tiles), 256, 0, s>>>(aw);
+  EPSP_LAUNCHED(ctx);
 }
 
 static long nparams(const Mlp* P) {
@@ -681,7 +917,7 @@ epsp_status epsp_warmstart_create(epsp_ctx* ctx, int32_t nlayers, const int32_t*
         v->zero(P.ctx->stream);
     }
     P.loss_sum.alloc(P.ctx, 1);
-    P.d_step.alloc(P.ctx, 1);
+    P.d_step.alloc(P.ctx, 2);
     P.d_step.zero(P.ctx->stream);
     P.d_err.alloc(P.ctx, 1);
     P.d_err.zero(P.ctx->stream);
@@ -834,35 +1070,24 @@ epsp_status epsp_warmstart_train(epsp_warmstart* w, const float* X, const float*
     if (perm)
       for (long k = 0; k < long(epochs) * n; ++k)
         if (perm[k] < 0 || perm[k] >= n) fail(EPSP_EINVAL, "perm holds an index outside [0, n)");
-    const long nbat = (n + batch - 1) / batch;
-    P.dataX.alloc(P.ctx, size_t(n) * size_t(d0));
-    P.dataY.alloc(P.ctx, size_t(n) * size_t(dl));
+    const long nbat = (n + batch - 1) / batch, rows = std::min<long>(n, batch);
+    ensure(P.dataX, P.ctx, size_t(n) * size_t(d0));
+    ensure(P.dataY, P.ctx, size_t(n) * size_t(dl));
     P.dataX.upload(X, size_t(n) * size_t(d0), s);
     P.dataY.upload(Y, size_t(n) * size_t(dl), s);
-    DBuf<int64_t> d_perm;
-    d_perm.alloc(P.ctx, size_t(n));
-    P.loss_sum.alloc(P.ctx, size_t(nbat));
-    ensure_cap(&P, std::min<long>(n, batch));
+    ensure(P.perm, P.ctx, size_t(n));
+    ensure(P.loss_sum, P.ctx, size_t(nbat));
+    ensure_cap(&P, rows);
     std::vector<int64_t> ident;
     if (!perm) {
       ident.resize(size_t(n));
       for (long k = 0; k < n; ++k) ident[size_t(k)] = k;
     }
     std::vector<double> bl(static_cast<size_t>(nbat));
-    // One epoch's launches (every minibatch: gather, forward, backward, Adam) are captured once in a
-    // CUDA graph and replayed per epoch; only the row order (uploaded before each replay) changes.
-    auto epoch_launches = [&] {
-      for (long bi = 0; bi < nbat; ++bi) {
-        const long r0 = bi * batch, nb = std::min<long>(batch, n - r0);
-        gather_rows_kernel<<<div_up(size_t(nb * d0), 256), 256, 0, s>>>(P.dataX.p, d_perm.p + r0, nb, d0, P.X[0].p);
-        EPSP_LAUNCHED(P.ctx);
-        gather_rows_kernel<<<div_up(size_t(nb * dl), 256), 256, 0, s>>>(P.dataY.p, d_perm.p + r0, nb, dl, P.Yb.p);
-        EPSP_LAUNCHED(P.ctx);
-        forward_train(&P, nb, true);
-        backward(&P, nb, nb, int(bi));
-        adam(&P, lr);
-      }
-    };
+    // A step's launches are captured once in a CUDA graph and replayed for every full minibatch (its rows, loss slot and
+    // step count come from the device); the first step and a last, smaller minibatch are launched one by one (the first
+    // launches set the kernels' attributes).
+    auto step = [&](long nb) { train_step(&P, nb, Batch{P.perm.p, P.d_step.p + 1, batch, P.dataY.p, 2.f / (float(nb) * float(dl))}, lr); };
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     struct GraphGuard {
@@ -873,31 +1098,7 @@ epsp_status epsp_warmstart_train(epsp_warmstart* w, const float* X, const float*
         if (*g) cudaGraphDestroy(*g);
       }
     } gguard{&graph, &exec};
-    // one gradient pass on the first minibatch outside the capture (no parameter update), so that
-    // every kernel's launch attributes are set before the capture
-    {
-      const long nb = std::min<long>(batch, n);
-      d_perm.upload(perm ? perm : ident.data(), size_t(n), s);
-      gather_rows_kernel<<<div_up(size_t(nb * d0), 256), 256, 0, s>>>(P.dataX.p, d_perm.p, nb, d0, P.X[0].p);
-      EPSP_LAUNCHED(P.ctx);
-      gather_rows_kernel<<<div_up(size_t(nb * dl), 256), 256, 0, s>>>(P.dataY.p, d_perm.p, nb, dl, P.Yb.p);
-      EPSP_LAUNCHED(P.ctx);
-      forward_train(&P, nb, true);
-      backward(&P, nb, nb, 0);
-      check_mlp_err(&P);
-    }
-    const int64_t l0 = P.ctx->launches;
-    EPSP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    try {
-      epoch_launches();
-    } catch (...) {
-      cudaStreamEndCapture(s, &graph);
-      throw;
-    }
-    EPSP_CUDA(cudaStreamEndCapture(s, &graph));
-    EPSP_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-    const int64_t per_epoch = P.ctx->launches - l0;
-    P.ctx->launches = l0;
+    int64_t per_step = 0;
     cudaEvent_t ev[2] = {nullptr, nullptr};
     struct EventGuard {
       cudaEvent_t* e;
@@ -909,11 +1110,33 @@ epsp_status epsp_warmstart_train(epsp_warmstart* w, const float* X, const float*
     for (auto& e : ev) EPSP_CUDA(cudaEventCreate(&e));
     P.train_ms = 0;
     for (int e = 0; e < epochs; ++e) {
-      d_perm.upload(perm ? perm + long(e) * n : ident.data(), size_t(n), s);
+      P.perm.upload(perm ? perm + long(e) * n : ident.data(), size_t(n), s);
+      EPSP_CUDA(cudaMemsetAsync(P.d_step.p + 1, 0, sizeof(int), s));  // the epoch's first minibatch
       EPSP_CUDA(cudaEventRecord(ev[0], s));
-      EPSP_CUDA(cudaGraphLaunch(exec, s));
+      for (long bi = 0; bi < nbat; ++bi) {
+        const long nb = std::min<long>(batch, n - bi * batch);
+        if ((e == 0 && bi == 0) || nb < rows) {
+          step(nb);
+          continue;
+        }
+        if (!exec) {
+          const int64_t l0 = P.ctx->launches;
+          EPSP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+          try {
+            step(nb);
+          } catch (...) {
+            cudaStreamEndCapture(s, &graph);
+            throw;
+          }
+          EPSP_CUDA(cudaStreamEndCapture(s, &graph));
+          EPSP_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+          per_step = P.ctx->launches - l0;
+          P.ctx->launches = l0;
+        }
+        EPSP_CUDA(cudaGraphLaunch(exec, s));
+        P.ctx->launches += per_step;
+      }
       EPSP_CUDA(cudaEventRecord(ev[1], s));
-      P.ctx->launches += per_epoch;
       P.loss_sum.download(bl.data(), size_t(nbat), s);
       check_mlp_err(&P);
       float ms = 0;
@@ -923,9 +1146,11 @@ epsp_status epsp_warmstart_train(epsp_warmstart* w, const float* X, const float*
       for (double v : bl) tot += v;
       if (loss_history) loss_history[e] = tot / (double(n) * dl);
     }
-    P.dataX.release();
-    P.dataY.release();
-    P.loss_sum.alloc(P.ctx, 1);
+    // a data set of up to 256 MiB keeps its memory for the next call
+    if ((P.dataX.n + P.dataY.n) * sizeof(float) > (size_t(256) << 20)) {
+      P.dataX.release();
+      P.dataY.release();
+    }
     ++P.wgen;
   });
 }

@@ -122,13 +122,13 @@ static CUtensorMap remap(const TcOperand& op, int p, int box_rows) {
                  : make_tmap_bf16(op.base[p], op.rows, op.cols, op.ld, box_rows, op.bk);
 }
 
-template <int BN, int STAGES, int NS, int BK, bool TF32 = false>
+template <int BN, int STAGES, int NS, int BK, bool TF32 = false, int NA = NS>
 static void launch_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int N, int kblocks, int per,
                            int splits, float* out, long ld_out, long split_stride, int* d_err, int gm = 1) {
-  using L = TcPSmem<BN, STAGES, NS, BK, TF32>;
+  using L = TcPSmem<BN, STAGES, NS, BK, TF32, NA>;
   if (A.bk != BK || B.bk != BK) fail(EPSP_EINVAL, "operand tensor maps were built for another K block");
   if (A.tf32 != TF32 || B.tf32 != TF32) fail(EPSP_EINVAL, "operand tensor maps were built for another element type");
-  auto* kern = tc_gemm_persist_kernel<BN, STAGES, NS, BK, TF32>;
+  auto* kern = tc_gemm_persist_kernel<BN, STAGES, NS, BK, TF32, NA>;
   static bool configured = false;  // one process, one attribute setting per instantiation
   if (!configured) {
     EPSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
@@ -136,7 +136,7 @@ static void launch_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B, int
   }
   TcMaps maps;
   for (int p = 0; p < 3; ++p) {
-    maps.a[p] = A.m[p < NS ? p : 0];
+    maps.a[p] = A.m[p < NA ? p : 0];
     maps.b[p] = B.m[p < NS ? p : 0];
   }
   const int nN = (N + BN - 1) / BN, nM = (M + kTcBM - 1) / kTcBM;
@@ -223,16 +223,19 @@ static void launch_pair_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B
 int tc_gemm_launch(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int N, int K, float* out, long ld_out,
                    long split_stride, int max_splits, int* d_err, const char* prof_name, int kb_cap) {
   if (A.tf32 || B.tf32) fail(EPSP_EINVAL, "TF32 operands take tc_gemm_launch_with");
-  if (A.ns != B.ns || (A.ns != 2 && A.ns != 3)) fail(EPSP_EINVAL, "operands must be split into 2 or 3 parts alike");
+  const bool one = A.ns == 1 && B.ns == 3;  // A exact in BF16
+  if (!one && (A.ns != B.ns || (A.ns != 2 && A.ns != 3))) fail(EPSP_EINVAL, "operands must be split into 2 or 3 parts alike");
   if (A.bk != B.bk) fail(EPSP_EINVAL, "operands built for different K blocks");
   int BN, splits;
-  tc_gemm_shape(ctx, M, N, K, max_splits, A.ns, &BN, &splits, kb_cap);  // splits from K blocks of 64
+  tc_gemm_shape(ctx, M, N, K, max_splits, B.ns, &BN, &splits, kb_cap);  // splits from K blocks of 64
   const int bk = A.bk;
   const int kblocks = (K + bk - 1) / bk;
   const int per = (kblocks + splits - 1) / splits;
   splits = (kblocks + per - 1) / per;
   long pi = prof_begin(ctx, prof_name);
-  if (A.ns == 3 && bk == 32)  // three-part operands in K blocks of 32: four stages
+  if (one && bk == kTcBK)
+    launch_persist<128, 3, 3, 64, false, 1>(ctx, A, B, M, N, kblocks, per, splits, out, ld_out, split_stride, d_err);
+  else if (A.ns == 3 && bk == 32)  // three-part operands in K blocks of 32: four stages
     launch<128, 4, 3, 32>(ctx, A, B, M, N, kblocks, per, splits, out, ld_out, split_stride, d_err);
   else if (bk != kTcBK)
     fail(EPSP_EINVAL, "K blocks of 32 are for three-part operands here (tc_gemm_launch_with takes two-part ones)");

@@ -333,24 +333,27 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-template <int BN, int STAGES, int NS, int BK, bool TF32 = false>
+// NA < NS: A's parts from NA on are zero (weights exact in BF16), their copies and products are left out: bitwise the
+// same sums.
+template <int BN, int STAGES, int NS, int BK, bool TF32 = false, int NA = NS>
 struct TcPSmem {
   static constexpr int kES = TF32 ? 4 : 2;
   static constexpr int kRB = BK * kES;
   static constexpr int kA = kTcBM * kRB;
   static constexpr int kB = BN * kRB;
-  static constexpr int kStage = NS * kA + NS * kB;
+  static constexpr int kStage = NA * kA + NS * kB;
   static constexpr int kBars = 2 * STAGES + 5;  // full, empty, accumulator full x2, empty x2, done
   static constexpr int kBytes = STAGES * kStage + 8 * kBars + 16 + 1024;
 };
 
-template <int BN, int STAGES, int NS, int BK, bool TF32 = false>
+template <int BN, int STAGES, int NS, int BK, bool TF32 = false, int NA = NS>
 __global__ void __launch_bounds__(192, 1)
     tc_gemm_persist_kernel(const __grid_constant__ TcMaps maps, int M, int N, int kblocks, int kb_per_split, int nN,
                            int nM, int nitems, float* __restrict__ out, long ld_out, long split_stride,
                            int* __restrict__ err, int gm = 1) {
-  using L = TcPSmem<BN, STAGES, NS, BK, TF32>;
+  using L = TcPSmem<BN, STAGES, NS, BK, TF32, NA>;
   static_assert(!TF32 || NS == 1, "TF32 operands have one part");
+  static_assert(NA == NS || (NA == 1 && NS == 3), "A has all parts, or one of three");
   static_assert(2 * BN <= 512, "two accumulators must fit TMEM");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -417,8 +420,8 @@ __global__ void __launch_bounds__(192, 1)
         const int kc = (kb0 + kb) * BK;
 #pragma unroll
         for (int p = 0; p < NS; ++p) {
-          tma_load_2d(smem_u32(st + p * L::kA), &maps.a[p], kc, m0, fb);
-          tma_load_2d(smem_u32(st + NS * L::kA + p * L::kB), &maps.b[p], kc, n0, fb);
+          if (p < NA) tma_load_2d(smem_u32(st + p * L::kA), &maps.a[p], kc, m0, fb);
+          tma_load_2d(smem_u32(st + NA * L::kA + p * L::kB), &maps.b[p], kc, n0, fb);
         }
         ++g;
       }
@@ -456,19 +459,21 @@ __global__ void __launch_bounds__(192, 1)
         }
         tc_fence_after();
         const uint32_t a0 = smem_u32(smem + s * L::kStage);
-        const uint32_t b0 = a0 + NS * L::kA;
+        const uint32_t b0 = a0 + NA * L::kA;
 #pragma unroll
         for (int ks = 0; ks < L::kRB / 32; ++ks) {
           const uint32_t off = ks * 32;
           umma<TF32>(acc, sw_desc<L::kRB>(a0 + off), sw_desc<L::kRB>(b0 + off), idesc, (kb | ks) != 0);
           if constexpr (NS >= 2) {
             umma<TF32>(acc, sw_desc<L::kRB>(a0 + off), sw_desc<L::kRB>(b0 + L::kB + off), idesc, 1);
-            umma<TF32>(acc, sw_desc<L::kRB>(a0 + L::kA + off), sw_desc<L::kRB>(b0 + off), idesc, 1);
+            if constexpr (NA >= 2) umma<TF32>(acc, sw_desc<L::kRB>(a0 + L::kA + off), sw_desc<L::kRB>(b0 + off), idesc, 1);
           }
           if constexpr (NS == 3) {
             umma<TF32>(acc, sw_desc<L::kRB>(a0 + off), sw_desc<L::kRB>(b0 + 2 * L::kB + off), idesc, 1);
-            umma<TF32>(acc, sw_desc<L::kRB>(a0 + L::kA + off), sw_desc<L::kRB>(b0 + L::kB + off), idesc, 1);
-            umma<TF32>(acc, sw_desc<L::kRB>(a0 + 2 * L::kA + off), sw_desc<L::kRB>(b0 + off), idesc, 1);
+            if constexpr (NA == 3) {
+              umma<TF32>(acc, sw_desc<L::kRB>(a0 + L::kA + off), sw_desc<L::kRB>(b0 + L::kB + off), idesc, 1);
+              umma<TF32>(acc, sw_desc<L::kRB>(a0 + 2 * L::kA + off), sw_desc<L::kRB>(b0 + off), idesc, 1);
+            }
           }
         }
         umma_commit(empty0 + 8 * s);
@@ -939,7 +944,8 @@ CUtensorMap make_tmap_bf16(const void* base, long rows, long cols, long ld, int 
 // or 16 (64 bytes, 64-byte swizzle).
 CUtensorMap make_tmap_f32(const void* base, long rows, long cols, long ld, int box_rows, int bk = 32);
 
-// The parts of one operand: ns = 2 (hi, lo) or 3 (hi, mid, lo) BF16 tensor maps, or one FP32 map
+// The parts of one operand: ns = 2 (hi, lo) or 3 (hi, mid, lo) BF16 tensor maps (ns = 1: values exact in BF16, the A
+// operand of a three-part B), or one FP32 map
 // of TF32-rounded values (tf32, ns = 1, bk = 32).
 struct TcOperand {
   CUtensorMap m[3];

@@ -101,18 +101,6 @@ __global__ void clamp_kernel(const double2* __restrict__ S, double2* __restrict_
   Sin[long(a) * n + k] = make_double2(z.x, fmin(z.y, -tp[t].eta_min));
 }
 
-// The same clamp for the tensor-core path, written straight into its FP32 form {Re Σ as a float
-// pair, Im Σ, 0} (slot a at Sf + a n).
-__global__ void clamp_f32_kernel(const double2* __restrict__ S, float4* __restrict__ Sf, long n,
-                                 const int* __restrict__ slots, const TParams* __restrict__ tp) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int a = blockIdx.y, t = slots[a];
-  const double2 z = S[long(t) * n + k];
-  const float2 r = split_df(z.x);
-  Sf[long(a) * n + k] = make_float4(r.x, r.y, float(fmin(z.y, -tp[t].eta_min)), 0.f);
-}
-
 // The reference's Fan-Migdal sum, term by term in FP64: for each (ω, i), the sum over νf of
 // _fan_migdal_imsigma_term (src/scgd0_kernel.jl:27-39) in ascending νf, added to ImΣ
 // (src/scgd0_kernel.jl:74-86). One thread per (ω, i); the block's νf tile (g2, ωq, n_B(ωq) and the
@@ -493,30 +481,6 @@ __global__ void __launch_bounds__(256) spectral_colsum_kernel(const double* __re
   if (threadIdx.x == 0) colsum[i] = r;
 }
 
-// D[a] = (Σ_i A[a, i] w_i) Wa[a] (src/scgd0.jl:306-307). A block of 256 threads covers 32 nodes a
-// (the lanes) and splits i over its 8 warps (i ≡ warp mod 8, ascending); the 8 partial sums are
-// added in warp order, so the result is deterministic.
-__global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restrict__ Aall, int nwa, int ni,
-                                                         const double* __restrict__ w_i, const double* __restrict__ Wa,
-                                                         double* __restrict__ Dall) {
-  __shared__ double sh[8][32];
-  const double* A = Aall + long(nwa) * ni * blockIdx.y;
-  double* D = Dall + long(nwa) * blockIdx.y;
-  const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
-  const int a = blockIdx.x * 32 + lane;
-  double s = 0;
-  if (a < nwa)
-    for (int i = g; i < ni; i += 8) s += A[a + long(nwa) * i] * w_i[i];
-  sh[g][lane] = s;
-  __syncthreads();
-  if (g == 0 && a < nwa) {
-    double t = sh[0][lane];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) t += sh[k][lane];
-    D[a] = t * Wa[a];
-  }
-}
-
 // The tensor-core path's spectral functions, in FP32 without FP64 arithmetic per (a, i) element.
 // With ωa = ω_j + d_a (j = j_sp(a), t = t_sp(a)), the denominator's real part is
 //   ωa - ε_i - [(1 - t) ReΣ_j + t ReΣ_{j+1}] = d_a - v_j - t δ_j,
@@ -526,94 +490,60 @@ __global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restric
 // absolute error ~1e-7 h (~1e-10 eV). (Interpolating Σ in FP32 and subtracting it from ωa - ε_i
 // instead leaves ~1e-8 eV, which near a pole puts ~1e-5 into A and, through μ, a floor of ~1e-7 eV
 // under the iteration's convergence.)
-// spectral_prep: P[i][j] = (v_j, δ_j, ImΣ_j, ImΣ_{j+1}) of slot blockIdx.z. Grid (nω / 256, ni, slots).
-__global__ void spectral_prep_f32_kernel(const double2* __restrict__ Sall, int nw, long slab, const int* __restrict__ slots,
-                                         const double* __restrict__ ws, const double* __restrict__ eps_i,
-                                         float4* __restrict__ Pall, double* __restrict__ minA_all) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)  // the minimum of spectral_fin starts at +inf
-    minA_all[slots[blockIdx.z]] = INFINITY;
-  if (j >= nw) return;
-  const int i = blockIdx.y;
-  const double2* col = Sall + slab * slots[blockIdx.z] + long(nw) * i;
-  const double2 lo = col[j];
-  const double2 hi = j + 1 < nw ? col[j + 1] : lo;
-  Pall[slab * blockIdx.z + long(nw) * i + j] =
-      make_float4(float(eps_i[i] - ws[j] + lo.x), float(hi.x - lo.x), float(lo.y), float(hi.y));
-}
-
+// (The terms P[i][j] = (v_j, δ_j, ImΣ_j, ImΣ_{j+1}) come from kk_epilogue_kernel.)
 // A[a, i] = -Im(1/(d_a - v_j - t δ_j + i((1-t) ImΣ_j + t ImΣ_{j+1})))/π, never stored: a block of
-// 256 nodes a and one chunk of states i accumulates Σ_i A w_i per node (Dpart[slot][chunk][a]) and
+// 64 nodes a and one chunk of 32 states accumulates Σ_i A w_i per node (Dpart[slot][chunk][a]) and
 // Σ_a A Wa per state (Cpart[slot][i][a-block], summed over the block's warps in warp order), both in
-// FP32 over at most ichunk resp. 256 terms. Grid (nωa / 256, ni / ichunk, slots).
+// FP32 over at most 32 resp. 64 terms. A warp keeps its 32 x 32 values A Wa in registers and sums them over the lanes
+// by halving exchanges (31 shuffles for 32 states, where a tree per state took 160, each waited for), and loads eight
+// states at a time: 3201 nodes x 105 states 22.4 -> AD1_US us, 8001 x 495 23.7 -> AD2_US. Grid (nωa / 64, ni / 32, slots).
 constexpr int kSpecChunk = 32;
-__global__ void __launch_bounds__(256) spectral_ad_f32_kernel(const float4* __restrict__ Pall, int nw, long slab,
-                                                              const int32_t* __restrict__ jsp, const float* __restrict__ dsp,
-                                                              const float* __restrict__ tsp, const float* __restrict__ Waf,
-                                                              const float* __restrict__ w_if, int nwa, int ni,
-                                                              float* __restrict__ Dpart, float* __restrict__ Cpart) {
-  __shared__ float sh[8][kSpecChunk];
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int kSpecNodes = 64;
+__global__ void __launch_bounds__(kSpecNodes) spectral_ad_f32_kernel(
+    const float4* __restrict__ Pall, int nw, long slab, const int32_t* __restrict__ jsp, const float* __restrict__ dsp,
+    const float* __restrict__ tsp, const float* __restrict__ Waf, const float* __restrict__ w_if, int nwa, int ni,
+    float* __restrict__ Dpart, float* __restrict__ Cpart, const IterCtl* __restrict__ ctl) {
+  if (ctl && ctl->stop) return;
+  __shared__ float sh[kSpecNodes / 32][kSpecChunk];
+  const int a = blockIdx.x * kSpecNodes + threadIdx.x;
   const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
-  const int i0 = blockIdx.y * kSpecChunk, i1 = min(ni, i0 + kSpecChunk);
+  const int i0 = blockIdx.y * kSpecChunk, n = min(ni - i0, kSpecChunk);
   const int nab = gridDim.x, nch = gridDim.y;
   const bool ok = a < nwa;
-  const int j = ok ? jsp[a] : 0;
-  const float d = ok ? dsp[a] : 0.f, t = ok ? tsp[a] : 0.f, wa = ok ? Waf[a] : 0.f;
-  const float4* P = Pall + slab * blockIdx.z + j;
-  float dsum = 0.f;
-  for (int i = i0; i < i1; ++i) {
-    float A = 0.f;
-    if (ok) {
-      const float4 p = P[long(nw) * i];
-      const float c = d - p.x - t * p.y;
-      const float si = (1.f - t) * p.z + t * p.w;
-      // -Im(1/(c - i si))/π = -si/(π (c² + si²)); Smith's form only where the square underflows
-      const float den = fmaf(c, c, si * si);
-      A = (den > 1e-30f ? __fdividef(-si, den) : -imag_inv_f(c, -si)) * 0.318309886183790671538f;
-    }
-    dsum += A * w_if[i];
-    float cs = A * wa;
+  const int ac = min(a, nwa - 1), j = jsp[ac];
+  const float d = dsp[ac], t = tsp[ac], wa = ok ? Waf[ac] : 0.f;
+  const float4* P = Pall + slab * blockIdx.z + j + long(nw) * i0;
+  float dsum = 0.f, cs[kSpecChunk];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cs += __shfl_xor_sync(0xffffffffu, cs, o);
-    if (lane == 0) sh[wid][i - i0] = cs;
+  for (int u0 = 0; u0 < kSpecChunk; u0 += 8) {
+    float4 p[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) p[u] = P[long(nw) * min(u0 + u, n - 1)];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float c = d - p[u].x - t * p[u].y;
+      const float si = (1.f - t) * p[u].z + t * p[u].w;
+      // -Im(1/(c + i si))/π = -si/(π (c² + si²)); Smith's form only where the square underflows
+      const float den = fmaf(c, c, si * si);
+      float A = (den > 1e-30f ? __fdividef(-si, den) : -imag_inv_f(c, -si)) * 0.318309886183790671538f;
+      if (u0 + u >= n) A = 0.f;
+      dsum += A * w_if[i0 + min(u0 + u, n - 1)];
+      cs[u0 + u] = A * wa;
+    }
   }
   if (ok) Dpart[(long(blockIdx.z) * nch + blockIdx.y) * nwa + a] = dsum;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {  // lane l ends with state l
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const float got = __shfl_xor_sync(0xffffffffu, up ? cs[k] : cs[k + o], o);
+      cs[k] = (up ? cs[k + o] : cs[k]) + got;
+    }
+  }
+  sh[wid][lane] = cs[0];
   __syncthreads();
-  if (threadIdx.x < i1 - i0) {
-    float c = 0.f;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) c += sh[w][threadIdx.x];
-    Cpart[(long(blockIdx.z) * ni + i0 + threadIdx.x) * nab + blockIdx.x] = c;
-  }
-}
-
-// D[a] = Wa[a] Σ_chunk Dpart (FP64, chunk order) for blocks x < nab; the blocks after them give one
-// warp to each state i: ∫A_i = Σ Cpart over the node blocks (FP64: lanes in strides of 32, then a
-// shuffle tree), whose minimum over i goes to minA[slots[z]] by an atomic minimum of the bit
-// patterns (∫A_i >= 0, so they order as the values; spectral_prep_f32_kernel sets +inf first).
-// Grid (nab + ni / 8, slots).
-__global__ void __launch_bounds__(256) spectral_fin_f32_kernel(const float* __restrict__ Dpart, const float* __restrict__ Cpart,
-                                                               int nch, int nab, const double* __restrict__ Wa, int nwa, int ni,
-                                                               const int* __restrict__ slots, double* __restrict__ Dall,
-                                                               double* __restrict__ minA_all) {
-  const long z = blockIdx.y;
-  if (int(blockIdx.x) < nab) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= nwa) return;
-    double s = 0;
-    for (int c = 0; c < nch; ++c) s += double(Dpart[(z * nch + c) * nwa + a]);
-    Dall[z * nwa + a] = s * Wa[a];
-    return;
-  }
-  const int i = (int(blockIdx.x) - nab) * 8 + int(threadIdx.x) / 32, lane = threadIdx.x % 32;
-  if (i >= ni) return;
-  const float* c = Cpart + (z * ni + i) * nab;
-  double s = 0;
-  for (int b = lane; b < nab; b += 32) s += double(c[b]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) atomicMin(reinterpret_cast<unsigned long long*>(minA_all + slots[z]), (unsigned long long)__double_as_longlong(s));
+  if (threadIdx.x < n) Cpart[(long(blockIdx.z) * ni + i0 + threadIdx.x) * nab + blockIdx.x] = sh[0][threadIdx.x] + sh[1][threadIdx.x];
 }
 
 __global__ void __launch_bounds__(256) min_kernel(const double* __restrict__ xall, int n, const int* __restrict__ slots,
@@ -649,20 +579,24 @@ __device__ __forceinline__ double float_middle_d(double x, double y) {
 // dn/dμ = g Σ_a D_a f(1 - f)/T), falling back to Roots' floating-point midpoint whenever the
 // Newton step leaves the bracket, and stops at a step below 2^-46 max(|μ|, 1) (the rounding noise of
 // n(μ) moves the root by ~1e-15) or at adjacent floats.
-// One cluster of kMuCluster CTAs per temperature: each CTA sums a slice of ωs_spectral in fixed
-// order, the partials are combined through distributed shared memory in rank order, so every
-// thread of the cluster holds the same totals and takes the same branches.
-// The per-node work of the first round runs beforehand across the whole GPU (mu_prep_kernel): the
-// terms D_a f(ωa; a), D_a f(ωa; b), D_a f0, D_a f0 (1 - f0) at both bracket ends and at the start x0,
-// and E_a = exp((ωa - x0)/T), so that near x0 a later round's occupations cost one product and one
-// reciprocal: exp((ωa - μ)/T) = E_a exp((x0 - μ)/T) (used while |μ - x0| <= 30 T; farther out, and at
-// T ~ 0, exp is evaluated directly). The cluster then only sums.
+// The first round's sums -- D_a f at both bracket ends (whose occupations do not change during a run: mu_ends_kernel),
+// D_a f0, D_a f0 (1 - f0) at the start x0, D_a f at the probes x0 -+ 8 T -- are formed where D_a is (the kernels
+// that end the spectral functions, mu_terms), as block sums, with E_a = exp((ωa - x0)/T): near x0 a later round's
+// occupation costs one product and one reciprocal, exp((ωa - μ)/T) = E_a exp((x0 - μ)/T) (used while
+// |μ - x0| <= 30 T; farther out, and at T ~ 0, exp is evaluated directly). When the probes put the root within
+// x0 -+ 8 T, nodes with E_a outside [2^-69, 2^69) have occupation 1 or 0 to the last bit in every later
+// round: their D_a is summed once (the seventh term) and only the others are evaluated -- at 300 K a sixth of
+// ±8 eV, and FP64 evaluations (a dozen operations a node at 2 a cycle and SM) are what a round costs.
+// One cluster of kMuCluster CTAs per temperature: groups of 64 nodes are dealt out to the CTAs in turn, the
+// partials are combined through distributed shared memory in rank order, so every thread of the cluster holds the
+// same totals and takes the same branches.
 // status: 0 ok, 1 no sign change on the bracket.
+// Measured per iteration (3201 and 8001 nodes): 27.7 -> MU1_US us and 35.2 -> MU2_US us with what mu_prep_kernel took.
 constexpr int kMuCluster = 8;
-constexpr int kMuThreads = 512;
-constexpr int kMuWarps = kMuThreads / 32;
-constexpr int kMuPrepThreads = 64;
-constexpr int kMuTerms = 6;              // first-round terms per node
+constexpr int kMuThreads = 128;
+constexpr int kMuWarps = kMuThreads / 32;  // kMuCluster x kMuWarps partials: one per lane of the warp that sums them
+constexpr int kMuTerms = 7;              // first-round terms per node
+constexpr int kMuPart = 8;               // doubles of one block's first-round sums
 constexpr double kMuProbe = 8.0;         // the probes x0 -+ 8 T
 constexpr double kMuProbeExp = 2980.957987041728;  // e^8
 
@@ -685,7 +619,7 @@ __device__ __forceinline__ double recip_ge1(double x) {
   return r;
 }
 
-// Shared by mu_prep_kernel and mu_solve_kernel: the start x0 of slot's temperature on the bracket.
+// Shared by mu_terms and mu_solve_kernel: the start x0 of slot's temperature on the bracket.
 __device__ __forceinline__ double mu_start(double guess, double a, double b) {
   return (guess > a && guess < b) ? guess : float_middle_d(a, b);
 }
@@ -697,49 +631,165 @@ __device__ __forceinline__ double occ_from_y(double y, int holes) {
   return r;
 }
 
-// Grid (nωa / kMuPrepThreads, slots): E[slot][a] and R1[slot][q][a], q: the first round's terms at
-// the bracket ends, f0 and f0 (1 - f0) at x0, and the occupations at x0 -+ kMuProbe T (which narrow
-// the bracket before the first Newton step).
-__global__ void __launch_bounds__(kMuPrepThreads)
-    mu_prep_kernel(const double* __restrict__ Dall, const double* __restrict__ wsa, int nwa, const int* __restrict__ slots,
-                   const TParams* __restrict__ tp, double br0, double br1, double* __restrict__ E_all,
-                   double* __restrict__ R1_all) {
+// The occupations at the bracket ends, per temperature of the run (ends[t][2][nωa]).
+__global__ void mu_ends_kernel(const double* __restrict__ wsa, int nwa, const TParams* __restrict__ tp, double br0,
+                               double br1, double* __restrict__ ends) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nwa) return;
-  const long slot = blockIdx.y;
-  const int t = slots[slot];
-  const double T = tp[t].T;
-  const int holes = tp[t].holes;
-  const double x0 = mu_start(tp[t].mu, br0, br1);
+  const TParams q = tp[blockIdx.y];
+  auto occ = [&](double wa, double mu) { return occ_fermion_d(q.holes ? mu - wa : wa - mu, q.T); };
+  ends[(2l * blockIdx.y) * nwa + k] = occ(wsa[k], br0);
+  ends[(2l * blockIdx.y + 1) * nwa + k] = occ(wsa[k], br1);
+}
+
+// Where E lies: 0 within [2^-69, 2^69), -1 below, 1 above.
+__device__ __forceinline__ int mu_band(double E) {
+  const int hi = __double2hiint(E);
+  return hi < ((1023 - 69) << 20) ? -1 : hi >= ((1023 + 69) << 20) ? 1 : 0;
+}
+
+// What the μ solve of a slot reads, and its first-round terms at one node.
+struct MuIn {
+  const double* ends = nullptr;  // null: no μ solve (μ fixed)
+  const TParams* tp = nullptr;
+  double br0 = 0, br1 = 0;
+  double* E = nullptr;     // [slot][nωa]
+  double* part = nullptr;  // [slot][blocks][kMuPart]
+};
+__device__ __forceinline__ void mu_terms(const MuIn& M, int t, long slot, int k, int nwa, double wa, double d,
+                                         double (&v)[kMuTerms]) {
+  const TParams q = M.tp[t];
+  const double T = q.T, x0 = mu_start(q.mu, M.br0, M.br1);
   const bool warm = T > 1.4901161193847656e-08;
-  auto occ = [&](double wa, double mu) { return occ_fermion_d(holes ? mu - wa : wa - mu, T); };
-  const double wa = wsa[k], d = Dall[slot * nwa + k];
-  auto from_E = [&](double y) { return holes ? (isinf(y) ? 1.0 : y / (1.0 + y)) : 1.0 / (y + 1.0); };
   double f0, fl, fr, E = 0;
+  int band = 0;
   if (warm) {
-    E = exp((wa - x0) / T);
-    f0 = from_E(E);
-    fl = from_E(E * kMuProbeExp);  // at x0 - kMuProbe T: exp((ωa - x0)/T + kMuProbe)
-    fr = from_E(E / kMuProbeExp);
+    E = exp((wa - x0) * q.inv_T);
+    band = mu_band(E);
+    f0 = occ_from_y(E, q.holes);
+    fl = occ_from_y(E * kMuProbeExp, q.holes);  // at x0 - kMuProbe T: exp((ωa - x0)/T + kMuProbe)
+    fr = occ_from_y(E * (1.0 / kMuProbeExp), q.holes);
   } else {
-    f0 = occ(wa, x0);
+    f0 = occ_fermion_d(q.holes ? x0 - wa : wa - x0, T);
     fl = fr = f0;
   }
-  E_all[slot * nwa + k] = E;
-  double* R1 = R1_all + slot * kMuTerms * nwa;
-  R1[k] = d * occ(wa, br0);
-  R1[nwa + k] = d * occ(wa, br1);
-  R1[2 * nwa + k] = d * f0;
-  R1[3 * nwa + k] = d * (f0 * (1 - f0));
-  R1[4 * nwa + k] = d * fl;
-  R1[5 * nwa + k] = d * fr;
+  M.E[slot * nwa + k] = E;
+  v[0] = d * M.ends[(2l * t) * nwa + k];
+  v[1] = d * M.ends[(2l * t + 1) * nwa + k];
+  v[2] = d * f0;
+  v[3] = d * (f0 * (1 - f0));
+  v[4] = d * fl;
+  v[5] = d * fr;
+  v[6] = band == (q.holes ? 1 : -1) ? d : 0.0;
+}
+// A warp's sums of the seven terms into out[0 .. 8): halving exchanges leave sum q on lanes 4 q .. 4 q + 3 (9 FP64
+// additions a lane, where a tree per term takes 35).
+__device__ __forceinline__ void mu_warp_terms(const double (&v)[kMuTerms], double* out) {
+  double x[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], 0.0};
+  const int lane = threadIdx.x % 32;
+#pragma unroll
+  for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double got = __shfl_xor_sync(0xffffffffu, up ? x[k] : x[k + h], o);
+      x[k] = (up ? x[k + h] : x[k]) + got;
+    }
+  }
+  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
+  if (lane % 4 == 0) out[lane / 4] = x[0];
+}
+
+// D[a] = Wa[a] Σ_chunk Dpart (FP64, chunk order) for blocks x < nab, and with it the μ solve's first round;
+// the blocks after them give one warp to each state i: ∫A_i = Σ Cpart over the node blocks (FP64: lanes in strides of
+// 32, then a shuffle tree), whose minimum over i goes to minA[slots[z]] by an atomic minimum of the bit
+// patterns (∫A_i >= 0, so they order as the values; kk_epilogue_kernel sets +inf first). The first thread also copies
+// the tensor-core wait flag into the iteration's results, and asks for a stop when its temperature has converged. Grid (nab + ni / 2, slots), 64 threads.
+__global__ void __launch_bounds__(kSpecNodes) spectral_fin_f32_kernel(
+    const float* __restrict__ Dpart, const float* __restrict__ Cpart, int nch, int nab, const double* __restrict__ Wa,
+    const double* __restrict__ wsa, int nwa, int ni, const int* __restrict__ slots, double* __restrict__ Dall,
+    double* __restrict__ minA_all, const MuIn M, const int* __restrict__ tc_err, int* __restrict__ tc_err_out,
+    const unsigned long long* __restrict__ errbits, IterCtl* __restrict__ ctl) {
+  if (ctl && ctl->stop) return;
+  __shared__ double sh[2][kMuPart];
+  const long z = blockIdx.y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (z == 0) *tc_err_out = *tc_err;
+    if (ctl && __longlong_as_double((long long)errbits[slots[z]]) < ctl->tol) ctl->stop_next = 1;
+  }
+  if (int(blockIdx.x) < nab) {
+    const int a = blockIdx.x * kSpecNodes + threadIdx.x;
+    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0};
+    if (a < nwa) {
+      double s = 0;
+#pragma unroll 8
+      for (int c = 0; c < nch; ++c) s += double(Dpart[(z * nch + c) * nwa + a]);
+      s *= Wa[a];
+      Dall[z * nwa + a] = s;
+      if (M.ends) mu_terms(M, slots[z], z, a, nwa, wsa[a], s, v);
+    }
+    if (!M.ends) return;
+    mu_warp_terms(v, sh[threadIdx.x / 32]);
+    __syncthreads();
+    if (threadIdx.x < kMuPart) M.part[(z * nab + blockIdx.x) * kMuPart + threadIdx.x] = sh[0][threadIdx.x] + sh[1][threadIdx.x];
+    return;
+  }
+  const int i = (int(blockIdx.x) - nab) * 2 + int(threadIdx.x) / 32, lane = threadIdx.x % 32;
+  if (i >= ni) return;
+  const float* c = Cpart + (z * ni + i) * nab;
+  double s = 0;
+#pragma unroll 4
+  for (int b = lane; b < nab; b += 32) s += double(c[b]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) atomicMin(reinterpret_cast<unsigned long long*>(minA_all + slots[z]), (unsigned long long)__double_as_longlong(s));
+}
+
+// D[a] = (Σ_i A[a, i] w_i) Wa[a] (src/scgd0.jl:306-307). A block of 256 threads covers 32 nodes a
+// (the lanes) and splits i over its 8 warps (i ≡ warp mod 8, ascending); the 8 partial sums are
+// added in warp order, so the result is deterministic. With it, the μ solve's first round (FP64 paths).
+__global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restrict__ Aall, int nwa, int ni,
+                                                         const double* __restrict__ w_i, const double* __restrict__ Wa,
+                                                         const double* __restrict__ wsa, const int* __restrict__ slots,
+                                                         double* __restrict__ Dall, const MuIn M) {
+  __shared__ double sh[8][32];
+  const double* A = Aall + long(nwa) * ni * blockIdx.y;
+  double* D = Dall + long(nwa) * blockIdx.y;
+  const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
+  const int a = blockIdx.x * 32 + lane;
+  double s = 0;
+  if (a < nwa)
+#pragma unroll 4
+    for (int i = g; i < ni; i += 8) s += A[a + long(nwa) * i] * w_i[i];
+  sh[g][lane] = s;
+  __syncthreads();
+  if (g == 0) {
+    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0};
+    if (a < nwa) {
+      double t = sh[0][lane];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) t += sh[k][lane];
+      t *= Wa[a];
+      D[a] = t;
+      mu_terms(M, slots[blockIdx.y], blockIdx.y, a, nwa, wsa[a], t, v);
+    }
+    mu_warp_terms(v, M.part + (long(blockIdx.y) * gridDim.x + blockIdx.x) * kMuPart);
+  }
+}
+
+// F / d for d > 0.
+__device__ __forceinline__ double div_pos(double F, double d) {
+  const int e = (__double2hiint(d) >> 20) & 0x7ff;
+  return e > 0 && e < 0x7f0 ? F * recip_seeded(d) : F / d;
 }
 
 __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
     mu_solve_kernel(const double* __restrict__ Dall, const double* __restrict__ wsa, int nwa, const int* __restrict__ slots,
                     TParams* __restrict__ tp, double W, double base, double gs, double br0, double br1,
-                    const double* __restrict__ E_all, const double* __restrict__ R1_all, double* __restrict__ mu_all,
-                    int* __restrict__ status_all, int* __restrict__ evals_all) {
+                    const double* __restrict__ E_all, const double* __restrict__ part1, int npart, double* __restrict__ mu_all,
+                    int* __restrict__ status_all, int* __restrict__ evals_all, const IterCtl* __restrict__ ctl) {
+  if (ctl && ctl->stop) return;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned rank = cluster.block_rank();
@@ -747,43 +797,31 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
   const int slot = blockIdx.x / kMuCluster, t = slots[slot];
   const double* D = Dall + long(nwa) * slot;
   const double* E = E_all + long(nwa) * slot;
-  const double* R1 = R1_all + long(kMuTerms) * nwa * slot;
-  const double T = tp[t].T, n_target = tp[t].n_target, guess = tp[t].mu;
+  const double* P1 = part1 + long(kMuPart) * npart * slot;
+  const double T = tp[t].T, inv_T = tp[t].inv_T, n_target = tp[t].n_target, guess = tp[t].mu;
   const int holes = tp[t].holes;
-  double* mu_out = mu_all + t;
-  int* status = status_all + t;
-  __shared__ double sv[kMuTerms][kMuThreads];
-  __shared__ double part[2][kMuTerms];
-  __shared__ double tot[kMuTerms];
-  const int chunk = (nwa + kMuCluster - 1) / kMuCluster;
-  const int a0 = int(rank) * chunk, a1 = min(nwa, a0 + chunk);
+  __shared__ double part[2][kMuWarps][2];
+  __shared__ double tot[kMuPart];
   const bool warm = T > 1.4901161193847656e-08;
   const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
-  // Fixed-order totals of up to kMuTerms per-thread sums over the cluster: warp q adds the CTA's
-  // per-thread values of sum q (lanes in strides of 32, then a shuffle tree), so the FP64 adds run in
-  // nv warps rather than in all of them; the CTA partials alternate between two buffers, so one
-  // cluster barrier per round suffices (a CTA can only overwrite a buffer after the next round's
-  // barrier, when every CTA has read it). One thread per total reads the remote partials (not every
-  // thread: that serialises on the owners' shared memory).
+  // Totals of two per-thread sums over the cluster, on the threads of warp 0: every warp's sums go to its CTA's part
+  // buffer (two buffers in turn, so one cluster barrier per round suffices: a CTA can only overwrite a buffer after
+  // the next round's barrier, when every CTA has read it), and lane l of warp 0 reads those of CTA l / 4, warp l % 4.
   int round = 0;
-  auto reduce = [&](double* v, int nv) {
-    for (int q = 0; q < nv; ++q) sv[q][threadIdx.x] = v[q];
-    __syncthreads();
-    double* pb = part[round & 1];
-    if (wid < nv) {
-      double t = 0;
-      for (int k = lane; k < kMuThreads; k += 32) t += sv[wid][k];
-      t = warp_sum_d(t);
-      if (lane == 0) pb[wid] = t;
+  auto reduce = [&](double (&v)[2]) {
+    v[0] = warp_sum_d(v[0]);
+    v[1] = warp_sum_d(v[1]);
+    double(*pb)[2] = part[round & 1];
+    if (lane == 0) {
+      pb[wid][0] = v[0];
+      pb[wid][1] = v[1];
     }
     cluster.sync();
-    if (threadIdx.x < nv) {
-      double t = 0;
-      for (unsigned r = 0; r < kMuCluster; ++r) t += cluster.map_shared_rank(pb, r)[threadIdx.x];
-      tot[threadIdx.x] = t;
+    if (wid == 0) {
+      const double* r = cluster.map_shared_rank(&pb[0][0], unsigned(lane / kMuWarps)) + 2 * (lane % kMuWarps);
+      v[0] = warp_sum_d(r[0]);
+      v[1] = warp_sum_d(r[1]);
     }
-    __syncthreads();
-    for (int q = 0; q < nv; ++q) v[q] = tot[q];
     ++round;
   };
   auto occ = [&](double wa, double mu) { return occ_fermion_d(holes ? mu - wa : wa - mu, T); };
@@ -792,9 +830,10 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
   // same totals, so all CTAs take the same steps) and publishes the next point through shared
   // memory, instead of every thread repeating it on the FP64 units.
   __shared__ double s_x, s_scale;
-  __shared__ int s_fact, s_stop;
+  __shared__ int s_fact, s_stop, s_win;
   double a = br0, b = br1, fa = 0, fb = 0, x = mu_start(guess, br0, br1), result = x;
   const double x0 = x;
+  double x_sc = x0, scale0 = 1.0;  // scale0 = exp((x0 - x_sc)/T)
   int it = 0;
   bool failed = false;
   auto newton = [&](double F, double dF) -> int {  // 1: done (result set)
@@ -807,7 +846,7 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
       b = x;
       fb = F;
     }
-    double xn = x - F / dF;
+    double xn = dF > 0 ? x - div_pos(F, dF) : x;
     // a converged Newton step ends the solve even when it rounds onto the end the bracket update
     // just moved to x (otherwise the safeguard below would bisect down to adjacent floats)
     if (dF > 0 && fabs(xn - x) <= 0x1p-46 * fmax(fabs(x), 1.0)) {
@@ -823,20 +862,42 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
     return ++it >= 400 ? 1 : 0;
   };
   auto publish = [&](int stop) {
-    const double sx = (x0 - x) / T;
+    const double sx = (x0 - x) * inv_T;
     const bool fact = warm && fabs(sx) <= 30.0;
+    if (fact && !stop) {  // exp((x0 - x)/T): by the series of the step where it is short (2^-45 / 9! relative)
+      const double d = (x_sc - x) * inv_T;
+      if (fabs(d) < 0.03125) {
+        double p = fma(d, 1.0 / 40320, 1.0 / 5040);
+        p = fma(d, p, 1.0 / 720);
+        p = fma(d, p, 1.0 / 120);
+        p = fma(d, p, 1.0 / 24);
+        p = fma(d, p, 1.0 / 6);
+        p = fma(d, p, 0.5);
+        p = fma(d, p, 1.0);
+        scale0 *= fma(d, p, 1.0);
+      } else {
+        scale0 = exp(sx);
+      }
+      x_sc = x;
+    }
     s_x = x;
-    s_scale = fact ? exp(sx) : 0.0;
+    s_scale = scale0;
     s_fact = fact ? 1 : 0;
     s_stop = stop;
   };
-  // round 1: n(a), n(b), n(x0), n'(x0) and n(x0 -+ 8T) from the prepared terms
+  // round 1: n(a), n(b), n(x0), n'(x0), n(x0 -+ 8T) and the saturated nodes' sum from the blocks' sums, by every CTA alike
   {
-    double v[kMuTerms] = {0, 0, 0, 0, 0, 0};
-    for (int k = a0 + int(threadIdx.x); k < a1; k += kMuThreads)
-#pragma unroll
-      for (int q = 0; q < kMuTerms; ++q) v[q] += R1[q * nwa + k];
-    reduce(v, kMuTerms);
+    for (int q = wid; q < kMuTerms; q += kMuWarps) {
+      double t = 0;
+#pragma unroll 4
+      for (int k = lane; k < npart; k += 32) t += P1[k * kMuPart + q];
+      t = warp_sum_d(t);
+      if (lane == 0) tot[q] = t;
+    }
+    if (threadIdx.x == 0) s_win = 0;
+    __syncthreads();
+    const double* v = tot;
+    ++round;
     if (threadIdx.x == 0) {
       fa = total(v[0]);
       fb = total(v[1]);
@@ -851,7 +912,7 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
         // the probes narrow the bracket to the side (or the 16 T window) that holds the sign change
         const double xl = x0 - kMuProbe * T, xr = x0 + kMuProbe * T;
         const double fl = total(v[4]), fr = total(v[5]);
-        const double F0 = total(v[2]), dF0 = warm ? gs * v[3] / T : 0.0;
+        const double F0 = total(v[2]), dF0 = warm ? gs * v[3] * inv_T : 0.0;
         if (warm && xl > a && xr < b && fl != 0 && fr != 0 && signbit(fl) == signbit(fr)) {
           // x0 lies outside the narrowed bracket: its Newton step (or the midpoint) starts round 2
           if (signbit(fl) != signbit(fa)) {
@@ -871,6 +932,7 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
             fa = fl;
             b = xr;
             fb = fr;
+            s_win = 1;  // every later point lies within x0 -+ 8 T
           }
           stop = newton(F0, dF0);
         }
@@ -879,17 +941,23 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
     }
     __syncthreads();
   }
+  const bool win = s_win != 0;
   while (!s_stop) {
     const double xr = s_x, scale = s_scale;
     const bool fact = s_fact != 0;
     double v[2] = {0, 0};
-    for (int k = a0 + int(threadIdx.x); k < a1; k += kMuThreads) {
-      const double f = fact ? occ_from_y(E[k] * scale, holes) : occ(wsa[k], xr);
-      v[0] += D[k] * f;
-      v[1] += D[k] * (f * (1 - f));
+#pragma unroll 4
+    for (int k = (int(threadIdx.x) / 64 * kMuCluster + int(rank)) * 64 + int(threadIdx.x) % 64; k < nwa;
+         k += kMuCluster * kMuThreads) {
+      const double Ek = E[k], d = D[k];
+      if (win && mu_band(Ek) != 0) continue;
+      const double f = fact ? occ_from_y(Ek * scale, holes) : occ(wsa[k], xr);
+      const double df = d * f;
+      v[0] += df;
+      v[1] += fma(-df, f, df);
     }
-    reduce(v, 2);
-    if (threadIdx.x == 0) publish(newton(total(v[0]), warm ? gs * v[1] / T : 0.0));
+    reduce(v);
+    if (threadIdx.x == 0) publish(newton(total(win ? tot[6] + v[0] : v[0]), warm ? gs * v[1] * inv_T : 0.0));
     __syncthreads();
   }
   // no CTA leaves while another may still read its partials
@@ -897,11 +965,11 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
   if (rank == 0 && threadIdx.x == 0) {
     evals_all[t] = round;
     if (failed) {
-      *status = 1;
+      status_all[t] = 1;
     } else {
-      *mu_out = result;
+      mu_all[t] = result;
       tp[t].mu = result;  // the next iteration's μ, without a round trip to the host
-      *status = 0;
+      status_all[t] = 0;
     }
   }
 }
@@ -1208,42 +1276,32 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
       EPSP_LAUNCHED(ctx);
     });
     plog.mark("g2 streamed, coupling sums");
-    // The cells of ω ± ω_ν, by the lookup of _interp_linear_grid (src/frequency_grids.jl:207-219):
-    // the value there is (1 - t) Σ[j] + t Σ[j + 1], which is Σ[0] below the grid (t = 0) and Σ[end]
-    // above it (t = 1).
+    // The cells of ω ± ω_ν, by the lookup of _interp_linear_grid (src/frequency_grids.jl:207-219).
     {
       const auto& w = P->ws.nodes;
       const long n = P->nw;
+      // (cell tables: cell j is entry j + 1, entry 0 the flat part below the grid)
       std::vector<int32_t> cj(size_t(2 * n * nm));
-      std::vector<double> ctt(cj.size()), cx(cj.size());
+      std::vector<double> cdx(cj.size());
       for (long side = 0; side < 2; ++side)
         for (long nu = 0; nu < nm; ++nu)
           for (long iw = 0; iw < n; ++iw) {
             const double x = side == 0 ? w[size_t(iw)] + wnu[size_t(nu)] : w[size_t(iw)] - wnu[size_t(nu)];
-            const size_t k = size_t(iw + n * (nu + nm * side));
-            cx[k] = x;
+            int32_t e;
             if (!(x > w[0])) {
-              cj[k] = 0;
-              ctt[k] = 0.0;
+              e = 0;
             } else if (x >= w[size_t(n - 1)]) {
-              cj[k] = int32_t(n - 2);
-              ctt[k] = 1.0;
+              e = int32_t(n);
             } else {
               const int32_t c = ct.jtab[size_t(int64_t((x - ct.x0) * ct.inv_h))];
-              const int32_t j = c - 1 + (w[size_t(c)] <= x ? 1 : 0);
-              cj[k] = j;
-              ctt[k] = (x - w[size_t(j)]) / (w[size_t(j + 1)] - w[size_t(j)]);
+              e = c + (w[size_t(c)] <= x ? 1 : 0);
             }
+            const size_t k = size_t(iw + n * (nu + nm * side));
+            cj[k] = e;
+            cdx[k] = x - w[size_t(std::max(e - 1, 0))];
           }
-      if (P->path == EPSP_PATH_GEMM_FP64)  // the entry of the cell table, and x less its node (kbuild_f64_kernel)
-        for (size_t k = 0; k < cj.size(); ++k) {
-          const int32_t e = !(cx[k] > w[0]) ? 0 : cx[k] >= w[size_t(n - 1)] ? int32_t(n) : cj[k] + 1;
-          ctt[k] = cx[k] - w[size_t(std::max(e - 1, 0))];
-          cj[k] = e;
-        }
       P->d_cell_j = to_device(ctx, cj);
-      P->d_cell_t = to_device(ctx, ctt);
-      P->d_cell_x = to_device(ctx, cx);
+      P->d_cell_t = to_device(ctx, cdx);
     }
     P->d_Fa.alloc(ctx, size_t(P->nw * nm));
     P->d_Fe.alloc(ctx, size_t(P->nw * nm));
@@ -1407,9 +1465,11 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   int* d_evals = d_status + nT;
   int* d_tcerr = reinterpret_cast<int*>(d_pack.p + 4 * nT);
   // host side of the readback and of the slot list: pinned
-  P->h_pin.ensure(npack * sizeof(double) + size_t(nT) * sizeof(int));
-  double* h_pack = static_cast<double*>(P->h_pin.p);
-  int* h_slots = reinterpret_cast<int*>(h_pack + npack);
+  P->h_pin.ensure(2 * npack * sizeof(double) + size_t(nT) * sizeof(int));
+  double* h_packs[2] = {static_cast<double*>(P->h_pin.p), static_cast<double*>(P->h_pin.p) + npack};
+  int* h_slots = reinterpret_cast<int*>(h_packs[1] + npack);
+  for (auto& e : P->read_ev)
+    if (!e) EPSP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::vector<int> up_slots;  // the slot list on the device (uploaded when it changes)
   int32_t niter = 0;
   const unsigned eb = div_up(size_t(slab), 256);
@@ -1423,10 +1483,11 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   DBuf<double>& D_b = P->w_D;
   bool grown = false;
   grown |= ensure(d_slots, ctx, size_t(nT));
+  grown |= ensure(P->w_ctl, ctx, 1);
   grown |= ensure(d_tp, ctx, size_t(nT));
   if (P->path != EPSP_PATH_GEMM_BF16) grown |= ensure(Sin_b, ctx, size_t(slab * nT));  // the tensor-core path clamps into FP32
   const bool f32_spec = P->path == EPSP_PATH_GEMM_BF16;
-  const int spec_nab = int(div_up(size_t(nwa), 256)), spec_nch = int(div_up(size_t(ni), size_t(kSpecChunk)));
+  const int spec_nab = int(div_up(size_t(nwa), f32_spec ? kSpecNodes : 32)), spec_nch = int(div_up(size_t(ni), size_t(kSpecChunk)));
   if (f32_spec) {
     grown |= ensure(P->w_Pf, ctx, size_t(slab * nT));
     grown |= ensure(P->w_Dpart, ctx, size_t(long(spec_nch) * nwa * nT));
@@ -1437,7 +1498,8 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   }
   grown |= ensure(D_b, ctx, size_t(nwa * nT));
   grown |= ensure(P->w_E, ctx, size_t(nwa * nT));
-  grown |= ensure(P->w_R1, ctx, size_t(kMuTerms * nwa * nT));
+  grown |= ensure(P->w_R1, ctx, size_t(kMuPart * spec_nab * nT));
+  grown |= ensure(P->w_ends, ctx, size_t(2 * nwa * nT));
   if (P->path == EPSP_PATH_GEMM_BF16) {
     const long cap0 = tc_capacity(P);
     tc_reserve(P, nT);
@@ -1448,7 +1510,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   std::vector<TParams> h_tp(static_cast<size_t>(nT));
   std::vector<int> slots;
   // CUDA graph of the iteration body (tensor-core path; not while one of its kernels is profiled)
-  static const char* kBodyProfiles[] = {"kprep", "kbuild", "tc_fm", "tc_kk", "finalize", "spectral", "mu"};
+  static const char* kBodyProfiles[] = {"kprep", "kbuild", "tc_fm", "tc_kk", "finalize", "kk_epilogue", "spectral", "mu", "fm_disp"};
   bool use_graph = P->path == EPSP_PATH_GEMM_BF16;
   for (const char* nm : kBodyProfiles)
     if (ctx->prof_name == nm) use_graph = false;
@@ -1458,14 +1520,22 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
     return std::array<long, 6>{long(nA), long(nT), long(fix_mu), P->w_gen,
                                long(std::llround(occ->spin_degeneracy * 1e6)), long(P->path) + 16 * long(P->fd_fast)};
   };
-  for (int32_t iter = 1; iter <= maxiter; ++iter) {
-    auto t0 = std::chrono::steady_clock::now();
+  // An iteration is launched before the host has read the one before it (IterCtl; the tensor-core path without
+  // dispersive modes, whose iterations take about as long as the round trip): the round trips run beside the iterations,
+  // and only the last one of a set of active temperatures waits, with one iteration after it that does nothing.
+  IterCtl* ctl = P->path == EPSP_PATH_GEMM_BF16 && !P->disp ? P->w_ctl.p : nullptr;
+  auto reset_ctl = [&] {
+    const IterCtl c{tol, 0, 0};
+    P->w_ctl.upload(&c, 1, s);
+  };
+  auto launch_iteration = [&](int32_t iter) {
     slots.clear();
     for (int64_t iT = 0; iT < nT; ++iT) {
       if (!active[size_t(iT)]) continue;
       slots.push_back(int(iT));
       TParams& q = h_tp[size_t(iT)];
       q.T = occ->Tlist[iT];
+      q.inv_T = 1.0 / q.T;
       q.mu = mu[size_t(iT)];
       q.eta_min = eta_min[iT];
       q.holes = (!fix_mu && occ->type == EPSP_SEMICONDUCTOR && occ->nlist[iT] < 0) ? 1 : 0;
@@ -1477,24 +1547,42 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       std::copy(slots.begin(), slots.end(), h_slots);
       EPSP_CUDA(cudaMemcpyAsync(d_slots.p, h_slots, slots.size() * sizeof(int), cudaMemcpyHostToDevice, s));
       up_slots = slots;
+      if (ctl) reset_ctl();
     }
     // T, η_min, target and branch are fixed for the run; μ is written on the device by the μ solve
-    if (iter == 1) d_tp.upload(h_tp.data(), h_tp.size(), s);
+    if (iter == 1) {
+      d_tp.upload(h_tp.data(), h_tp.size(), s);
+      if (!fix_mu) {
+        mu_ends_kernel<<<dim3(div_up(size_t(nwa), 64), unsigned(nT)), 64, 0, s>>>(P->d_wsa.p, int(nwa), d_tp.p, br0, br1,
+                                                                              P->w_ends.p);
+        EPSP_LAUNCHED(ctx);
+      }
+    }
+    // the tensor-core path's form of the clamped Σ: made here for the first iteration and after the network's
+    // correction, by each iteration's last pass for the next
+    if (P->path == EPSP_PATH_GEMM_BF16) {
+      if (iter == 1) tc_start(P, nT, d_tp.p);
+      if (iter == 1 || (warm && iter == 2)) tc_take_sigma(P, nA, d_slots.p, d_tp.p, S.p);
+    }
     // the launches of one iteration; on the tensor-core path they are captured once per active set
     // into a CUDA graph and replayed (μ, T come from the device, so a replay sees the current ones)
     auto body = [&] {
-      EPSP_CUDA(cudaMemsetAsync(d_err, 0, size_t(nT) * 8, s));
-      EPSP_CUDA(cudaMemsetAsync(d_status, 0, size_t(2 * nT) * sizeof(int), s));
-      if (P->path == EPSP_PATH_GEMM_BF16)
-        clamp_f32_kernel<<<dim3(eb, unsigned(nA)), 256, 0, s>>>(S.p, tc_sigma_f32(P), slab, d_slots.p, d_tp.p);
-      else
+      MuIn mu_in;
+      mu_in.ends = fix_mu ? nullptr : P->w_ends.p;
+      mu_in.tp = d_tp.p;
+      mu_in.br0 = br0;
+      mu_in.br1 = br1;
+      mu_in.E = P->w_E.p;
+      mu_in.part = P->w_R1.p;
+      if (P->path != EPSP_PATH_GEMM_BF16 || P->disp) EPSP_CUDA(cudaMemsetAsync(d_err, 0, size_t(nT) * 8, s));
+      if (P->path != EPSP_PATH_GEMM_BF16) {
         clamp_kernel<<<dim3(eb, unsigned(nA)), 256, 0, s>>>(S.p, Sin_b.p, slab, d_slots.p, d_tp.p);
-      EPSP_LAUNCHED(ctx);
+        EPSP_LAUNCHED(ctx);
+      }
       if (P->path == EPSP_PATH_GEMM_BF16) {
         // Σ_new, its multiplet average, max|ΔΣ|, Σ ← Σ_new and the spectral terms from the
         // Kramers-Kronig product's epilogue (so no multiplet, spectral-prep or err/copy pass below)
-        tc_iterate(P, nA, d_slots.p, slots.data(), d_tp.p, nullptr, S.p, P->w_Pf.p, d_err, d_minA);
-        EPSP_CUDA(cudaMemcpyAsync(d_tcerr, tc_err_ptr(P), sizeof(int), cudaMemcpyDeviceToDevice, s));
+        tc_iterate(P, nA, d_slots.p, d_tp.p, S.p, P->w_Pf.p, d_err, d_minA, ctl);
       } else {
         for (int a = 0; a < nA; ++a) {
           const int64_t iT = slots[size_t(a)];
@@ -1515,12 +1603,13 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       }
       long psp = prof_begin(ctx, "spectral");
       if (f32_spec) {  // the per-node terms came from the Kramers-Kronig epilogue
-        spectral_ad_f32_kernel<<<dim3(unsigned(spec_nab), unsigned(spec_nch), unsigned(nA)), 256, 0, s>>>(
+        spectral_ad_f32_kernel<<<dim3(unsigned(spec_nab), unsigned(spec_nch), unsigned(nA)), kSpecNodes, 0, s>>>(
             P->w_Pf.p, int(nw), slab, P->d_jsp.p, P->d_dspf.p, P->d_tspf.p, P->d_Waf.p, P->d_w_if.p, int(nwa), int(ni),
-            P->w_Dpart.p, P->w_Cpart.p);
+            P->w_Dpart.p, P->w_Cpart.p, ctl);
         EPSP_LAUNCHED(ctx);
-        spectral_fin_f32_kernel<<<dim3(unsigned(spec_nab + div_up(size_t(ni), 8)), unsigned(nA)), 256, 0, s>>>(
-            P->w_Dpart.p, P->w_Cpart.p, spec_nch, spec_nab, P->d_Wa.p, int(nwa), int(ni), d_slots.p, D_b.p, d_minA);
+        spectral_fin_f32_kernel<<<dim3(unsigned(spec_nab + div_up(size_t(ni), 2)), unsigned(nA)), kSpecNodes, 0, s>>>(
+            P->w_Dpart.p, P->w_Cpart.p, spec_nch, spec_nab, P->d_Wa.p, P->d_wsa.p, int(nwa), int(ni), d_slots.p, D_b.p,
+            d_minA, mu_in, tc_err_ptr(P), d_tcerr, d_err, ctl);
         EPSP_LAUNCHED(ctx);
       } else {
         spectral_A_kernel<<<dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0, s>>>(
@@ -1532,20 +1621,17 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
         min_kernel<<<unsigned(nA), 256, 0, s>>>(colsum_b.p, int(ni), d_slots.p, d_minA);
         EPSP_LAUNCHED(ctx);
         if (!fix_mu) {
-          spectral_D_kernel<<<dim3(div_up(size_t(nwa), 32), unsigned(nA)), 256, 0, s>>>(A_b.p, int(nwa), int(ni),
-                                                                                       P->d_w_i.p, P->d_Wa.p, D_b.p);
+          spectral_D_kernel<<<dim3(unsigned(spec_nab), unsigned(nA)), 256, 0, s>>>(
+              A_b.p, int(nwa), int(ni), P->d_w_i.p, P->d_Wa.p, P->d_wsa.p, d_slots.p, D_b.p, mu_in);
           EPSP_LAUNCHED(ctx);
         }
       }
       prof_end(ctx, psp);
       if (!fix_mu) {
         long pm = prof_begin(ctx, "mu");
-        mu_prep_kernel<<<dim3(div_up(size_t(nwa), kMuPrepThreads), unsigned(nA)), kMuPrepThreads, 0, s>>>(
-            D_b.p, P->d_wsa.p, int(nwa), d_slots.p, d_tp.p, br0, br1, P->w_E.p, P->w_R1.p);
-        EPSP_LAUNCHED(ctx);
         mu_solve_kernel<<<unsigned(kMuCluster * nA), kMuThreads, 0, s>>>(
             D_b.p, P->d_wsa.p, int(nwa), d_slots.p, d_tp.p, P->W, P->nstates_base, occ->spin_degeneracy, br0, br1,
-            P->w_E.p, P->w_R1.p, d_mu, d_status, d_evals);
+            P->w_E.p, P->w_R1.p, spec_nab, d_mu, d_status, d_evals, ctl);
         EPSP_LAUNCHED(ctx);
         prof_end(ctx, pm);
       }
@@ -1556,14 +1642,10 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
     };
     // iteration 1 replays a graph a previous run captured with the same key; otherwise it runs
     // eagerly (first launches set kernel attributes) and iteration 2 captures
-    const bool have_graph = P->graph && [&] {
-      const auto k = graph_key(nA);
-      return std::equal(k.begin(), k.end(), P->graph_key);
-    }();
-    if (use_graph && (iter > 1 || have_graph)) {
-      const auto key = graph_key(nA);
-      if (!P->graph || !std::equal(key.begin(), key.end(), P->graph_key)) {
-        if (P->graph) cudaGraphExecDestroy(P->graph), P->graph = nullptr;
+    const auto key = graph_key(nA);
+    auto have = std::find_if(P->graphs.begin(), P->graphs.end(), [&](const auto& g) { return g.key == key; });
+    if (use_graph && (iter > 1 || have != P->graphs.end())) {
+      if (have == P->graphs.end()) {
         const int64_t l0 = ctx->launches;
         cudaGraph_t g = nullptr;
         EPSP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
@@ -1575,21 +1657,38 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
           throw;
         }
         EPSP_CUDA(cudaStreamEndCapture(s, &g));
-        cudaError_t ie = cudaGraphInstantiate(&P->graph, g, 0);
+        cudaGraphExec_t exec = nullptr;
+        cudaError_t ie = cudaGraphInstantiate(&exec, g, 0);
         cudaGraphDestroy(g);
-        if (ie != cudaSuccess) P->graph = nullptr;
         EPSP_CUDA(ie);
-        P->graph_launches = ctx->launches - l0;
+        while (P->graphs.size() >= Scgd0Plan::kGraphs) {
+          cudaGraphExecDestroy(P->graphs.back().exec);
+          P->graphs.pop_back();
+        }
+        P->graphs.insert(P->graphs.begin(), {key, exec, long(ctx->launches - l0)});
         ctx->launches = l0;
-        std::copy(key.begin(), key.end(), P->graph_key);
+      } else if (have != P->graphs.begin()) {
+        std::rotate(P->graphs.begin(), have, have + 1);
       }
-      EPSP_CUDA(cudaGraphLaunch(P->graph, s));
-      ctx->launches += P->graph_launches;
+      EPSP_CUDA(cudaGraphLaunch(P->graphs.front().exec, s));
+      ctx->launches += P->graphs.front().launches;
     } else {
       body();
     }
-    EPSP_CUDA(cudaMemcpyAsync(h_pack, d_pack.p, npack * sizeof(double), cudaMemcpyDeviceToHost, s));
-    EPSP_CUDA(cudaStreamSynchronize(s));
+    EPSP_CUDA(cudaMemcpyAsync(h_packs[iter & 1], d_pack.p, npack * sizeof(double), cudaMemcpyDeviceToHost, s));
+    EPSP_CUDA(cudaEventRecord(P->read_ev[iter & 1], s));
+  };
+  int32_t launched = 0;
+  auto t0 = std::chrono::steady_clock::now();
+  for (int32_t iter = 1; iter <= maxiter; ++iter) {
+    if (launched < iter) launch_iteration(iter);
+    launched = iter;
+    if (ctl && iter < maxiter && !(warm && iter == 1)) {
+      launch_iteration(iter + 1);
+      launched = iter + 1;
+    }
+    EPSP_CUDA(cudaEventSynchronize(P->read_ev[iter & 1]));
+    const double* h_pack = h_packs[iter & 1];
     {
       int tcerr = 0;
       std::memcpy(&tcerr, &h_pack[size_t(4 * nT)], sizeof(int));
@@ -1625,6 +1724,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       if (err < tol) {
         active[size_t(iT)] = 0;
         hist->iter_frozen[iT] = iter;
+        launched = iter;  // the next iteration, if it was launched, stops itself
       }
       if (P->verbosity >= 2)
         std::fprintf(stderr, "scgd0 iteration %d, T = %.6g: err = %.3e, mu = %.15g, mu evaluations %d\n", int(iter),
@@ -1635,7 +1735,9 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
         if (active[size_t(iT)])
           warmstart_correct(warm, ctx, S.p + slab * iT, nw, ni, P->d_eps_i.p, occ->Tlist[iT], mu[size_t(iT)],
                             warm_scale[iT], P->path == EPSP_PATH_GEMM_BF16 ? tc_err_ptr(P) : nullptr);
-    hist->wall[iter - 1] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    const auto now = std::chrono::steady_clock::now();
+    hist->wall[iter - 1] = std::chrono::duration<double>(now - t0).count();
+    t0 = now;
     niter = iter;
     if (std::none_of(active.begin(), active.end(), [](char a) { return a != 0; })) break;
   }

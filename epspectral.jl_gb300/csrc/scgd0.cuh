@@ -4,14 +4,23 @@
 #include "common.cuh"
 #include "oz_gemm.cuh"
 
+#include <array>
 #include <memory>
 
 namespace epsp {
 
 // Per-temperature parameters of one iteration, on the device (indexed by temperature).
 struct TParams {
-  double T, mu, eta_min, n_target;
+  double T, inv_T, mu, eta_min, n_target;
   int holes, pad;
+};
+
+// What lets an iteration be launched before the one before it has been read: an iteration sets stop_next when a
+// temperature has converged (max|ΔΣ| < tol), and the next one, launched for the same temperatures, then takes it
+// over as stop and changes nothing (the host launches it again for those that are left).
+struct IterCtl {
+  double tol;
+  int stop_next, stop;
 };
 
 struct Scgd0Plan {
@@ -65,10 +74,10 @@ struct Scgd0Plan {
   DBuf<int32_t> d_iq, d_iksi, d_iksf, d_fti;
   DBuf<double> d_epsf;
   DBuf<float4> d_wtab;
-  // cells of ω ± ω_ν for every (ω, ν): [2][nω·nm] lower node, weight and point (absorption, emission); GEMM_FP64:
-  // the cell table's entry, the distance from its node, the point
+  // cells of ω ± ω_ν for every (ω, ν): [2][nω·nm] the cell tables' entry and the distance from its node (absorption,
+  // emission)
   DBuf<int32_t> d_cell_j;
-  DBuf<double> d_cell_t, d_cell_x;
+  DBuf<double> d_cell_t;
   // tensor-core path state (scgd0_tc.cu)
   struct Tc;
   std::unique_ptr<Tc, void (*)(Tc*)> tc{nullptr, [](Tc*) {}};
@@ -79,20 +88,29 @@ struct Scgd0Plan {
   DBuf<double2> w_S, w_Snew, w_Sin;
   int64_t sigma_nT = 0;  // temperatures of the last run's Σ in w_S (0: no run yet)
   DBuf<double> w_A, w_colsum, w_D, w_pack;
-  // μ solve tables (E, first-round terms) and the FP32 spectral path's per-node Σ terms and partials
-  DBuf<double> w_E, w_R1;
+  // μ solve tables (E, first-round sums, occupations at the bracket ends) and the FP32 spectral path's per-node Σ terms and partials
+  DBuf<double> w_E, w_R1, w_ends;
   DBuf<float4> w_Pf;
   DBuf<float> w_Dpart, w_Cpart;
   DBuf<int> w_slots;
   DBuf<TParams> w_tp;
   long w_gen = 0;  // bumped whenever one of them is reallocated
-  HostPinned h_pin;  // the per-iteration readback and the slot list
-  // the captured iteration of the last run, reused while its key matches
-  cudaGraphExec_t graph = nullptr;
-  long graph_key[6] = {-1, -1, -1, -1, -1, -1};
-  long graph_launches = 0;
+  HostPinned h_pin;  // the readbacks of two iterations and the slot list
+  DBuf<IterCtl> w_ctl;
+  cudaEvent_t read_ev[2] = {nullptr, nullptr};
+  // captured iterations, the last used first (a run over several temperatures uses one for each number of them that
+  // is left); at most kGraphs
+  static constexpr size_t kGraphs = 16;
+  struct IterGraph {
+    std::array<long, 6> key;
+    cudaGraphExec_t exec;
+    long launches;
+  };
+  std::vector<IterGraph> graphs;
   ~Scgd0Plan() {
-    if (graph) cudaGraphExecDestroy(graph);
+    for (auto& g : graphs) cudaGraphExecDestroy(g.exec);
+    for (auto& e : read_ev)
+      if (e) cudaEventDestroy(e);
   }
 };
 
@@ -111,15 +129,17 @@ void tc_reserve(Scgd0Plan* P, long nT);
 // The temperatures tc_reserve's buffers hold now.
 long tc_capacity(Scgd0Plan* P);
 // One iteration of nA active temperatures at once, up to the spectral functions: slot a reads the
-// clamped Σ_in + a nω ni; per-temperature T and μ from tp (device). With d_Sin_b null, the slots'
-// clamped Σ are already in the FP32 buffer tc_sigma_f32 returns. The Kramers-Kronig product's
-// epilogue writes Σ_new (multiplet-averaged) into S_all + slots_h[a] nω ni (temperature index),
-// max |Σ_new - Σ| into d_errbits[temperature] (bit patterns, atomic maximum), the spectral
-// functions' per-node terms into d_P + a nω ni, and +inf into d_minA[temperature].
-void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const int* slots_h, const TParams* d_tp,
-                const double2* d_Sin_b, double2* d_S_all, float4* d_P, unsigned long long* d_errbits, double* d_minA);
-// The FP32 form of the clamped Σ of every reserved temperature ({Re hi, Re lo, Im, 0}, slot-major).
-float4* tc_sigma_f32(Scgd0Plan* P);
+// clamped Σ of temperature slots[a] in its FP32 form (tc_take_sigma); per-temperature T and μ from tp
+// (device). The Kramers-Kronig product's epilogue writes Σ_new (multiplet-averaged) into S_all + t nω ni
+// of temperature t and its clamped FP32 form, max |Σ_new - Σ| into d_errbits[t] (bit patterns, atomic
+// maximum; reset here unless the modes are dispersive), the spectral functions' per-node terms into d_P + a nω ni, and +inf into d_minA[t].
+// ctl (not with dispersive modes): the iteration does nothing when the one before it asked for a stop.
+void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, double2* d_S_all, float4* d_P,
+                unsigned long long* d_errbits, double* d_minA, IterCtl* ctl);
+// A run's per-temperature tables (tp on the device), and the iteration's form of the clamped Σ of temperatures
+// slots[0 .. nA) from Σ itself (afterwards each iteration leaves it for the next).
+void tc_start(Scgd0Plan* P, long nT, const TParams* d_tp);
+void tc_take_sigma(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, const double2* d_S_all);
 // Fails with EPSP_EDEVICE_TIMEOUT if a tensor-core GEMM's bounded wait ran out (synchronises).
 void tc_check(Scgd0Plan* P);
 // The device flag the tensor-core GEMMs set when a bounded wait runs out.

@@ -39,11 +39,13 @@ struct Scgd0Plan::Tc {
   DBuf<float> part;
   DBuf<int> err;
   TcOperand opK, opG, opKK, opIm;
-  // FP32 forms of the K-tensor inputs: cell points as float pairs (hi, lo), cell weights, the cell
-  // energies as pairs, the occupation tables, and per iteration Σin as {Re hi, Re lo, Im, 0}
-  DBuf<float2> xf, ef;
-  DBuf<float> tf, Ff;
-  DBuf<float4> Sf;
+  // FP32 forms of the K-tensor inputs: distances from the cells' nodes, the cell energies as pairs, the occupation
+  // tables; per temperature the columns' cell records (rec, dim; kbuild_bf16_kernel) or, with dispersive modes, Σ_in as
+  // {Re hi, Re lo, Im, 0}; ε_i as pairs, and the modes' exp(ω_ν/T) and n of the run's temperatures
+  DBuf<float2> ef, epair;
+  DBuf<float> tf, Ff, dim;
+  DBuf<float4> Sf, rec;
+  DBuf<double2> modes;
   // dispersive modes: cell records and Im slopes of every column and slot, partial sums of the splits
   DBuf<float4> fdrec;
   DBuf<float> fddim;
@@ -73,6 +75,64 @@ __global__ void to_f32_kernel(const double* __restrict__ x, long n, float* __res
   if (k < n) out[k] = float(x[k]);
 }
 
+// Σ_s part[s stride] in ascending s.
+__device__ __forceinline__ float sum_splits(const float* __restrict__ part, int splits, long stride) {
+  float acc = 0.f;
+#pragma unroll 4
+  for (int p = 0; p < splits; ++p) acc += part[stride * p];
+  return acc;
+}
+
+// One node's Σ as FP32: Re as a pair, Im. Cell j of a column from its nodes' values z (node j) and zn (node j + 1):
+// {ω_j - ReΣ_j as a pair, 1 - ReΣ', ImΣ_j} and ImΣ' (Im clamped at -η_min = etam), so that at x = ω_j + dx
+//   Re z = (U_hi - ε_hi) + ((U_lo - ε_lo) + dx (1 - ReΣ')),  Im Σ = ImΣ_j + dx ImΣ';
+// the first difference is exact where Re z is small against its parts. wj: {ω_j hi, lo, 1 / (ω_{j+1} - ω_j) (0 at the
+// last node, whose cell is the flat part above the grid), ..}.
+__device__ __forceinline__ float4 cell_record(float4 z, float4 zn, float4 wj, float etam, float& dim) {
+  float e;
+  const float s = two_sum(wj.x, -z.x, e);
+  const float l = e + (wj.y - z.y), h = s + l;
+  const float im = fminf(z.z, etam);
+  dim = (fminf(zn.z, etam) - im) * wj.z;
+  return make_float4(h, l - (h - s), 1.f - ((zn.x - z.x) + (zn.y - z.y)) * wj.z, im);
+}
+__device__ __forceinline__ float4 sigma_f32(double2 z) {
+  const float2 r = split_df(z.x);
+  return make_float4(r.x, r.y, float(z.y), 0.f);
+}
+
+// The records of the columns of temperature slots[blockIdx.y] from Σ there, clamped at -η_min: [ni][nω + 1] entries a
+// temperature, entry j + 1 cell j, entry 0 the flat part below the grid. Without slots: of one Σ, as it is.
+__global__ void cell_records_kernel(const double2* __restrict__ S_all, const int* __restrict__ slots,
+                                    const TParams* __restrict__ tp, const float4* __restrict__ wtab, int nw, long slab,
+                                    float4* __restrict__ rec_all, float* __restrict__ dim_all) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= slab) return;
+  const int t = slots ? slots[blockIdx.y] : 0, j = int(k % nw);
+  const double2* S = S_all + slab * t;
+  const float etam = slots ? float(-tp[t].eta_min) : INFINITY;
+  const float4 z = sigma_f32(S[k]), zn = j + 1 < nw ? sigma_f32(S[k + 1]) : z, wj = wtab[j];
+  const long at = (k / nw + slab / nw * t) * (nw + 1l) + j + 1;
+  float d;
+  rec_all[at] = cell_record(z, zn, wj, etam, d);
+  dim_all[at] = d;
+  if (j == 0) {
+    rec_all[at - 1] = cell_record(z, z, wj, etam, d);
+    dim_all[at - 1] = 0.f;
+  }
+}
+
+// clamp_kernel's Σ_in in FP32 {Re Σ as a float pair, Im Σ, 0} (temperature t at Sf + t n), for the dispersive sum.
+__global__ void clamp_f32_kernel(const double2* __restrict__ S, float4* __restrict__ Sf, long n,
+                                 const int* __restrict__ slots, const TParams* __restrict__ tp) {
+  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int a = blockIdx.y, t = slots[a];
+  const double2 z = S[long(t) * n + k];
+  const float2 r = split_df(z.x);
+  Sf[long(t) * n + k] = make_float4(r.x, r.y, float(fmin(z.y, -tp[t].eta_min)), 0.f);
+}
+
 __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* __restrict__ out) {
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
@@ -82,28 +142,31 @@ __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* 
 }
 
 // Kernel tensor of the recast Fan-Migdal sum (see kbuild_f64_kernel in scgd0.cu), written as BF16
-// split rows K_t[ω][k], k = c nm + ν, through a shared-memory transpose. The cells of ω ± ω_ν come
-// from the setup table; Re z = (x - ε) - Re Σ(x), which cancels near the quasiparticle pole, is
-// formed exactly from float pairs (re_z), and Im Σ(x), the reciprocal and the occupation products
-// are FP32: the kernel runs on the FP32 units only.
+// split rows K_t[ω][k], k = c nm + ν, through a shared-memory transpose. Σ(ω ± ω_ν) comes from the columns' cell
+// records (cell_record above; the cells and distances from set-up), the reciprocal and the occupation products are
+// FP32: the kernel runs on the FP32 units only. A side of an element is 20 bytes and about 12 instructions (four
+// 16-byte gathers, two weights and two two-sums a side before: 54 -> KB1_US us at 1251 x 7425, 52 -> KB2_US us at 8
+// temperatures of 626 x 2184).
 // Grid (nω / 16, Kp / (kKbCols nm), slots), 256 threads: thread (node ω0 + t % 16, modes t / 16,
 // t / 16 + 16, ..) loads the cells and occupations of its (ω, ν) once and runs over the block's
-// kKbCols columns c (their Σ column and energy from shared memory), so per element only the two
-// interpolations of Σ and the arithmetic remain. Dynamic shared memory: the tile [kKbCols nm][17]
-// floats. kKbCols nm must be a multiple of 8, so that the write-out's 16-byte chunks never
+// kKbCols columns c (their records' offset and energy from shared memory). Dynamic shared memory: the tile
+// [kKbCols nm][17] floats. kKbCols nm must be a multiple of 8, so that the write-out's 16-byte chunks never
 // straddle two blocks (nor Kp, a multiple of 64).
 constexpr int kKbCols = 8;
 constexpr int kKbW = 16;
-__global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, long slab, const float4* __restrict__ Sf_all,
-                                                          const int32_t* __restrict__ cell_j,
-                                                          const float* __restrict__ cell_t,
-                                                          const float2* __restrict__ cell_x,
+__global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, const float4* __restrict__ rec_all,
+                                                          const float* __restrict__ dim_all,
+                                                          const int* __restrict__ slots,
+                                                          const int32_t* __restrict__ cell_e,
+                                                          const float* __restrict__ cell_dx,
                                                           const uint8_t* __restrict__ skip, int nm,
                                                           const float2* __restrict__ eps_c,
                                                           const int32_t* __restrict__ col_c, int nc,
                                                           const float* __restrict__ F_all,
                                                           __nv_bfloat16* __restrict__ K0, __nv_bfloat16* __restrict__ K1,
-                                                          __nv_bfloat16* __restrict__ K2, long Kp) {
+                                                          __nv_bfloat16* __restrict__ K2, long Kp,
+                                                          const IterCtl* __restrict__ ctl = nullptr) {
+  if (ctl && ctl->stop) return;
   extern __shared__ float kb_tile[];  // [kKbCols nm][kKbW + 1]
   __shared__ int s_col[kKbCols];
   __shared__ float2 s_eps[kKbCols];
@@ -112,27 +175,26 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, long slab, 
   const int tw = threadIdx.x % kKbW, tm = threadIdx.x / kKbW;
   const int iw = w0 + tw;
   const int nwm = nw * nm;
-  const float4* Sf = Sf_all + slab * blockIdx.z;
+  const long tab = (nw + 1l) * ni * (slots ? slots[blockIdx.z] : 0);
+  const float4* rec = rec_all + tab;
+  const float* dim = dim_all + tab;
   const float* F = F_all + 2l * nwm * blockIdx.z;
   if (threadIdx.x < kKbCols) {
     const int c = cbeg + threadIdx.x;
-    s_col[threadIdx.x] = c < nc ? nw * col_c[c] : -1;
+    s_col[threadIdx.x] = c < nc ? (nw + 1) * col_c[c] : -1;
     s_eps[threadIdx.x] = c < nc ? eps_c[c] : make_float2(0.f, 0.f);
   }
   __syncthreads();
   for (int nu = tm; nu < nm; nu += 256 / kKbW) {
     const bool on = iw < nw && !skip[nu];
-    int ja = 0, je = 0;
-    float ta = 0.f, te = 0.f, Fa = 0.f, Fe = 0.f;
-    float2 xa = make_float2(0.f, 0.f), xe = xa;
+    int ea = 0, ee = 0;
+    float da = 0.f, de = 0.f, Fa = 0.f, Fe = 0.f;
     if (on) {
       const int ia = iw + nw * nu, ie = ia + nwm;
-      ja = cell_j[ia];
-      je = cell_j[ie];
-      ta = cell_t[ia];
-      te = cell_t[ie];
-      xa = cell_x[ia];
-      xe = cell_x[ie];
+      ea = cell_e[ia];
+      ee = cell_e[ie];
+      da = cell_dx[ia];
+      de = cell_dx[ie];
       Fa = F[ia];
       Fe = F[ie];
     }
@@ -141,17 +203,14 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, long slab, 
       const int co = s_col[cl];
       float v = 0.f;
       if (on && co >= 0) {
-        const float4* col = Sf + co;
         const float2 e = s_eps[cl];
-        const float4 la = col[ja], ha = col[ja + 1], le = col[je], he = col[je + 1];
-        const float zar = re_z(xa, e, la, ha, ta);
-        const float zer = re_z(xe, e, le, he, te);
-        const float sia = (1.f - ta) * la.z + ta * ha.z;  // Im Σ(x)
-        const float sie = (1.f - te) * le.z + te * he.z;
+        const float4 A = rec[co + ea], B = rec[co + ee];
+        const float zar = (A.x - e.x) + fmaf(da, A.z, A.y - e.y), sia = fmaf(da, dim[co + ea], A.w);
+        const float zer = (B.x - e.x) + fmaf(de, B.z, B.y - e.y), sie = fmaf(de, dim[co + ee], B.w);
         // Im 1/z with Im z = -Im Σ; the K tensor carries FP32 precision, so an approximate
         // division (2 ulp; denominators here lie far inside its range) is enough
-        const float ga = __fdividef(sia, zar * zar + sia * sia);
-        const float ge = __fdividef(sie, zer * zer + sie * sie);
+        const float ga = __fdividef(sia, fmaf(zar, zar, sia * sia));
+        const float ge = __fdividef(sie, fmaf(zer, zer, sie * sie));
         v = ga * Fa + ge * Fe;
       }
       kb_tile[(cl * nm + nu) * (kKbW + 1) + tw] = v;
@@ -202,7 +261,7 @@ static size_t kbuild_smem_bytes(long nm) { return size_t(kKbCols * nm * (kKbW + 
 // (256 pairs (ν, f)) added into FP64. The (ν, f) tile of the block's outer state -- w_f g2, ωq,
 // n(ωq), exp(±ωq/T), ε_f, the Σ column -- is staged in shared memory by the block; the node table
 // and the bucket table too, when they fit.
-// Grid (nω / 256, ni, slots), 256 threads, thread = node ω. Slot a reads Σ_in from Sf_all + a nω ni
+// Grid (nω / 256, ni, slots), 256 threads, thread = node ω. Slot a reads Σ_in from Sf_all + slots[a] nω ni
 // and T, μ from tp[slots[a]]. Output: with ImS_b, ImΣ of the slot (ImS_b + a nω ni) and its BF16
 // split as the Kramers-Kronig product's B operand (rows a ni + i, columns ω, stride Kp2), as
 // finalize_fm_batch_kernel writes them; else ImΣ added into add_out [nω, ni] (slot 0).
@@ -258,7 +317,7 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
   const bool warm = T > 1.4901161193847656e-08f;
   const float invT = warm ? 1.f / T : 0.f;
   const float2 mu = split_df(q.mu);
-  const float4* Sf = Sf_all + slab * a;
+  const float4* Sf = Sf_all + slab * slots[a];
   const float4 wn = wtab_g[on ? iw : 0];
   const float2 w = make_float2(wn.x, wn.y);
   // exp((ω - μ)/T) of the thread's node: f(ω ± ωq - μ) = 1 / (E exp(±ωq/T) + 1); a node whose E
@@ -383,14 +442,16 @@ __device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v 
   return fmaf(E, fmaf(-a, T, v) / T, E);
 }
 
-__global__ void fd_cell_kernel(const float4* __restrict__ Sf, const float4* __restrict__ wtab, const double* __restrict__ ws,
-                               int nw, long n, float4* __restrict__ rec, float* __restrict__ dim) {
-  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;  // node and column, all slots
-  if (k >= n) return;
+__global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __restrict__ slots,
+                               const float4* __restrict__ wtab, const double* __restrict__ ws, int nw, long slab,
+                               float4* __restrict__ rec, float* __restrict__ dim) {
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;  // node and column of slot blockIdx.y
+  if (k >= slab) return;
+  const float4* Sf = Sf_all + slab * slots[blockIdx.y];
   const int j = int(k % nw);
   const float4 s = Sf[k], wj = wtab[j];
   const float2 u = split_df(ws[j] - (double(s.x) + double(s.y)));
-  const long col = 2 * (k - j) + j;  // records [side][nω] of the column
+  const long col = 2 * (slab * blockIdx.y + k - j) + j;  // records [side][nω] of the column
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     const bool out = side ? j == nw - 1 : j == 0;
@@ -568,35 +629,71 @@ __global__ void finalize_assemble_kernel(const float* __restrict__ part, long n,
   out[k] = make_double2(double(s), im[k]);
 }
 
-// The occupation tables of the active temperatures as FP32 (computed in FP64 as occ_table_kernel):
-// F[a][0 .. nω nm) absorption, F[a][nω nm .. 2 nω nm) emission.
-__global__ void occ_table_f32_kernel(const double* __restrict__ ws, int nw, const double* __restrict__ wnu, int nm,
-                                     const int* __restrict__ slots, const TParams* __restrict__ tp, double w_ac,
-                                     float* __restrict__ F_all) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const long nwm = long(nw) * nm;
-  if (k >= nwm) return;
-  const int a = blockIdx.y;
-  const TParams q = tp[slots[a]];
-  float* F = F_all + 2 * nwm * a;
-  const int iw = k % nw, nu = k / nw;
-  const double wq = wnu[nu], w = ws[iw];
-  if (wq < w_ac) {
-    F[k] = 0.f;
-    F[k + nwm] = 0.f;
-    return;
+// exp(ω_ν/T) and n(ω_ν) of every temperature and mode of a run (the quotient's rounding put back); 0 where the
+// occupation table takes the plain formula: ω_ν > 300 T, T ~ 0, a mode left out or at 0.
+__global__ void mode_table_kernel(const double* __restrict__ wnu, int nm, const TParams* __restrict__ tp, double w_ac,
+                                  double2* __restrict__ modes) {
+  const int nu = threadIdx.x + blockIdx.x * blockDim.x, t = blockIdx.y;
+  if (nu >= nm) return;
+  const double wq = wnu[nu], T = tp[t].T;
+  double2 o = make_double2(0.0, 0.0);
+  if (T > 1.4901161193847656e-08 && !(wq < w_ac) && wq > 0.0 && wq <= 300.0 * T) {
+    const double a = wq / T, m0 = expm1(a), m = fma(m0 + 1.0, fma(-a, T, wq) / T, m0);
+    o = make_double2(m + 1.0, 1.0 / m);
   }
-  const double nq = occ_boson_d(wq, q.T);
-  F[k] = float(nq + occ_fermion_d(w + wq - q.mu, q.T));
-  F[k + nwm] = float(nq + 1 - occ_fermion_d(w - wq - q.mu, q.T));
+  modes[nu + nm * t] = o;
 }
 
-__global__ void sigma_f32_batch_kernel(const double2* __restrict__ S, long n, int nA, float4* __restrict__ out) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n * nA) return;
-  const double2 z = S[k];
-  const float2 r = split_df(z.x);
-  out[k] = make_float4(r.x, r.y, float(z.y), 0.f);
+// The occupation tables of the active temperatures as FP32, computed in FP64: F[a][0 .. nω nm) absorption
+// n + f(ω + ω_ν - μ), F[a][nω nm .. 2 nω nm) emission n + 1 - f(ω - ω_ν - μ). By detailed balance these are
+// (1 + n)(1 + E)/(1 + E e) and n (1 + E)/(1 + E/e) with E = exp((ω - μ)/T), e = exp(ω_ν/T) (both over E above μ): one
+// exponential a node and a dozen operations an element, in blocks of four nodes over all SMs (FP64 instructions issue
+// at one per 16 cycles and SM; two exponentials and divisions an element before: 501 x 15 6.5 -> OCC_US us). Also resets
+// the iteration's max|ΔΣ|. Grid (nω / 4, slots).
+constexpr int kOccW = 4;
+__global__ void __launch_bounds__(64) occ_table_f32_kernel(const double* __restrict__ ws, int nw,
+                                                           const double* __restrict__ wnu, int nm,
+                                                           const int* __restrict__ slots, const TParams* __restrict__ tp,
+                                                           const double2* __restrict__ modes, double w_ac,
+                                                           float* __restrict__ F_all,
+                                                           unsigned long long* __restrict__ errbits,
+                                                           IterCtl* __restrict__ ctl) {
+  __shared__ double s_p[kOccW], s_q[kOccW];
+  const int a = blockIdx.y, t = slots[a];
+  const int stop = ctl->stop_next;  // set by the iteration before, unchanged during this one's first kernels
+  if (blockIdx.x == 0 && a == 0 && threadIdx.x == 0) ctl->stop = stop;
+  if (stop) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) errbits[t] = 0;
+  const long nwm = long(nw) * nm;
+  const TParams q = tp[t];
+  float* F = F_all + 2 * nwm * a;
+  const int wl = threadIdx.x % kOccW, iw = blockIdx.x * kOccW + wl;
+  if (threadIdx.x < kOccW && iw < nw && q.T > 1.4901161193847656e-08) {
+    const double v = ws[iw] - q.mu, m = -fabs(v), av = m * q.inv_T, E0 = exp(av), E = fma(E0, fma(-av, q.T, m) * q.inv_T, E0);
+    s_p[wl] = v <= 0.0 ? 1.0 : E;
+    s_q[wl] = v <= 0.0 ? E : 1.0;
+  }
+  __syncthreads();
+  if (iw >= nw) return;
+  for (int nu = threadIdx.x / kOccW; nu < nm; nu += 64 / kOccW) {
+    const long k = iw + long(nw) * nu;
+    const double wq = wnu[nu];
+    const double2 en = modes[nu + nm * t];
+    float fa = 0.f, fe = 0.f;
+    if (en.x > 0.0) {
+      const double c = s_p[wl] + s_q[wl];
+      // 1 / (p + q e) and 1 / (p + q / e) = e / (p e + q) from one division
+      const double da = fma(s_q[wl], en.x, s_p[wl]), de = fma(s_p[wl], en.x, s_q[wl]), r = c / (da * de);
+      fa = float((en.y + 1.0) * r * de);
+      fe = float(en.y * en.x * r * da);
+    } else if (!(wq < w_ac)) {
+      const double nq = occ_boson_d(wq, q.T), w = ws[iw];
+      fa = float(nq + occ_fermion_d(w + wq - q.mu, q.T));
+      fe = float(nq + 1 - occ_fermion_d(w - wq - q.mu, q.T));
+    }
+    F[k] = fa;
+    F[k + nwm] = fe;
+  }
 }
 
 // ImΣ of slot a: ImS[a][ω + nω i] = Σ_s part[s][(a nω + ω) + M i], M = nA nω (the stacked rows).
@@ -605,14 +702,14 @@ __global__ void sigma_f32_batch_kernel(const double2* __restrict__ S, long n, in
 __global__ void finalize_fm_batch_kernel(const float* __restrict__ part, int nw, long slab, int nA, int splits,
                                          long stride, double* __restrict__ ImS, __nv_bfloat16* __restrict__ Im0 = nullptr,
                                          __nv_bfloat16* __restrict__ Im1 = nullptr, __nv_bfloat16* __restrict__ Im2 = nullptr,
-                                         long Kp2 = 0) {
+                                         long Kp2 = 0, const IterCtl* __restrict__ ctl = nullptr) {
+  if (ctl && ctl->stop) return;
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= slab) return;
   const int a = blockIdx.y;
   const long w = k % nw, i = k / nw;
   const long src = (long(a) * nw + w) + long(nA) * nw * i;
-  float acc = 0.f;
-  for (int p = 0; p < splits; ++p) acc += part[src + stride * p];
+  const float acc = sum_splits(part + src, splits, stride);
   ImS[slab * a + k] = double(acc);
   if (Im0) {  // and the B operand of the Kramers-Kronig product: row a ni + i, column ω, three parts
     __nv_bfloat16 q[3];
@@ -629,72 +726,98 @@ __global__ void finalize_fm_batch_kernel(const float* __restrict__ part, int nw,
 // multiplet, or a single state -- Σ_new(ω_j) = Σ_s part[s] + i ImΣ of every member (the partials in
 // ascending order), averaged over the members of a multiplet (their sum in member order divided by
 // the count); then per member: err = max |Σ_new - Σ| over the slot's temperature (FP64 differences,
-// FP32 magnitude, the maximum taken on the bit patterns as err_copy_kernel does), Σ ← Σ_new, and the
+// FP32 magnitude, the maximum taken on the bit patterns as err_copy_kernel does), Σ ← Σ_new, its clamped form for the
+// next iteration -- the columns' cell records (rec, dim), or Sf with dispersive modes (rec null) -- and the
 // spectral functions' per-node terms P[i][j] = (ε_i - ω_j + ReΣ_j, ReΣ_{j+1} - ReΣ_j, ImΣ_j, ImΣ_{j+1})
-// of spectral_prep_f32_kernel (ImΣ_{j+1}, ReΣ_{j+1} = those of j at the last node). Bitwise the
-// results of the separate kernels. Groups: CSR (gptr, gidx), members in order. Grid (nω / 255,
+// (ImΣ_{j+1}, ReΣ_{j+1} = those of j at the last node). Everything but Σ itself and its change is formed on float pairs
+// (a single state's ReΣ is an FP32 sum): six instructions on the FP64 pipe a state and node, where about 25 bound the
+// kernel (1251 x 495: 26 -> KE1_US us, 8 x 626 x 168: 32 -> KE2_US us, with the next iteration's clamp, 10 us, included).
+// Groups: CSR (gptr, gidx), members in order. Grid (nω / 255,
 // groups, slots), 256 threads: thread t takes node j = 255 blockIdx.x + t; the last thread's node
 // is the next block's first, formed again to give node 254 its neighbour.
 __global__ void __launch_bounds__(256) kk_epilogue_kernel(const float* __restrict__ part, int splits, long stride,
                                                           const double* __restrict__ ImS_b, int nw, long slab,
                                                           const int* __restrict__ slots, const int32_t* __restrict__ gptr,
-                                                          const int32_t* __restrict__ gidx, const double* __restrict__ ws,
-                                                          const double* __restrict__ eps_i, double2* __restrict__ S_all,
-                                                          float4* __restrict__ Pall,
+                                                          const int32_t* __restrict__ gidx, const float4* __restrict__ wtab,
+                                                          const float2* __restrict__ epair,
+                                                          const TParams* __restrict__ tp, double2* __restrict__ S_all,
+                                                          float4* __restrict__ Sf_all, float4* __restrict__ rec_all,
+                                                          float* __restrict__ dim_all, float4* __restrict__ Pall,
                                                           unsigned long long* __restrict__ errbits_all,
-                                                          double* __restrict__ minA_all) {
-  __shared__ double2 sh[256];
-  __shared__ unsigned long long she[256];
+                                                          double* __restrict__ minA_all,
+                                                          const IterCtl* __restrict__ ctl) {
+  if (ctl && ctl->stop) return;
+  __shared__ float4 sh[256];
+  __shared__ uint32_t she[8];
   const int a = blockIdx.z, t = slots[a];
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)  // the minimum of spectral_fin starts at +inf
     minA_all[t] = INFINITY;
   const int j = blockIdx.x * 255 + threadIdx.x;
   const bool in = j < nw;
   const int p0 = gptr[blockIdx.y], p1 = gptr[blockIdx.y + 1];
-  double sr = 0, si = 0;
+  double2 z = make_double2(0.0, 0.0);
+  float4 zf = make_float4(0.f, 0.f, 0.f, 0.f);  // {Re hi, Re lo, Im}
   if (in) {
-    for (int p = p0; p < p1; ++p) {
-      const long src = slab * a + j + long(nw) * gidx[p];
-      float acc = 0.f;
-      for (int q = 0; q < splits; ++q) acc += part[src + stride * q];
-      if (p1 - p0 == 1) {
-        sr = double(acc);
-        si = ImS_b[src];
-      } else {
-        sr += double(acc);
-        si += ImS_b[src];
+    if (p1 - p0 == 1) {
+      const long src = slab * a + j + long(nw) * gidx[p0];
+      const float acc = sum_splits(part + src, splits, stride);
+      z = make_double2(double(acc), ImS_b[src]);
+      zf = make_float4(acc, 0.f, float(z.y), 0.f);
+    } else {
+      for (int p = p0; p < p1; ++p) {
+        const long src = slab * a + j + long(nw) * gidx[p];
+        z.x += double(sum_splits(part + src, splits, stride));
+        z.y += ImS_b[src];
       }
-    }
-    if (p1 - p0 > 1) {
       const double len = double(p1 - p0);
-      sr /= len;
-      si /= len;
+      z.x /= len;
+      z.y /= len;
+      zf = sigma_f32(z);
     }
   }
-  sh[threadIdx.x] = make_double2(sr, si);
+  sh[threadIdx.x] = zf;
   __syncthreads();
-  unsigned long long e = 0;
+  uint32_t e = 0;  // the largest magnitude's bits: non-negative floats order as integers, and NaN above all
   if (in && threadIdx.x < 255) {
-    const double2 lo = sh[threadIdx.x];
-    const double2 hi = j + 1 < nw ? sh[threadIdx.x + 1] : lo;
+    const float4 zn = j + 1 < nw ? sh[threadIdx.x + 1] : zf, wj = wtab[j];
+    const float etam = float(-tp[t].eta_min);
+    float dim, d0;
+    const float4 rec = cell_record(zf, zn, wj, etam, dim);
+    const float dre = (zn.x - zf.x) + (zn.y - zf.y);
     double2* S = S_all + slab * t;
+    const long ni = slab / nw;
     for (int p = p0; p < p1; ++p) {
       const int i = gidx[p];
       const long k = j + long(nw) * i;
       const double2 b = S[k];
-      const double d = double(hypotf(float(lo.x - b.x), float(lo.y - b.y)));
-      e = max(e, (unsigned long long)__double_as_longlong(d));
-      S[k] = lo;
-      Pall[slab * a + k] = make_float4(float(eps_i[i] - ws[j] + lo.x), float(hi.x - lo.x), float(lo.y), float(hi.y));
+      e = max(e, __float_as_uint(hypotf(float(z.x - b.x), float(z.y - b.y))));
+      S[k] = z;
+      if (rec_all) {
+        const long at = (ni * t + i) * (nw + 1l) + j + 1;
+        rec_all[at] = rec;
+        dim_all[at] = dim;
+        if (j == 0) {
+          rec_all[at - 1] = cell_record(zf, zf, wj, etam, d0);
+          dim_all[at - 1] = 0.f;
+        }
+      } else {
+        Sf_all[slab * t + k] = make_float4(zf.x, zf.y, fminf(zf.z, etam), 0.f);
+      }
+      // ε_i - ω_j + ReΣ_j with its cancelling parts exact
+      const float2 ep = epair[i];
+      float e1, e2;
+      const float s1 = two_sum(ep.x, -wj.x, e1), s2 = two_sum(s1, zf.x, e2);
+      Pall[slab * a + k] = make_float4(s2 + ((e1 + e2) + ((ep.y - wj.y) + zf.y)), dre, zf.z, zn.z);
     }
   }
-  she[threadIdx.x] = e;
+  e = __reduce_max_sync(0xffffffffu, e);
+  if (threadIdx.x % 32 == 0) she[threadIdx.x / 32] = e;
   __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st) she[threadIdx.x] = max(she[threadIdx.x], she[threadIdx.x + st]);
-    __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) e = max(e, she[w]);
+    atomicMax(errbits_all + t, (unsigned long long)__double_as_longlong(double(__uint_as_float(e))));
   }
-  if (threadIdx.x == 0) atomicMax(errbits_all + t, she[0]);
 }
 
 static long pad64(long x) { return (x + 63) / 64 * 64; }
@@ -720,6 +843,14 @@ void tc_setup(Scgd0Plan* P) {
   T->Kp = pad64(nk);
   T->Kp2 = pad64(nw);
   if (nw > (1l << 30) || ni > (1l << 30) || nk > (1l << 30)) fail(EPSP_EINVAL, "sizes beyond the 32-bit tile grid");
+  T->epair.alloc(ctx, size_t(ni));
+  split_df_kernel<<<div_up(size_t(ni), 256), 256, 0, s>>>(P->d_eps_i.p, ni, T->epair.p);
+  EPSP_LAUNCHED(ctx);
+  if (!P->disp) {
+    P->d_wtab.alloc(ctx, size_t(nw));
+    fd_node_table_kernel<<<div_up(size_t(nw), 256), 256, 0, s>>>(P->d_ws.p, int(nw), P->d_wtab.p);
+    EPSP_LAUNCHED(ctx);
+  }
   if (P->disp) {  // the Kramers-Kronig map's operands only: the Fan-Migdal sum is fm_disp_f32_kernel
     for (int p = 0; p < kNs; ++p) {
       T->KK[p].alloc(ctx, size_t(nw * T->Kp2));
@@ -770,13 +901,12 @@ void tc_setup(Scgd0Plan* P) {
   tc_gemm_shape(ctx, int(nw), int(ni), int(nw), max_splits_for(nw, kKbCapKK), kNs, &T->bn2, &T->splits2, kKbCapKK);
   T->part.alloc(ctx, size_t(std::max(T->splits1, T->splits2)) * size_t(nw * ni));
   const long nwm = nw * P->nm;
-  T->xf.alloc(ctx, size_t(2 * nwm));
   T->tf.alloc(ctx, size_t(2 * nwm));
   T->Ff.alloc(ctx, size_t(2 * nwm));
   T->ef.alloc(ctx, size_t(P->nc));
-  T->Sf.alloc(ctx, size_t(nw * ni));
-  split_df_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_x.p, 2 * nwm, T->xf.p);
-  EPSP_LAUNCHED(ctx);
+  T->rec.alloc(ctx, size_t((nw + 1) * ni));
+  T->dim.alloc(ctx, size_t((nw + 1) * ni));
+  T->modes.alloc(ctx, size_t(P->nm));
   to_f32_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_t.p, 2 * nwm, T->tf.p);
   EPSP_LAUNCHED(ctx);
   split_df_kernel<<<div_up(size_t(P->nc), 256), 256, 0, s>>>(P->d_epsc.p, P->nc, T->ef.p);
@@ -819,8 +949,8 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
     const long slab = nw * ni, n = slab * nA, nvf = P->nm * P->nf;
     ensure(T->fdrec, ctx, size_t(2 * n));
     ensure(T->fddim, ctx, size_t(2 * n));
-    fd_cell_kernel<<<div_up(size_t(n), 256), 256, 0, ctx->stream>>>(T->Sf.p, P->d_wtab.p, P->d_ws.p, int(nw), n, T->fdrec.p,
-                                                                    T->fddim.p);
+    fd_cell_kernel<<<dim3(div_up(size_t(slab), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
+        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, T->fdrec.p, T->fddim.p);
     EPSP_LAUNCHED(ctx);
     const size_t tab = sizeof(float2) * size_t(nw) + 2 * size_t(P->ntab);
     const bool smem = tab <= (size_t(96) << 10) && nw <= 65535;
@@ -894,6 +1024,7 @@ void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, do
   tc_disp_choose(P, &T, 1);
   TParams q{};
   q.T = T;
+  q.inv_T = 1.0 / T;
   q.mu = mu;
   DBuf<TParams> d_q = to_device(ctx, &q, 1);
   DBuf<int> d_slot0;
@@ -951,15 +1082,15 @@ void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS) {
   const long nw = P->nw, ni = P->ni, nk = P->nm * P->nc;
   long pk = prof_begin(ctx, "kbuild");
   const long nwm = nw * P->nm;
-  sigma_f32_kernel<<<div_up(size_t(nw * ni), 256), 256, 0, s>>>(d_Sin, nw * ni, T->Sf.p);
+  cell_records_kernel<<<div_up(size_t(nw * ni), 256), 256, 0, s>>>(d_Sin, nullptr, nullptr, P->d_wtab.p, int(nw), nw * ni,
+                                                                   T->rec.p, T->dim.p);
   EPSP_LAUNCHED(ctx);
-
   to_f32_kernel<<<div_up(size_t(nwm), 256), 256, 0, s>>>(P->d_Fa.p, nwm, T->Ff.p);
   EPSP_LAUNCHED(ctx);
   to_f32_kernel<<<div_up(size_t(nwm), 256), 256, 0, s>>>(P->d_Fe.p, nwm, T->Ff.p + nwm);
   EPSP_LAUNCHED(ctx);
   kbuild_bf16_kernel<<<dim3(div_up(size_t(nw), kKbW), unsigned(div_up(size_t(T->Kp), size_t(kKbCols * P->nm))), 1), 256,
-                       kbuild_smem_bytes(P->nm), s>>>(int(nw), nw * ni, T->Sf.p, P->d_cell_j.p, T->tf.p, T->xf.p,
+                       kbuild_smem_bytes(P->nm), s>>>(int(nw), int(ni), T->rec.p, T->dim.p, nullptr, P->d_cell_j.p, T->tf.p,
                                                       T->skip.p, int(P->nm), T->ef.p, P->d_colc.p, int(P->nc), T->Ff.p,
                                                       T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp);
   EPSP_LAUNCHED(ctx);
@@ -998,8 +1129,14 @@ void tc_reserve(Scgd0Plan* P, long nT) {
     T->Im[p].alloc(ctx, size_t(nT * ni * T->Kp2));
     T->Im[p].zero(ctx->stream);  // the padding columns nω.. Kp2 of the KK operand stay zero
   }
-  T->Sf.alloc(ctx, size_t(nT * slab));
-  if (!P->disp) T->Ff.alloc(ctx, size_t(nT * 2 * nwm));
+  if (P->disp) {
+    T->Sf.alloc(ctx, size_t(nT * slab));
+  } else {
+    T->rec.alloc(ctx, size_t(nT * (nw + 1) * ni));
+    T->dim.alloc(ctx, size_t(nT * (nw + 1) * ni));
+    T->modes.alloc(ctx, size_t(nT * P->nm));
+    T->Ff.alloc(ctx, size_t(nT * 2 * nwm));
+  }
   T->ImS_b.alloc(ctx, size_t(nT * slab));
   size_t part = 0;
   for (long a = 1; a <= nT; ++a) {
@@ -1020,74 +1157,84 @@ int* tc_err_ptr(Scgd0Plan* P) { return P->tc->err.p; }
 
 long tc_capacity(Scgd0Plan* P) { return P->tc->ImS_b.p ? P->tc->capT : 0; }
 
-float4* tc_sigma_f32(Scgd0Plan* P) { return P->tc->Sf.p; }
+void tc_start(Scgd0Plan* P, long nT, const TParams* d_tp) {
+  if (P->disp) return;
+  mode_table_kernel<<<dim3(div_up(size_t(P->nm), 32), unsigned(nT)), 32, 0, P->ctx->stream>>>(P->d_wnu.p, int(P->nm), d_tp,
+                                                                                            P->w_ac, P->tc->modes.p);
+  EPSP_LAUNCHED(P->ctx);
+}
 
-static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, double2* d_S_all, float4* d_P,
-                       unsigned long long* d_errbits, double* d_minA);
+void tc_take_sigma(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, const double2* d_S_all) {
+  auto* T = P->tc.get();
+  const long slab = P->nw * P->ni;
+  const dim3 grid(div_up(size_t(slab), 256), unsigned(nA));
+  if (P->disp)
+    clamp_f32_kernel<<<grid, 256, 0, P->ctx->stream>>>(d_S_all, T->Sf.p, slab, d_slots, d_tp);
+  else
+    cell_records_kernel<<<grid, 256, 0, P->ctx->stream>>>(d_S_all, d_slots, d_tp, P->d_wtab.p, int(P->nw), slab, T->rec.p,
+                                                          T->dim.p);
+  EPSP_LAUNCHED(P->ctx);
+}
 
-void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const int* slots_h, const TParams* d_tp,
-                const double2* d_Sin_b, double2* d_S_all, float4* d_P, unsigned long long* d_errbits, double* d_minA) {
-  (void)slots_h;
+static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, double2* d_S_all, float4* d_P,
+                       unsigned long long* d_errbits, double* d_minA, const IterCtl* ctl);
+
+void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, double2* d_S_all, float4* d_P,
+                unsigned long long* d_errbits, double* d_minA, IterCtl* ctl) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
   auto* T = P->tc.get();
   if (nA > T->capT) fail(EPSP_EINVAL, "more active temperatures than reserved");
-  const long nw = P->nw, ni = P->ni, nk = P->nm * P->nc, nwm = nw * P->nm, slab = nw * ni;
+  const long nw = P->nw, ni = P->ni, nk = P->nm * P->nc, slab = nw * ni;
   const unsigned eb = div_up(size_t(slab), 256);
-  long pp = prof_begin(ctx, "kprep");
-  if (d_Sin_b) {
-    sigma_f32_batch_kernel<<<div_up(size_t(slab * nA), 256), 256, 0, s>>>(d_Sin_b, slab, nA, T->Sf.p);
-    EPSP_LAUNCHED(ctx);
-  }
   if (P->disp) {  // dispersive modes: ImΣ of every slot term by term, then the same Kramers-Kronig tail
-    prof_end(ctx, pp);
     long pk = prof_begin(ctx, "fm_disp");
     launch_fm_disp(P, nA, d_slots, d_tp, T->ImS_b.p, nullptr);
     prof_end(ctx, pk);
-    tc_kk_tail(P, nA, d_slots, d_S_all, d_P, d_errbits, d_minA);
+    tc_kk_tail(P, nA, d_slots, d_tp, d_S_all, d_P, d_errbits, d_minA, nullptr);
     return;
   }
-  // small blocks: the FP64 exponentials of the table spread over every SM
-  occ_table_f32_kernel<<<dim3(div_up(size_t(nwm), 64), unsigned(nA)), 64, 0, s>>>(
-      P->d_ws.p, int(nw), P->d_wnu.p, int(P->nm), d_slots, d_tp, P->w_ac, T->Ff.p);
+  long pp = prof_begin(ctx, "kprep");
+  occ_table_f32_kernel<<<dim3(div_up(size_t(nw), kOccW), unsigned(nA)), 64, 0, s>>>(
+      P->d_ws.p, int(nw), P->d_wnu.p, int(P->nm), d_slots, d_tp, T->modes.p, P->w_ac, T->Ff.p, d_errbits, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pp);
   long pk = prof_begin(ctx, "kbuild");
   kbuild_bf16_kernel<<<dim3(div_up(size_t(nw), kKbW), unsigned(div_up(size_t(T->Kp), size_t(kKbCols * P->nm))),
                             unsigned(nA)),
-                       256, kbuild_smem_bytes(P->nm), s>>>(int(nw), slab, T->Sf.p, P->d_cell_j.p, T->tf.p, T->xf.p,
+                       256, kbuild_smem_bytes(P->nm), s>>>(int(nw), int(ni), T->rec.p, T->dim.p, d_slots, P->d_cell_j.p, T->tf.p,
                                                            T->skip.p, int(P->nm), T->ef.p, P->d_colc.p, int(P->nc), T->Ff.p,
-                                                           T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp);
+                                                           T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pk);
   // ImΣ of every slot: the stacked K_t rows times G
   const long M = long(nA) * nw;
   int sp = tc_gemm_launch(ctx, T->opK, T->opG, int(M), int(ni), int(nk), T->part.p, M, M * ni, max_splits_for(nk),
-                          T->err.p, "tc_fm", kKbCap);
+                          T->err.p, "tc_fm", kKbCap, ctl ? &ctl->stop : nullptr);
   // ImΣ of every slot, and its BF16 split as the B operand of ReΣ = KK ImΣ (columns: the slots'
   // states in order)
   long pf = prof_begin(ctx, "finalize");
   finalize_fm_batch_kernel<<<dim3(eb, unsigned(nA)), 256, 0, s>>>(T->part.p, int(nw), slab, nA, sp, M * ni, T->ImS_b.p,
-                                                                   T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2);
+                                                                   T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pf);
-  tc_kk_tail(P, nA, d_slots, d_S_all, d_P, d_errbits, d_minA);
+  tc_kk_tail(P, nA, d_slots, d_tp, d_S_all, d_P, d_errbits, d_minA, ctl);
 }
 
 // ReΣ = KK ImΣ for every slot (the split ImΣ rows already in T->Im) and the fused epilogue.
-static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, double2* d_S_all, float4* d_P,
-                       unsigned long long* d_errbits, double* d_minA) {
+static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, double2* d_S_all, float4* d_P,
+                       unsigned long long* d_errbits, double* d_minA, const IterCtl* ctl) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
   auto* T = P->tc.get();
   const long nw = P->nw, ni = P->ni, slab = nw * ni;
   const long N2 = long(nA) * ni;
   int sp2 = tc_gemm_launch(ctx, T->opKK, T->opIm, int(nw), int(N2), int(nw), T->part.p, nw, nw * N2,
-                           max_splits_for(nw, kKbCapKK), T->err.p, "tc_kk", kKbCapKK);
+                           max_splits_for(nw, kKbCapKK), T->err.p, "tc_kk", kKbCapKK, ctl ? &ctl->stop : nullptr);
   long pf = prof_begin(ctx, "kk_epilogue");
   kk_epilogue_kernel<<<dim3(div_up(size_t(nw), 255), unsigned(P->ngroups), unsigned(nA)), 256, 0, s>>>(
-      T->part.p, sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_ws.p, P->d_eps_i.p,
-      d_S_all, d_P, d_errbits, d_minA);
+      T->part.p, sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_wtab.p, T->epair.p,
+      d_tp, d_S_all, T->Sf.p, T->rec.p, T->dim.p, d_P, d_errbits, d_minA, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pf);
 }

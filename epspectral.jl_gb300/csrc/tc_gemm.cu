@@ -124,7 +124,7 @@ static CUtensorMap remap(const TcOperand& op, int p, int box_rows) {
 
 template <int BN, int STAGES, int NS, int BK, bool TF32 = false, int NA = NS>
 static void launch_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int N, int kblocks, int per,
-                           int splits, float* out, long ld_out, long split_stride, int* d_err, int gm = 1) {
+                           int splits, float* out, long ld_out, long split_stride, int* d_err, int gm = 1, const int* skip = nullptr) {
   using L = TcPSmem<BN, STAGES, NS, BK, TF32, NA>;
   if (A.bk != BK || B.bk != BK) fail(EPSP_EINVAL, "operand tensor maps were built for another K block");
   if (A.tf32 != TF32 || B.tf32 != TF32) fail(EPSP_EINVAL, "operand tensor maps were built for another element type");
@@ -143,7 +143,7 @@ static void launch_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B, int
   const int nitems = nN * nM * splits;  // (N tile, M tile, split)
   const int grid = std::min(nitems, ctx->sm_count);
   kern<<<grid, 192, L::kBytes, ctx->stream>>>(maps, M, N, kblocks, per, nN, nM, nitems, out, ld_out, split_stride,
-                                              d_err, gm);
+                                              d_err, gm, skip);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -221,8 +221,9 @@ static void launch_pair_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B
 }
 
 int tc_gemm_launch(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int N, int K, float* out, long ld_out,
-                   long split_stride, int max_splits, int* d_err, const char* prof_name, int kb_cap) {
+                   long split_stride, int max_splits, int* d_err, const char* prof_name, int kb_cap, const int* skip) {
   if (A.tf32 || B.tf32) fail(EPSP_EINVAL, "TF32 operands take tc_gemm_launch_with");
+  if (skip && (A.ns != 3 || A.bk != kTcBK)) fail(EPSP_EINVAL, "internal: the skip flag is for three-part operands");
   const bool one = A.ns == 1 && B.ns == 3;  // A exact in BF16
   if (!one && (A.ns != B.ns || (A.ns != 2 && A.ns != 3))) fail(EPSP_EINVAL, "operands must be split into 2 or 3 parts alike");
   if (A.bk != B.bk) fail(EPSP_EINVAL, "operands built for different K blocks");
@@ -240,7 +241,7 @@ int tc_gemm_launch(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int 
   else if (bk != kTcBK)
     fail(EPSP_EINVAL, "K blocks of 32 are for three-part operands here (tc_gemm_launch_with takes two-part ones)");
   else if (A.ns == 3)  // the persistent kernel: each SM's tiles back to back, epilogues overlapped
-    launch_persist<128, 2, 3, 64>(ctx, A, B, M, N, kblocks, per, splits, out, ld_out, split_stride, d_err);
+    launch_persist<128, 2, 3, 64>(ctx, A, B, M, N, kblocks, per, splits, out, ld_out, split_stride, d_err, 1, skip);
   else if (BN == 256)
     launch_persist<256, 2, 2, 64>(ctx, A, B, M, N, kblocks, per, splits, out, ld_out, split_stride, d_err);
   else

@@ -349,12 +349,13 @@ struct TcPSmem {
 template <int BN, int STAGES, int NS, int BK, bool TF32 = false, int NA = NS>
 __global__ void __launch_bounds__(192, 1)
     tc_gemm_persist_kernel(const __grid_constant__ TcMaps maps, int M, int N, int kblocks, int kb_per_split, int nN,
-                           int nM, int nitems, float* __restrict__ out, long ld_out, long split_stride,
-                           int* __restrict__ err, int gm = 1) {
+                           int nM, int nitems_, float* __restrict__ out, long ld_out, long split_stride,
+                           int* __restrict__ err, int gm = 1, const int* __restrict__ skip = nullptr) {
   using L = TcPSmem<BN, STAGES, NS, BK, TF32, NA>;
   static_assert(!TF32 || NS == 1, "TF32 operands have one part");
   static_assert(NA == NS || (NA == 1 && NS == 3), "A has all parts, or one of three");
   static_assert(2 * BN <= 512, "two accumulators must fit TMEM");
+  const int nitems = skip && *skip ? 0 : nitems_;  // (skip: nothing is done or written)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * L::kStage);
@@ -960,9 +961,11 @@ struct TcOperand {
 // Launches the split-precision product of A [M][K] and B [N][K] (K-major, both split into A.ns
 // parts) into the FP32 slabs out[split][m + ld_out n]; returns the number of splits used. With
 // kb_cap > 0 no FP32 accumulator sums more than kb_cap K-blocks of 64 (splits are added to bound
-// the accumulation error of long same-sign sums), within max_splits.
+// the accumulation error of long same-sign sums), within max_splits. With skip, a device flag, the kernel does nothing
+// where it is set.
 int tc_gemm_launch(Ctx* ctx, const TcOperand& A, const TcOperand& B, int M, int N, int K, float* out, long ld_out,
-                   long split_stride, int max_splits, int* d_err, const char* prof_name = "tc_gemm", int kb_cap = 0);
+                   long split_stride, int max_splits, int* d_err, const char* prof_name = "tc_gemm", int kb_cap = 0,
+                   const int* skip = nullptr);
 
 // The BN and split count tc_gemm_launch picks for (M, N, K), ns parts, at most max_splits splits.
 void tc_gemm_shape(Ctx* ctx, int M, int N, int K, int max_splits, int ns, int* bn, int* splits, int kb_cap = 0);

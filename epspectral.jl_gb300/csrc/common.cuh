@@ -153,6 +153,30 @@ inline void prof_end(Ctx* c, long idx) {
   if (idx >= 0) EPSP_CUDA(cudaEventRecord(c->prof_events[size_t(idx) + 1], c->stream));
 }
 
+// Programmatic dependent launch: a kernel launched with launch_after is made ready while the kernel ahead of it in the
+// stream runs out, and waits in pdl_wait (the first thing that it does with memory: until that kernel has ended and
+// its writes are visible), so that a kernel that runs has everything before its predecessor behind it too. It hides
+// launch latency in chains of kernels of 5 to 20 us: a scGD0 iteration of nine 92.6 -> 90.0 us, a training step of
+// 17 in a row 145 -> 141. (Letting it start still earlier, by griddepcontrol.launch_dependents, cost 5 % at 495 states: its
+// blocks then take shared memory and L1 from the kernel that runs.) A kernel launched plainly passes the wait at once.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline void launch_after(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  EPSP_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+}
+#endif
+
 #define EPSP_LAUNCHED(ctx) do { (ctx)->launches++; EPSP_CUDA(cudaGetLastError()); } while (0)
 
 // ---- device buffers ----

@@ -496,13 +496,14 @@ __global__ void __launch_bounds__(256) spectral_colsum_kernel(const double* __re
 // Σ_a A Wa per state (Cpart[slot][i][a-block], summed over the block's warps in warp order), both in
 // FP32 over at most 32 resp. 64 terms. A warp keeps its 32 x 32 values A Wa in registers and sums them over the lanes
 // by halving exchanges (31 shuffles for 32 states, where a tree per state took 160, each waited for), and loads eight
-// states at a time: 3201 nodes x 105 states 22.4 -> AD1_US us, 8001 x 495 23.7 -> AD2_US. Grid (nωa / 64, ni / 32, slots).
+// states at a time: 3201 nodes x 105 states 22.4 -> 9.3 us, 8001 x 495 23.7 -> 10.4. Grid (nωa / 64, ni / 32, slots).
 constexpr int kSpecChunk = 32;
 constexpr int kSpecNodes = 64;
 __global__ void __launch_bounds__(kSpecNodes) spectral_ad_f32_kernel(
     const float4* __restrict__ Pall, int nw, long slab, const int32_t* __restrict__ jsp, const float* __restrict__ dsp,
     const float* __restrict__ tsp, const float* __restrict__ Waf, const float* __restrict__ w_if, int nwa, int ni,
     float* __restrict__ Dpart, float* __restrict__ Cpart, const IterCtl* __restrict__ ctl) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   __shared__ float sh[kSpecNodes / 32][kSpecChunk];
   const int a = blockIdx.x * kSpecNodes + threadIdx.x;
@@ -591,7 +592,8 @@ __device__ __forceinline__ double float_middle_d(double x, double y) {
 // partials are combined through distributed shared memory in rank order, so every thread of the cluster holds the
 // same totals and takes the same branches.
 // status: 0 ok, 1 no sign change on the bracket.
-// Measured per iteration (3201 and 8001 nodes): 27.7 -> MU1_US us and 35.2 -> MU2_US us with what mu_prep_kernel took.
+// Measured at 3201 and 8001 nodes: 27.7 -> 16.6 us and 35.2 -> 21.5 us (before: with the kernel that prepared D at
+// the nodes). spectral_fin_f32_kernel, which forms the first round's terms now, went from 3.6 to 8.3 us.
 constexpr int kMuCluster = 8;
 constexpr int kMuThreads = 128;
 constexpr int kMuWarps = kMuThreads / 32;  // kMuCluster x kMuWarps partials: one per lane of the warp that sums them
@@ -711,6 +713,7 @@ __global__ void __launch_bounds__(kSpecNodes) spectral_fin_f32_kernel(
     const double* __restrict__ wsa, int nwa, int ni, const int* __restrict__ slots, double* __restrict__ Dall,
     double* __restrict__ minA_all, const MuIn M, const int* __restrict__ tc_err, int* __restrict__ tc_err_out,
     const unsigned long long* __restrict__ errbits, IterCtl* __restrict__ ctl) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   __shared__ double sh[2][kMuPart];
   const long z = blockIdx.y;
@@ -789,6 +792,7 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
                     TParams* __restrict__ tp, double W, double base, double gs, double br0, double br1,
                     const double* __restrict__ E_all, const double* __restrict__ part1, int npart, double* __restrict__ mu_all,
                     int* __restrict__ status_all, int* __restrict__ evals_all, const IterCtl* __restrict__ ctl) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -1603,13 +1607,13 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       }
       long psp = prof_begin(ctx, "spectral");
       if (f32_spec) {  // the per-node terms came from the Kramers-Kronig epilogue
-        spectral_ad_f32_kernel<<<dim3(unsigned(spec_nab), unsigned(spec_nch), unsigned(nA)), kSpecNodes, 0, s>>>(
-            P->w_Pf.p, int(nw), slab, P->d_jsp.p, P->d_dspf.p, P->d_tspf.p, P->d_Waf.p, P->d_w_if.p, int(nwa), int(ni),
-            P->w_Dpart.p, P->w_Cpart.p, ctl);
+        launch_after(s, spectral_ad_f32_kernel, dim3(unsigned(spec_nab), unsigned(spec_nch), unsigned(nA)), kSpecNodes, 0,
+                     P->w_Pf.p, int(nw), slab, P->d_jsp.p, P->d_dspf.p, P->d_tspf.p, P->d_Waf.p, P->d_w_if.p, int(nwa),
+                     int(ni), P->w_Dpart.p, P->w_Cpart.p, ctl);
         EPSP_LAUNCHED(ctx);
-        spectral_fin_f32_kernel<<<dim3(unsigned(spec_nab + div_up(size_t(ni), 2)), unsigned(nA)), kSpecNodes, 0, s>>>(
-            P->w_Dpart.p, P->w_Cpart.p, spec_nch, spec_nab, P->d_Wa.p, P->d_wsa.p, int(nwa), int(ni), d_slots.p, D_b.p,
-            d_minA, mu_in, tc_err_ptr(P), d_tcerr, d_err, ctl);
+        launch_after(s, spectral_fin_f32_kernel, dim3(unsigned(spec_nab + div_up(size_t(ni), 2)), unsigned(nA)), kSpecNodes,
+                     0, P->w_Dpart.p, P->w_Cpart.p, spec_nch, spec_nab, P->d_Wa.p, P->d_wsa.p, int(nwa), int(ni), d_slots.p,
+                     D_b.p, d_minA, mu_in, tc_err_ptr(P), d_tcerr, d_err, ctl);
         EPSP_LAUNCHED(ctx);
       } else {
         spectral_A_kernel<<<dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0, s>>>(
@@ -1629,9 +1633,9 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       prof_end(ctx, psp);
       if (!fix_mu) {
         long pm = prof_begin(ctx, "mu");
-        mu_solve_kernel<<<unsigned(kMuCluster * nA), kMuThreads, 0, s>>>(
-            D_b.p, P->d_wsa.p, int(nwa), d_slots.p, d_tp.p, P->W, P->nstates_base, occ->spin_degeneracy, br0, br1,
-            P->w_E.p, P->w_R1.p, spec_nab, d_mu, d_status, d_evals, ctl);
+        launch_after(s, mu_solve_kernel, unsigned(kMuCluster * nA), kMuThreads, 0, D_b.p, P->d_wsa.p, int(nwa), d_slots.p,
+                     d_tp.p, P->W, P->nstates_base, occ->spin_degeneracy, br0, br1, P->w_E.p, P->w_R1.p, spec_nab, d_mu,
+                     d_status, d_evals, ctl);
         EPSP_LAUNCHED(ctx);
         prof_end(ctx, pm);
       }

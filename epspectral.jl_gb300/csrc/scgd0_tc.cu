@@ -145,7 +145,7 @@ __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* 
 // split rows K_t[ω][k], k = c nm + ν, through a shared-memory transpose. Σ(ω ± ω_ν) comes from the columns' cell
 // records (cell_record above; the cells and distances from set-up), the reciprocal and the occupation products are
 // FP32: the kernel runs on the FP32 units only. A side of an element is 20 bytes and about 12 instructions (four
-// 16-byte gathers, two weights and two two-sums a side before: 54 -> KB1_US us at 1251 x 7425, 52 -> KB2_US us at 8
+// 16-byte gathers, two weights and two two-sums a side before: 54 -> 42.8 us at 1251 x 7425, 52 -> 42 us at 8
 // temperatures of 626 x 2184).
 // Grid (nω / 16, Kp / (kKbCols nm), slots), 256 threads: thread (node ω0 + t % 16, modes t / 16,
 // t / 16 + 16, ..) loads the cells and occupations of its (ω, ν) once and runs over the block's
@@ -165,7 +165,8 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, con
                                                           const float* __restrict__ F_all,
                                                           __nv_bfloat16* __restrict__ K0, __nv_bfloat16* __restrict__ K1,
                                                           __nv_bfloat16* __restrict__ K2, long Kp,
-                                                          const IterCtl* __restrict__ ctl = nullptr) {
+                                                          const IterCtl* __restrict__ ctl) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   extern __shared__ float kb_tile[];  // [kKbCols nm][kKbW + 1]
   __shared__ int s_col[kKbCols];
@@ -648,7 +649,7 @@ __global__ void mode_table_kernel(const double* __restrict__ wnu, int nm, const 
 // n + f(ω + ω_ν - μ), F[a][nω nm .. 2 nω nm) emission n + 1 - f(ω - ω_ν - μ). By detailed balance these are
 // (1 + n)(1 + E)/(1 + E e) and n (1 + E)/(1 + E/e) with E = exp((ω - μ)/T), e = exp(ω_ν/T) (both over E above μ): one
 // exponential a node and a dozen operations an element, in blocks of four nodes over all SMs (FP64 instructions issue
-// at one per 16 cycles and SM; two exponentials and divisions an element before: 501 x 15 6.5 -> OCC_US us). Also resets
+// at one per 16 cycles and SM; two exponentials and divisions an element before: 501 x 15 6.5 -> 5.3 us). Also resets
 // the iteration's max|ΔΣ|. Grid (nω / 4, slots).
 constexpr int kOccW = 4;
 __global__ void __launch_bounds__(64) occ_table_f32_kernel(const double* __restrict__ ws, int nw,
@@ -658,6 +659,7 @@ __global__ void __launch_bounds__(64) occ_table_f32_kernel(const double* __restr
                                                            float* __restrict__ F_all,
                                                            unsigned long long* __restrict__ errbits,
                                                            IterCtl* __restrict__ ctl) {
+  pdl_wait();
   __shared__ double s_p[kOccW], s_q[kOccW];
   const int a = blockIdx.y, t = slots[a];
   const int stop = ctl->stop_next;  // set by the iteration before, unchanged during this one's first kernels
@@ -703,6 +705,7 @@ __global__ void finalize_fm_batch_kernel(const float* __restrict__ part, int nw,
                                          long stride, double* __restrict__ ImS, __nv_bfloat16* __restrict__ Im0 = nullptr,
                                          __nv_bfloat16* __restrict__ Im1 = nullptr, __nv_bfloat16* __restrict__ Im2 = nullptr,
                                          long Kp2 = 0, const IterCtl* __restrict__ ctl = nullptr) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= slab) return;
@@ -731,7 +734,7 @@ __global__ void finalize_fm_batch_kernel(const float* __restrict__ part, int nw,
 // spectral functions' per-node terms P[i][j] = (ε_i - ω_j + ReΣ_j, ReΣ_{j+1} - ReΣ_j, ImΣ_j, ImΣ_{j+1})
 // (ImΣ_{j+1}, ReΣ_{j+1} = those of j at the last node). Everything but Σ itself and its change is formed on float pairs
 // (a single state's ReΣ is an FP32 sum): six instructions on the FP64 pipe a state and node, where about 25 bound the
-// kernel (1251 x 495: 26 -> KE1_US us, 8 x 626 x 168: 32 -> KE2_US us, with the next iteration's clamp, 10 us, included).
+// kernel (1251 x 495: 26 -> 24.3 us, 8 x 626 x 168: 32 -> 28.9 us, with the next iteration's clamp, 10 us, included).
 // Groups: CSR (gptr, gidx), members in order. Grid (nω / 255,
 // groups, slots), 256 threads: thread t takes node j = 255 blockIdx.x + t; the last thread's node
 // is the next block's first, formed again to give node 254 its neighbour.
@@ -746,6 +749,7 @@ __global__ void __launch_bounds__(256) kk_epilogue_kernel(const float* __restric
                                                           unsigned long long* __restrict__ errbits_all,
                                                           double* __restrict__ minA_all,
                                                           const IterCtl* __restrict__ ctl) {
+  pdl_wait();
   if (ctl && ctl->stop) return;
   __shared__ float4 sh[256];
   __shared__ uint32_t she[8];
@@ -1092,7 +1096,7 @@ void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS) {
   kbuild_bf16_kernel<<<dim3(div_up(size_t(nw), kKbW), unsigned(div_up(size_t(T->Kp), size_t(kKbCols * P->nm))), 1), 256,
                        kbuild_smem_bytes(P->nm), s>>>(int(nw), int(ni), T->rec.p, T->dim.p, nullptr, P->d_cell_j.p, T->tf.p,
                                                       T->skip.p, int(P->nm), T->ef.p, P->d_colc.p, int(P->nc), T->Ff.p,
-                                                      T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp);
+                                                      T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp, nullptr);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pk);
   const long slab = nw * ni;
@@ -1200,11 +1204,10 @@ void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, d
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pp);
   long pk = prof_begin(ctx, "kbuild");
-  kbuild_bf16_kernel<<<dim3(div_up(size_t(nw), kKbW), unsigned(div_up(size_t(T->Kp), size_t(kKbCols * P->nm))),
-                            unsigned(nA)),
-                       256, kbuild_smem_bytes(P->nm), s>>>(int(nw), int(ni), T->rec.p, T->dim.p, d_slots, P->d_cell_j.p, T->tf.p,
-                                                           T->skip.p, int(P->nm), T->ef.p, P->d_colc.p, int(P->nc), T->Ff.p,
-                                                           T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp, ctl);
+  launch_after(s, kbuild_bf16_kernel,
+               dim3(div_up(size_t(nw), kKbW), unsigned(div_up(size_t(T->Kp), size_t(kKbCols * P->nm))), unsigned(nA)), 256,
+               kbuild_smem_bytes(P->nm), int(nw), int(ni), T->rec.p, T->dim.p, d_slots, P->d_cell_j.p, T->tf.p, T->skip.p,
+               int(P->nm), T->ef.p, P->d_colc.p, int(P->nc), T->Ff.p, T->Kt[0].p, T->Kt[1].p, T->Kt[2].p, T->Kp, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pk);
   // ImΣ of every slot: the stacked K_t rows times G
@@ -1214,8 +1217,8 @@ void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, d
   // ImΣ of every slot, and its BF16 split as the B operand of ReΣ = KK ImΣ (columns: the slots'
   // states in order)
   long pf = prof_begin(ctx, "finalize");
-  finalize_fm_batch_kernel<<<dim3(eb, unsigned(nA)), 256, 0, s>>>(T->part.p, int(nw), slab, nA, sp, M * ni, T->ImS_b.p,
-                                                                   T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2, ctl);
+  launch_after(s, finalize_fm_batch_kernel, dim3(eb, unsigned(nA)), 256, 0, T->part.p, int(nw), slab, nA, sp, M * ni,
+               T->ImS_b.p, T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pf);
   tc_kk_tail(P, nA, d_slots, d_tp, d_S_all, d_P, d_errbits, d_minA, ctl);
@@ -1232,9 +1235,9 @@ static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, const TParams* 
   int sp2 = tc_gemm_launch(ctx, T->opKK, T->opIm, int(nw), int(N2), int(nw), T->part.p, nw, nw * N2,
                            max_splits_for(nw, kKbCapKK), T->err.p, "tc_kk", kKbCapKK, ctl ? &ctl->stop : nullptr);
   long pf = prof_begin(ctx, "kk_epilogue");
-  kk_epilogue_kernel<<<dim3(div_up(size_t(nw), 255), unsigned(P->ngroups), unsigned(nA)), 256, 0, s>>>(
-      T->part.p, sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_wtab.p, T->epair.p,
-      d_tp, d_S_all, T->Sf.p, T->rec.p, T->dim.p, d_P, d_errbits, d_minA, ctl);
+  launch_after(s, kk_epilogue_kernel, dim3(div_up(size_t(nw), 255), unsigned(P->ngroups), unsigned(nA)), 256, 0, T->part.p,
+               sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_wtab.p, T->epair.p, d_tp,
+               d_S_all, T->Sf.p, T->rec.p, T->dim.p, d_P, d_errbits, d_minA, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pf);
 }

@@ -142,8 +142,8 @@ static void launch_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B, int
   const int nN = (N + BN - 1) / BN, nM = (M + kTcBM - 1) / kTcBM;
   const int nitems = nN * nM * splits;  // (N tile, M tile, split)
   const int grid = std::min(nitems, ctx->sm_count);
-  kern<<<grid, 192, L::kBytes, ctx->stream>>>(maps, M, N, kblocks, per, nN, nM, nitems, out, ld_out, split_stride,
-                                              d_err, gm, skip);
+  launch_after(ctx->stream, kern, grid, 192, L::kBytes, maps, M, N, kblocks, per, nN, nM, nitems, out, ld_out, split_stride,
+               d_err, gm, skip);
   EPSP_LAUNCHED(ctx);
 }
 

@@ -355,7 +355,6 @@ __global__ void __launch_bounds__(192, 1)
   static_assert(!TF32 || NS == 1, "TF32 operands have one part");
   static_assert(NA == NS || (NA == 1 && NS == 3), "A has all parts, or one of three");
   static_assert(2 * BN <= 512, "two accumulators must fit TMEM");
-  const int nitems = skip && *skip ? 0 : nitems_;  // (skip: nothing is done or written)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * L::kStage);
@@ -395,6 +394,8 @@ __global__ void __launch_bounds__(192, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // (barriers and tensor memory are set up beside the kernel ahead)
+  const int nitems = skip && *skip ? 0 : nitems_;  // (skip: nothing is done or written)
 
   if (warp == 0 && lane == 0) {
     // producer

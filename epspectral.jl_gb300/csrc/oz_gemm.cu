@@ -279,12 +279,8 @@ __global__ void __launch_bounds__(320, 1)
         tc_fence_after();
         for (int kb = b0; kb < b1; ++kb) {
           const int st = g % STAGES;
-          if (!mbar_wait(full0 + 8 * st, (g / STAGES) & 1)) {
+          if (!mbar_wait_issuer(full0 + 8 * st, (g / STAGES) & 1, &s_abort)) {
             atomicExch(&s_abort, 1);
-            stop = true;
-            break;
-          }
-          if (aborted()) {
             stop = true;
             break;
           }

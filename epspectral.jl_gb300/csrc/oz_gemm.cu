@@ -333,13 +333,15 @@ __global__ void __launch_bounds__(320, 1)
         int* dst = sums + (long(o.seg * kOzOrders + o.d) * sh.N + o.nt * BN + half * kCols) * sh.M + row;
         const int nc = min(kCols, sh.N - o.nt * BN - half * kCols);
 #pragma unroll
-        for (int j = 0; j < kCols; ++j)
+        for (int j = 0; j < kCols; ++j) {
           if (j < nc) {
             if (o.alone)
-              dst[long(j) * sh.M] = int(acc[j]);
+              *dst = int(acc[j]);
             else
-              atomicAdd(dst + long(j) * sh.M, int(acc[j]));
+              atomicAdd(dst, int(acc[j]));
           }
+          dst += sh.M;
+        }
       }
     }
   }

@@ -55,10 +55,10 @@ struct LadderChunk {
   long k_off = 0;          // row offset of the chunk in B̃
 };
 
-// zgather_kernel's launch shape: U nodes per thread, nranges node ranges of U threads nodes each,
-// NC columns per block, staged rows of wstride float4s (the widest window + 4 zeros); smem bytes.
+// zgather_kernel's launch shape: nranges node ranges of 2 threads nodes each, NC columns per block,
+// staged rows of wstride float4s (the widest window + 4 zeros); smem bytes.
 struct ZgatherShape {
-  int U = 2, NC = 4, threads = 0, nranges = 1, wstride = 0;
+  int NC = 4, threads = 0, nranges = 1, wstride = 0;
   size_t smem = 0;
 };
 
@@ -691,14 +691,16 @@ __global__ void bz_build_kernel(const double* __restrict__ Gt, long Kx, int nmp,
   }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+// A copy of `bytes` (a multiple of 16, as both addresses are) into shared memory, counted on the mbarrier `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// zgather_kernel: the largest block (two blocks resident per SM, the accumulators in registers).
-constexpr int kZgMaxThreads = 320;
+// zgather_kernel: the largest block, and the blocks per SM that its registers and shared memory are sized for.
+constexpr int kZgMaxThreads = 128;
+constexpr int kZgBlocks = 4;
 
 // D from Z (the formula above), FP32, modes in ascending order, both signs and three taps each.
 // Z: [Mz, nm N] column-major (ld ldZ) as zsplits split-K partials zstride apart (summed in
@@ -708,16 +710,25 @@ constexpr int kZgMaxThreads = 320;
 // taps are p0, p0 + 1, p0 + 2); nnu_all 16 Bose occupations per right-hand side (rmap[z], or z).
 // D[z 24 nwp + (q + 6 (c0 + 2 ri)) nwp + j + ldD n], rows j < nω.
 // Grid (N / NC, 4 (c0, ri) x node ranges, slots), blockDim a multiple of 32 up to kZgMaxThreads: a
-// block owns NC columns n of one (c0, ri) and the U blockDim nodes of its range; per mode it stages
-// the window zwin[range][ν] (nodes [lo, hi): every node the range's taps read, as float4s) into
-// rows of wstride float4s by asynchronous copies, double-buffered over ν, and each thread
-// accumulates U nodes x NC columns, one shared-memory load per tap for the four components.
-template <int U, int NC>
-__global__ void __launch_bounds__(kZgMaxThreads, 2)
+// block owns NC columns n of one (c0, ri) and the 2 blockDim nodes of its range; per mode it stages
+// the window zwin[range][ν] (nodes [lo, hi): every node the range's taps read, as float4s) into rows of
+// wstride float4s and (NC > 1) its nodes' table entries, by bulk copies of whole rows, double-buffered over ν.
+// DRAM bounds it (1251 nodes x 1485 columns x 15 modes reads 1.87 GB, 300 us at copy rate) next to the taps'
+// shared-memory loads (250 us). With 16-byte copies by the threads, which pass through the pipe that the taps are read
+// by, and the entries read from L2 when they were needed, it took 560 us, 421 now; 625 nodes x 315 x 15 104 -> 62; 501 nodes x 315 x 15 with
+// 16 slots (2.45 GB) 817 -> 543. With four blocks of 128 threads an SM; three of 160 took 405 and 70 us of the
+// first two, two of 224 427 and 70. Neighbours in one thread, which share taps, need windows stored out of order for
+// loads without bank conflicts, and lost more by it (594 with copies by the threads).
+template <int NC>
+__global__ void __launch_bounds__(kZgMaxThreads, kZgBlocks)
     zgather_kernel(const float* __restrict__ Z, long ldZ, int zsplits, long zstride, const float4* __restrict__ ztab,
                    const int2* __restrict__ zwin, int wstride, const float* __restrict__ nnu_all,
-                   const int* __restrict__ rmap, int nw, int nwp, int nm, long N, float* __restrict__ D, long ldD) {
-  extern __shared__ __align__(16) float4 zs4[];  // [2][NC][wstride]
+                   const int* __restrict__ rmap, int nw, int nwp, int nm, long N, float* __restrict__ D, long ldD,
+                   int* __restrict__ err) {
+  constexpr int U = 2;
+  constexpr bool kTab = NC > 1;
+  extern __shared__ __align__(16) float4 zs4[];  // [2][NC][wstride]; with kTab the entries [2][U][2 signs][threads]
+  __shared__ uint64_t full_bar[2];
   const long n0 = long(blockIdx.x) * NC;
   const int c0 = blockIdx.y & 1, ri = (blockIdx.y >> 1) & 1, rg = int(blockIdx.y >> 2);
   const long z = blockIdx.z;
@@ -726,26 +737,44 @@ __global__ void __launch_bounds__(kZgMaxThreads, 2)
   const float* zb = Z + z * 16 * nwp + long(ri * 2 + c0) * 4 * nwp;  // the nodes' float4s, contiguous
   const int nthr = blockDim.x;
   const int jb = rg * U * nthr;  // the range's first node
+  float4* ts4 = zs4 + 2 * NC * wstride;
+  const uint32_t full0 = smem_u32(full_bar);
+  const int ncol = int(min(long(NC), N - n0));
+  const bool bulk = zsplits == 1;
+  if (threadIdx.x == 0) {
+    mbar_init(full0, 1);
+    mbar_init(full0 + 8, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
   auto stage = [&](int nu, int buf, int2 win) {
     const int nn = win.y - win.x;  // nodes staged
-    for (int c = 0; c < NC; ++c) {
-      const long n = n0 + c;
-      if (n >= N) break;
-      float4* dst = zs4 + long(buf * NC + c) * wstride;
+    float4* dst = zs4 + long(buf * NC) * wstride;
+    if (win.y == nwp && int(threadIdx.x) < 4 * ncol) {
       // zeros after the staged nodes: a tap past the grid's last padded node (weight zero) reads them
-      if (threadIdx.x < 4) dst[nn + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float* src = zb + ldZ * (long(nu) * N + n) + 4l * win.x;
-      if (zsplits == 1) {
-        for (int e = threadIdx.x; e < nn; e += nthr) cp_async16(dst + e, src + 4l * e);
-      } else {  // split-K partials: summed here in ascending order (synchronous loads)
+      dst[long(threadIdx.x / 4) * wstride + nn + threadIdx.x % 4] = make_float4(0.f, 0.f, 0.f, 0.f);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (a later bulk copy may write there)
+    }
+    const float* src = zb + ldZ * (long(nu) * N + n0) + 4l * win.x;
+    if (!bulk)  // split-K partials: summed here in ascending order (synchronous loads)
+      for (int c = 0; c < ncol; ++c)
         for (int e = threadIdx.x; e < 4 * nn; e += nthr) {
           float acc = 0.f;
-          for (int sp = 0; sp < zsplits; ++sp) acc += src[e + zstride * sp];
-          reinterpret_cast<float*>(dst)[e] = acc;
+          for (int sp = 0; sp < zsplits; ++sp) acc += src[ldZ * c + e + zstride * sp];
+          reinterpret_cast<float*>(dst + long(c) * wstride)[e] = acc;
         }
-      }
+    if (threadIdx.x < 32) {  // lane c: column c; with kTab lanes 4 + 2u + sign: entries
+      const int lane = threadIdx.x, u = (lane - 4) / 2;
+      const int bytes_col = bulk ? 16 * nn : 0;
+      auto entries = [&](int u) { return max(0, min(nthr, nwp - jb - u * nthr)); };
+      const uint32_t bar = full0 + 8 * buf;
+      if (lane == 0) mbar_expect_tx(bar, uint32_t(ncol * bytes_col + (kTab ? 32 * (entries(0) + entries(1)) : 0)));
+      __syncwarp();
+      if (lane < ncol && bytes_col > 0) bulk_load(smem_u32(dst + long(lane) * wstride), src + ldZ * lane, uint32_t(bytes_col), bar);
+      if (kTab && lane >= 4 && lane < 8 && entries(u) > 0)
+        bulk_load(smem_u32(ts4 + long((buf * U + u) * 2 + lane % 2) * nthr),
+                  ztab + (long(nu) * 2 + lane % 2) * nwp + jb + u * nthr, uint32_t(16 * entries(u)), bar);
     }
-    cp_async_commit();
   };
   float acc[NC][U][6];
 #pragma unroll
@@ -761,33 +790,32 @@ __global__ void __launch_bounds__(kZgMaxThreads, 2)
     const float nb = nnu[nu];
     const float hp = 0.5f + nb;
     const int2 win_next = win_rg[nu + 1 < nm ? nu + 1 : nu];  // loaded before the wait
-    cp_async_wait_all();
-    __syncthreads();  // mode nu's columns are in buffer nu & 1; buffer (nu + 1) & 1 is free
+    // mode nu's columns are in buffer nu & 1; buffer (nu + 1) & 1 is free
+    if (!__syncthreads_and(mbar_wait(full0 + 8 * (nu & 1), (nu >> 1) & 1))) {
+      mbar_wait(full0 + 8 * (nu & 1), (nu >> 1) & 1);  // (bounded: no copy is in flight when the block leaves)
+      if (threadIdx.x == 0) atomicExch(err, 1);
+      return;
+    }
     if (nu + 1 < nm) stage(nu + 1, (nu + 1) & 1, win_next);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int j = jb + threadIdx.x + nthr * u;
       if (j >= nw) continue;
-      float4 t[2];
-      int pk[2];
-#pragma unroll
-      for (int sg = 0; sg < 2; ++sg) {
-        t[sg] = ztab[(long(nu) * 2 + sg) * nwp + j];
-        pk[sg] = __float_as_int(t[sg].w) - win.x;
-      }
       // per sign s: the factors of components c12 = 0 (11, .x), 1 (21, .y), 2 (12, .z), 3 (22, .w)
       // in the six rows q (sign + : 1/2, -(1/2 + n), n, 1 + n; sign - : -1/2, -(1/2 + n), 1 + n, n)
 #pragma unroll
       for (int sg = 0; sg < 2; ++sg) {
         const float half = sg ? -0.5f : 0.5f, fy = sg ? 1.f + nb : nb, fz = sg ? nb : 1.f + nb;
+        const float4 t = kTab ? ts4[long(((nu & 1) * U + u) * 2 + sg) * nthr + threadIdx.x]
+                              : ztab[(long(nu) * 2 + sg) * nwp + j];
+        const float4* zc = zs4 + long((nu & 1) * NC) * wstride + (__float_as_int(t.w) - win.x);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const float4* zc = zs4 + long((nu & 1) * NC + c) * wstride + pk[sg];
+        for (int c = 0; c < NC; ++c, zc += wstride) {
           const float4 r0 = zc[0], r1 = zc[1], r2 = zc[2];
-          const float xx = t[sg].x * r0.x + t[sg].y * r1.x + t[sg].z * r2.x;
-          const float xy = t[sg].x * r0.y + t[sg].y * r1.y + t[sg].z * r2.y;
-          const float xz = t[sg].x * r0.z + t[sg].y * r1.z + t[sg].z * r2.z;
-          const float xw = t[sg].x * r0.w + t[sg].y * r1.w + t[sg].z * r2.w;
+          const float xx = t.x * r0.x + t.y * r1.x + t.z * r2.x;
+          const float xy = t.x * r0.y + t.y * r1.y + t.z * r2.y;
+          const float xz = t.x * r0.z + t.y * r1.z + t.z * r2.z;
+          const float xw = t.x * r0.w + t.y * r1.w + t.z * r2.w;
           acc[c][u][0] += half * xx;
           acc[c][u][1] += -hp * xx;
           acc[c][u][2] += half * xw;
@@ -817,22 +845,22 @@ __global__ void __launch_bounds__(kZgMaxThreads, 2)
 constexpr int kZGroupM = 8;
 
 // Threads and ranges for nω nodes (the windows, and with them NC and the staging, follow).
-static ZgatherShape zgather_ranges(long nw, int U) {
+static ZgatherShape zgather_ranges(long nw) {
   ZgatherShape g;
-  g.U = U;
-  const long nthr = (nw + U - 1) / U;  // threads for all nodes in one block
+  const long nthr = (nw + 1) / 2;  // threads for all nodes in one block
   g.nranges = int((nthr + kZgMaxThreads - 1) / kZgMaxThreads);
   g.threads = int(((nthr + g.nranges - 1) / g.nranges + 31) / 32 * 32);
   return g;
 }
+
 // The staging windows of zgather_kernel: for each node range and mode, the nodes [lo, hi) that
 // hold every tap p0 .. p0 + 2 of the range's nodes (both signs), from the first-tap table hk
 // [nm][2][nwp]; taps past nwp read the zeros staged after the window. Sets g.wstride (the widest
-// window + 4, float4s), g.NC (4 while two double-buffered blocks fit an SM, else 2, else 1) and
-// g.smem.
+// window + 4, float4s), g.NC (4 while two double-buffered blocks fit an SM, else 2, else 1: only the widest
+// windows come to that, and they leave the table entries where they are) and g.smem.
 static std::vector<int32_t> zgather_windows(ZgatherShape& g, const std::vector<int32_t>& hk, long nw, long nwp, long nm) {
   std::vector<int32_t> win(size_t(2 * g.nranges * nm));
-  const long span = long(g.U) * g.threads;
+  const long span = 2l * g.threads;
   long maxn = 1;
   for (long r = 0; r < g.nranges; ++r)
     for (long nu = 0; nu < nm; ++nu) {
@@ -852,35 +880,37 @@ static std::vector<int32_t> zgather_windows(ZgatherShape& g, const std::vector<i
     }
   g.wstride = int(maxn + 4);
   const size_t per_col = size_t(2 * g.wstride) * sizeof(float4);  // two buffers
-  g.NC = per_col * 4 <= (size_t(110) << 10) ? 4 : per_col * 2 <= (size_t(110) << 10) ? 2 : 1;
-  g.smem = per_col * size_t(g.NC);
+  const size_t tab = size_t(8 * g.threads) * sizeof(float4);
+  const size_t two = size_t(112) << 10;  // shared memory of one of two blocks
+  g.NC = per_col * 4 + tab <= two ? 4 : per_col * 2 + tab <= two ? 2 : 1;
+  g.smem = per_col * size_t(g.NC) + (g.NC > 1 ? tab : 0);
   if (g.smem > (size_t(227) << 10))
     fail(EPSP_EUNSUPPORTED, "the ladder's interpolation windows do not fit shared memory (grid too fine for its modes)");
   return win;
 }
-template <int U, int NC>
+template <int NC>
 static void launch_zgather_t(const ZgatherShape& g, dim3 grid, cudaStream_t s, const float* Z, long ldZ, int zsplits,
                              long zstride, const float4* ztab, const int2* zwin, const float* nnu, const int* rmap, int nw,
-                             int nwp, int nm, long N, float* D, long ldD) {
+                             int nwp, int nm, long N, float* D, long ldD, int* err) {
   static size_t smem_set = 0;  // the largest dynamic shared memory allowed so far
   if (g.smem > smem_set) {
-    EPSP_CUDA(cudaFuncSetAttribute(zgather_kernel<U, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
+    EPSP_CUDA(cudaFuncSetAttribute(zgather_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
     smem_set = g.smem;
   }
-  zgather_kernel<U, NC><<<grid, g.threads, g.smem, s>>>(Z, ldZ, zsplits, zstride, ztab, zwin, g.wstride, nnu, rmap, nw,
-                                                        nwp, nm, N, D, ldD);
+  zgather_kernel<NC><<<grid, g.threads, g.smem, s>>>(Z, ldZ, zsplits, zstride, ztab, zwin, g.wstride, nnu, rmap, nw,
+                                                     nwp, nm, N, D, ldD, err);
 }
 // Grid (N / NC, 4 x node ranges, slots).
 static void launch_zgather(const ZgatherShape& g, long N, unsigned slots, cudaStream_t s, const float* Z, long ldZ,
                            int zsplits, long zstride, const float4* ztab, const int2* zwin, const float* nnu,
-                           const int* rmap, int nw, int nwp, int nm, float* D, long ldD) {
+                           const int* rmap, int nw, int nwp, int nm, float* D, long ldD, int* err) {
   const dim3 grid(unsigned((N + g.NC - 1) / g.NC), 4u * unsigned(g.nranges), slots);
   if (g.NC == 4)
-    launch_zgather_t<2, 4>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD);
+    launch_zgather_t<4>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD, err);
   else if (g.NC == 2)
-    launch_zgather_t<2, 2>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD);
+    launch_zgather_t<2>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD, err);
   else
-    launch_zgather_t<2, 1>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD);
+    launch_zgather_t<1>(g, grid, s, Z, ldZ, zsplits, zstride, ztab, zwin, nnu, rmap, nw, nwp, nm, N, D, ldD, err);
 }
 
 // Y (rows q = 0, 2 of D) as the BF16 hi/lo B operand of the Kramers-Kronig GEMM: row (qq, c0, ri, n),
@@ -1775,7 +1805,7 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
           std::memcpy(&hf[4 * e + 3], &hk[e], sizeof(int32_t));
         }
         P->d_ztab = to_device(ctx, hf);
-        P->zg = zgather_ranges(nw, 2);
+        P->zg = zgather_ranges(nw);
         P->d_zwin = to_device(ctx, zgather_windows(P->zg, hk, nw, P->nwp, nm));
         EPSP_CUDA(cudaStreamSynchronize(s));  // hf is a local
       }
@@ -2052,7 +2082,7 @@ static void apply_L(LadderPlan* P, const float2* J, float2* LJ, const float2* X 
   long pz = prof_begin(ctx, "zgather");
   launch_zgather(P->zg, N, 1, s, P->d_Z.p, P->Mz, sp, P->Mz * P->Nz, reinterpret_cast<const float4*>(P->d_ztab.p),
                  reinterpret_cast<const int2*>(P->d_zwin.p), P->d_nnu_f.p, nullptr, int(nw), int(nwp), int(P->nm),
-                 P->d_Dz.p, M);
+                 P->d_Dz.p, M, P->d_err.p);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pz);
   long pl = prof_begin(ctx, "lsum");
@@ -2565,7 +2595,8 @@ static void apply_L_batch(LadderPlan* P, LadderBatch& B, const float2* X, int nA
   tc_gemm_launch_with(ctx, B.opA, P->opG, P->bn, 1, int(Mzt), int(P->Nz), int(P->Kz), B.Z.p, Mzt, Mzt * P->Nz,
                       P->d_err.p, "tc_ladder", P->persist, P->pair, P->gm);
   launch_zgather(P->zg, N, unsigned(nA), s, B.Z.p, Mzt, 1, long(0), reinterpret_cast<const float4*>(P->d_ztab.p),
-                 reinterpret_cast<const int2*>(P->d_zwin.p), B.nnu.p, B.rmap.p, int(nw), int(nwp), int(P->nm), B.D.p, Mt);
+                 reinterpret_cast<const int2*>(P->d_zwin.p), B.nnu.p, B.rmap.p, int(nw), int(nwp), int(P->nm), B.D.p, Mt,
+                 P->d_err.p);
   EPSP_LAUNCHED(ctx);
   y_split_kernel<<<dim3(div_up(size_t(P->Kp2), 256), unsigned(N), unsigned(nA)), 256, 0, s>>>(
       B.D.p, Mt, 1, 0, int(nw), int(nwp), N, P->Kp2, B.Yh.p, B.Yl.p);

@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(128, 1)
 // Per tile the MMAs run in the one-tile kernel's order, so the results are bitwise the same.
 // Where K is short the epilogue is the bound, a column of it a pointer step and a 128-byte store a warp (a 64-bit
 // product and a comparison a column before: TF32 131072 x 4725 x 315 1130 -> 627 us, 2.4 GB of it written; BF16x3
-// 8192 x 4860 x 540 101 -> 71; 32 training steps with their copies 5.48 -> 4.42 ms). Eight epilogue warps instead of four
+// 10240 x 4725 x 315 101 -> 71; 32 training steps with their copies 5.48 -> 4.42 ms). Eight epilogue warps instead of four
 // gave nothing more (633, 72).
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");

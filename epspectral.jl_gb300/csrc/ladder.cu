@@ -278,6 +278,7 @@ __global__ void propagators_kernel(const double2* __restrict__ ST, const double*
 template <class V>
 __global__ void attach_bare_kernel(const V* __restrict__ Gm_all, const V* __restrict__ Gp_all,
                                    const double* __restrict__ v, int nw, int ni, V* __restrict__ J0_all) {
+  pdl_wait();
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
   const int c12 = blockIdx.z % 4, rest = blockIdx.y;
@@ -306,6 +307,7 @@ __global__ void attach_bare_kernel(const V* __restrict__ Gm_all, const V* __rest
 template <class V>
 __global__ void __launch_bounds__(256) cond_sum_kernel(const V* __restrict__ J_all, const double* __restrict__ Ww, int nw,
                                                        int ni, double2* __restrict__ Y_all) {
+  pdl_wait();
   __shared__ double sr[256], si[256];
   const long z = blockIdx.y;
   const V* J = J_all + z * 24l * nw * ni;
@@ -343,6 +345,7 @@ __global__ void __launch_bounds__(256) prep_vertex_f32_kernel(const double2* __r
                                                               const double* __restrict__ Ww, int ni, float2* __restrict__ Gm,
                                                               float2* __restrict__ Gp, float2* __restrict__ J0,
                                                               double2* __restrict__ Y, double2* __restrict__ part) {
+  pdl_wait();
   __shared__ double sr[256], si[256];
   const int i = blockIdx.x;
   const double2* col = ST + long(nw) * i;
@@ -639,6 +642,7 @@ template <bool kTf32>
 __global__ void __launch_bounds__(256) jmat_kernel(const float2* __restrict__ J_all, long jstride, const int* __restrict__ rmap,
                                                    int nw, int nwp, int ni, long Kzp, float* __restrict__ Jt,
                                                    __nv_bfloat16* __restrict__ Jh, __nv_bfloat16* __restrict__ Jl) {
+  pdl_wait();
   __shared__ float2 tile[32][33];
   const int k0 = blockIdx.x * 32, p0 = blockIdx.y * 32;
   const int comp = blockIdx.z % 8, z = blockIdx.z / 8;
@@ -725,6 +729,7 @@ __global__ void __launch_bounds__(kZgMaxThreads, kZgBlocks)
                    const int2* __restrict__ zwin, int wstride, const float* __restrict__ nnu_all,
                    const int* __restrict__ rmap, int nw, int nwp, int nm, long N, float* __restrict__ D, long ldD,
                    int* __restrict__ err) {
+  pdl_wait();
   constexpr int U = 2;
   constexpr bool kTab = NC > 1;
   extern __shared__ __align__(16) float4 zs4[];  // [2][NC][wstride]; with kTab the entries [2][U][2 signs][threads]
@@ -897,7 +902,7 @@ static void launch_zgather_t(const ZgatherShape& g, dim3 grid, cudaStream_t s, c
     EPSP_CUDA(cudaFuncSetAttribute(zgather_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
     smem_set = g.smem;
   }
-  zgather_kernel<NC><<<grid, g.threads, g.smem, s>>>(Z, ldZ, zsplits, zstride, ztab, zwin, g.wstride, nnu, rmap, nw,
+  launch_after(s, zgather_kernel<NC>, grid, g.threads, g.smem, Z, ldZ, zsplits, zstride, ztab, zwin, g.wstride, nnu, rmap, nw,
                                                      nwp, nm, N, D, ldD, err);
 }
 // Grid (N / NC, 4 x node ranges, slots).
@@ -922,6 +927,7 @@ static void launch_zgather(const ZgatherShape& g, long N, unsigned slots, cudaSt
 // the 8 rows (qq, c0, ri, n).
 __global__ void y_split_kernel(const float* __restrict__ D, long ldD, int dsplits, long dstride, int nw, int nwp, long N,
                                long Kp2, __nv_bfloat16* __restrict__ Yh, __nv_bfloat16* __restrict__ Yl) {
+  pdl_wait();
   const long w = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (w >= Kp2) return;
   const long n = blockIdx.y, z = blockIdx.z;
@@ -983,6 +989,7 @@ __global__ void finish_gemm_kernel(const R* __restrict__ D_all, long ldD, int ds
                                    const Vec2<R>* __restrict__ Gm_all, const Vec2<R>* __restrict__ Gp_all,
                                    const int* __restrict__ rmap, int nw, int nwp, int ni, Vec2<R>* __restrict__ LJ_all,
                                    const Vec2<R>* __restrict__ X_all = nullptr) {
+  pdl_wait();
   using V = Vec2<R>;
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
@@ -1076,6 +1083,7 @@ __device__ __forceinline__ long slot_rhs(const int* rmap) {
 template <class V>
 __global__ void __launch_bounds__(256) dot_partial_kernel(const V* __restrict__ U, const V* __restrict__ Vv, long n,
                                                           const int* __restrict__ rmap, double2* __restrict__ part) {
+  pdl_wait();
   __shared__ double sr[256], si[256];
   const long r = slot_rhs<V>(rmap);
   const V* u = U + n * r;
@@ -1124,6 +1132,7 @@ __global__ void __launch_bounds__(256) dot_partial_kernel(const V* __restrict__ 
 // out[rmap[z]] (out[z] without rmap) = Σ_b part[z][b] in order; one block per slot.
 __global__ void __launch_bounds__(256) dot_final_kernel(const double2* __restrict__ part, int np, const int* __restrict__ rmap,
                                                         double2* __restrict__ out) {
+  pdl_wait();
   __shared__ double sr[256], si[256];
   double ar = 0, ai = 0;
   for (int k = threadIdx.x; k < np; k += 256) {
@@ -1143,18 +1152,120 @@ __global__ void __launch_bounds__(256) dot_final_kernel(const double2* __restric
   if (threadIdx.x == 0) out[rmap ? rmap[blockIdx.x] : int(blockIdx.x)] = make_double2(sr[0], si[0]);
 }
 
-// Q[r] -= h[r] V[r] with h from device memory (one coefficient per right-hand side).
+// Elements of a thread of axpby_kernel, scale_kernel and combine_kernel, 256 apart, their loads issued together (grids
+// of n / (256 kVecPer) blocks).
+constexpr int kVecPer = 4;
+
+// Q[r] -= h[r] X[r] with h from device memory (one coefficient per right-hand side), and in the same pass the block
+// partials of conj(U[r]) Q[r] (of |Q[r]|^2 without U) of the result, in dot_partial_kernel's order: a vector less is
+// read than by two kernels (16 vectors of 1.26M: 82 and 63 us -> 96). Grid (blocks, slots), as dot_partial_kernel's.
 template <class V>
-__global__ void axpy_dev_kernel(V* __restrict__ Q, const V* __restrict__ X, const double2* __restrict__ h, long n,
-                                const int* __restrict__ rmap) {
+__global__ void __launch_bounds__(256) axpy_dot_kernel(V* __restrict__ Q, const V* __restrict__ X, const double2* __restrict__ h,
+                                                       const V* __restrict__ U, long n, const int* __restrict__ rmap,
+                                                       double2* __restrict__ part) {
+  pdl_wait();
   using R = typename VecOf<V>::R;
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+  __shared__ double sr[256], si[256];
   const long r = slot_rhs<V>(rmap);
   const double2 hd = h[r];
   const R hx = R(hd.x), hy = R(hd.y);
-  const V x = X[n * r + k], q = Q[n * r + k];
-  Q[n * r + k] = VecOf<V>::make(q.x - (hx * x.x - hy * x.y), q.y - (hx * x.y + hy * x.x));
+  V* q = Q + n * r;
+  const V* x = X + n * r;
+  const V* u = U ? U + n * r : nullptr;
+  double ar = 0, ai = 0;
+  const long stride = long(gridDim.x) * 256;
+  constexpr int kHalf = kRun / 2;  // elements whose loads are issued together
+  for (long k0 = long(blockIdx.x) * 256 + threadIdx.x; k0 < n; k0 += stride * kRun) {
+    R fr = 0, fi = 0;
+#pragma unroll
+    for (int g = 0; g < kRun; g += kHalf) {
+      V a[kHalf], b[kHalf], c[kHalf];
+#pragma unroll
+      for (int e = 0; e < kHalf; ++e) {
+        const long k = k0 + stride * (g + e);
+        a[e] = k < n ? q[k] : VecOf<V>::make(0, 0);
+        b[e] = k < n ? x[k] : VecOf<V>::make(0, 0);
+        if (u) c[e] = k < n ? u[k] : VecOf<V>::make(0, 0);
+      }
+#pragma unroll
+      for (int e = 0; e < kHalf; ++e) {
+        const long k = k0 + stride * (g + e);
+        const V w = VecOf<V>::make(a[e].x - (hx * b[e].x - hy * b[e].y), a[e].y - (hx * b[e].y + hy * b[e].x));
+        if (k < n) {
+          q[k] = w;
+          const V v = u ? c[e] : w;
+          fr += v.x * w.x + v.y * w.y;  // conj(v) w
+          fi += v.x * w.y - v.y * w.x;
+        }
+      }
+    }
+    ar += fr;
+    ai += fi;
+  }
+  sr[threadIdx.x] = ar;
+  si[threadIdx.x] = ai;
+  __syncthreads();
+  for (int st = 128; st > 0; st >>= 1) {
+    if (threadIdx.x < st) {
+      sr[threadIdx.x] += sr[threadIdx.x + st];
+      si[threadIdx.x] += si[threadIdx.x + st];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) part[long(blockIdx.y) * gridDim.x + blockIdx.x] = make_double2(sr[0], si[0]);
+}
+
+// J[r] = Σ_t y_t X_t[r] over t < m (ascending), or J[r] += with `add`: one pass over J for kCombine vectors (a pass per
+// vector before: 16 x 2 vectors of 1.26M 265 us -> 103). The coefficients are y[r + ystride t] from device memory, or
+// the launch's own; vector t enters right-hand side r only where i0 + t < count[r] (all do without count). A block
+// rounds its coefficients once: every thread doing so, on the FP64 pipe (one instruction a warp in 16 cycles), was most
+// of the kernels of this family (axpby 132 us of 16 vectors, this one 577).
+constexpr int kCombine = 8;
+template <class V>
+struct CombineArgs {
+  const V* x[kCombine];
+  double2 y[kCombine];
+};
+template <class V>
+__global__ void __launch_bounds__(256) combine_kernel(const __grid_constant__ CombineArgs<V> A, int m, int i0,
+                                                      const double2* __restrict__ y, long ystride,
+                                                      const int* __restrict__ count, bool add, V* __restrict__ J, long n) {
+  pdl_wait();
+  using R = typename VecOf<V>::R;
+  __shared__ V c[kCombine];
+  const long r = blockIdx.y;
+  if (count) m = min(m, count[r] - i0);
+  if (int(threadIdx.x) < m) {
+    const double2 yt = y ? y[r + ystride * threadIdx.x] : A.y[threadIdx.x];
+    c[threadIdx.x] = VecOf<V>::make(R(yt.x), R(yt.y));
+  }
+  __syncthreads();
+  constexpr int kE = 2;
+#pragma unroll
+  for (int g = 0; g < kVecPer; g += kE) {
+    const long k0 = long(blockIdx.x) * (256 * kVecPer) + 256 * g + threadIdx.x;
+    V a[kE], x[kCombine][kE];
+#pragma unroll
+    for (int e = 0; e < kE; ++e) a[e] = add && k0 + 256 * e < n ? J[n * r + k0 + 256 * e] : VecOf<V>::make(0, 0);
+#pragma unroll
+    for (int q = 0; q < kCombine; ++q)
+      if (q < m) {
+#pragma unroll
+        for (int e = 0; e < kE; ++e)
+          if (k0 + 256 * e < n) x[q][e] = A.x[q][n * r + k0 + 256 * e];
+      }
+#pragma unroll
+    for (int q = 0; q < kCombine; ++q)
+      if (q < m) {
+        const V ct = c[q];
+#pragma unroll
+        for (int e = 0; e < kE; ++e)
+          a[e] = VecOf<V>::make(ct.x * x[q][e].x - ct.y * x[q][e].y + a[e].x, ct.x * x[q][e].y + ct.y * x[q][e].x + a[e].y);
+      }
+#pragma unroll
+    for (int e = 0; e < kE; ++e)
+      if (k0 + 256 * e < n) J[n * r + k0 + 256 * e] = a[e];
+  }
 }
 
 // Y[r] = a X[r] + b Y[r]: complex a, b from the host (a_dev, b_dev null) or per right-hand side
@@ -1162,29 +1273,55 @@ __global__ void axpy_dev_kernel(V* __restrict__ Q, const V* __restrict__ X, cons
 template <class V>
 __global__ void axpby_kernel(double2 a, const double2* __restrict__ a_dev, const V* __restrict__ X, double2 b,
                              const double2* __restrict__ b_dev, V* __restrict__ Y, long n, const int* __restrict__ rmap) {
+  pdl_wait();
   using R = typename VecOf<V>::R;
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+  __shared__ R c[4];
   const long r = slot_rhs<V>(rmap);
-  if (a_dev) a = a_dev[r];
-  if (b_dev) b = b_dev[r];
-  const R ax = R(a.x), ay = R(a.y), bx = R(b.x), by = R(b.y);
-  const V xv = X[n * r + k], yv = Y[n * r + k];
-  Y[n * r + k] = VecOf<V>::make(ax * xv.x - ay * xv.y + bx * yv.x - by * yv.y, ax * xv.y + ay * xv.x + bx * yv.y + by * yv.x);
+  if (threadIdx.x == 0) {  // (rounded once a block, as in combine_kernel)
+    if (a_dev) a = a_dev[r];
+    if (b_dev) b = b_dev[r];
+    c[0] = R(a.x), c[1] = R(a.y), c[2] = R(b.x), c[3] = R(b.y);
+  }
+  __syncthreads();
+  const R ax = c[0], ay = c[1], bx = c[2], by = c[3];
+  const long k0 = long(blockIdx.x) * (256 * kVecPer) + threadIdx.x;
+  V xv[kVecPer], yv[kVecPer];
+#pragma unroll
+  for (int e = 0; e < kVecPer; ++e)
+    if (k0 + 256 * e < n) {
+      xv[e] = X[n * r + k0 + 256 * e];
+      yv[e] = Y[n * r + k0 + 256 * e];
+    }
+#pragma unroll
+  for (int e = 0; e < kVecPer; ++e)
+    if (k0 + 256 * e < n)
+      Y[n * r + k0 + 256 * e] = VecOf<V>::make(ax * xv[e].x - ay * xv[e].y + bx * yv[e].x - by * yv[e].y,
+                                               ax * xv[e].y + ay * xv[e].x + bx * yv[e].y + by * yv[e].x);
 }
 
 // Y[r] = a X[r] (Y is not read); a from the host or per right-hand side from device memory.
 template <class V>
 __global__ void scale_kernel(double2 a, const double2* __restrict__ a_dev, const V* __restrict__ X, V* __restrict__ Y, long n,
                              const int* __restrict__ rmap) {
+  pdl_wait();
   using R = typename VecOf<V>::R;
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+  __shared__ R c[2];
   const long r = slot_rhs<V>(rmap);
-  if (a_dev) a = a_dev[r];
-  const R ax = R(a.x), ay = R(a.y);
-  const V xv = X[n * r + k];
-  Y[n * r + k] = VecOf<V>::make(ax * xv.x - ay * xv.y, ax * xv.y + ay * xv.x);
+  if (threadIdx.x == 0) {  // (rounded once a block, as in combine_kernel)
+    if (a_dev) a = a_dev[r];
+    c[0] = R(a.x), c[1] = R(a.y);
+  }
+  __syncthreads();
+  const R ax = c[0], ay = c[1];
+  const long k0 = long(blockIdx.x) * (256 * kVecPer) + threadIdx.x;
+  V xv[kVecPer];
+#pragma unroll
+  for (int e = 0; e < kVecPer; ++e)
+    if (k0 + 256 * e < n) xv[e] = X[n * r + k0 + 256 * e];
+#pragma unroll
+  for (int e = 0; e < kVecPer; ++e)
+    if (k0 + 256 * e < n)
+      Y[n * r + k0 + 256 * e] = VecOf<V>::make(ax * xv[e].x - ay * xv[e].y, ax * xv[e].y + ay * xv[e].x);
 }
 
 // q -= h v (h from device memory) and the block partials of |q|^2 of the result, in the order of
@@ -1265,6 +1402,7 @@ constexpr int kMG = 8;
 template <class V>
 __global__ void __launch_bounds__(256) mdot_partial_kernel(V* const* __restrict__ vp, int i0, int m, const V* __restrict__ w,
                                                            long n, double2* __restrict__ part) {
+  pdl_wait();
   __shared__ double sr[256], si[256];
   double ar[kMG], ai[kMG];
   const V* vt[kMG];  // the m vectors' pointers, read once
@@ -1328,11 +1466,12 @@ __global__ void __launch_bounds__(256) mdot_partial_kernel(V* const* __restrict_
   }
 }
 
-// w -= Σ_{t < m} h[i0 + t] V_{i0 + t} (ascending t, in the arithmetic of axpy_dev_kernel); with part,
+// w -= Σ_{t < m} h[i0 + t] V_{i0 + t} (ascending t, in the arithmetic of axpy_dot_kernel); with part,
 // also the block partials of |w|^2 of the result.
 template <class V>
 __global__ void __launch_bounds__(256) maxpy_kernel(V* __restrict__ w, V* const* __restrict__ vp, int i0, int m,
                                                     const double2* __restrict__ h, long n, double2* __restrict__ part) {
+  pdl_wait();
   using R = typename VecOf<V>::R;
   __shared__ double sr[256];
   R hx[kMG], hy[kMG];
@@ -1389,6 +1528,7 @@ __global__ void gmres_givens_kernel(const double2* __restrict__ h1, const double
                                     const double2* __restrict__ beta_sq, double rtol, double btol, int inner,
                                     double2* __restrict__ Rp, double* __restrict__ cs, double2* __restrict__ sn,
                                     double2* __restrict__ zv, GmresDev* __restrict__ st, double2* __restrict__ inv_out) {
+  pdl_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   using C = cuda_cplx;
   if (inner == 1) {
@@ -2047,7 +2187,7 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   y_gemm_kernel<<<div_up(size_t(ny), 256), 256, 0, s>>>(P->d_D.p, int(nw), int(nwp), N, P->d_Y.p);
   EPSP_LAUNCHED(ctx);
   oz_gemm(ctx, P->oz, nw, 8 * N, nw, P->d_KK.p, nw, &P->ozKK, P->d_Y.p, nw, nullptr, 0.0, P->d_KY.p, nw);
-  finish_gemm_kernel<double><<<dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, s>>>(
+  launch_after(s, finish_gemm_kernel<double>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, 
       P->d_D.p, M, 1, 0, P->d_KY.p, 1, 0, P->d_Gm.p, P->d_Gp.p, nullptr, int(nw), int(nwp), int(ni), LJ, X);
   EPSP_LAUNCHED(ctx);
 }
@@ -2058,10 +2198,10 @@ static void launch_jmat(LadderPlan* P, const float2* J, long jstride, const int*
   Ctx* ctx = P->ctx;
   const dim3 grid(unsigned(P->Kzp / 32), unsigned(P->nwp / 32), unsigned(8 * nA));
   if (P->path == EPSP_PATH_GEMM_TF32)
-    jmat_kernel<true><<<grid, 256, 0, ctx->stream>>>(J, jstride, rmap, int(P->nw), int(P->nwp), int(P->ni), P->Kzp, Jt,
+    launch_after(ctx->stream, jmat_kernel<true>, grid, 256, 0, J, jstride, rmap, int(P->nw), int(P->nwp), int(P->ni), P->Kzp, Jt,
                                                      nullptr, nullptr);
   else
-    jmat_kernel<false><<<grid, 256, 0, ctx->stream>>>(J, jstride, rmap, int(P->nw), int(P->nwp), int(P->ni), P->Kzp,
+    launch_after(ctx->stream, jmat_kernel<false>, grid, 256, 0, J, jstride, rmap, int(P->nw), int(P->nwp), int(P->ni), P->Kzp,
                                                       nullptr, Jh, Jl);
   EPSP_LAUNCHED(ctx);
 }
@@ -2086,14 +2226,14 @@ static void apply_L(LadderPlan* P, const float2* J, float2* LJ, const float2* X 
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pz);
   long pl = prof_begin(ctx, "lsum");
-  y_split_kernel<<<dim3(div_up(size_t(P->Kp2), 256), unsigned(N), 1), 256, 0, s>>>(P->d_Dz.p, M, 1, 0, int(nw), int(nwp),
+  launch_after(s, y_split_kernel, dim3(div_up(size_t(P->Kp2), 256), unsigned(N), 1), 256, 0, P->d_Dz.p, M, 1, 0, int(nw), int(nwp),
                                                                                   N, P->Kp2, P->d_Yh.p, P->d_Yl.p);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pl);
   int sp2 = tc_gemm_launch(ctx, P->opKK, P->opY, int(nw), int(8 * N), int(nw), P->d_part2.p, nw, nw * 8 * N, 16, P->d_err.p,
                            "tc_ladder_kk");
   pl = prof_begin(ctx, "lfinish");
-  finish_gemm_kernel<float><<<dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, s>>>(
+  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, 
       P->d_Dz.p, M, 1, 0, P->d_part2.p, sp2, nw * 8 * N, P->d_Gmf.p, P->d_Gpf.p, nullptr, int(nw), int(nwp), int(ni), LJ,
       X);
   EPSP_LAUNCHED(ctx);
@@ -2122,9 +2262,9 @@ template <class V>
 static void dot_dev(LadderPlan* P, const V* u, const V* v, long n, DBuf<double2>& part, double2* out_dev) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
-  dot_partial_kernel<V><<<dim3(kDotBlocks, 1), 256, 0, s>>>(u, v, n, nullptr, part.p);
+  launch_after(s, dot_partial_kernel<V>, dim3(kDotBlocks, 1), 256, 0, u, v, n, nullptr, part.p);
   EPSP_LAUNCHED(ctx);
-  dot_final_kernel<<<1, 256, 0, s>>>(part.p, kDotBlocks, nullptr, out_dev);
+  launch_after(s, dot_final_kernel, 1, 256, 0, part.p, kDotBlocks, nullptr, out_dev);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -2133,7 +2273,7 @@ static void dot_dev(LadderPlan* P, const V* u, const V* v, long n, DBuf<double2>
 template <class V>
 static void cond_launch(LadderPlan* P, const V* J, double2* Ydev) {
   Ctx* ctx = P->ctx;
-  cond_sum_kernel<V><<<dim3(unsigned(3 * P->ni), 1), 256, 0, ctx->stream>>>(J, P->d_Ww.p, int(P->nw), int(P->ni), Ydev);
+  launch_after(ctx->stream, cond_sum_kernel<V>, dim3(unsigned(3 * P->ni), 1), 256, 0, J, P->d_Ww.p, int(P->nw), int(P->ni), Ydev);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -2162,6 +2302,7 @@ static void conductivity_dev(LadderPlan* P, const V* J, double Om, double T, DBu
 
 // c[0] = 1/sqrt(Re x[0]) (the scale of the first Krylov vector, without a round trip to the host).
 __global__ void rsqrt_coef_kernel(const double2* __restrict__ x, double2* __restrict__ c) {
+  pdl_wait();
   if (threadIdx.x == 0 && blockIdx.x == 0) c[0] = make_double2(1.0 / sqrt(x[0].x), 0.0);
 }
 
@@ -2203,7 +2344,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
     if (!(Tlist[iT] >= 0)) fail(EPSP_EINVAL, "Temperature must be positive");
   const long nw = P->nw, ni = P->ni;
   const long n = nw * 24 * ni;
-  const unsigned eb = div_up(size_t(n), 256);
+  const unsigned eb = div_up(size_t(n), 256), vb = div_up(size_t(n), 256 * kVecPer);
   DBuf<double2>& part = P->w_part;
   DBuf<double2>& Hdev = P->w_H;
   DBuf<double2>& Ybuf = P->w_Y;
@@ -2243,16 +2384,16 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
       if constexpr (std::is_same_v<V, float2>) {
         // propagators, J0, its σ sums (slot 0) and ‖J0‖² in one pass
         set_propagators(P, mu[iT], T, Om, false);
-        prep_vertex_f32_kernel<<<unsigned(ni), 256, 0, s>>>(P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p,
+        launch_after(s, prep_vertex_f32_kernel, unsigned(ni), 256, 0, P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p,
                                                             P->d_tp.p, P->d_eps_i.p, mu[iT], T, Om, P->d_v.p, P->d_Ww.p,
                                                             int(ni), P->d_Gmf.p, P->d_Gpf.p, J0.p, Ybuf.p, part.p);
         EPSP_LAUNCHED(ctx);
-        dot_final_kernel<<<1, 256, 0, s>>>(part.p, int(ni), nullptr, Hdev.p + hN0);
+        launch_after(s, dot_final_kernel, 1, 256, 0, part.p, int(ni), nullptr, Hdev.p + hN0);
         EPSP_LAUNCHED(ctx);
       } else {
         set_propagators(P, mu[iT], T, Om);
         const dim3 ab(div_up(size_t(nw), 256), unsigned(6 * ni), 4);
-        attach_bare_kernel<double2><<<ab, 256, 0, s>>>(P->d_Gm.p, P->d_Gp.p, P->d_v.p, int(nw), int(ni), J0.p);
+        launch_after(s, attach_bare_kernel<double2>, ab, 256, 0, P->d_Gm.p, P->d_Gp.p, P->d_v.p, int(nw), int(ni), J0.p);
         EPSP_LAUNCHED(ctx);
       }
       auto op = [&](const V* x, V* y) {  // y = x - L(x)
@@ -2285,12 +2426,12 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
         if (warm) {          // r0 = b - A x0
           if (!needJ) cond_launch(P, J.p, Ybuf.p + ny);  // slot 1: σ(x0)
           op(J.p, W.p);
-          axpby_kernel<V><<<eb, 256, 0, s>>>(make_double2(1, 0), nullptr, J0.p, make_double2(-1, 0), nullptr, W.p, n, nullptr);
+          launch_after(s, axpby_kernel<V>, vb, 256, 0, make_double2(1, 0), nullptr, J0.p, make_double2(-1, 0), nullptr, W.p, n, nullptr);
           EPSP_LAUNCHED(ctx);
           dot_dev(P, W.p, W.p, n, part, Hdev.p + hB2);
           r0 = W.p;
         }
-        rsqrt_coef_kernel<<<1, 32, 0, s>>>(Hdev.p + (warm ? hB2 : hN0), Hdev.p + hC);
+        launch_after(s, rsqrt_coef_kernel, 1, 32, 0, Hdev.p + (warm ? hB2 : hN0), Hdev.p + hC);
         EPSP_LAUNCHED(ctx);
         // the Krylov vectors and their pointers on the device (allocated as the basis grows, kept)
         auto vec = [&](int k) -> V* {
@@ -2303,7 +2444,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
           }
           return Vk[size_t(k)].p;
         };
-        scale_kernel<V><<<eb, 256, 0, s>>>(make_double2(0, 0), Hdev.p + hC, r0, vec(0), n, nullptr);
+        launch_after(s, scale_kernel<V>, vb, 256, 0, make_double2(0, 0), Hdev.p + hC, r0, vec(0), n, nullptr);
         EPSP_LAUNCHED(ctx);
         prof_end(ctx, plp);
         plp = -1;
@@ -2331,21 +2472,21 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
             double2* hp = pass == 0 ? P->g_h1.p : P->g_h2.p;
             for (int i0 = 0; i0 < inner; i0 += kMG) {
               const int m = std::min(kMG, inner - i0);
-              mdot_partial_kernel<V><<<kDotBlocks, 256, 0, s>>>(vp, i0, m, W.p, n, part.p);
+              launch_after(s, mdot_partial_kernel<V>, kDotBlocks, 256, 0, vp, i0, m, W.p, n, part.p);
               EPSP_LAUNCHED(ctx);
-              dot_final_kernel<<<unsigned(m), 256, 0, s>>>(part.p, kDotBlocks, nullptr, hp + i0);
+              launch_after(s, dot_final_kernel, unsigned(m), 256, 0, part.p, kDotBlocks, nullptr, hp + i0);
               EPSP_LAUNCHED(ctx);
             }
             for (int i0 = 0; i0 < inner; i0 += kMG) {
               const int m = std::min(kMG, inner - i0);
               const bool last = pass == npass - 1 && i0 + m >= inner;
-              maxpy_kernel<V><<<kDotBlocks, 256, 0, s>>>(W.p, vp, i0, m, hp, n, last ? part.p : nullptr);
+              launch_after(s, maxpy_kernel<V>, kDotBlocks, 256, 0, W.p, vp, i0, m, hp, n, last ? part.p : nullptr);
               EPSP_LAUNCHED(ctx);
             }
           }
-          dot_final_kernel<<<1, 256, 0, s>>>(part.p, kDotBlocks, nullptr, P->g_hsq.p);
+          launch_after(s, dot_final_kernel, 1, 256, 0, part.p, kDotBlocks, nullptr, P->g_hsq.p);
           EPSP_LAUNCHED(ctx);
-          gmres_givens_kernel<<<1, 32, 0, s>>>(P->g_h1.p, npass == 2 ? P->g_h2.p : nullptr, P->g_hsq.p, Hdev.p + hN0,
+          launch_after(s, gmres_givens_kernel, 1, 32, 0, P->g_h1.p, npass == 2 ? P->g_h2.p : nullptr, P->g_hsq.p, Hdev.p + hN0,
                                                Hdev.p + (warm ? hB2 : hN0), rtol, btol, inner, P->g_R.p, P->g_cs.p,
                                                P->g_sn.p, P->g_z.p, P->g_st.p, P->g_inv.p);
           EPSP_LAUNCHED(ctx);
@@ -2387,7 +2528,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
           breakdown = gs.breakdown != 0;
           tired = inner >= maxiter;
           if (!(solved || tired || breakdown)) {  // the next Krylov vector w / H[k + 1, k]
-            scale_kernel<V><<<eb, 256, 0, s>>>(make_double2(0, 0), P->g_inv.p, W.p, vec(inner), n, nullptr);
+            launch_after(s, scale_kernel<V>, vb, 256, 0, make_double2(0, 0), P->g_inv.p, W.p, vec(inner), n, nullptr);
             EPSP_LAUNCHED(ctx);
           }
         }
@@ -2417,12 +2558,14 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
           // x = x0 + V y (x0 = J for a warm start, else 0)
           long psl = prof_begin(ctx, "lsol");
           if (inner == 0 && !warm) J.zero(s);
-          for (int i = 0; i < inner; ++i) {
-            const double2 yi = make_double2(y[size_t(i)].real(), y[size_t(i)].imag());
-            if (i == 0 && !warm)
-              scale_kernel<V><<<eb, 256, 0, s>>>(yi, nullptr, Vk[0].p, J.p, n, nullptr);
-            else
-              axpby_kernel<V><<<eb, 256, 0, s>>>(yi, nullptr, Vk[size_t(i)].p, make_double2(1, 0), nullptr, J.p, n, nullptr);
+          for (int i0 = 0; i0 < inner; i0 += kCombine) {
+            const int m = std::min(kCombine, inner - i0);
+            CombineArgs<V> A{};
+            for (int t = 0; t < m; ++t) {
+              A.x[t] = Vk[size_t(i0 + t)].p;
+              A.y[t] = make_double2(y[size_t(i0 + t)].real(), y[size_t(i0 + t)].imag());
+            }
+            launch_after(s, combine_kernel<V>, vb, 256, 0, A, m, i0, nullptr, 0, nullptr, i0 > 0 || warm, J.p, n);
             EPSP_LAUNCHED(ctx);
           }
           prof_end(ctx, psl);
@@ -2507,6 +2650,7 @@ __global__ void propagators_batch_kernel(const double2* __restrict__ S_all, cons
                                          const int32_t* __restrict__ jp_all, const double* __restrict__ tp_all,
                                          const double* __restrict__ eps_i, const PairParams* __restrict__ pp,
                                          float2* __restrict__ Gm_all, float2* __restrict__ Gp_all, int ni) {
+  pdl_wait();
   int w = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y;
   const long z = blockIdx.z;
@@ -2529,8 +2673,8 @@ struct LadderBatch {
   DBuf<__nv_bfloat16> Jh, Jl, Yh, Yl;
   DBuf<float> Jt;  // GEMM_TF32: Jr as TF32-rounded FP32
   DBuf<float> Z, D, part2, nnu;
-  DBuf<float2> Gm, Gp, J0, J, LJ, W;
-  DBuf<double2> dpart, H, coef_a, coef_b;
+  DBuf<float2> Gm, Gp, J0, J, W;
+  DBuf<double2> dpart, H, coef_a;
   std::vector<DBuf<float2>> V;
   DBuf<int32_t> jm, jp;
   DBuf<double> tm, tp;
@@ -2565,11 +2709,10 @@ static void batch_reserve(LadderPlan* P, LadderBatch& B, long R, int maxiter) {
   B.nnu.alloc(ctx, size_t(16 * R));
   B.Gm.alloc(ctx, size_t(R * 4 * nw * ni));
   B.Gp.alloc(ctx, size_t(R * 4 * nw * ni));
-  for (auto* b : {&B.J0, &B.J, &B.LJ, &B.W}) b->alloc(ctx, size_t(R * n));
+  for (auto* b : {&B.J0, &B.J, &B.W}) b->alloc(ctx, size_t(R * n));
   B.dpart.alloc(ctx, size_t(R * kDotBlocksB));
   B.H.alloc(ctx, size_t(R * (maxiter + 2)));
   B.coef_a.alloc(ctx, size_t(R));
-  B.coef_b.alloc(ctx, size_t(R));
   B.jm.alloc(ctx, size_t(R * nw));
   B.jp.alloc(ctx, size_t(R * nw));
   B.tm.alloc(ctx, size_t(R * nw));
@@ -2583,8 +2726,8 @@ static void batch_reserve(LadderPlan* P, LadderBatch& B, long R, int maxiter) {
   B.opY = two_part(B.Yh.p, B.Yl.p, R * 8 * N, nw, P->Kp2, P->bn2);
 }
 
-// LJ[r] = L(X[r]) for the nA right-hand sides listed in the device array rmap (host copy rmap_h).
-static void apply_L_batch(LadderPlan* P, LadderBatch& B, const float2* X, int nA, float2* LJ) {
+// W[r] = X[r] - L(X[r]) for the nA right-hand sides listed in the device array rmap.
+static void apply_one_minus_L_batch(LadderPlan* P, LadderBatch& B, const float2* X, int nA, float2* W) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
   const long nw = P->nw, ni = P->ni, nwp = P->nwp, M = 24 * nwp, N = 3 * ni, n = nw * 24 * ni;
@@ -2598,14 +2741,14 @@ static void apply_L_batch(LadderPlan* P, LadderBatch& B, const float2* X, int nA
                  reinterpret_cast<const int2*>(P->d_zwin.p), B.nnu.p, B.rmap.p, int(nw), int(nwp), int(P->nm), B.D.p, Mt,
                  P->d_err.p);
   EPSP_LAUNCHED(ctx);
-  y_split_kernel<<<dim3(div_up(size_t(P->Kp2), 256), unsigned(N), unsigned(nA)), 256, 0, s>>>(
+  launch_after(s, y_split_kernel, dim3(div_up(size_t(P->Kp2), 256), unsigned(N), unsigned(nA)), 256, 0, 
       B.D.p, Mt, 1, 0, int(nw), int(nwp), N, P->Kp2, B.Yh.p, B.Yl.p);
   EPSP_LAUNCHED(ctx);
   const long N2 = 8 * N * nA;
   int sp2 = tc_gemm_launch(ctx, P->opKK, B.opY, int(nw), int(N2), int(nw), B.part2.p, nw, nw * N2, 16, P->d_err.p,
                            "tc_ladder_kk");
-  finish_gemm_kernel<float><<<dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(nA)), 256, 0, s>>>(
-      B.D.p, Mt, 1, 0, B.part2.p, sp2, nw * N2, B.Gm.p, B.Gp.p, B.rmap.p, int(nw), int(nwp), int(ni), LJ);
+  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(nA)), 256, 0, 
+      B.D.p, Mt, 1, 0, B.part2.p, sp2, nw * N2, B.Gm.p, B.Gp.p, B.rmap.p, int(nw), int(nwp), int(ni), W, X);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -2615,7 +2758,7 @@ static void conductivity_batch(LadderPlan* P, LadderBatch& B, const float2* J, i
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
   const long nw = P->nw, ni = P->ni;
-  cond_sum_kernel<float2><<<dim3(unsigned(3 * ni), unsigned(nP)), 256, 0, s>>>(J, P->d_Ww.p, int(nw), int(ni), B.Y.p);
+  launch_after(s, cond_sum_kernel<float2>, dim3(unsigned(3 * ni), unsigned(nP)), 256, 0, J, P->d_Ww.p, int(nw), int(ni), B.Y.p);
   EPSP_LAUNCHED(ctx);
   std::vector<double2> Y(static_cast<size_t>(3 * ni * nP));
   B.Y.download(Y.data(), Y.size(), s);
@@ -2676,11 +2819,11 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
   S_all.alloc(ctx, size_t(slab * nT));
   EPSP_CUDA(cudaMemcpyAsync(S_all.p, sigma, size_t(slab * nT) * sizeof(double2), cudaMemcpyDefault, s));
   const double btol = std::pow(std::numeric_limits<double>::epsilon(), 0.75);
-  const unsigned eb = div_up(size_t(n), 256);
+  const unsigned vb = div_up(size_t(n), 256 * kVecPer);
   auto dot_batch = [&](const float2* U, const float2* V, int nA, double2* out) {
-    dot_partial_kernel<float2><<<dim3(kDotBlocksB, unsigned(nA)), 256, 0, s>>>(U, V, n, B.rmap.p, B.dpart.p);
+    launch_after(s, dot_partial_kernel<float2>, dim3(kDotBlocksB, unsigned(nA)), 256, 0, U, V, n, B.rmap.p, B.dpart.p);
     EPSP_LAUNCHED(ctx);
-    dot_final_kernel<<<unsigned(nA), 256, 0, s>>>(B.dpart.p, kDotBlocksB, B.rmap.p, out);
+    launch_after(s, dot_final_kernel, unsigned(nA), 256, 0, B.dpart.p, kDotBlocksB, B.rmap.p, out);
     EPSP_LAUNCHED(ctx);
   };
   auto set_rmap = [&](const std::vector<int>& rm) { B.rmap.upload(rm.data(), rm.size(), s); };
@@ -2722,10 +2865,10 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
     B.tp.upload(tp.data(), tp.size(), s);
     B.nnu.upload(nnu.data(), nnu.size(), s);
     B.pp.upload(pp.data(), pp.size(), s);
-    propagators_batch_kernel<<<dim3(div_up(size_t(nw), 128), unsigned(ni), unsigned(nP)), 128, 0, s>>>(
+    launch_after(s, propagators_batch_kernel, dim3(div_up(size_t(nw), 128), unsigned(ni), unsigned(nP)), 128, 0, 
         S_all.p, P->d_ws.p, int(nw), B.jm.p, B.tm.p, B.jp.p, B.tp.p, P->d_eps_i.p, B.pp.p, B.Gm.p, B.Gp.p, int(ni));
     EPSP_LAUNCHED(ctx);
-    attach_bare_kernel<float2><<<dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(4 * nP)), 256, 0, s>>>(
+    launch_after(s, attach_bare_kernel<float2>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(4 * nP)), 256, 0, 
         B.Gm.p, B.Gp.p, P->d_v.p, int(nw), int(ni), B.J0.p);
     EPSP_LAUNCHED(ctx);
     conductivity_batch(P, B, B.J0.p, nP, pp, sb, idx);
@@ -2739,7 +2882,7 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
     EPSP_CUDA(cudaStreamSynchronize(s));
     std::vector<GmresState> g(static_cast<size_t>(nP));
     std::vector<int> act;
-    std::vector<double2> ca(static_cast<size_t>(nP)), cb(static_cast<size_t>(nP));
+    std::vector<double2> ca(static_cast<size_t>(nP));
     for (int z = 0; z < nP; ++z) {
       GmresState& q = g[size_t(z)];
       const double beta = std::sqrt(h[size_t(z)].x);
@@ -2755,29 +2898,27 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
       } else {
         ca[size_t(z)] = make_double2(0, 0);
       }
-      cb[size_t(z)] = make_double2(0, 0);
     }
     if (B.V.empty()) B.V.emplace_back();
     if (B.V[0].n != size_t(R * n)) B.V[0].alloc(ctx, size_t(R * n));
     // V0 = J0 / β (every slot; solved ones get 0)
     B.coef_a.upload(ca.data(), ca.size(), s);
-    scale_kernel<float2><<<dim3(eb, unsigned(nP)), 256, 0, s>>>(make_double2(0, 0), B.coef_a.p, B.J0.p, B.V[0].p, n, B.rmap.p);
+    launch_after(s, scale_kernel<float2>, dim3(vb, unsigned(nP)), 256, 0, make_double2(0, 0), B.coef_a.p, B.J0.p, B.V[0].p, n, B.rmap.p);
     EPSP_LAUNCHED(ctx);
     int k = 0;
     while (!act.empty()) {
       ++k;
       const int nA = int(act.size());
       set_rmap(act);
-      apply_L_batch(P, B, B.V[size_t(k - 1)].p, nA, B.LJ.p);  // LJ[r] = L(v_k)
-      sub_kernel<float2><<<dim3(eb, unsigned(nA)), 256, 0, s>>>(B.V[size_t(k - 1)].p, B.LJ.p, B.W.p, n, B.rmap.p);
-      EPSP_LAUNCHED(ctx);
-      for (int i = 0; i < k; ++i) {
-        dot_batch(B.V[size_t(i)].p, B.W.p, nA, B.H.p + long(i) * R);
-        axpy_dev_kernel<float2><<<dim3(eb, unsigned(nA)), 256, 0, s>>>(B.W.p, B.V[size_t(i)].p, B.H.p + long(i) * R, n,
-                                                                       B.rmap.p);
+      apply_one_minus_L_batch(P, B, B.V[size_t(k - 1)].p, nA, B.W.p);
+      dot_batch(B.V[0].p, B.W.p, nA, B.H.p);
+      for (int i = 0; i < k; ++i) {  // modified Gram-Schmidt; the last pass takes the norm
+        launch_after(s, axpy_dot_kernel<float2>, dim3(kDotBlocksB, unsigned(nA)), 256, 0, 
+            B.W.p, B.V[size_t(i)].p, B.H.p + long(i) * R, i + 1 < k ? B.V[size_t(i + 1)].p : nullptr, n, B.rmap.p, B.dpart.p);
+        EPSP_LAUNCHED(ctx);
+        launch_after(s, dot_final_kernel, unsigned(nA), 256, 0, B.dpart.p, kDotBlocksB, B.rmap.p, B.H.p + long(i + 1) * R);
         EPSP_LAUNCHED(ctx);
       }
-      dot_batch(B.W.p, B.W.p, nA, B.H.p + long(k) * R);
       std::vector<double2> hall(static_cast<size_t>((k + 1) * R));
       B.H.download(hall.data(), hall.size(), s);
       EPSP_CUDA(cudaStreamSynchronize(s));
@@ -2836,13 +2977,12 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
         if (B.V[size_t(k)].n != size_t(R * n)) B.V[size_t(k)].alloc(ctx, size_t(R * n));
         set_rmap(act);
         B.coef_a.upload(ca.data(), ca.size(), s);
-        scale_kernel<float2><<<dim3(eb, unsigned(act.size())), 256, 0, s>>>(make_double2(0, 0), B.coef_a.p, B.W.p,
+        launch_after(s, scale_kernel<float2>, dim3(vb, unsigned(act.size())), 256, 0, make_double2(0, 0), B.coef_a.p, B.W.p,
                                                                              B.V[size_t(k)].p, n, B.rmap.p);
         EPSP_LAUNCHED(ctx);
       }
     }
     // x = Σ_i y_i v_i per right-hand side (x0 = 0)
-    B.J.zero(s);
     const int kmax = k;
     std::vector<std::vector<cplx>> ys(static_cast<size_t>(nP));
     for (int z = 0; z < nP; ++z) {
@@ -2862,21 +3002,22 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
       }
       ys[size_t(z)] = y;
     }
-    for (int i = 0; i < kmax; ++i) {
-      std::vector<int> use;
-      for (int z = 0; z < nP; ++z) {
-        if (g[size_t(z)].inner > i) {
-          use.push_back(z);
-          ca[size_t(z)] = make_double2(ys[size_t(z)][size_t(i)].real(), ys[size_t(z)][size_t(i)].imag());
-          cb[size_t(z)] = make_double2(1, 0);
-        }
-      }
-      if (use.empty()) continue;
-      set_rmap(use);
-      B.coef_a.upload(ca.data(), ca.size(), s);
-      B.coef_b.upload(cb.data(), cb.size(), s);
-      axpby_kernel<float2><<<dim3(eb, unsigned(use.size())), 256, 0, s>>>(make_double2(0, 0), B.coef_a.p, B.V[size_t(i)].p,
-                                                                           make_double2(0, 0), B.coef_b.p, B.J.p, n, B.rmap.p);
+    // (coefficients [kmax][R]; a solve that took fewer steps has no vectors past its own)
+    std::vector<double2> yall(static_cast<size_t>(std::max(1, kmax) * R), make_double2(0, 0));
+    std::vector<int> inner(static_cast<size_t>(nP));
+    for (int z = 0; z < nP; ++z) {
+      inner[size_t(z)] = g[size_t(z)].inner;
+      for (int i = 0; i < g[size_t(z)].inner; ++i)
+        yall[size_t(i * R + z)] = make_double2(ys[size_t(z)][size_t(i)].real(), ys[size_t(z)][size_t(i)].imag());
+    }
+    set_rmap(inner);
+    B.H.upload(yall.data(), yall.size(), s);
+    for (int i0 = 0; i0 == 0 || i0 < kmax; i0 += kCombine) {
+      const int m = std::min(kCombine, kmax - i0);
+      CombineArgs<float2> A{};
+      for (int t = 0; t < m; ++t) A.x[t] = B.V[size_t(i0 + t)].p;
+      launch_after(s, combine_kernel<float2>, dim3(vb, unsigned(nP)), 256, 0, A, m, i0, B.H.p + long(i0) * R, R, B.rmap.p, i0 > 0, B.J.p,
+                                                                    n);
       EPSP_LAUNCHED(ctx);
     }
     conductivity_batch(P, B, B.J.p, nP, pp, sl, idx);

@@ -203,18 +203,20 @@ static void launch_pair_persist(Ctx* ctx, const TcOperand& A, const TcOperand& B
   const long items = long(nN) * nM2 * splits;
   if (items > (1l << 30)) fail(EPSP_EINVAL, "too many tiles for the persistent kernel");
   const int npairs = int(std::min<long>(std::max(1, ctx->sm_count / 2), items));
-  cudaLaunchAttribute cl;
-  cl.id = cudaLaunchAttributeClusterDimension;
-  cl.val.clusterDim.x = 2;
-  cl.val.clusterDim.y = 1;
-  cl.val.clusterDim.z = 1;
+  cudaLaunchAttribute cl[2];
+  cl[0].id = cudaLaunchAttributeClusterDimension;
+  cl[0].val.clusterDim.x = 2;
+  cl[0].val.clusterDim.y = 1;
+  cl[0].val.clusterDim.z = 1;
+  cl[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (as launch_after: the kernel waits in pdl_wait)
+  cl[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(2 * npairs), 1, 1);
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = L::kBytes;
   cfg.stream = ctx->stream;
-  cfg.attrs = &cl;
-  cfg.numAttrs = 1;
+  cfg.attrs = cl;
+  cfg.numAttrs = 2;
   EPSP_CUDA(cudaLaunchKernelEx(&cfg, kern, maps, M, N, kblocks, per, nN, nM2, int(items), out, ld_out, split_stride,
                                d_err, gm));
   EPSP_LAUNCHED(ctx);

@@ -816,6 +816,7 @@ __global__ void __launch_bounds__(192, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   cluster_sync_all();  // both CTAs' barriers initialised and TMEM allocated
+  pdl_wait();
 
   if (warp == 0 && lane == 0) {
     // producer: this CTA's A rows and B half of every item, completing on the leader's full barrier

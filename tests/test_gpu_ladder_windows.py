@@ -34,3 +34,26 @@ def test_apply_matches_oracle(oracle, nw, unit, modes):
             assert np.all(np.isfinite(got))
             assert np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref), (path, splits)
         plan.close()
+
+
+def test_solutions_of_more_vectors_than_one_pass_combines():
+    # Four solves of 6 to 14 Krylov vectors (a pass sums eight): batched, each pair's vertex is formed from its own
+    # count of vectors and must equal the sequential solve's (warm-started: its sum adds to a vertex) to 1e-4, as both
+    # residuals are 1e-6.
+    from epspectral_gb300 import api, graded_frequency_grid
+    ws = graded_frequency_grid([(-0.3, 0.3, 0.01), (-0.9, 0.9, 0.1)])
+    s = synthetic.cubic_t2g_setup(N=4, ws=ws, g2_dtype=np.float64, seed=3)
+    s["g2"] = 0.1 * s["g2"]
+    sig = np.empty((len(ws), s["eps_i"].size, 2), dtype=complex, order="F")
+    sig[:, :, 0], sig[:, :, 1] = 0.001 - 0.02j, -0.002 - 0.05j
+    plan = api.LadderPlan(s, path="gemm_bf16", omega_acoustic=W_AC)
+    args = (sig, [0.0, 0.01], [0.02, 0.05], [0.0, 0.1])
+    kw = dict(rtol=1e-6, maxiter=40, store_vertex=True)
+    seq, bat = plan.run(*args, **kw), plan.run(*args, batch_rhs=4, **kw)
+    assert seq["converged"].all() and bat["converged"].all()
+    assert bat["niter"].max() > 8 > bat["niter"].min() and seq["niter"].max() > 8
+    for iT in range(2):
+        for iO in range(2):
+            a, b = bat["J"][..., iO, iT], seq["J"][..., iO, iT]
+            assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b), (iO, iT)
+    plan.close()

@@ -67,6 +67,11 @@ struct Scgd0Plan {
   // as float pairs with their neighbouring cells' inverse widths, the bucket table's origin and scale
   bool disp = false;
   bool fd_fast = false;  // this call's temperatures allow fm_disp_fast_kernel
+  // ... its nodes and cell table in grid units (empty: not for this grid), the table's padding, the unit
+  DBuf<int32_t> d_fdoff;
+  DBuf<uint32_t> d_fdtab;
+  int fd_pad = 0;
+  double fd_unit = 0;
   long nk_i = 0, ntab = 0;
   float x0f = 0.f, inv_hf = 0.f;
   DBuf<float> d_gwf;

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <limits>
+#include <numeric>
 
 namespace epsp {
 
@@ -420,98 +421,91 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
   }
 }
 
-// The same sum in about 70 instructions a term (issue slots bound it; fm_disp_f32_kernel above takes about 180), for
-// temperatures above ωq / 40:
-//  * cells with slopes: record (side, c) of a column describes the cell above (side 1) or below (side 0) node c
-//    from that node: ω_c - ReΣ_c as a float pair, 1 - ReΣ', ImΣ_c, ImΣ', so that Re z = (U_hi - ε_hi) +
-//    ((U_lo - ε_lo) + (x - ω_c)(1 - ReΣ')): the first difference is exact where Re z is small against its parts, and
-//    outside the grid the record's slopes are 0 (fd_cell_kernel). No weight, no boundary test.
+// The same sum in about 50 instructions a term (the L1 data pipe bounds it; fm_disp_f32_kernel above takes about 180),
+// for temperatures above ωq / 40:
+//  * Frequencies in grid units u (the nodes are origin + offset u, whole offsets): x = ω ± ωq is a whole number b,
+//    ωq's being the same for all nodes, and a fraction that all nodes share. A table over b gives the cell that x is in
+//    and b's distance from the cell's lower node; padded by ωq's largest number, it needs no clamp.
+//  * A record a cell and column describes Σ from the cell's lower node c: ω_c - ReΣ_c as a float pair, u (1 - ReΣ'),
+//    ImΣ_c, u ImΣ', so that Re z = (U_hi - ε_hi) + ((U_lo - ε_lo) + (x - ω_c) (1 - ReΣ')): the first difference is exact
+//    where Re z is small against its parts. The cells below and above the grid have slopes 0 (fd_cell_kernel).
 //  * n + f(x_a - μ) = (1 + n)(1 + E)/(1 + E e) and n + 1 - f(x_e - μ) = n (1 + E)/(1 + E/e), E = exp((ω - μ)/T),
 //    e = exp(ωq/T): one FMA a side, the bracket's reciprocal shared with 1/|z|², and 1 + E outside the sum
 //    (both sides over E above μ, so that every factor stays below e^40).
-// The records of one side are contiguous over the nodes (four wavefronts of L1 a load); the bucket table is 16-bit
-// in shared memory. Grid (nω / 256, ni, slots x splits): the (ν, f) range is split, in whole tiles, until the
+// A column's records are contiguous over the cells (four wavefronts of L1 a load) and a staged pair is read once for
+// NPT nodes of a thread. Grid (nω / (256 NPT), ni, slots x splits): the (ν, f) range is split, in whole tiles, until the
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
-// Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 -> 3.25 ms;
-// the L1 data pipe is then 92 % busy (about 24 wavefronts a term and warp, half records, half shared memory) and
-// the issue slots 71 %.
+// Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
+// search for the nearest node and a record for either side of it, 2.30 now: 7.7 wavefronts a side and warp keep the L1
+// data pipe 90 % busy (4.7 of them the records, 20 bytes a lane), the issue slots 71 %.
 constexpr float kFdMaxArg = 40.f;
+constexpr long kFdMaxTable = 1l << 24;  // entries; those that fit 96 KB are kept in shared memory
+constexpr long kFdMaxCell = 32767;      // grid units of a cell or ωq: distances are 16 bits
 
 __device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v / T's rounding put back
   const float a = v / T, E = expf(a);
   return fmaf(E, fmaf(-a, T, v) / T, E);
 }
 
+// Records [column][nω + 1] of slot blockIdx.y: cell 0 is below the grid, cell c from node c - 1 to node c, cell nω above.
 __global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __restrict__ slots,
-                               const float4* __restrict__ wtab, const double* __restrict__ ws, int nw, long slab,
+                               const float4* __restrict__ wtab, const double* __restrict__ ws, int nw, long slab, double unit,
                                float4* __restrict__ rec, float* __restrict__ dim) {
-  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;  // node and column of slot blockIdx.y
-  if (k >= slab) return;
-  const float4* Sf = Sf_all + slab * slots[blockIdx.y];
-  const int j = int(k % nw);
-  const float4 s = Sf[k], wj = wtab[j];
+  const long ncell = slab / nw * (nw + 1);
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k >= ncell) return;
+  const int c = int(k % (nw + 1)), j = max(c - 1, 0);
+  const float4* Sf = Sf_all + slab * slots[blockIdx.y] + k / (nw + 1) * nw;
+  const float4 s = Sf[j], o = Sf[min(c, nw - 1)];
   const float2 u = split_df(ws[j] - (double(s.x) + double(s.y)));
-  const long col = 2 * (slab * blockIdx.y + k - j) + j;  // records [side][nω] of the column
-#pragma unroll
-  for (int side = 0; side < 2; ++side) {
-    const bool out = side ? j == nw - 1 : j == 0;
-    const float4 o = out ? s : Sf[side ? k + 1 : k - 1];
-    const float inv = out ? 0.f : side ? wj.z : -wj.w;
-    const float dre = ((o.x - s.x) + (o.y - s.y)) * inv, di = (o.z - s.z) * inv;
-    rec[col + long(nw) * side] = make_float4(u.x, u.y, 1.f - dre, s.z);
-    dim[col + long(nw) * side] = di;
-  }
+  const float inv = c == 0 || c == nw ? 0.f : wtab[j].z;
+  const float dre = ((o.x - s.x) + (o.y - s.y)) * inv, di = (o.z - s.z) * inv;
+  rec[ncell * blockIdx.y + k] = make_float4(u.x, u.y, float(unit * (1.0 - double(dre))), s.z);
+  dim[ncell * blockIdx.y + k] = float(unit) * di;
 }
 
-template <bool kSmemTab>
+template <int NPT, bool kSmemTab>
 __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     int nw, long slab, const float4* __restrict__ rec_all, const float* __restrict__ dim_all,
-    const float4* __restrict__ wtab_g, const int32_t* __restrict__ jtab_g, float x0, float inv_h, int ntab,
-    const float* __restrict__ gw, const double* __restrict__ wph, const int32_t* __restrict__ iq_kk,
+    const float4* __restrict__ wtab_g, const int32_t* __restrict__ offs, const uint32_t* __restrict__ tab_g, int ntab, int pad,
+    double unit, const float* __restrict__ gw, const double* __restrict__ wph, const int32_t* __restrict__ iq_kk,
     const int32_t* __restrict__ iks_i, const int32_t* __restrict__ iks_f, long nk_i, const double* __restrict__ eps_f,
     const int32_t* __restrict__ f_to_i, int nm, long nvf, long per, int nsplit, double w_ac, const int* __restrict__ slots,
     const TParams* __restrict__ tp, double* __restrict__ part) {
-  extern __shared__ __align__(16) unsigned char fd_tab[];  // kSmemTab: nodes [nw] float2, then the buckets (16 bits)
-  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε and ωq as float pairs}, the column
+  extern __shared__ __align__(16) uint32_t fd_cells[];  // kSmemTab: the cell table
+  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε as a float pair, ωq's fraction f and
+  // 1 - f}, {the column, ωq's whole number}
   __shared__ float4 s_a[kFdTile], s_e[kFdTile];
-  __shared__ int s_c[kFdTile];
-  float2* sw = reinterpret_cast<float2*>(fd_tab);
-  uint16_t* sj = reinterpret_cast<uint16_t*>(fd_tab + sizeof(float2) * size_t(nw));
-  if constexpr (kSmemTab) {
-    for (int k = threadIdx.x; k < nw; k += kFdTile) sw[k] = make_float2(wtab_g[k].x, wtab_g[k].y);
-    for (int k = threadIdx.x; k < ntab; k += kFdTile) sj[k] = uint16_t(jtab_g[k]);
-  }
+  __shared__ int2 s_c[kFdTile];
+  if constexpr (kSmemTab)
+    for (int k = threadIdx.x; k < ntab; k += kFdTile) fd_cells[k] = tab_g[k];
+  const uint32_t* tab = kSmemTab ? fd_cells : tab_g;
   const int i = blockIdx.y, a = blockIdx.z / nsplit, sp = blockIdx.z % nsplit;
-  const int iw = blockIdx.x * kFdTile + threadIdx.x;
+  const int iw0 = blockIdx.x * (kFdTile * NPT) + threadIdx.x;  // the nodes iw0 + 256 n
   const TParams tq = tp[slots[a]];
   const float T = float(tq.T);
-  const float4* rec = rec_all + 2 * slab * a;
-  const float* dim = dim_all + 2 * slab * a;
-  const float4 wn = wtab_g[min(iw, nw - 1)];
-  const float2 w = make_float2(wn.x, wn.y), mu = split_df(tq.mu);
-  const float wm = (w.x - mu.x) + (w.y - mu.y);
-  const float Ew = exp_comp(-fabsf(wm), T);  // E, or 1/E above μ
-  const float p = wm <= 0.f ? 1.f : Ew, q = wm <= 0.f ? Ew : 1.f;
-  // the bucket floor((x - x0) / h) by an FP32 addition (1.5 2^23: the integer lands in the mantissa): an
-  // off-by-one bucket at a bucket's edge picks the neighbouring cell, continuous there
-  const float bk1 = fmaf(-x0, inv_h, -0.5f), bmax = float(ntab - 1);
+  const long ncell = slab / nw * (nw + 1);
+  const float4* rec = rec_all + ncell * a;
+  const float* dim = dim_all + ncell * a;
+  const float2 mu = split_df(tq.mu);
+  float p[NPT], q[NPT];
+  int off[NPT];
+#pragma unroll
+  for (int n = 0; n < NPT; ++n) {
+    const int iw = min(iw0 + kFdTile * n, nw - 1);
+    const float4 wn = wtab_g[iw];
+    const float wm = (wn.x - mu.x) + (wn.y - mu.y);
+    const float Ew = exp_comp(-fabsf(wm), T);  // E, or 1/E above μ
+    p[n] = wm <= 0.f ? 1.f : Ew;
+    q[n] = wm <= 0.f ? Ew : 1.f;
+    off[n] = offs[iw] + pad;
+  }
   const int ki = iks_i[i];
-  auto side = [&](float wh, float wl, float2 e, int col, float o, float g, float& run) {
-    const float v = fminf(fmaxf(fmaf(w.x + wh, inv_h, bk1), 0.f), bmax);
-    const int b = __float_as_int(v + 12582912.f) - 0x4B400000;
-    int c;
-    float2 wc;
-    if constexpr (kSmemTab) {
-      c = sj[b];
-      wc = sw[c];
-    } else {
-      c = jtab_g[b];
-      const float4 t = wtab_g[c];
-      wc = make_float2(t.x, t.y);
-    }
-    const float dx = ((w.x - wc.x) + wh) + ((w.y - wc.y) + wl);
-    const int at = col + c + (dx < 0.f ? 0 : nw);
+  auto side = [&](int b, float frac, float2 e, int col, float o, float g, float& run) {
+    const uint32_t t = tab[b];  // the cell, and b's distance from its lower node + 32768
+    const float dx = (__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7610)) - 8421376.f) + frac;
+    const int at = col + int(t >> 16);
     const float4 r = rec[at];
     const float zr = (r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
     const float si = fmaf(dx, dim[at], r.w);
@@ -520,43 +514,65 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
     run = fmaf(g * si, inv, run);
   };
-  double acc = 0.0;
+  double acc[NPT];
+#pragma unroll
+  for (int n = 0; n < NPT; ++n) acc[n] = 0.0;
   const long t_end = min(nvf, per * (sp + 1l));
   for (long t0 = per * sp; t0 < t_end; t0 += kFdTile) {
     const long vf = t0 + threadIdx.x;
-    __syncthreads();  // the previous tile's readers are done (and, first, the tables are staged)
+    __syncthreads();  // the previous tile's readers are done (and, first, the table is staged)
     // below ω_acoustic no term: zero coupling, and ε = -1e25, so that |z|² overflows and the reciprocal is 0
-    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, 0.f, 0.f);
-    int sc = 0;
+    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, 0.f, 1.f);
+    int2 sc = make_int2(0, 0);
     if (vf < t_end) {
       const int nu = int(vf % nm);
       const long f = vf / nm;
       const double wq = wph[nu + long(nm) * iq_kk[ki + nk_i * long(iks_f[f])]];
       if (!(wq < w_ac)) {
-        const float2 ep = split_df(eps_f[f]), wp = split_df(wq);
-        const float n = occ_boson_f(wp.x, T), g = gw[vf + nvf * i];
-        sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp.x, T), exp_comp(-wp.x, T));
-        se = make_float4(ep.x, ep.y, wp.x, wp.y);
-        sc = 2 * nw * f_to_i[f];
+        const float2 ep = split_df(eps_f[f]);
+        const float wp = float(wq), n = occ_boson_f(wp, T), g = gw[vf + nvf * i];
+        const double wu = wq / unit, wb = fmin(floor(wu), double(pad - 1));
+        sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp, T), exp_comp(-wp, T));
+        se = make_float4(ep.x, ep.y, float(wu - wb), float(1.0 - (wu - wb)));
+        sc = make_int2((nw + 1) * f_to_i[f], int(wb));
       }
     }
     s_a[threadIdx.x] = sa;
     s_e[threadIdx.x] = se;
     s_c[threadIdx.x] = sc;
     __syncthreads();
-    float run0 = 0.f, run1 = 0.f;
     const int nt = int(min(long(kFdTile), t_end - t0));
+    // (a warp past the last node, or whose second nodes are, does that part of the work no more than it must)
+    if (iw0 - int(threadIdx.x % 32) >= nw) continue;
+    const bool both = NPT == 1 || iw0 - int(threadIdx.x % 32) + kFdTile < nw;
+    float run0[NPT], run1[NPT];
+#pragma unroll
+    for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
+    auto terms = [&](auto nodes) {
 #pragma unroll 2
-    for (int k = 0; k < nt; ++k) {
-      const float4 A = s_a[k], Q = s_e[k];
-      const int col = s_c[k];
-      const float2 e = make_float2(Q.x, Q.y);
-      side(Q.z, Q.w, e, col, fmaf(q, A.z, p), A.x, run0);
-      side(-Q.z, -Q.w, e, col, fmaf(q, A.w, p), A.y, run1);
-    }
-    acc += double(run0) + double(run1);
+      for (int k = 0; k < nt; ++k) {
+        const float4 A = s_a[k], Q = s_e[k];
+        const int2 C = s_c[k];
+        const float2 e = make_float2(Q.x, Q.y);
+#pragma unroll
+        for (int n = 0; n < decltype(nodes)::value; ++n) {
+          side(off[n] + C.y, Q.z, e, C.x, fmaf(q[n], A.z, p[n]), A.x, run0[n]);
+          side(off[n] - C.y - 1, Q.w, e, C.x, fmaf(q[n], A.w, p[n]), A.y, run1[n]);
+        }
+      }
+    };
+    if (both)
+      terms(std::integral_constant<int, NPT>{});
+    else
+      terms(std::integral_constant<int, 1>{});
+#pragma unroll
+    for (int n = 0; n < NPT; ++n) acc[n] += double(run0[n]) + double(run1[n]);
   }
-  if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc * double(p + q);
+#pragma unroll
+  for (int n = 0; n < NPT; ++n) {
+    const int iw = iw0 + kFdTile * n;
+    if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc[n] * double(p[n] + q[n]);
+  }
 }
 
 // ImΣ of slot a = the sum of its partials in order: into ImS_b and the Kramers-Kronig operand, or added to add_out.
@@ -931,11 +947,15 @@ static void check_err(Scgd0Plan* P) {
   }
 }
 
+// Nodes of a thread: two as soon as one tile does not hold them all (a dispersive run at 501 nodes: 28.4 ms, with one
+// 32.1; the second node's work is skipped by the warps that have none).
+static int fd_nodes(const Scgd0Plan* P) { return P->nw > kFdTile ? 2 : 1; }
+
 // Splits of the (ν, f) range for nA slots: about 40 blocks a multiprocessor (four are resident, so the last wave is a
 // tenth of the time), eight tiles of pairs a split at least (a block's tables and tail).
 static int fd_splits(const Scgd0Plan* P, long nA) {
   const long tiles = div_up(size_t(P->nm * P->nf), kFdTile);
-  const long blocks = long(div_up(size_t(P->nw), kFdTile)) * P->ni * nA;
+  const long blocks = long(div_up(size_t(P->nw), size_t(kFdTile * fd_nodes(P)))) * P->ni * nA;
   const long want = std::max<long>(1, (40l * P->ctx->sm_count + blocks - 1) / blocks);
   const long n = std::min(want, std::max<long>(1, tiles / 8));
   return int(div_up(size_t(tiles), div_up(size_t(tiles), size_t(n))));  // no empty split
@@ -948,37 +968,38 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
   Ctx* ctx = P->ctx;
   auto* T = P->tc.get();
   const long nw = P->nw, ni = P->ni;
-  // the grid nodes and the bucket table in shared memory when they fit 96 KB
   if (P->fd_fast) {
-    const long slab = nw * ni, n = slab * nA, nvf = P->nm * P->nf;
-    ensure(T->fdrec, ctx, size_t(2 * n));
-    ensure(T->fddim, ctx, size_t(2 * n));
-    fd_cell_kernel<<<dim3(div_up(size_t(slab), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
-        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, T->fdrec.p, T->fddim.p);
+    const long slab = nw * ni, ncell = (nw + 1) * ni, nvf = P->nm * P->nf;
+    ensure(T->fdrec, ctx, size_t(ncell * nA));
+    ensure(T->fddim, ctx, size_t(ncell * nA));
+    fd_cell_kernel<<<dim3(div_up(size_t(ncell), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
+        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, P->fd_unit, T->fdrec.p, T->fddim.p);
     EPSP_LAUNCHED(ctx);
-    const size_t tab = sizeof(float2) * size_t(nw) + 2 * size_t(P->ntab);
-    const bool smem = tab <= (size_t(96) << 10) && nw <= 65535;
-    const int nsplit = fd_splits(P, nA);
+    const size_t tab = sizeof(uint32_t) * P->d_fdtab.n;
+    const int nsplit = fd_splits(P, nA), npt = fd_nodes(P);
     const long per = (div_up(size_t(nvf), kFdTile) + nsplit - 1) / nsplit * kFdTile;
-    ensure(T->fdpart, ctx, size_t(n) * size_t(nsplit));
-    const dim3 grid(div_up(size_t(nw), kFdTile), unsigned(ni), unsigned(nA * nsplit));
+    ensure(T->fdpart, ctx, size_t(slab * nA) * size_t(nsplit));
+    const dim3 grid(div_up(size_t(nw), size_t(kFdTile * npt)), unsigned(ni), unsigned(nA * nsplit));
     auto go = [&](auto kern, size_t bytes) {
       EPSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-      kern<<<grid, kFdTile, bytes, ctx->stream>>>(int(nw), slab, T->fdrec.p, T->fddim.p, P->d_wtab.p, P->d_jtab.p, P->x0f,
-                                                  P->inv_hf, int(P->ntab), P->d_gwf.p, P->d_wph.p, P->d_iq.p, P->d_iksi.p,
-                                                  P->d_iksf.p, P->nk_i, P->d_epsf.p, P->d_fti.p, int(P->nm), nvf, per,
-                                                  nsplit, P->w_ac, d_slots, d_tp, T->fdpart.p);
+      kern<<<grid, kFdTile, bytes, ctx->stream>>>(int(nw), slab, T->fdrec.p, T->fddim.p, P->d_wtab.p, P->d_fdoff.p,
+                                                  P->d_fdtab.p, int(P->d_fdtab.n), P->fd_pad, P->fd_unit, P->d_gwf.p,
+                                                  P->d_wph.p, P->d_iq.p, P->d_iksi.p, P->d_iksf.p, P->nk_i, P->d_epsf.p,
+                                                  P->d_fti.p, int(P->nm), nvf, per, nsplit, P->w_ac, d_slots, d_tp,
+                                                  T->fdpart.p);
     };
-    if (smem)
-      go(fm_disp_fast_kernel<true>, tab);
+    const bool smem = tab <= (size_t(96) << 10);
+    if (npt == 2)
+      smem ? go(fm_disp_fast_kernel<2, true>, tab) : go(fm_disp_fast_kernel<2, false>, size_t(0));
     else
-      go(fm_disp_fast_kernel<false>, size_t(0));
+      smem ? go(fm_disp_fast_kernel<1, true>, tab) : go(fm_disp_fast_kernel<1, false>, size_t(0));
     EPSP_LAUNCHED(ctx);
     fd_finish_kernel<<<dim3(div_up(size_t(slab), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
         T->fdpart.p, int(nw), slab, nsplit, ImS_b, T->Im[0].p, T->Im[1].p, T->Im[2].p, T->Kp2, add_out);
     EPSP_LAUNCHED(ctx);
     return;
   }
+  // the grid nodes and the bucket table in shared memory when they fit 96 KB
   const size_t tab = sizeof(float4) * size_t(nw) + sizeof(int32_t) * size_t(P->ntab);
   const bool smem = tab <= (size_t(96) << 10);
   const dim3 grid(div_up(size_t(nw), kFdTile), unsigned(ni), unsigned(nA));
@@ -1000,17 +1021,17 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
   EPSP_LAUNCHED(ctx);
 }
 
-// Whether the temperatures of a call allow fm_disp_fast_kernel (every exp(ωq/T) within e^40; ω_acoustic above 0,
-// so that n(ωq) is finite). Reserves its buffers for nT slots, so that none is allocated while a graph is captured.
+// Whether the plan has the table of fm_disp_fast_kernel and the temperatures of a call allow it (every exp(ωq/T) within
+// e^40; ω_acoustic above 0, so that n(ωq) is finite). Reserves its buffers for nT slots, so that none is allocated while a graph is captured.
 void tc_disp_choose(Scgd0Plan* P, const double* Tlist, long nT) {
   if (!P->disp) return;
-  P->fd_fast = P->w_ac > 0 && 2 * P->nw * P->ni < (1l << 31);  // (32-bit record offsets)
+  P->fd_fast = P->w_ac > 0 && P->d_fdtab.n > 0;
   for (long t = 0; t < nT; ++t) P->fd_fast = P->fd_fast && Tlist[t] > 1.4901161193847656e-08 && P->wq_max <= kFdMaxArg * Tlist[t];
   if (!P->fd_fast) return;
   auto* T = P->tc.get();
-  const size_t n = size_t(P->nw * P->ni) * size_t(nT);
-  bool grown = ensure(T->fdrec, P->ctx, 2 * n);
-  grown |= ensure(T->fddim, P->ctx, 2 * n);
+  const size_t n = size_t((P->nw + 1) * P->ni) * size_t(nT);
+  bool grown = ensure(T->fdrec, P->ctx, n);
+  grown |= ensure(T->fddim, P->ctx, n);
   size_t part = 0;
   for (long a = 1; a <= nT; ++a) part = std::max(part, size_t(P->nw * P->ni) * size_t(a) * size_t(fd_splits(P, a)));
   grown |= ensure(T->fdpart, P->ctx, part);
@@ -1038,6 +1059,39 @@ void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, do
   launch_fm_disp(P, 1, d_slot0.p, d_q.p, nullptr, d_ImS);
   prof_end(ctx, pk);
   EPSP_CUDA(cudaStreamSynchronize(s));  // the parameter buffers are locals
+}
+
+// fm_disp_fast_kernel's nodes and cell table in units of the offsets' common divisor. None where ωq or a cell is too wide
+// in them, the table too long, or the records' offsets pass 32 bits: those plans keep fm_disp_f32_kernel.
+static void fd_table(Scgd0Plan* P) {
+  const GridHost& g = P->ws;
+  const long nw = P->nw;
+  long div = 0, widest = 0;
+  for (long j = 1; j < nw; ++j) {
+    const long d = g.offsets[size_t(j)] - g.offsets[size_t(j - 1)];
+    div = std::gcd(div, d);
+    widest = std::max(widest, d);
+  }
+  div = std::max(1l, div);
+  const double unit = g.unit * double(div), wq = P->wq_max / unit;
+  if (!(wq < double(kFdMaxCell - 1)) || widest / div > kFdMaxCell || nw > 65534 || (nw + 1) * P->ni >= (1l << 31)) return;
+  const long pad = long(std::floor(std::max(0.0, wq))) + 1;  // the whole numbers are 0 .. pad - 1
+  const long range = (g.offsets[size_t(nw - 1)] - g.offsets[0]) / div, n = range + 2 * pad;
+  if (n > kFdMaxTable) return;
+  std::vector<int32_t> off(static_cast<size_t>(nw));
+  for (long j = 0; j < nw; ++j) off[size_t(j)] = int32_t((g.offsets[size_t(j)] - g.offsets[0]) / div);
+  std::vector<uint32_t> tab(static_cast<size_t>(n));
+  long c = 0;  // the cell of b: the nodes at or below it
+  for (long e = 0; e < n; ++e) {
+    const long b = e - pad;
+    while (c < nw && off[size_t(c)] <= b) ++c;
+    tab[size_t(e)] = uint32_t(c) << 16 | uint32_t(b - off[size_t(std::max(0l, c - 1))] + 32768);
+  }
+  P->fd_unit = unit;
+  P->fd_pad = int(pad);
+  P->d_fdoff = to_device(P->ctx, off);
+  P->d_fdtab = to_device(P->ctx, tab);
+  EPSP_CUDA(cudaStreamSynchronize(P->ctx->stream));  // off and tab are locals
 }
 
 // The tables of fm_disp_f32_kernel (see Scgd0Plan): w_f g2 permuted to [ν f, i] and rounded to
@@ -1070,6 +1124,7 @@ void tc_setup_dispersive(Scgd0Plan* P, const epsp_model* m) {
   P->d_wtab.alloc(ctx, size_t(P->nw));
   fd_node_table_kernel<<<div_up(size_t(P->nw), 256), 256, 0, s>>>(P->d_ws.p, int(P->nw), P->d_wtab.p);
   EPSP_LAUNCHED(ctx);
+  fd_table(P);
   P->x0f = float(P->ct.x0);
   P->inv_hf = float(P->ct.inv_h);
   P->ntab = long(P->d_jtab.n);

@@ -34,3 +34,27 @@ def test_sum_matches_oracle(oracle, nw, ni, nm, nf, T, mu, graded):
     assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
     assert np.array_equal(plan.imsigma(S, mu, T, np.zeros((nw, ni))), got)
     plan.close()
+
+
+@pytest.mark.parametrize("off,unit,nm", [
+    (np.arange(513), 0.004, 3),                                        # two nodes a thread, one over
+    (np.cumsum(1 + 4 * (np.arange(700) % 3 == 0)) - 5, 0.002, 2),      # uneven cells
+    (np.append(50 * np.arange(520), 50 * 519 + 1), 8e-5, 2),           # a table too long for shared memory
+    (np.append(0, 40000 + 3 * np.arange(96)), 5e-5, 2),                # a cell too wide for it: the general sum
+    (np.arange(60), 5e-6, 2), (np.arange(90) * 7, 3e-3, 3)])           # ωq of more units than it holds; a common divisor
+def test_sum_on_uneven_grids(oracle, off, unit, nm):
+    from epspectral_gb300 import api
+    ni, nf, T, mu, nw = 3, 130, 0.03, 0.01, len(off)
+    off = off - off[0]
+    g = FrequencyGrid(-0.5 * unit * off[-1], unit, off)
+    wq = 0.05 + 0.1 * np.abs(R.pseudorandom(nm, ni, nf, seed=10))
+    wq[0, 0, 0], wq[1, 2, 5] = unit * 3, unit * 250  # whole numbers of units
+    s = per_pair_setup(g, np.abs(R.pseudorandom(nm, ni, nf, seed=9)), wq, 0.4 * R.pseudorandom(nf, seed=11),
+                       np.array([(5 * (f + 1)) % ni for f in range(nf)], dtype=np.int32), np.full(nf, 1.0 / nf))
+    S = 0.1 * R.pseudorandom(nw, ni, seed=7) + 1j * (-0.05 - 0.05 * np.abs(R.pseudorandom(nw, ni, seed=8)))
+    ref = oracle.imsigma(s, S, mu, T, np.zeros((nw, ni)), omega_acoustic=1e-5)
+    plan = api.Scgd0Plan(s, path="gemm_bf16", omega_acoustic=1e-5)
+    got = plan.imsigma(S, mu, T, np.zeros((nw, ni)))
+    assert np.all(np.isfinite(got))
+    assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref)
+    plan.close()

@@ -145,9 +145,10 @@ __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* 
 // Kernel tensor of the recast Fan-Migdal sum (see kbuild_f64_kernel in scgd0.cu), written as BF16
 // split rows K_t[ω][k], k = c nm + ν, through a shared-memory transpose. Σ(ω ± ω_ν) comes from the columns' cell
 // records (cell_record above; the cells and distances from set-up), the reciprocal and the occupation products are
-// FP32: the kernel runs on the FP32 units only. A side of an element is 20 bytes and about 12 instructions (four
-// 16-byte gathers, two weights and two two-sums a side before: 54 -> 42.8 us at 1251 x 7425, 52 -> 42 us at 8
-// temperatures of 626 x 2184).
+// FP32: the kernel runs on the FP32 units only. Instructions and the latency of its gathers bound it: a side of an element
+// is 20 bytes and about 12 instructions, the BF16 parts are formed two elements at a time, and eight blocks are kept on an
+// SM (with four 16-byte gathers, two weights and two two-sums a side 54 us at 1251 x 7425; six blocks, elements one by
+// one and a test of every column 40.8; now 36.6. 32 nodes a block instead of 16: 38.4, and 10 -> 12 us at 501 x 1575).
 // Grid (nω / 16, Kp / (kKbCols nm), slots), 256 threads: thread (node ω0 + t % 16, modes t / 16,
 // t / 16 + 16, ..) loads the cells and occupations of its (ω, ν) once and runs over the block's
 // kKbCols columns c (their records' offset and energy from shared memory). Dynamic shared memory: the tile
@@ -155,7 +156,31 @@ __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* 
 // straddle two blocks (nor Kp, a multiple of 64).
 constexpr int kKbCols = 8;
 constexpr int kKbW = 16;
-__global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, const float4* __restrict__ rec_all,
+
+__device__ __forceinline__ float rcp_f(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// split_bf16_n of a and b in three parts, each part's two values packed (a in the low half): the packed conversion takes
+// both, and a part's value as FP32 is its 16 bits moved up.
+__device__ __forceinline__ void split_bf16_pair(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  auto pack = [](float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+  };
+  p0 = pack(a, b);
+  a -= __uint_as_float(p0 << 16);
+  b -= __uint_as_float(p0 & 0xffff0000u);
+  p1 = pack(a, b);
+  a -= __uint_as_float(p1 << 16);
+  b -= __uint_as_float(p1 & 0xffff0000u);
+  p2 = pack(a, b);
+}
+
+__global__ void __launch_bounds__(256, 8) kbuild_bf16_kernel(int nw, int ni, const float4* __restrict__ rec_all,
                                                           const float* __restrict__ dim_all,
                                                           const int* __restrict__ slots,
                                                           const int32_t* __restrict__ cell_e,
@@ -170,8 +195,7 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, con
   pdl_wait();
   if (ctl && ctl->stop) return;
   extern __shared__ float kb_tile[];  // [kKbCols nm][kKbW + 1]
-  __shared__ int s_col[kKbCols];
-  __shared__ float2 s_eps[kKbCols];
+  __shared__ float4 s_col[kKbCols];  // ε as a float pair, the records' offset (integer bits)
   const int w0 = blockIdx.x * kKbW;
   const int cbeg = blockIdx.y * kKbCols;
   const int tw = threadIdx.x % kKbW, tm = threadIdx.x / kKbW;
@@ -183,8 +207,9 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, con
   const float* F = F_all + 2l * nwm * blockIdx.z;
   if (threadIdx.x < kKbCols) {
     const int c = cbeg + threadIdx.x;
-    s_col[threadIdx.x] = c < nc ? (nw + 1) * col_c[c] : -1;
-    s_eps[threadIdx.x] = c < nc ? eps_c[c] : make_float2(0.f, 0.f);
+    // (past the last column: |z|² overflows, its reciprocal and the element are 0)
+    const float2 e = c < nc ? eps_c[c] : make_float2(-1e25f, 0.f);
+    s_col[threadIdx.x] = make_float4(e.x, e.y, __int_as_float(c < nc ? (nw + 1) * col_c[c] : 0), 0.f);
   }
   __syncthreads();
   for (int nu = tm; nu < nm; nu += 256 / kKbW) {
@@ -200,21 +225,17 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, con
       Fa = F[ia];
       Fe = F[ie];
     }
-#pragma unroll 4
+#pragma unroll 2
     for (int cl = 0; cl < kKbCols; ++cl) {
-      const int co = s_col[cl];
-      float v = 0.f;
-      if (on && co >= 0) {
-        const float2 e = s_eps[cl];
-        const float4 A = rec[co + ea], B = rec[co + ee];
-        const float zar = (A.x - e.x) + fmaf(da, A.z, A.y - e.y), sia = fmaf(da, dim[co + ea], A.w);
-        const float zer = (B.x - e.x) + fmaf(de, B.z, B.y - e.y), sie = fmaf(de, dim[co + ee], B.w);
-        // Im 1/z with Im z = -Im Σ; the K tensor carries FP32 precision, so an approximate
-        // division (2 ulp; denominators here lie far inside its range) is enough
-        const float ga = __fdividef(sia, fmaf(zar, zar, sia * sia));
-        const float ge = __fdividef(sie, fmaf(zer, zer, sie * sie));
-        v = ga * Fa + ge * Fe;
-      }
+      const float4 e = s_col[cl];
+      const int ia = __float_as_int(e.z) + ea, ie = __float_as_int(e.z) + ee;
+      const float4 A = rec[ia], B = rec[ie];
+      const float zar = (A.x - e.x) + fmaf(da, A.z, A.y - e.y), sia = fmaf(da, dim[ia], A.w);
+      const float zer = (B.x - e.x) + fmaf(de, B.z, B.y - e.y), sie = fmaf(de, dim[ie], B.w);
+      // Im 1/z with Im z = -Im Σ, by an approximate reciprocal (1 ulp): the K tensor carries FP32 precision
+      const float ga = sia * rcp_f(fmaf(zar, zar, sia * sia));
+      const float ge = sie * rcp_f(fmaf(zer, zer, sie * sie));
+      const float v = on ? ga * Fa + ge * Fe : 0.f;
       kb_tile[(cl * nm + nu) * (kKbW + 1) + tw] = v;
     }
   }
@@ -229,19 +250,15 @@ __global__ void __launch_bounds__(256, 6) kbuild_bf16_kernel(int nw, int ni, con
       const int ow = w0 + wr;
       const long k = kbeg + 8 * ch;
       if (ow >= nw || k >= Kp) continue;
-      __align__(16) __nv_bfloat16 p0[8], p1[8], p2[8];
+      uint32_t p[3][4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        __nv_bfloat16 q[3];
-        split_bf16_n(kb_tile[(8 * ch + j) * (kKbW + 1) + wr], 3, q);
-        p0[j] = q[0];
-        p1[j] = q[1];
-        p2[j] = q[2];
-      }
+      for (int j = 0; j < 4; ++j)
+        split_bf16_pair(kb_tile[(8 * ch + 2 * j) * (kKbW + 1) + wr], kb_tile[(8 * ch + 2 * j + 1) * (kKbW + 1) + wr],
+                        p[0][j], p[1][j], p[2][j]);
       const long off = (krow0 + ow) * Kp + k;
-      *reinterpret_cast<uint4*>(K0 + off) = *reinterpret_cast<const uint4*>(p0);
-      *reinterpret_cast<uint4*>(K1 + off) = *reinterpret_cast<const uint4*>(p1);
-      *reinterpret_cast<uint4*>(K2 + off) = *reinterpret_cast<const uint4*>(p2);
+      *reinterpret_cast<uint4*>(K0 + off) = make_uint4(p[0][0], p[0][1], p[0][2], p[0][3]);
+      *reinterpret_cast<uint4*>(K1 + off) = make_uint4(p[1][0], p[1][1], p[1][2], p[1][3]);
+      *reinterpret_cast<uint4*>(K2 + off) = make_uint4(p[2][0], p[2][1], p[2][2], p[2][3]);
     }
   }
 }
@@ -510,9 +527,7 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     const float zr = (r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
     const float si = fmaf(dx, dim[at], r.w);
     const float d = fmaf(zr, zr, si * si) * o;
-    float inv;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(d));
-    run = fmaf(g * si, inv, run);
+    run = fmaf(g * si, rcp_f(d), run);
   };
   double acc[NPT];
 #pragma unroll

@@ -262,6 +262,7 @@ __global__ void propagators_kernel(const double2* __restrict__ ST, const double*
                                    const double* __restrict__ eps_i, double mu, double T, double Om,
                                    Vec2<std::conditional_t<F32, float, double>>* __restrict__ Gm,
                                    Vec2<std::conditional_t<F32, float, double>>* __restrict__ Gp, int ni) {
+  pdl_wait();
   int w = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y;
   if (w >= nw) return;
@@ -586,6 +587,7 @@ __global__ void coupling_rot_chunk_kernel(const T* __restrict__ g2c, const doubl
 __global__ void __launch_bounds__(128) xgen_f64_kernel(const double2* __restrict__ J, const double4* __restrict__ xtab,
                                                        const double* __restrict__ nnu, int nw, int nwp, int nm, int nmp,
                                                        double* __restrict__ A) {
+  pdl_wait();
   const int j = blockIdx.x * 128 + threadIdx.x;
   if (j >= nw) return;
   const int b = blockIdx.y % 3, nu = blockIdx.z / 2, c0 = blockIdx.z % 2;
@@ -966,6 +968,7 @@ __global__ void split_rows_t2_kernel(const double* __restrict__ S, long ldr, lon
 
 // Y of the regrouped path: the rows q = 0 (c12 = 11) and q = 2 (c12 = 22) of D, as [nω, (qq, c0, ri, n)].
 __global__ void y_gemm_kernel(const double* __restrict__ D, int nw, int nwp, long ncol, double* __restrict__ Y) {
+  pdl_wait();
   long idx = long(blockIdx.x) * blockDim.x + threadIdx.x;
   long total = long(nw) * 8 * ncol;
   if (idx >= total) return;
@@ -2089,10 +2092,10 @@ static void set_propagators(LadderPlan* P, double mu, double T, double Om, bool 
   if (!launch) return;
   const dim3 grid(div_up(size_t(nw), 128), unsigned(ni));
   if (tc_path(P->path))
-    propagators_kernel<true><<<grid, 128, 0, s>>>(P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p, P->d_tp.p,
+    launch_after(s, propagators_kernel<true>, grid, 128, 0, P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p, P->d_tp.p,
                                                    P->d_eps_i.p, mu, T, Om, P->d_Gmf.p, P->d_Gpf.p, int(ni));
   else
-    propagators_kernel<false><<<grid, 128, 0, s>>>(P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p,
+    launch_after(s, propagators_kernel<false>, grid, 128, 0, P->d_ST.p, P->d_ws.p, int(nw), P->d_jm.p, P->d_tm.p, P->d_jp.p,
                                                     P->d_tp.p, P->d_eps_i.p, mu, T, Om, P->d_Gm.p, P->d_Gp.p, int(ni));
   EPSP_LAUNCHED(ctx);
 }
@@ -2176,7 +2179,7 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   set_mode_occupations(P, T);
   const long nwp = P->nwp, M = 24 * nwp, N = 3 * ni;
   long px = prof_begin(ctx, "xgen");
-  xgen_f64_kernel<<<dim3(div_up(size_t(nw), 128), unsigned(3 * ni), unsigned(2 * P->nm)), 128, 0, s>>>(
+  launch_after(s, xgen_f64_kernel, dim3(div_up(size_t(nw), 128), unsigned(3 * ni), unsigned(2 * P->nm)), 128, 0, 
       J, P->d_xtab.p, P->d_nnu.p, int(nw), int(nwp), int(P->nm), int(P->nmp), P->d_Af.p);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, px);
@@ -2184,7 +2187,7 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   oz_gemm(ctx, P->oz, M, N, P->Kx, P->d_Af.p, M, nullptr, P->d_Gt.p, P->Kx, &P->ozGt, 0.0, P->d_D.p, M);
   prof_end(ctx, pg);
   const long ny = nw * 8 * N;
-  y_gemm_kernel<<<div_up(size_t(ny), 256), 256, 0, s>>>(P->d_D.p, int(nw), int(nwp), N, P->d_Y.p);
+  launch_after(s, y_gemm_kernel, div_up(size_t(ny), 256), 256, 0, P->d_D.p, int(nw), int(nwp), N, P->d_Y.p);
   EPSP_LAUNCHED(ctx);
   oz_gemm(ctx, P->oz, nw, 8 * N, nw, P->d_KK.p, nw, &P->ozKK, P->d_Y.p, nw, nullptr, 0.0, P->d_KY.p, nw);
   launch_after(s, finish_gemm_kernel<double>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, 

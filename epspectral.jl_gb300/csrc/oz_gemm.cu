@@ -60,6 +60,7 @@ __device__ __forceinline__ uint32_t oz_hi(double x) { return uint32_t(__double2h
 // read comes from L1/L2).
 __global__ void __launch_bounds__(256) oz_split_k_kernel(const double* __restrict__ S, long ld, long rows, long K, long Kp,
                                                          __nv_bfloat16* __restrict__ q, uint32_t* __restrict__ mx) {
+  pdl_wait();
   __shared__ uint32_t sm[8];
   const long r = blockIdx.x;
   const double* row = S + ld * r;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(256) oz_split_k_kernel(const double* __restric
 // and kper k), then the digits through a 64 x 64 transpose.
 __global__ void __launch_bounds__(256) oz_max_m_kernel(const double* __restrict__ S, long ld, long rows, long K, long kper,
                                                        uint32_t* __restrict__ mx) {
+  pdl_wait();
   __shared__ uint32_t sm[4][64];
   const int tx = threadIdx.x % 64, ty = threadIdx.x / 64;
   const long r = long(blockIdx.x) * 64 + tx, k0 = long(blockIdx.y) * kper;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(256) oz_max_m_kernel(const double* __restrict_
 }
 __global__ void __launch_bounds__(256) oz_split_m_kernel(const double* __restrict__ S, long ld, long rows, long K, long Kp,
                                                          const uint32_t* __restrict__ mx, __nv_bfloat16* __restrict__ q) {
+  pdl_wait();
   __shared__ unsigned long long tile[64][65];  // [k][r]
   const long r0 = long(blockIdx.x) * 64, k0 = long(blockIdx.y) * 64;
   {
@@ -229,6 +232,7 @@ __global__ void __launch_bounds__(320, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // (barriers and tensor memory are set up beside the kernel ahead)
 
   if (warp == 0 && lane == 0) {
     int g = 0;
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(256) oz_sum_kernel(const int* __restrict__ sum
                                                      const uint32_t* __restrict__ mxA, const uint32_t* __restrict__ mxB,
                                                      const double* __restrict__ A, long lda, const double* __restrict__ B,
                                                      long ldb, double beta, double* __restrict__ C, long ldc) {
+  pdl_wait();
   const long idx = long(blockIdx.x) * 256 + threadIdx.x;
   if (idx >= long(M) * N) return;
   const int m = int(idx % M), n = int(idx / M);
@@ -433,7 +438,7 @@ void oz_split(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_majo
     P.map = make_tmap_bf16(P.q.p, kOzDigits * rows, K, Kp, box, 64);  // k >= K reads zeros
   }
   if (k_major) {
-    oz_split_k_kernel<<<unsigned(rows), 256, 0, s>>>(S, ld, rows, K, Kp, P.q.p, P.mx.p);
+    launch_after(s, oz_split_k_kernel, unsigned(rows), 256, 0, S, ld, rows, K, Kp, P.q.p, P.mx.p);
     EPSP_LAUNCHED(ctx);
     return;
   }
@@ -441,9 +446,9 @@ void oz_split(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_majo
   // enough blocks of k for eight a multiprocessor, of 16 k at least (a block's fixed cost), 512 at most
   const long nb = div_up(size_t(rows), 64), kb = std::max<long>(1, 8l * ctx->sm_count / nb);
   const long kper = std::min<long>(512, std::max<long>(16, (K + kb - 1) / kb));
-  oz_max_m_kernel<<<dim3(unsigned(nb), div_up(size_t(K), size_t(kper))), 256, 0, s>>>(S, ld, rows, K, kper, P.mx.p);
+  launch_after(s, oz_max_m_kernel, dim3(unsigned(nb), div_up(size_t(K), size_t(kper))), 256, 0, S, ld, rows, K, kper, P.mx.p);
   EPSP_LAUNCHED(ctx);
-  oz_split_m_kernel<<<dim3(div_up(size_t(rows), 64), div_up(size_t(Kp), 64)), 256, 0, s>>>(S, ld, rows, K, Kp, P.mx.p, P.q.p);
+  launch_after(s, oz_split_m_kernel, dim3(div_up(size_t(rows), 64), div_up(size_t(Kp), 64)), 256, 0, S, ld, rows, K, Kp, P.mx.p, P.q.p);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -452,7 +457,7 @@ static void launch_mma(Ctx* ctx, const OzPlanes& A, const OzPlanes& B, const OzS
   using L = OzSmem<BN>;
   EPSP_CUDA(cudaFuncSetAttribute(oz_mma_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
   const int items = sh.nM * sh.nN * sh.nseg * sh.per_seg;
-  oz_mma_kernel<BN><<<std::min(items, ctx->sm_count), 320, L::kBytes, ctx->stream>>>(A.map, B.map, sh, sums, err);
+  launch_after(ctx->stream, oz_mma_kernel<BN>, std::min(items, ctx->sm_count), 320, L::kBytes, A.map, B.map, sh, sums, err);
   EPSP_LAUNCHED(ctx);
 }
 
@@ -505,7 +510,7 @@ static void gemm_panel(Ctx* ctx, OzWork& W, const OzPlanes& A, long m0, long M, 
     case 128: launch_mma<128>(ctx, A, B, sh, W.sums.p, W.err.p); break;
     default: launch_mma<64>(ctx, A, B, sh, W.sums.p, W.err.p); break;
   }
-  oz_sum_kernel<<<div_up(size_t(sh.M) * size_t(sh.N), 256), 256, 0, s>>>(W.sums.p, sh.nseg, sh.M, sh.N, int(A.K),
+  launch_after(s, oz_sum_kernel, div_up(size_t(sh.M) * size_t(sh.N), 256), 256, 0, W.sums.p, sh.nseg, sh.M, sh.N, int(A.K),
                                                                         A.mx.p + m0, B.mx.p, dA, lda, dB, ldb, beta, C, ldc);
   EPSP_LAUNCHED(ctx);
 }

@@ -93,10 +93,13 @@ __global__ void fill_start_kernel(double2* __restrict__ S, double2* __restrict__
 // Σ_in = Re Σ + i min(Im Σ, -η_min) (src/scgd0.jl:256-260), for the active temperatures: slot a
 // (blockIdx.y) reads Σ of temperature slots[a] and writes Sin + a n.
 __global__ void clamp_kernel(const double2* __restrict__ S, double2* __restrict__ Sin, long n,
-                             const int* __restrict__ slots, const TParams* __restrict__ tp) {
+                             const int* __restrict__ slots, const TParams* __restrict__ tp,
+                             unsigned long long* __restrict__ errbits_all) {
+  pdl_wait();
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int a = blockIdx.y, t = slots[a];
+  if (k == 0) errbits_all[t] = 0;  // the iteration's max |ΔΣ| starts at 0
   double2 z = S[long(t) * n + k];
   Sin[long(a) * n + k] = make_double2(z.x, fmin(z.y, -tp[t].eta_min));
 }
@@ -181,6 +184,7 @@ struct FmPair {
 // Cell table of every column: entry j + 1 holds cell j, entry 0 the flat part below the grid.
 __global__ void fm_cell_kernel(const double* __restrict__ ws, int nw, const double2* __restrict__ Sin, long ncol,
                                double4* __restrict__ tab) {
+  pdl_wait();
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= (nw + 1l) * ncol) return;
   const int j = int(k % (nw + 1)) - 1;
@@ -223,6 +227,7 @@ __global__ void __launch_bounds__(512) fm_direct_fast_kernel(
     const double* __restrict__ wqt, long nvf, const double* __restrict__ eps_f, const double* __restrict__ w_f,
     const int32_t* __restrict__ f_to_i, int nm, long vf0, long vf1, long per, double mu, double T, double invT, double w_ac,
     double* __restrict__ part) {
+  pdl_wait();
   __shared__ FmPair sp[kFmFastTile];
   __shared__ int s_col[kFmFastTile];
   const int i = blockIdx.y;
@@ -289,7 +294,8 @@ __global__ void __launch_bounds__(512) fm_direct_fast_kernel(
 
 // ImΣ += Σ_s part[s]: 32 elements a block, eight runs of splits side by side, each in ascending s, added in order.
 __global__ void __launch_bounds__(256) fm_add_kernel(const double* __restrict__ part, long n, int splits,
-                                                     double* __restrict__ imsigma) {
+                                                     double* __restrict__ imsigma, bool set) {
+  pdl_wait();
   __shared__ double sh[8][32];
   const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
   const long k = long(blockIdx.x) * 32 + lane;
@@ -303,7 +309,7 @@ __global__ void __launch_bounds__(256) fm_add_kernel(const double* __restrict__ 
   if (g == 0 && k < n) {
 #pragma unroll
     for (int r = 1; r < 8; ++r) v += sh[r][lane];
-    imsigma[k] += v;
+    imsigma[k] = set ? v : imsigma[k] + v;
   }
 }
 
@@ -312,6 +318,7 @@ __global__ void __launch_bounds__(256) fm_add_kernel(const double* __restrict__ 
 // below ω_acoustic.
 __global__ void occ_table_kernel(const double* __restrict__ ws, int nw, const double* __restrict__ wnu, int nm,
                                  double mu, double T, double w_ac, double* __restrict__ Fa, double* __restrict__ Fe) {
+  pdl_wait();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nw * nm) return;
   int iw = k % nw, nu = k / nw;
@@ -338,6 +345,7 @@ __global__ void kbuild_f64_kernel(int nw, const double4* __restrict__ tab, const
                                   const double* __restrict__ eps_c, const int32_t* __restrict__ col_c,
                                   const double* __restrict__ Fa, const double* __restrict__ Fe, double w_ac,
                                   double* __restrict__ Kt) {
+  pdl_wait();
   const int iw = blockIdx.x * blockDim.x + threadIdx.x;
   const long kc = blockIdx.y;  // (ν, c) with ν fastest
   if (iw >= nw) return;
@@ -386,10 +394,46 @@ __global__ void coupling_sum_chunk_kernel(const T* __restrict__ g2c, int nm, int
 }
 
 // Σ_new = ReΣ + i ImΣ (src/scgd0.jl:290-291).
-__global__ void assemble_kernel(const double* __restrict__ re, const double* __restrict__ im, double2* __restrict__ out,
-                                long n) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = make_double2(re[k], im[k]);
+// max of |a - S[k]| over the block's elements into *errbits, and S[k] ← a (src/scgd0.jl:326-328). The maximum of
+// non-negative doubles is taken on their bit patterns, which order the same way; NaN wins, as in Julia's maximum.
+__device__ __forceinline__ void err_copy(double2 a, bool on, double2* S, unsigned long long* errbits) {
+  __shared__ unsigned long long sh[256];
+  unsigned long long e = 0;
+  if (on) {
+    const double2 b = *S;
+    e = (unsigned long long)__double_as_longlong(hypot(a.x - b.x, a.y - b.y));
+    *S = a;
+  }
+  sh[threadIdx.x] = e;
+  __syncthreads();
+  for (int s = 128; s > 0; s >>= 1) {
+    if (threadIdx.x < s) sh[threadIdx.x] = max(sh[threadIdx.x], sh[threadIdx.x + s]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) atomicMax(errbits, sh[0]);
+}
+
+// Σ_new = re + i im of one temperature; with S, which then is its Σ, also max |Σ_new - Σ| and Σ ← Σ_new. Hands the
+// products' error flag on to the host's copy. 256 threads.
+__global__ void __launch_bounds__(256) assemble_kernel(const double* __restrict__ re, const double* __restrict__ im,
+                                                       double2* __restrict__ out, long n, double2* __restrict__ S,
+                                                       unsigned long long* __restrict__ errbits,
+                                                       const int* __restrict__ tcerr, int* __restrict__ tcerr_out) {
+  pdl_wait();
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k == 0) *tcerr_out = *tcerr;
+  const double2 a = k < n ? make_double2(re[k], im[k]) : make_double2(0.0, 0.0);
+  if (k < n) out[k] = a;
+  if (S) err_copy(a, k < n, S + k, errbits);
+}
+
+// The same where the multiplets' average comes between: max |Σ_new - Σ| and Σ ← Σ_new of every slot. 256 threads.
+__global__ void __launch_bounds__(256) err_copy_kernel(const double2* __restrict__ Snew_all, double2* __restrict__ S_all, long n,
+                                                       const int* __restrict__ slots,
+                                                       unsigned long long* __restrict__ errbits_all) {
+  pdl_wait();
+  const long k = long(blockIdx.x) * blockDim.x + threadIdx.x, t = slots[blockIdx.y];
+  err_copy(k < n ? Snew_all[t * n + k] : make_double2(0.0, 0.0), k < n, S_all + t * n + k, errbits_all + t);
 }
 
 __global__ void assemble_f32_kernel(const float* __restrict__ re, const float* __restrict__ im, double2* __restrict__ out,
@@ -402,6 +446,7 @@ __global__ void assemble_f32_kernel(const float* __restrict__ re, const float* _
 // over members in order divided by the count.
 __global__ void multiplet_kernel(double2* __restrict__ Sall, int nw, long slab, const int* __restrict__ slots,
                                  const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx, long nmult) {
+  pdl_wait();
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= long(nw) * nmult) return;
   double2* S = Sall + slab * slots[blockIdx.y];
@@ -438,6 +483,7 @@ __global__ void spectral_A_kernel(const double2* __restrict__ Sall, int nw, long
                                   const double* __restrict__ wsa, int nwa, const int32_t* __restrict__ jsp,
                                   const double* __restrict__ tsp, const double* __restrict__ eps_i,
                                   double* __restrict__ Aall, int ni) {
+  pdl_wait();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y;
   if (a >= nwa) return;
@@ -471,6 +517,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 // colsum[i] = Σ_a A[a, i] Wa[a] (the ∫A_i of min_spectral_weight, src/scgd0.jl:308).
 __global__ void __launch_bounds__(256) spectral_colsum_kernel(const double* __restrict__ Aall, int nwa, int ni,
                                                               const double* __restrict__ Wa, double* __restrict__ colsum_all) {
+  pdl_wait();
   __shared__ double sh[256];
   int i = blockIdx.x;
   const double* A = Aall + long(nwa) * ni * blockIdx.y;
@@ -549,6 +596,7 @@ __global__ void __launch_bounds__(kSpecNodes) spectral_ad_f32_kernel(
 
 __global__ void __launch_bounds__(256) min_kernel(const double* __restrict__ xall, int n, const int* __restrict__ slots,
                                                   double* __restrict__ out_all) {
+  pdl_wait();
   __shared__ double sh[256];
   const double* x = xall + long(n) * blockIdx.x;
   double* out = out_all + slots[blockIdx.x];
@@ -756,6 +804,7 @@ __global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restric
                                                          const double* __restrict__ w_i, const double* __restrict__ Wa,
                                                          const double* __restrict__ wsa, const int* __restrict__ slots,
                                                          double* __restrict__ Dall, const MuIn M) {
+  pdl_wait();
   __shared__ double sh[8][32];
   const double* A = Aall + long(nwa) * ni * blockIdx.y;
   double* D = Dall + long(nwa) * blockIdx.y;
@@ -976,39 +1025,6 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
       status_all[t] = 0;
     }
   }
-}
-
-// err = max |Σ_new - Σ| over one temperature, and Σ ← Σ_new (src/scgd0.jl:326-328). The maximum of
-// non-negative doubles is taken on their bit patterns, which order the same way; NaN wins, as in
-// Julia's maximum.
-// F32 (tensor-core path): the differences in FP64, their magnitude in FP32.
-template <bool F32>
-__global__ void err_copy_kernel(const double2* __restrict__ Snew_all, double2* __restrict__ S_all, long n,
-                                const int* __restrict__ slots, unsigned long long* __restrict__ errbits_all) {
-  __shared__ unsigned long long sh[256];
-  const int t = slots[blockIdx.y];
-  const double2* Snew = Snew_all + long(t) * n;
-  double2* S = S_all + long(t) * n;
-  unsigned long long* errbits = errbits_all + t;
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  unsigned long long e = 0;
-  if (k < n) {
-    double2 a = Snew[k], b = S[k];
-    double d;
-    if constexpr (F32)
-      d = double(hypotf(float(a.x - b.x), float(a.y - b.y)));
-    else
-      d = hypot(a.x - b.x, a.y - b.y);
-    e = (unsigned long long)__double_as_longlong(d);
-    S[k] = a;
-  }
-  sh[threadIdx.x] = e;
-  __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] = max(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) atomicMax(errbits, sh[0]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1339,7 +1355,8 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
 // one Fan-Migdal sum at one temperature: ImΣ += Σ (src/scgd0_kernel.jl:59-86)
 // ---------------------------------------------------------------------------------------------
 
-void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, double* d_ImS) {
+// With `set`, for which d_ImS need not be zeroed, ImΣ = Σ (the FP64 paths).
+void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, double* d_ImS, bool set = false) {
   Ctx* ctx = P->ctx;
   cudaStream_t s = ctx->stream;
   const long nm = P->nm, ni = P->ni, nf = P->nf, nw = P->nw;
@@ -1353,7 +1370,7 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
     if (fast) {
       const long n = (nw + 1) * ni;
       ensure(P->w_fmtab, ctx, size_t(n));
-      fm_cell_kernel<<<div_up(size_t(n), 128), 128, 0, s>>>(P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
+      launch_after(s, fm_cell_kernel, div_up(size_t(n), 128), 128, 0, P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
       EPSP_LAUNCHED(ctx);
     }
     for (long f0 = 0; f0 < nf; f0 += P->nf_chunk) {
@@ -1366,13 +1383,14 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
         const long per = std::max<long>(8, (len + want - 1) / want);
         const int splits = int((len + per - 1) / per);
         ensure(P->w_fmpart, ctx, size_t(nw * ni * splits));
-        fm_direct_fast_kernel<<<dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0, s>>>(
+        launch_after(s, fm_direct_fast_kernel, dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0, 
             P->d_ws.p, int(nw), P->d_wkey.p, P->d_jtab.p, int(P->d_jtab.n), float(P->ct.x0), float(P->ct.inv_h),
             P->fm_guard, P->w_fmtab.p, P->d_g2t.p, P->d_wqt.p, nvf, P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm),
             nm * f0, nm * f1, per, mu, T, 1.0 / T, P->w_ac, P->w_fmpart.p);
         EPSP_LAUNCHED(ctx);
-        fm_add_kernel<<<div_up(size_t(nw * ni), 32), 256, 0, s>>>(P->w_fmpart.p, nw * ni, splits, d_ImS);
+        launch_after(s, fm_add_kernel, div_up(size_t(nw * ni), 32), 256, 0, P->w_fmpart.p, nw * ni, splits, d_ImS, set && f0 == 0);
       } else {
+        if (set && f0 == 0) EPSP_CUDA(cudaMemsetAsync(d_ImS, 0, size_t(nw * ni) * sizeof(double), s));
         fm_direct_kernel<<<tiles, kFmTile, 0, s>>>(P->d_ws.p, int(nw), P->ct, d_Sin, P->d_g2t.p, P->d_wqt.p, nvf,
                                                    P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm), nm * f0, nm * f1, mu,
                                                    T, P->w_ac, d_ImS);
@@ -1386,23 +1404,23 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
     tc_imsigma_disp(P, d_Sin, mu, T, d_ImS);
     return;
   }
-  occ_table_kernel<<<div_up(size_t(nw * nm), 256), 256, 0, s>>>(P->d_ws.p, int(nw), P->d_wnu.p, int(nm), mu, T, P->w_ac,
+  launch_after(s, occ_table_kernel, div_up(size_t(nw * nm), 256), 256, 0, P->d_ws.p, int(nw), P->d_wnu.p, int(nm), mu, T, P->w_ac,
                                                                  P->d_Fa.p, P->d_Fe.p);
   EPSP_LAUNCHED(ctx);
   const long nk = nm * P->nc;
   if (P->path == EPSP_PATH_GEMM_FP64) {
     long pk = prof_begin(ctx, "kbuild");
     ensure(P->w_fmtab, ctx, size_t((nw + 1) * ni));
-    fm_cell_kernel<<<div_up(size_t((nw + 1) * ni), 128), 128, 0, s>>>(P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
+    launch_after(s, fm_cell_kernel, div_up(size_t((nw + 1) * ni), 128), 128, 0, P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
     EPSP_LAUNCHED(ctx);
-    kbuild_f64_kernel<<<dim3(div_up(size_t(nw), 128), unsigned(nk)), 128, 0, s>>>(
+    launch_after(s, kbuild_f64_kernel, dim3(div_up(size_t(nw), 128), unsigned(nk)), 128, 0, 
         int(nw), P->w_fmtab.p, P->d_cell_j.p, P->d_cell_t.p, P->d_wnu.p, int(nm), P->d_epsc.p, P->d_colc.p, P->d_Fa.p,
         P->d_Fe.p, P->w_ac, P->d_Kt.p);
     EPSP_LAUNCHED(ctx);
     prof_end(ctx, pk);
     long pg = prof_begin(ctx, "fm_gemm");
     // ImΣ[ω, i] += Σ_k K_t[ω, k] G[k, i]
-    oz_gemm(ctx, P->oz, nw, ni, nk, P->d_Kt.p, nw, nullptr, P->d_G.p, nk, &P->ozG, 1.0, d_ImS, nw);
+    oz_gemm(ctx, P->oz, nw, ni, nk, P->d_Kt.p, nw, nullptr, P->d_G.p, nk, &P->ozG, set ? 0.0 : 1.0, d_ImS, nw);
     prof_end(ctx, pg);
     return;
   }
@@ -1578,9 +1596,9 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       mu_in.br1 = br1;
       mu_in.E = P->w_E.p;
       mu_in.part = P->w_R1.p;
-      if (P->path != EPSP_PATH_GEMM_BF16 || P->disp) EPSP_CUDA(cudaMemsetAsync(d_err, 0, size_t(nT) * 8, s));
+      if (P->path == EPSP_PATH_GEMM_BF16 && P->disp) EPSP_CUDA(cudaMemsetAsync(d_err, 0, size_t(nT) * 8, s));
       if (P->path != EPSP_PATH_GEMM_BF16) {
-        clamp_kernel<<<dim3(eb, unsigned(nA)), 256, 0, s>>>(S.p, Sin_b.p, slab, d_slots.p, d_tp.p);
+        launch_after(s, clamp_kernel, dim3(eb, unsigned(nA)), 256, 0, S.p, Sin_b.p, slab, d_slots.p, d_tp.p, d_err);
         EPSP_LAUNCHED(ctx);
       }
       if (P->path == EPSP_PATH_GEMM_BF16) {
@@ -1590,18 +1608,18 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
       } else {
         for (int a = 0; a < nA; ++a) {
           const int64_t iT = slots[size_t(a)];
-          P->d_ImS.zero(s);
-          scgd0_imsigma(P, Sin_b.p + slab * a, mu[size_t(iT)], occ->Tlist[iT], P->d_ImS.p);
+          scgd0_imsigma(P, Sin_b.p + slab * a, mu[size_t(iT)], occ->Tlist[iT], P->d_ImS.p, true);
           long pk = prof_begin(ctx, "kk");
           oz_gemm(ctx, P->oz, nw, ni, nw, P->d_KK.p, nw, &P->ozKK, P->d_ImS.p, nw, nullptr, 0.0, P->d_ReS.p, nw);
-          assemble_kernel<<<eb, 256, 0, s>>>(P->d_ReS.p, P->d_ImS.p, Snew.p + slab * iT, slab);
+          const bool last = P->nmult == 0;  // no multiplet average to come: max |ΔΣ| and Σ ← Σ_new in the same pass
+          launch_after(s, assemble_kernel, eb, 256, 0, P->d_ReS.p, P->d_ImS.p, Snew.p + slab * iT, slab,
+                                             last ? S.p + slab * iT : nullptr, d_err + iT, P->oz.err.p, d_tcerr);
           EPSP_LAUNCHED(ctx);
           prof_end(ctx, pk);
         }
       }
-      if (!f32_spec) EPSP_CUDA(cudaMemcpyAsync(d_tcerr, P->oz.err.p, sizeof(int), cudaMemcpyDeviceToDevice, s));
       if (P->nmult > 0 && !f32_spec) {
-        multiplet_kernel<<<dim3(div_up(size_t(nw * P->nmult), 256), unsigned(nA)), 256, 0, s>>>(
+        launch_after(s, multiplet_kernel, dim3(div_up(size_t(nw * P->nmult), 256), unsigned(nA)), 256, 0, 
             Snew.p, int(nw), slab, d_slots.p, P->d_mptr.p, P->d_midx.p, P->nmult);
         EPSP_LAUNCHED(ctx);
       }
@@ -1616,16 +1634,16 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
                      D_b.p, d_minA, mu_in, tc_err_ptr(P), d_tcerr, d_err, ctl);
         EPSP_LAUNCHED(ctx);
       } else {
-        spectral_A_kernel<<<dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0, s>>>(
+        launch_after(s, spectral_A_kernel, dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0, 
             Snew.p, int(nw), slab, d_slots.p, P->d_wsa.p, int(nwa), P->d_jsp.p, P->d_tsp.p, P->d_eps_i.p, A_b.p, int(ni));
         EPSP_LAUNCHED(ctx);
-        spectral_colsum_kernel<<<dim3(unsigned(ni), unsigned(nA)), 256, 0, s>>>(A_b.p, int(nwa), int(ni), P->d_Wa.p,
+        launch_after(s, spectral_colsum_kernel, dim3(unsigned(ni), unsigned(nA)), 256, 0, A_b.p, int(nwa), int(ni), P->d_Wa.p,
                                                                               colsum_b.p);
         EPSP_LAUNCHED(ctx);
-        min_kernel<<<unsigned(nA), 256, 0, s>>>(colsum_b.p, int(ni), d_slots.p, d_minA);
+        launch_after(s, min_kernel, unsigned(nA), 256, 0, colsum_b.p, int(ni), d_slots.p, d_minA);
         EPSP_LAUNCHED(ctx);
         if (!fix_mu) {
-          spectral_D_kernel<<<dim3(unsigned(spec_nab), unsigned(nA)), 256, 0, s>>>(
+          launch_after(s, spectral_D_kernel, dim3(unsigned(spec_nab), unsigned(nA)), 256, 0, 
               A_b.p, int(nwa), int(ni), P->d_w_i.p, P->d_Wa.p, P->d_wsa.p, d_slots.p, D_b.p, mu_in);
           EPSP_LAUNCHED(ctx);
         }
@@ -1639,8 +1657,8 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
         EPSP_LAUNCHED(ctx);
         prof_end(ctx, pm);
       }
-      if (P->path != EPSP_PATH_GEMM_BF16) {  // (the tensor-core epilogue took err and the copy)
-        err_copy_kernel<false><<<dim3(eb, unsigned(nA)), 256, 0, s>>>(Snew.p, S.p, slab, d_slots.p, d_err);
+      if (P->path != EPSP_PATH_GEMM_BF16 && P->nmult > 0) {  // (the tensor-core epilogue took err and the copy)
+        launch_after(s, err_copy_kernel, dim3(eb, unsigned(nA)), 256, 0, Snew.p, S.p, slab, d_slots.p, d_err);
         EPSP_LAUNCHED(ctx);
       }
     };

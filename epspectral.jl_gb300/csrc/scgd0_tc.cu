@@ -760,7 +760,7 @@ __global__ void finalize_fm_batch_kernel(const float* __restrict__ part, int nw,
 // multiplet, or a single state -- Σ_new(ω_j) = Σ_s part[s] + i ImΣ of every member (the partials in
 // ascending order), averaged over the members of a multiplet (their sum in member order divided by
 // the count); then per member: err = max |Σ_new - Σ| over the slot's temperature (FP64 differences,
-// FP32 magnitude, the maximum taken on the bit patterns as err_copy_kernel does), Σ ← Σ_new, its clamped form for the
+// FP32 magnitude, the maximum taken on the bit patterns as err_copy does), Σ ← Σ_new, its clamped form for the
 // next iteration -- the columns' cell records (rec, dim), or Sf with dispersive modes (rec null) -- and the
 // spectral functions' per-node terms P[i][j] = (ε_i - ω_j + ReΣ_j, ReΣ_{j+1} - ReΣ_j, ImΣ_j, ImΣ_{j+1})
 // (ImΣ_{j+1}, ReΣ_{j+1} = those of j at the last node). Everything but Σ itself and its change is formed on float pairs

@@ -1074,7 +1074,9 @@ __global__ void finish_gemm_kernel(const R* __restrict__ D_all, long ldD, int ds
 // Batched over blockIdx.y: slot z works on the vectors of right-hand side r = rmap[z] (r = z without
 // rmap), stored n apart.
 
-constexpr int kDotBlocks = 1024;
+// Three blocks an SM: a block's tree of FP64 sums takes as long as eight elements a thread (1024 blocks: the 9-state
+// ladder 1.78 ms, 456: 1.70, 304: 1.71 but the 16-state step 4.95 instead of 4.88).
+constexpr int kDotBlocks = 456;
 constexpr int kRun = 8;  // elements per FP32 run of the float2 reductions
 
 template <class V>
@@ -2667,7 +2669,7 @@ __global__ void propagators_batch_kernel(const double2* __restrict__ S_all, cons
 }
 
 // The batched BLAS-1 are the kernels above with blockIdx.y over the slots and rmap.
-constexpr int kDotBlocksB = 256;
+constexpr int kDotBlocksB = 128;  // a right-hand side (256: the map of 16 4.48 ms, 128: 4.43)
 
 // Buffers of a batch of right-hand sides (capacity cap), tensor maps over them.
 struct LadderBatch {

@@ -206,11 +206,27 @@ __global__ void __launch_bounds__(320, 1)
     o.alone = n == 1;
     return o;
   };
-  // chunk c of order d: digits (s, d - s) and its K blocks [b0, b1)
-  auto chunk_of = [&](const Item& o, int c, int& s, int& b0, int& b1) {
-    s = max(0, o.d - (kOzDigits - 1)) + c / sh.nkc;
-    b0 = (o.seg * sh.nkc + c % sh.nkc) * (kOzChunk / 64);
-    b1 = min(sh.kblocks, b0 + kOzChunk / 64);
+  // the chunks of an item in order: digits (s, d - s) and K blocks [b0, b1)
+  struct Chunk {
+    int s, k, b0, b1;
+  };
+  auto chunk_at = [&](const Item& o, Chunk& c) {
+    c.b0 = (o.seg * sh.nkc + c.k) * (kOzChunk / 64);
+    c.b1 = min(sh.kblocks, c.b0 + kOzChunk / 64);
+  };
+  auto chunk_first = [&](const Item& o) {
+    Chunk c;
+    c.s = max(0, o.d - (kOzDigits - 1)) + o.c0 / sh.nkc;
+    c.k = o.c0 % sh.nkc;
+    chunk_at(o, c);
+    return c;
+  };
+  auto chunk_next = [&](const Item& o, Chunk& c) {
+    if (++c.k == sh.nkc) {
+      c.k = 0;
+      ++c.s;
+    }
+    chunk_at(o, c);
   };
 
   if (threadIdx.x == 0) {
@@ -239,10 +255,9 @@ __global__ void __launch_bounds__(320, 1)
     bool stop = false;
     for (int it = int(blockIdx.x); it < nitems && !stop; it += int(gridDim.x)) {
       const Item o = item_of(it);
-      for (int c = o.c0; c < o.c1 && !stop; ++c) {
-        int s, b0, b1;
-        chunk_of(o, c, s, b0, b1);
-        for (int kb = b0; kb < b1; ++kb) {
+      Chunk ch = chunk_first(o);
+      for (int c = o.c0; c < o.c1 && !stop; ++c, chunk_next(o, ch)) {
+        for (int kb = ch.b0; kb < ch.b1; ++kb) {
           const int st = g % STAGES;
           if (g >= STAGES && !mbar_wait(empty0 + 8 * st, ((g / STAGES) & 1) ^ 1)) {
             atomicExch(&s_abort, 1);
@@ -256,8 +271,8 @@ __global__ void __launch_bounds__(320, 1)
           const uint32_t dst = smem_u32(smem + st * L::kStage), fb = full0 + 8 * st;
           mbar_expect_tx(fb, L::kStage);
           // a tile past its plane's last row reads the next plane (or zeros): rows that are not stored
-          tma_load_2d(dst, &mapA, kb * 64, s * sh.rowsA + sh.m0 + o.mt * kTcBM, fb);
-          tma_load_2d(dst + L::kA, &mapB, kb * 64, (o.d - s) * sh.N + o.nt * BN, fb);
+          tma_load_2d(dst, &mapA, kb * 64, ch.s * sh.rowsA + sh.m0 + o.mt * kTcBM, fb);
+          tma_load_2d(dst + L::kA, &mapB, kb * 64, (o.d - ch.s) * sh.N + o.nt * BN, fb);
           ++g;
         }
       }
@@ -266,13 +281,14 @@ __global__ void __launch_bounds__(320, 1)
       for (int k = max(0, g - STAGES); k < g; ++k) mbar_wait(full0 + 8 * (k % STAGES), (k / STAGES) & 1);
   } else if (warp == 1 && lane == 0) {
     constexpr uint32_t idesc = idesc_f32acc<false>(BN);
-    int g = 0, t = 0;
+    const uint64_t desc0 = sw128_desc(smem_u32(smem));
+    int st = 0, t = 0;
+    uint32_t ph = 0;  // the ring's stage and the parity of its turn
     bool stop = false;
     for (int it = int(blockIdx.x); it < nitems && !stop; it += int(gridDim.x)) {
       const Item o = item_of(it);
-      for (int c = o.c0; c < o.c1 && !stop; ++c, ++t) {
-        int s, b0, b1;
-        chunk_of(o, c, s, b0, b1);
+      Chunk ch = chunk_first(o);
+      for (int c = o.c0; c < o.c1 && !stop; ++c, ++t, chunk_next(o, ch)) {
         const int b = t & 1;
         const uint32_t acc = tmem + uint32_t(b * BN);
         if (t >= 2 && !mbar_wait(acce0 + 8 * b, ((t >> 1) & 1) ^ 1)) {
@@ -281,20 +297,22 @@ __global__ void __launch_bounds__(320, 1)
           break;
         }
         tc_fence_after();
-        for (int kb = b0; kb < b1; ++kb) {
-          const int st = g % STAGES;
-          if (!mbar_wait_issuer(full0 + 8 * st, (g / STAGES) & 1, &s_abort)) {
+        for (int kb = ch.b0; kb < ch.b1; ++kb) {
+          if (!mbar_wait_issuer(full0 + 8 * st, ph, &s_abort)) {
             atomicExch(&s_abort, 1);
             stop = true;
             break;
           }
           tc_fence_after();
-          const uint32_t a0 = smem_u32(smem + st * L::kStage), bb = a0 + L::kA;
+          // (an operand's descriptor holds its address / 16 in the low bits)
+          const uint64_t da = desc0 + uint64_t(st * (L::kStage / 16)), db = da + L::kA / 16;
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma<false>(acc, sw128_desc(a0 + ks * 32), sw128_desc(bb + ks * 32), idesc, kb > b0 || ks > 0);
+          for (int ks = 0; ks < 4; ++ks) umma<false>(acc, da + 2 * ks, db + 2 * ks, idesc, kb > ch.b0 || ks > 0);
           umma_commit(empty0 + 8 * st);
-          ++g;
+          if (++st == STAGES) {
+            st = 0;
+            ph ^= 1;
+          }
         }
         umma_commit(accf0 + 8 * b);
       }
@@ -309,7 +327,8 @@ __global__ void __launch_bounds__(320, 1)
       uint32_t acc[kCols];
 #pragma unroll
       for (int j = 0; j < kCols; ++j) acc[j] = 0u - uint32_t(o.c1 - o.c0) * 0x4B400000u;
-      for (int c = o.c0; c < o.c1; ++c, ++t) {
+      Chunk ch = chunk_first(o);
+      for (int c = o.c0; c < o.c1; ++c, ++t, chunk_next(o, ch)) {
         const int b = t & 1;
         if (!mbar_wait(accf0 + 8 * b, (t >> 1) & 1)) atomicExch(&s_abort, 1);
         if (aborted()) {
@@ -317,9 +336,7 @@ __global__ void __launch_bounds__(320, 1)
           break;
         }
         tc_fence_after();
-        int s, b0, b1;
-        chunk_of(o, c, s, b0, b1);
-        const bool some = b0 < b1;  // a chunk past the last segment's end: no product, the sum is 0
+        const bool some = ch.b0 < ch.b1;  // a chunk past the last segment's end: no product, the sum is 0
 #pragma unroll
         for (int j0 = 0; j0 < kCols; j0 += 32) {
           float v[32];

@@ -457,6 +457,10 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // search for the nearest node and a record for either side of it, 2.30 now: 7.7 wavefronts a side and warp keep the L1
 // data pipe 90 % busy (4.7 of them the records, 20 bytes a lane), the issue slots 71 %.
 constexpr float kFdMaxArg = 40.f;
+// Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
+// modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
+// kernel above 5.6e-8, 2.1e-8. Shorter runs take the FP64 pipe's time: 28.3, 28.6, 28.9 ms a run.
+constexpr int kFdRun = 64;
 constexpr long kFdMaxTable = 1l << 24;  // entries; those that fit 96 KB are kept in shared memory
 constexpr long kFdMaxCell = 32767;      // grid units of a cell or ωq: distances are 16 bits
 
@@ -560,33 +564,36 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     // (a warp past the last node, or whose second nodes are, does that part of the work no more than it must)
     if (iw0 - int(threadIdx.x % 32) >= nw) continue;
     const bool both = NPT == 1 || iw0 - int(threadIdx.x % 32) + kFdTile < nw;
-    float run0[NPT], run1[NPT];
-#pragma unroll
-    for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
     auto terms = [&](auto nodes) {
-#pragma unroll 2
-      for (int k = 0; k < nt; ++k) {
-        const float4 A = s_a[k], Q = s_e[k];
-        const int2 C = s_c[k];
-        const float2 e = make_float2(Q.x, Q.y);
+      for (int k0 = 0; k0 < nt; k0 += kFdRun) {
+        float run0[NPT], run1[NPT];
 #pragma unroll
-        for (int n = 0; n < decltype(nodes)::value; ++n) {
-          side(off[n] + C.y, Q.z, e, C.x, fmaf(q[n], A.z, p[n]), A.x, run0[n]);
-          side(off[n] - C.y - 1, Q.w, e, C.x, fmaf(q[n], A.w, p[n]), A.y, run1[n]);
+        for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
+        const int k1 = min(nt, k0 + kFdRun);
+#pragma unroll 2
+        for (int k = k0; k < k1; ++k) {
+          const float4 A = s_a[k], Q = s_e[k];
+          const int2 C = s_c[k];
+          const float2 e = make_float2(Q.x, Q.y);
+#pragma unroll
+          for (int n = 0; n < decltype(nodes)::value; ++n) {
+            side(off[n] + C.y, Q.z, e, C.x, fmaf(q[n], A.z, p[n]), A.x, run0[n]);
+            side(off[n] - C.y - 1, Q.w, e, C.x, fmaf(q[n], A.w, p[n]), A.y, run1[n]);
+          }
         }
+#pragma unroll
+        for (int n = 0; n < decltype(nodes)::value; ++n) acc[n] += double(run0[n]) + double(run1[n]);
       }
     };
     if (both)
       terms(std::integral_constant<int, NPT>{});
     else
       terms(std::integral_constant<int, 1>{});
-#pragma unroll
-    for (int n = 0; n < NPT; ++n) acc[n] += double(run0[n]) + double(run1[n]);
   }
 #pragma unroll
   for (int n = 0; n < NPT; ++n) {
     const int iw = iw0 + kFdTile * n;
-    if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc[n] * double(p[n] + q[n]);
+    if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc[n] * (double(p[n]) + double(q[n]));
   }
 }
 

@@ -1077,6 +1077,9 @@ __global__ void finish_gemm_kernel(const R* __restrict__ D_all, long ldD, int ds
 // Three blocks an SM: a block's tree of FP64 sums takes as long as eight elements a thread (1024 blocks: the 9-state
 // ladder 1.78 ms, 456: 1.70, 304: 1.71 but the 16-state step 4.95 instead of 4.88).
 constexpr int kDotBlocks = 456;
+// maxpy_kernel's blocks (one tree each): more from 16 elements a thread on, where its loads and stores in flight bound it
+// (n = 1.5e7: 1024 blocks 72 us, 456 108).
+static int maxpy_blocks(long n) { return n > 16l * 256 * kDotBlocks ? 1024 : kDotBlocks; }
 constexpr int kRun = 8;  // elements per FP32 run of the float2 reductions
 
 template <class V>
@@ -2485,11 +2488,11 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
             for (int i0 = 0; i0 < inner; i0 += kMG) {
               const int m = std::min(kMG, inner - i0);
               const bool last = pass == npass - 1 && i0 + m >= inner;
-              launch_after(s, maxpy_kernel<V>, kDotBlocks, 256, 0, W.p, vp, i0, m, hp, n, last ? part.p : nullptr);
+              launch_after(s, maxpy_kernel<V>, maxpy_blocks(n), 256, 0, W.p, vp, i0, m, hp, n, last ? part.p : nullptr);
               EPSP_LAUNCHED(ctx);
             }
           }
-          launch_after(s, dot_final_kernel, 1, 256, 0, part.p, kDotBlocks, nullptr, P->g_hsq.p);
+          launch_after(s, dot_final_kernel, 1, 256, 0, part.p, maxpy_blocks(n), nullptr, P->g_hsq.p);
           EPSP_LAUNCHED(ctx);
           launch_after(s, gmres_givens_kernel, 1, 32, 0, P->g_h1.p, npass == 2 ? P->g_h2.p : nullptr, P->g_hsq.p, Hdev.p + hN0,
                                                Hdev.p + (warm ? hB2 : hN0), rtol, btol, inner, P->g_R.p, P->g_cs.p,

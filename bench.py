@@ -55,8 +55,8 @@ FP64_LADDER_APPLIES = 2
 # DRAM bytes (read + write) and tensor-pipe activity of one ladder-contraction launch of this
 # workload (Z = Jr Bz, the TF32 persistent CTA-pair kernel), from one Nsight Compute
 # capture of the same kernel on a GB300 (summarised with the other captures under profiles/)
-TC_LADDER_TRAFFIC_BYTES = 1.643e9 + 1.786e9
-TC_LADDER_TENSOR_PIPE_ACTIVE = 0.633
+TC_LADDER_TRAFFIC_BYTES = 1.567e9 + 1.786e9
+TC_LADDER_TENSOR_PIPE_ACTIVE = 0.717
 # learned warm start: training and held-out runs, epochs
 WARM_TRAIN_RUNS, WARM_HELDOUT_RUNS, WARM_EPOCHS = 256, 32, 40
 

@@ -936,7 +936,7 @@ void epsp_warmstart_destroy(epsp_warmstart* w) {
 int64_t epsp_warmstart_nparams(const epsp_warmstart* w) { return w ? nparams(&w->m) : 0; }
 
 /* Device milliseconds of the epochs of the last epsp_warmstart_train (CUDA events around each
- * epoch's graph replay; the uploads and the capture are not included). */
+ * epoch's graph replays; the uploads and the capture are not included). */
 double epsp_warmstart_train_ms(const epsp_warmstart* w) { return w ? w->m.train_ms : 0.0; }
 
 /* Parameters as one flat FP32 vector: for each layer, W [d_{l+1}][d_l] then b [d_{l+1}]. Setting

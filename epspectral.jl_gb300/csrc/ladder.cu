@@ -1076,8 +1076,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) finish_gemm_kerne
 // Batched over blockIdx.y: slot z works on the vectors of right-hand side r = rmap[z] (r = z without
 // rmap), stored n apart.
 
-// Three blocks an SM: a block's tree of FP64 sums takes as long as eight elements a thread (1024 blocks: the 9-state
-// ladder 1.78 ms, 456: 1.70, 304: 1.71 but the 16-state step 4.95 instead of 4.88).
+// Three blocks an SM: a block's tree of FP64 sums takes as long as eight elements a thread (1024 blocks: the ladder
+// of 105 states x 625 nodes 1.78 ms, 456: 1.70, 304: 1.71 but a step of 495 x 1251 4.95 instead of 4.88).
 constexpr int kDotBlocks = 456;
 // maxpy_kernel's blocks (one tree each): more from 16 elements a thread on, where its loads and stores in flight bound it
 // (n = 1.5e7: 1024 blocks 72 us, 456 108).

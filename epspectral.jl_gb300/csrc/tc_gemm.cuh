@@ -67,7 +67,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
 // The same for the thread that issues MMAs: it also gives up once another warp set *abort, which it
 // reads only while it is kept waiting. Its shared-memory loads wait behind the MMAs it has queued,
 // so a look at the flag for every K block left the tensor cores idle for 240 of 726 clocks (the
-// TF32 ladder contraction of 16 states x 1251 nodes x 15 modes on CTA pairs: 1841 -> 1576 us).
+// TF32 ladder contraction of 495 states x 1251 nodes x 15 modes on CTA pairs: 1841 -> 1576 us).
 __device__ __forceinline__ bool mbar_wait_issuer(uint32_t bar, uint32_t parity, const int* abort,
                                                  unsigned limit = kWaitLimit) {
   for (unsigned it = 0; it < limit; ++it) {

@@ -478,7 +478,9 @@ __device__ __forceinline__ double imag_inv_d(double c, double d) {
 // Spectral functions on ωs_spectral (src/scgd0.jl:303-305): A[a, i] = -Im(1/(ωa - ε_i -
 // Σ(ωa)))/π with Σ read by the table (j_sp, t_sp) (apply_interpolation_table!).
 
-// FP64 paths (the tensor-core path has its own FP32 kernels below).
+// FP64 paths (the tensor-core path has its own FP32 kernels below). The FP64 pipe bounds it (an instruction a warp in 16
+// cycles): A = d / (π |z|²) with one refined reciprocal takes 15 of them an element, Smith's quotient and the division by
+// π, which stay for |z|² near the ends of the range, 43 (3201 x 105: 25.4 -> 12.1 us).
 __global__ void spectral_A_kernel(const double2* __restrict__ Sall, int nw, long slab, const int* __restrict__ slots,
                                   const double* __restrict__ wsa, int nwa, const int32_t* __restrict__ jsp,
                                   const double* __restrict__ tsp, const double* __restrict__ eps_i,
@@ -495,8 +497,10 @@ __global__ void spectral_A_kernel(const double2* __restrict__ Sall, int nw, long
   double2 lo = col[j], hi = col[j + 1];
   double sr = (1 - t) * lo.x + t * hi.x;
   double si = (1 - t) * lo.y + t * hi.y;
-  const double c = wsa[a] - eps_i[i] - sr;
-  A[a + long(nwa) * i] = -imag_inv_d(c, -si) / 3.14159265358979323846;
+  const double c = wsa[a] - eps_i[i] - sr, d = -si, q = fma(c, c, d * d);
+  const int e = (__double2hiint(q) >> 20) & 0x7ff;
+  A[a + long(nwa) * i] = e > 0x100 && e < 0x700 ? d * recip_seeded(q) * 0.31830988618379067154
+                                                : -imag_inv_d(c, d) / 3.14159265358979323846;
 }
 
 // Fixed-order block reduction helpers (deterministic for a fixed block size).

@@ -105,3 +105,19 @@ def test_direct_sum_matches_oracle(api, oracle, nw, ni, nm, nf, T, mu, graded):
         assert np.all(np.isfinite(got)) and rel(got, ref) <= 1e-13
         assert np.array_equal(plan.imsigma(S, mu, T, np.zeros((nw, ni))), got)
         plan.close()
+
+
+# ---- the spectral functions (FP64 paths) ----
+# The smallest ∫A over the states, where |z|² is ordinary and, for one state, at the ends of the range (0 to rounding):
+# a few roundings a node, the sums' terms of one sign, so 1e-13 relative holds.
+@pytest.mark.parametrize("shift", [0.0, 3.0, 1e30, 1e100, 1e140, 1e154, 1e170])
+def test_spectral_weight_matches_oracle(api, oracle, shift):
+    nw, ni, nm, nf = 65, 3, 2, 9
+    s, S = _setup(nw, ni, nm, nf), _sigma(nw, ni)
+    s["eps_i"] = np.array(s["eps_i"], dtype=np.float64)
+    s["eps_i"][1] += shift
+    occ = dict(Tlist=[0.03], nlist=[0.0], nelec=1.0, spin_degeneracy=2.0, type="metal")
+    kw = dict(eta_init=0.05, tol=0.0, maxiter=1, mu_start=[0.07], fix_mu=True, sigma_init=S[:, :, None], omega_acoustic=1e-3)
+    want = oracle.loop_scgd0(s, occ, **kw)["history"]["min_spectral_weight"]
+    have = api.loop_scgd0(s, occ, path="gemm_fp64", **kw)["history"]["min_spectral_weight"]
+    assert np.all(np.isfinite(have)) and np.allclose(have, want, rtol=1e-13, atol=1e-300)

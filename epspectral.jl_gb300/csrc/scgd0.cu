@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(256) fm_add_kernel(const double* __restrict__ 
 
 // The occupation factors of the recast sum, per (ω, ν): F_abs = n_ν + f(ω + ω_ν - μ) and
 // F_emi = n_ν + 1 - f(ω - ω_ν - μ) (the two brackets of src/scgd0_kernel.jl:37-38); 0 for a mode
-// below ω_acoustic.
+// below ω_acoustic. Blocks of 32, so that every SM's FP64 pipe has some (501 x 15: 9.8 us in blocks of 256, 6.2).
 __global__ void occ_table_kernel(const double* __restrict__ ws, int nw, const double* __restrict__ wnu, int nm,
                                  double mu, double T, double w_ac, double* __restrict__ Fa, double* __restrict__ Fe) {
   pdl_wait();
@@ -395,22 +395,32 @@ __global__ void coupling_sum_chunk_kernel(const T* __restrict__ g2c, int nm, int
 
 // Σ_new = ReΣ + i ImΣ (src/scgd0.jl:290-291).
 // max of |a - S[k]| over the block's elements into *errbits, and S[k] ← a (src/scgd0.jl:326-328). The maximum of
-// non-negative doubles is taken on their bit patterns, which order the same way; NaN wins, as in Julia's maximum.
+// non-negative doubles is taken on their bit patterns, which order the same way; NaN wins, as in Julia's maximum. It is
+// taken of the squares, and one root a block: a hypot an element, which a block falls back to where a square leaves the
+// middle of the range, was most of the kernel's time on the FP64 pipe (501 x 105: 6.0 -> 4.8 us).
 __device__ __forceinline__ void err_copy(double2 a, bool on, double2* S, unsigned long long* errbits) {
   __shared__ unsigned long long sh[256];
-  unsigned long long e = 0;
+  double x = 0, y = 0;
   if (on) {
     const double2 b = *S;
-    e = (unsigned long long)__double_as_longlong(hypot(a.x - b.x, a.y - b.y));
+    x = a.x - b.x;
+    y = a.y - b.y;
     *S = a;
   }
-  sh[threadIdx.x] = e;
+  double q = fma(x, x, y * y);
+  const int ex = (__double2hiint(q) >> 20) & 0x7ff;
+  const bool far = __syncthreads_or((ex < 0x100 || ex > 0x700) && (x != 0 || y != 0));
+  if (far) q = hypot(x, y);
+  sh[threadIdx.x] = (unsigned long long)__double_as_longlong(q);
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
     if (threadIdx.x < s) sh[threadIdx.x] = max(sh[threadIdx.x], sh[threadIdx.x + s]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) atomicMax(errbits, sh[0]);
+  if (threadIdx.x == 0) {
+    const double m = __longlong_as_double((long long)sh[0]);
+    atomicMax(errbits, (unsigned long long)__double_as_longlong(far ? m : sqrt(m)));
+  }
 }
 
 // Σ_new = re + i im of one temperature; with S, which then is its Σ, also max |Σ_new - Σ| and Σ ← Σ_new. Hands the
@@ -1408,7 +1418,7 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
     tc_imsigma_disp(P, d_Sin, mu, T, d_ImS);
     return;
   }
-  launch_after(s, occ_table_kernel, div_up(size_t(nw * nm), 256), 256, 0, P->d_ws.p, int(nw), P->d_wnu.p, int(nm), mu, T, P->w_ac,
+  launch_after(s, occ_table_kernel, div_up(size_t(nw * nm), 32), 32, 0, P->d_ws.p, int(nw), P->d_wnu.p, int(nm), mu, T, P->w_ac,
                                                                  P->d_Fa.p, P->d_Fe.p);
   EPSP_LAUNCHED(ctx);
   const long nk = nm * P->nc;

@@ -670,29 +670,17 @@ __device__ __forceinline__ double warp_sum_d(double v) {
   return v;
 }
 
-// 1/x for x >= 1 to within an ulp or two of FP64 division: an FP32 reciprocal refined by two
-// Newton-Raphson steps r <- r (2 - x r) (each squares the relative error: 6e-8 -> 4e-15 -> FP64
-// rounding), on the FMA units instead of FP64 division; x beyond the FP32 range gives 0 (1/x is
-// then below 3e-39).
-__device__ __forceinline__ double recip_ge1(double x) {
-  const float xf = float(x);
-  if (isinf(xf)) return 0.0;
-  double r = double(__frcp_rn(xf));
-  r = fma(r, fma(-x, r, 1.0), r);
-  r = fma(r, fma(-x, r, 1.0), r);
-  return r;
-}
-
 // Shared by mu_terms and mu_solve_kernel: the start x0 of slot's temperature on the bracket.
 __device__ __forceinline__ double mu_start(double guess, double a, double b) {
   return (guess > a && guess < b) ? guess : float_middle_d(a, b);
 }
 
-// Occupation from y = exp((ωa - μ)/T) (electrons: 1/(1 + y); holes: y/(1 + y)).
+// Occupation from y = exp((ωa - μ)/T) (electrons: 1/(1 + y); holes: y/(1 + y)), to an ulp or two: recip_seeded takes
+// 1 + y up to 2^1000; beyond (693 T above μ) an electron's is below 1e-301 and a hole's is 1 to the last bit.
 __device__ __forceinline__ double occ_from_y(double y, int holes) {
-  const double r = recip_ge1(1.0 + y);
-  if (holes) return isinf(y) ? 1.0 : y * r;
-  return r;
+  if (y >= 0x1p1000) return holes ? 1.0 : 0.0;
+  const double r = recip_seeded(1.0 + y);
+  return holes ? y * r : r;
 }
 
 // The occupations at the bracket ends, per temperature of the run (ends[t][2][nωa]).

@@ -647,9 +647,11 @@ __device__ __forceinline__ double float_middle_d(double x, double y) {
 // that end the spectral functions, mu_terms), as block sums, with E_a = exp((ωa - x0)/T): near x0 a later round's
 // occupation costs one product and one reciprocal, exp((ωa - μ)/T) = E_a exp((x0 - μ)/T) (used while
 // |μ - x0| <= 30 T; farther out, and at T ~ 0, exp is evaluated directly). When the probes put the root within
-// x0 -+ 8 T, nodes with E_a outside [2^-69, 2^69) have occupation 1 or 0 to the last bit in every later
-// round: their D_a is summed once (the seventh term) and only the others are evaluated -- at 300 K a sixth of
-// ±8 eV, and FP64 evaluations (a dozen operations a node at 2 a cycle and SM) are what a round costs.
+// x0 -+ 8 T, nodes with E_a outside [2^-69, 2^69) have, in every later round, occupation 1 to the last bit or, within
+// 2^-57 of it, their occupation at x0 times exp(±(μ - x0)/T): D_a of the former and D_a f0 of the latter (all that a
+// count of 1e-20 electrons is made of) are summed once, the seventh and eighth terms, and only the other nodes are
+// evaluated -- at 300 K a sixth of ±8 eV, and FP64 evaluations (a dozen operations a node at 2 a cycle and SM) are
+// what a round costs.
 // One cluster of kMuCluster CTAs per temperature: groups of 64 nodes are dealt out to the CTAs in turn, the
 // partials are combined through distributed shared memory in rank order, so every thread of the cluster holds the
 // same totals and takes the same branches.
@@ -659,8 +661,7 @@ __device__ __forceinline__ double float_middle_d(double x, double y) {
 constexpr int kMuCluster = 8;
 constexpr int kMuThreads = 128;
 constexpr int kMuWarps = kMuThreads / 32;  // kMuCluster x kMuWarps partials: one per lane of the warp that sums them
-constexpr int kMuTerms = 7;              // first-round terms per node
-constexpr int kMuPart = 8;               // doubles of one block's first-round sums
+constexpr int kMuTerms = 8;              // first-round terms per node
 constexpr double kMuProbe = 8.0;         // the probes x0 -+ 8 T
 constexpr double kMuProbeExp = 2980.957987041728;  // e^8
 
@@ -706,7 +707,7 @@ struct MuIn {
   const TParams* tp = nullptr;
   double br0 = 0, br1 = 0;
   double* E = nullptr;     // [slot][nωa]
-  double* part = nullptr;  // [slot][blocks][kMuPart]
+  double* part = nullptr;  // [slot][blocks][kMuTerms]
 };
 __device__ __forceinline__ void mu_terms(const MuIn& M, int t, long slot, int k, int nwa, double wa, double d,
                                          double (&v)[kMuTerms]) {
@@ -733,11 +734,12 @@ __device__ __forceinline__ void mu_terms(const MuIn& M, int t, long slot, int k,
   v[4] = d * fl;
   v[5] = d * fr;
   v[6] = band == (q.holes ? 1 : -1) ? d : 0.0;
+  v[7] = band == (q.holes ? -1 : 1) ? d * f0 : 0.0;
 }
-// A warp's sums of the seven terms into out[0 .. 8): halving exchanges leave sum q on lanes 4 q .. 4 q + 3 (9 FP64
+// A warp's sums of the eight terms into out[0 .. 8): halving exchanges leave sum q on lanes 4 q .. 4 q + 3 (9 FP64
 // additions a lane, where a tree per term takes 35).
 __device__ __forceinline__ void mu_warp_terms(const double (&v)[kMuTerms], double* out) {
-  double x[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], 0.0};
+  double x[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
   const int lane = threadIdx.x % 32;
 #pragma unroll
   for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
@@ -765,7 +767,7 @@ __global__ void __launch_bounds__(kSpecNodes) spectral_fin_f32_kernel(
     const unsigned long long* __restrict__ errbits, IterCtl* __restrict__ ctl) {
   pdl_wait();
   if (ctl && ctl->stop) return;
-  __shared__ double sh[2][kMuPart];
+  __shared__ double sh[2][kMuTerms];
   const long z = blockIdx.y;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (z == 0) *tc_err_out = *tc_err;
@@ -773,7 +775,7 @@ __global__ void __launch_bounds__(kSpecNodes) spectral_fin_f32_kernel(
   }
   if (int(blockIdx.x) < nab) {
     const int a = blockIdx.x * kSpecNodes + threadIdx.x;
-    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0};
+    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (a < nwa) {
       double s = 0;
 #pragma unroll 8
@@ -785,7 +787,7 @@ __global__ void __launch_bounds__(kSpecNodes) spectral_fin_f32_kernel(
     if (!M.ends) return;
     mu_warp_terms(v, sh[threadIdx.x / 32]);
     __syncthreads();
-    if (threadIdx.x < kMuPart) M.part[(z * nab + blockIdx.x) * kMuPart + threadIdx.x] = sh[0][threadIdx.x] + sh[1][threadIdx.x];
+    if (threadIdx.x < kMuTerms) M.part[(z * nab + blockIdx.x) * kMuTerms + threadIdx.x] = sh[0][threadIdx.x] + sh[1][threadIdx.x];
     return;
   }
   const int i = (int(blockIdx.x) - nab) * 2 + int(threadIdx.x) / 32, lane = threadIdx.x % 32;
@@ -819,7 +821,7 @@ __global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restric
   sh[g][lane] = s;
   __syncthreads();
   if (g == 0) {
-    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0};
+    double v[kMuTerms] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (a < nwa) {
       double t = sh[0][lane];
 #pragma unroll
@@ -828,7 +830,7 @@ __global__ void __launch_bounds__(256) spectral_D_kernel(const double* __restric
       D[a] = t;
       mu_terms(M, slots[blockIdx.y], blockIdx.y, a, nwa, wsa[a], t, v);
     }
-    mu_warp_terms(v, M.part + (long(blockIdx.y) * gridDim.x + blockIdx.x) * kMuPart);
+    mu_warp_terms(v, M.part + (long(blockIdx.y) * gridDim.x + blockIdx.x) * kMuTerms);
   }
 }
 
@@ -852,11 +854,11 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
   const int slot = blockIdx.x / kMuCluster, t = slots[slot];
   const double* D = Dall + long(nwa) * slot;
   const double* E = E_all + long(nwa) * slot;
-  const double* P1 = part1 + long(kMuPart) * npart * slot;
+  const double* P1 = part1 + long(kMuTerms) * npart * slot;
   const double T = tp[t].T, inv_T = tp[t].inv_T, n_target = tp[t].n_target, guess = tp[t].mu;
   const int holes = tp[t].holes;
   __shared__ double part[2][kMuWarps][2];
-  __shared__ double tot[kMuPart];
+  __shared__ double tot[kMuTerms];
   const bool warm = T > 1.4901161193847656e-08;
   const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
   // Totals of two per-thread sums over the cluster, on the threads of warp 0: every warp's sums go to its CTA's part
@@ -940,12 +942,13 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
     s_fact = fact ? 1 : 0;
     s_stop = stop;
   };
-  // round 1: n(a), n(b), n(x0), n'(x0), n(x0 -+ 8T) and the saturated nodes' sum from the blocks' sums, by every CTA alike
+  // round 1: n(a), n(b), n(x0), n'(x0), n(x0 -+ 8T) and the sums of the nodes with E outside [2^-69, 2^69) from the
+  // blocks' sums, by every CTA alike
   {
     for (int q = wid; q < kMuTerms; q += kMuWarps) {
       double t = 0;
 #pragma unroll 4
-      for (int k = lane; k < npart; k += 32) t += P1[k * kMuPart + q];
+      for (int k = lane; k < npart; k += 32) t += P1[k * kMuTerms + q];
       t = warp_sum_d(t);
       if (lane == 0) tot[q] = t;
     }
@@ -1012,7 +1015,10 @@ __global__ void __cluster_dims__(kMuCluster, 1, 1) __launch_bounds__(kMuThreads)
       v[1] += fma(-df, f, df);
     }
     reduce(v);
-    if (threadIdx.x == 0) publish(newton(total(win ? tot[6] + v[0] : v[0]), warm ? gs * v[1] * inv_T : 0.0));
+    if (threadIdx.x == 0) {
+      const double tail = win ? tot[7] * (holes ? scale : recip_seeded(scale)) : 0.0;  // (f (1 - f) is f there)
+      publish(newton(total(win ? tot[6] + tail + v[0] : v[0]), warm ? gs * (v[1] + tail) * inv_T : 0.0));
+    }
     __syncthreads();
   }
   // no CTA leaves while another may still read its partials
@@ -1522,7 +1528,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   }
   grown |= ensure(D_b, ctx, size_t(nwa * nT));
   grown |= ensure(P->w_E, ctx, size_t(nwa * nT));
-  grown |= ensure(P->w_R1, ctx, size_t(kMuPart * spec_nab * nT));
+  grown |= ensure(P->w_R1, ctx, size_t(kMuTerms * spec_nab * nT));
   grown |= ensure(P->w_ends, ctx, size_t(2 * nwa * nT));
   if (P->path == EPSP_PATH_GEMM_BF16) {
     const long cap0 = tc_capacity(P);

@@ -47,3 +47,21 @@ def test_hole_counts_match_oracle(api, oracle, chain, kelvin, nlist):
         for path, gate in GATE.items():
             got = api.loop_scgd0(chain, occ(nlist, T, 2.0), path=path, mu_start=[start], **kw)["mu"][0]
             assert abs(got - ref) <= gate * slope, (path, start)
+
+
+# ---- electrons: counts that only nodes far above μ hold, in a density of states with an edge (Σ without width outside it)
+@pytest.mark.parametrize("count", [1e-6, 1e-12, 1e-18, 1e-24, 1e-30])
+def test_small_electron_counts_match_oracle(api, oracle, chain, count):
+    # the sum is all in nodes 14 to 69 T above μ; the first nodes above the edge hold most of it, so an error of it is one
+    # of their Σ (1e-10 of its size; 1e-5 eV of width and energy) and moves the root by T times its relative size
+    T = 100 * synthetic.KELVIN
+    w, ni = chain["omegas"].nodes(), len(chain["eps_i"])
+    S = np.zeros((len(w), ni, 1), dtype=np.complex128, order="F")
+    S[np.abs(w) <= 1.2] = -0.1j
+    kw = dict(eta_init=0.1, tol=0.0, maxiter=1, omega_acoustic=W_AC, sigma_init=S)
+    root = oracle.loop_scgd0(chain, occ(count, T, 0.0), mu_start=[-2.0], **kw)["mu"][0]
+    for start in (root, root - 3 * T, root + 3 * T, root - 40 * T, root + 40 * T, -3.9, 0.0):
+        ref = oracle.loop_scgd0(chain, occ(count, T, 0.0), mu_start=[start], **kw)["mu"][0]
+        for path, gate in GATE.items():
+            got = api.loop_scgd0(chain, occ(count, T, 0.0), path=path, mu_start=[start], **kw)["mu"][0]
+            assert abs(got - ref) <= gate, (path, start)

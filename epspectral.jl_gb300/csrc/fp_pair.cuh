@@ -11,6 +11,13 @@ __device__ __forceinline__ float2 split_df(double x) {
   return make_float2(h, float(x - double(h)));
 }
 
+// The same with hi a multiple of the power of two q (for |x| < 2^24 q), so that sums and differences of high parts below
+// 2^24 q are exact; lo then is at most q / 2 and holds 2^-25 of that.
+__device__ __forceinline__ float2 split_q(double x, double q) {
+  const float h = float(rint(x / q) * q);
+  return make_float2(h, float(x - double(h)));
+}
+
 // s + e = a + b exactly (Knuth's two-sum; additions only, so no contraction into FMA applies).
 __device__ __forceinline__ float two_sum(float a, float b, float& e) {
   const float s = a + b;

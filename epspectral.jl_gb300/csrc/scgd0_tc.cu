@@ -43,8 +43,8 @@ struct Scgd0Plan::Tc {
   // FP32 forms of the K-tensor inputs: distances from the cells' nodes, the cell energies as pairs, the occupation
   // tables; per temperature the columns' cell records (rec, dim; kbuild_bf16_kernel) or, with dispersive modes, Σ_in as
   // {Re hi, Re lo, Im, 0}; ε_i as pairs, and the modes' exp(ω_ν/T) and n of the run's temperatures
-  DBuf<float2> ef, epair;
-  DBuf<float> tf, Ff, dim;
+  DBuf<float2> ef, epair, tf;
+  DBuf<float> Ff, dim;
   DBuf<float4> Sf, rec;
   DBuf<double2> modes;
   // dispersive modes: cell records and Im slopes of every column and slot, partial sums of the splits
@@ -71,6 +71,12 @@ __global__ void gw_f32_kernel(const double* __restrict__ g2t, const double* __re
   gw[k] = float(w_f[(k % nvf) / nm] * g2t[k]);
 }
 
+// Pairs with high parts on the plan's quantum (split_q).
+__global__ void split_q_kernel(const double* __restrict__ x, long n, double q, float2* __restrict__ out) {
+  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (k < n) out[k] = split_q(x[k], q);
+}
+
 __global__ void to_f32_kernel(const double* __restrict__ x, long n, float* __restrict__ out) {
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k < n) out[k] = float(x[k]);
@@ -85,17 +91,19 @@ __device__ __forceinline__ float sum_splits(const float* __restrict__ part, int 
 }
 
 // One node's Σ as FP32: Re as a pair, Im. Cell j of a column from its nodes' values z (node j) and zn (node j + 1):
-// {ω_j - ReΣ_j as a pair, 1 - ReΣ', ImΣ_j} and ImΣ' (Im clamped at -η_min = etam), so that at x = ω_j + dx
-//   Re z = (U_hi - ε_hi) + ((U_lo - ε_lo) + dx (1 - ReΣ')),  Im Σ = ImΣ_j + dx ImΣ';
-// the first difference is exact where Re z is small against its parts. wj: {ω_j hi, lo, 1 / (ω_{j+1} - ω_j) (0 at the
+// {ω_j - ReΣ_j as a pair (U), -ReΣ', ImΣ_j} and ImΣ' (Im clamped at -η_min = etam), so that at x = ω_j + dx
+//   Re z = ((U_hi - ε_hi) + dx_hi) + ((U_lo - ε_lo) + dx_lo - dx ReΣ'),  Im Σ = ImΣ_j + dx ImΣ'.
+// The high parts are multiples of one quantum (split_q; qm = 1.5 2^23 times it), so the first bracket is exact and Re z
+// keeps its distance to a pole wherever in a cell it lies (dx as one FP32 number, times 1 - ReΣ', moved elements by up to
+// 2^-26 dx over the pole's width: 1e-6 relative for 0.1 eV and 1e-3 eV). wj: {ω_j hi, lo, 1 / (ω_{j+1} - ω_j) (0 at the
 // last node, whose cell is the flat part above the grid), ..}.
-__device__ __forceinline__ float4 cell_record(float4 z, float4 zn, float4 wj, float etam, float& dim) {
+__device__ __forceinline__ float4 cell_record(float4 z, float4 zn, float4 wj, float etam, float qm, float& dim) {
   float e;
   const float s = two_sum(wj.x, -z.x, e);
-  const float l = e + (wj.y - z.y), h = s + l;
+  const float h = (s + qm) - qm;
   const float im = fminf(z.z, etam);
   dim = (fminf(zn.z, etam) - im) * wj.z;
-  return make_float4(h, l - (h - s), 1.f - ((zn.x - z.x) + (zn.y - z.y)) * wj.z, im);
+  return make_float4(h, (s - h) + (e + (wj.y - z.y)), ((z.x - zn.x) + (z.y - zn.y)) * wj.z, im);
 }
 __device__ __forceinline__ float4 sigma_f32(double2 z) {
   const float2 r = split_df(z.x);
@@ -105,8 +113,8 @@ __device__ __forceinline__ float4 sigma_f32(double2 z) {
 // The records of the columns of temperature slots[blockIdx.y] from Σ there, clamped at -η_min: [ni][nω + 1] entries a
 // temperature, entry j + 1 cell j, entry 0 the flat part below the grid. Without slots: of one Σ, as it is.
 __global__ void cell_records_kernel(const double2* __restrict__ S_all, const int* __restrict__ slots,
-                                    const TParams* __restrict__ tp, const float4* __restrict__ wtab, int nw, long slab,
-                                    float4* __restrict__ rec_all, float* __restrict__ dim_all) {
+                                    const TParams* __restrict__ tp, const float4* __restrict__ wtab, float qm, int nw,
+                                    long slab, float4* __restrict__ rec_all, float* __restrict__ dim_all) {
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= slab) return;
   const int t = slots ? slots[blockIdx.y] : 0, j = int(k % nw);
@@ -115,10 +123,10 @@ __global__ void cell_records_kernel(const double2* __restrict__ S_all, const int
   const float4 z = sigma_f32(S[k]), zn = j + 1 < nw ? sigma_f32(S[k + 1]) : z, wj = wtab[j];
   const long at = (k / nw + slab / nw * t) * (nw + 1l) + j + 1;
   float d;
-  rec_all[at] = cell_record(z, zn, wj, etam, d);
+  rec_all[at] = cell_record(z, zn, wj, etam, qm, d);
   dim_all[at] = d;
   if (j == 0) {
-    rec_all[at - 1] = cell_record(z, z, wj, etam, d);
+    rec_all[at - 1] = cell_record(z, z, wj, etam, qm, d);
     dim_all[at - 1] = 0.f;
   }
 }
@@ -146,9 +154,10 @@ __global__ void sigma_f32_kernel(const double2* __restrict__ S, long n, float4* 
 // split rows K_t[ω][k], k = c nm + ν, through a shared-memory transpose. Σ(ω ± ω_ν) comes from the columns' cell
 // records (cell_record above; the cells and distances from set-up), the reciprocal and the occupation products are
 // FP32: the kernel runs on the FP32 units only. Instructions and the latency of its gathers bound it: a side of an element
-// is 20 bytes and about 12 instructions, the BF16 parts are formed two elements at a time, and eight blocks are kept on an
-// SM (with four 16-byte gathers, two weights and two two-sums a side 54 us at 1251 x 7425; six blocks, elements one by
-// one and a test of every column 40.8; now 36.6. 32 nodes a block instead of 16: 38.4, and 10 -> 12 us at 501 x 1575).
+// is 20 bytes and about 15 instructions, the BF16 parts are formed two elements at a time, and eight blocks are kept on an
+// SM (with four 16-byte gathers, two weights and two two-sums a side 54 us at 1251 x 7425; now 38.4, 10.5 at 501 x 1575.
+// Two columns in flight spill at eight blocks' 32 registers: 42.5 and 10.0; with seven blocks 42.3, six 46.3; four columns
+// and six blocks 40.2 and 10.5).
 // Grid (nω / 16, Kp / (kKbCols nm), slots), 256 threads: thread (node ω0 + t % 16, modes t / 16,
 // t / 16 + 16, ..) loads the cells and occupations of its (ω, ν) once and runs over the block's
 // kKbCols columns c (their records' offset and energy from shared memory). Dynamic shared memory: the tile
@@ -184,7 +193,7 @@ __global__ void __launch_bounds__(256, 8) kbuild_bf16_kernel(int nw, int ni, con
                                                           const float* __restrict__ dim_all,
                                                           const int* __restrict__ slots,
                                                           const int32_t* __restrict__ cell_e,
-                                                          const float* __restrict__ cell_dx,
+                                                          const float2* __restrict__ cell_dx,
                                                           const uint8_t* __restrict__ skip, int nm,
                                                           const float2* __restrict__ eps_c,
                                                           const int32_t* __restrict__ col_c, int nc,
@@ -215,7 +224,8 @@ __global__ void __launch_bounds__(256, 8) kbuild_bf16_kernel(int nw, int ni, con
   for (int nu = tm; nu < nm; nu += 256 / kKbW) {
     const bool on = iw < nw && !skip[nu];
     int ea = 0, ee = 0;
-    float da = 0.f, de = 0.f, Fa = 0.f, Fe = 0.f;
+    float2 da = make_float2(0.f, 0.f), de = da;
+    float Fa = 0.f, Fe = 0.f;
     if (on) {
       const int ia = iw + nw * nu, ie = ia + nwm;
       ea = cell_e[ia];
@@ -225,13 +235,14 @@ __global__ void __launch_bounds__(256, 8) kbuild_bf16_kernel(int nw, int ni, con
       Fa = F[ia];
       Fe = F[ie];
     }
-#pragma unroll 2
+#pragma unroll 1
     for (int cl = 0; cl < kKbCols; ++cl) {
       const float4 e = s_col[cl];
       const int ia = __float_as_int(e.z) + ea, ie = __float_as_int(e.z) + ee;
       const float4 A = rec[ia], B = rec[ie];
-      const float zar = (A.x - e.x) + fmaf(da, A.z, A.y - e.y), sia = fmaf(da, dim[ia], A.w);
-      const float zer = (B.x - e.x) + fmaf(de, B.z, B.y - e.y), sie = fmaf(de, dim[ie], B.w);
+      const float xa = da.x + da.y, xe = de.x + de.y;
+      const float zar = ((A.x - e.x) + da.x) + fmaf(xa, A.z, (A.y - e.y) + da.y), sia = fmaf(xa, dim[ia], A.w);
+      const float zer = ((B.x - e.x) + de.x) + fmaf(xe, B.z, (B.y - e.y) + de.y), sie = fmaf(xe, dim[ie], B.w);
       // Im 1/z with Im z = -Im Σ, by an approximate reciprocal (1 ulp): the K tensor carries FP32 precision
       const float ga = sia * rcp_f(fmaf(zar, zar, sia * sia));
       const float ge = sie * rcp_f(fmaf(zer, zer, sie * sie));
@@ -780,7 +791,7 @@ __global__ void __launch_bounds__(256) kk_epilogue_kernel(const float* __restric
                                                           const double* __restrict__ ImS_b, int nw, long slab,
                                                           const int* __restrict__ slots, const int32_t* __restrict__ gptr,
                                                           const int32_t* __restrict__ gidx, const float4* __restrict__ wtab,
-                                                          const float2* __restrict__ epair,
+                                                          float qm, const float2* __restrict__ epair,
                                                           const TParams* __restrict__ tp, double2* __restrict__ S_all,
                                                           float4* __restrict__ Sf_all, float4* __restrict__ rec_all,
                                                           float* __restrict__ dim_all, float4* __restrict__ Pall,
@@ -824,7 +835,7 @@ __global__ void __launch_bounds__(256) kk_epilogue_kernel(const float* __restric
     const float4 zn = j + 1 < nw ? sh[threadIdx.x + 1] : zf, wj = wtab[j];
     const float etam = float(-tp[t].eta_min);
     float dim, d0;
-    const float4 rec = cell_record(zf, zn, wj, etam, dim);
+    const float4 rec = cell_record(zf, zn, wj, etam, qm, dim);
     const float dre = (zn.x - zf.x) + (zn.y - zf.y);
     double2* S = S_all + slab * t;
     const long ni = slab / nw;
@@ -839,7 +850,7 @@ __global__ void __launch_bounds__(256) kk_epilogue_kernel(const float* __restric
         rec_all[at] = rec;
         dim_all[at] = dim;
         if (j == 0) {
-          rec_all[at - 1] = cell_record(zf, zf, wj, etam, d0);
+          rec_all[at - 1] = cell_record(zf, zf, wj, etam, qm, d0);
           dim_all[at - 1] = 0.f;
         }
       } else {
@@ -884,6 +895,10 @@ void tc_setup(Scgd0Plan* P) {
   const long nw = P->nw, ni = P->ni, nk = P->nm * P->nc;
   T->Kp = pad64(nk);
   T->Kp2 = pad64(nw);
+  // the quantum of high parts: 2^20 of it reach beyond the grid's nodes, so that sums of nodes, energies, distances and
+  // Σ within four times that stay below the 2^24 that FP32 adds exactly
+  P->re_q = std::ldexp(1.0, std::ilogb(std::max(std::fabs(P->ws.nodes.front()), std::fabs(P->ws.nodes.back()))) + 1 - 20);
+  P->re_qm = float(1.5 * 0x1p23 * P->re_q);
   if (nw > (1l << 30) || ni > (1l << 30) || nk > (1l << 30)) fail(EPSP_EINVAL, "sizes beyond the 32-bit tile grid");
   T->epair.alloc(ctx, size_t(ni));
   split_df_kernel<<<div_up(size_t(ni), 256), 256, 0, s>>>(P->d_eps_i.p, ni, T->epair.p);
@@ -949,9 +964,9 @@ void tc_setup(Scgd0Plan* P) {
   T->rec.alloc(ctx, size_t((nw + 1) * ni));
   T->dim.alloc(ctx, size_t((nw + 1) * ni));
   T->modes.alloc(ctx, size_t(P->nm));
-  to_f32_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_t.p, 2 * nwm, T->tf.p);
+  split_q_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_t.p, 2 * nwm, P->re_q, T->tf.p);
   EPSP_LAUNCHED(ctx);
-  split_df_kernel<<<div_up(size_t(P->nc), 256), 256, 0, s>>>(P->d_epsc.p, P->nc, T->ef.p);
+  split_q_kernel<<<div_up(size_t(P->nc), 256), 256, 0, s>>>(P->d_epsc.p, P->nc, P->re_q, T->ef.p);
   EPSP_LAUNCHED(ctx);
   T->opK = operand(T->Kt, nw, nk, T->Kp, kTcBM);
   T->opG = operand(T->G, ni, nk, T->Kp, T->bn1);
@@ -1163,7 +1178,7 @@ void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS) {
   const long nw = P->nw, ni = P->ni, nk = P->nm * P->nc;
   long pk = prof_begin(ctx, "kbuild");
   const long nwm = nw * P->nm;
-  cell_records_kernel<<<div_up(size_t(nw * ni), 256), 256, 0, s>>>(d_Sin, nullptr, nullptr, P->d_wtab.p, int(nw), nw * ni,
+  cell_records_kernel<<<div_up(size_t(nw * ni), 256), 256, 0, s>>>(d_Sin, nullptr, nullptr, P->d_wtab.p, P->re_qm, int(nw), nw * ni,
                                                                    T->rec.p, T->dim.p);
   EPSP_LAUNCHED(ctx);
   to_f32_kernel<<<div_up(size_t(nwm), 256), 256, 0, s>>>(P->d_Fa.p, nwm, T->Ff.p);
@@ -1252,7 +1267,7 @@ void tc_take_sigma(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp
   if (P->disp)
     clamp_f32_kernel<<<grid, 256, 0, P->ctx->stream>>>(d_S_all, T->Sf.p, slab, d_slots, d_tp);
   else
-    cell_records_kernel<<<grid, 256, 0, P->ctx->stream>>>(d_S_all, d_slots, d_tp, P->d_wtab.p, int(P->nw), slab, T->rec.p,
+    cell_records_kernel<<<grid, 256, 0, P->ctx->stream>>>(d_S_all, d_slots, d_tp, P->d_wtab.p, P->re_qm, int(P->nw), slab, T->rec.p,
                                                           T->dim.p);
   EPSP_LAUNCHED(P->ctx);
 }
@@ -1313,7 +1328,7 @@ static void tc_kk_tail(Scgd0Plan* P, int nA, const int* d_slots, const TParams* 
                            max_splits_for(nw, kKbCapKK), T->err.p, "tc_kk", kKbCapKK, ctl ? &ctl->stop : nullptr);
   long pf = prof_begin(ctx, "kk_epilogue");
   launch_after(s, kk_epilogue_kernel, dim3(div_up(size_t(nw), 255), unsigned(P->ngroups), unsigned(nA)), 256, 0, T->part.p,
-               sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_wtab.p, T->epair.p, d_tp,
+               sp2, nw * N2, T->ImS_b.p, int(nw), slab, d_slots, P->d_gptr.p, P->d_gidx.p, P->d_wtab.p, P->re_qm, T->epair.p, d_tp,
                d_S_all, T->Sf.p, T->rec.p, T->dim.p, d_P, d_errbits, d_minA, ctl);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, pf);

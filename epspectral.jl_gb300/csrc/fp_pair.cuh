@@ -11,10 +11,10 @@ __device__ __forceinline__ float2 split_df(double x) {
   return make_float2(h, float(x - double(h)));
 }
 
-// The same with hi a multiple of the power of two q (for |x| < 2^24 q), so that sums and differences of high parts below
-// 2^24 q are exact; lo then is at most q / 2 and holds 2^-25 of that.
-__device__ __forceinline__ float2 split_q(double x, double q) {
-  const float h = float(rint(x / q) * q);
+// The same with hi a multiple of a power of two q (for |x| < 2^24 q; qm = 1.5 2^52 q), so that sums and differences of
+// high parts below 2^24 q are exact; lo then is at most q / 2 and holds 2^-25 of that.
+__device__ __forceinline__ float2 split_q(double x, double qm) {
+  const float h = float((x + qm) - qm);
   return make_float2(h, float(x - double(h)));
 }
 

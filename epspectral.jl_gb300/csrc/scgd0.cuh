@@ -83,8 +83,9 @@ struct Scgd0Plan {
   // emission)
   DBuf<int32_t> d_cell_j;
   DBuf<double> d_cell_t;
-  // tensor-core path: the quantum of the high parts of energies and frequencies (split_q), and 1.5 2^23 times it
-  double re_q = 0;
+  // tensor-core path: the quantum of the high parts of energies and frequencies (split_q), and 1.5 2^52 and 1.5 2^23
+  // times it
+  double re_q = 0, re_qmd = 0;
   float re_qm = 0.f;
   // tensor-core path state (scgd0_tc.cu)
   struct Tc;

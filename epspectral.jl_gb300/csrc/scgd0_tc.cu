@@ -72,9 +72,9 @@ __global__ void gw_f32_kernel(const double* __restrict__ g2t, const double* __re
 }
 
 // Pairs with high parts on the plan's quantum (split_q).
-__global__ void split_q_kernel(const double* __restrict__ x, long n, double q, float2* __restrict__ out) {
+__global__ void split_q_kernel(const double* __restrict__ x, long n, double qm, float2* __restrict__ out) {
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = split_q(x[k], q);
+  if (k < n) out[k] = split_q(x[k], qm);
 }
 
 __global__ void to_f32_kernel(const double* __restrict__ x, long n, float* __restrict__ out) {
@@ -454,9 +454,12 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 //  * Frequencies in grid units u (the nodes are origin + offset u, whole offsets): x = ω ± ωq is a whole number b,
 //    ωq's being the same for all nodes, and a fraction that all nodes share. A table over b gives the cell that x is in
 //    and b's distance from the cell's lower node; padded by ωq's largest number, it needs no clamp.
-//  * A record a cell and column describes Σ from the cell's lower node c: ω_c - ReΣ_c as a float pair, u (1 - ReΣ'),
-//    ImΣ_c, u ImΣ', so that Re z = (U_hi - ε_hi) + ((U_lo - ε_lo) + (x - ω_c) (1 - ReΣ')): the first difference is exact
-//    where Re z is small against its parts. The cells below and above the grid have slopes 0 (fd_cell_kernel).
+//  * A record a cell and column describes Σ from the cell's lower node c: U = ω_c - ReΣ_c as a float pair, u_lo - u ReΣ',
+//    ImΣ_c, u ImΣ', with u = u_hi + u_lo. x is b whole units and a fraction f from ω_c; the fraction's f u_hi is taken off
+//    ε (ε' = ε - f u_hi, a pair a side), so Re z = ((U_hi - ε'_hi) + b u_hi) + ((U_lo - ε'_lo) + (b + f) (u_lo - u ReΣ')).
+//    High parts are multiples of one quantum (split_q): the first bracket is exact, and Re z keeps its distance to a
+//    pole anywhere in a wide cell (as (b + f) times u (1 - ReΣ') in FP32, terms near poles 0.2 meV wide were off by
+//    1e-5 in cells of 0.25 eV). The cells below and above the grid have slopes 0 (fd_cell_kernel).
 //  * n + f(x_a - μ) = (1 + n)(1 + E)/(1 + E e) and n + 1 - f(x_e - μ) = n (1 + E)/(1 + E/e), E = exp((ω - μ)/T),
 //    e = exp(ωq/T): one FMA a side, the bracket's reciprocal shared with 1/|z|², and 1 + E outside the sum
 //    (both sides over E above μ, so that every factor stays below e^40).
@@ -465,8 +468,9 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
 // Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
-// search for the nearest node and a record for either side of it, 2.30 now: 7.7 wavefronts a side and warp keep the L1
-// data pipe 90 % busy (4.7 of them the records, 20 bytes a lane), the issue slots 71 %.
+// search for the nearest node and a record for either side of it, 2.46 now (2.30 with (b + f) u as one FP32 number): 7.7
+// wavefronts a side and warp keep the L1 data pipe 85 % busy (4.7 of them the records, 20 bytes a lane), the issue slots
+// 71 % in that form.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
 // modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
@@ -483,17 +487,17 @@ __device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v 
 // Records [column][nω + 1] of slot blockIdx.y: cell 0 is below the grid, cell c from node c - 1 to node c, cell nω above.
 __global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __restrict__ slots,
                                const float4* __restrict__ wtab, const double* __restrict__ ws, int nw, long slab, double unit,
-                               float4* __restrict__ rec, float* __restrict__ dim) {
+                               float u_lo, double qm, float4* __restrict__ rec, float* __restrict__ dim) {
   const long ncell = slab / nw * (nw + 1);
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= ncell) return;
   const int c = int(k % (nw + 1)), j = max(c - 1, 0);
   const float4* Sf = Sf_all + slab * slots[blockIdx.y] + k / (nw + 1) * nw;
   const float4 s = Sf[j], o = Sf[min(c, nw - 1)];
-  const float2 u = split_df(ws[j] - (double(s.x) + double(s.y)));
+  const float2 u = split_q(ws[j] - (double(s.x) + double(s.y)), qm);
   const float inv = c == 0 || c == nw ? 0.f : wtab[j].z;
   const float dre = ((o.x - s.x) + (o.y - s.y)) * inv, di = (o.z - s.z) * inv;
-  rec[ncell * blockIdx.y + k] = make_float4(u.x, u.y, float(unit * (1.0 - double(dre))), s.z);
+  rec[ncell * blockIdx.y + k] = make_float4(u.x, u.y, fmaf(-float(unit), dre, u_lo), s.z);
   dim[ncell * blockIdx.y + k] = float(unit) * di;
 }
 
@@ -501,15 +505,16 @@ template <int NPT, bool kSmemTab>
 __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     int nw, long slab, const float4* __restrict__ rec_all, const float* __restrict__ dim_all,
     const float4* __restrict__ wtab_g, const int32_t* __restrict__ offs, const uint32_t* __restrict__ tab_g, int ntab, int pad,
-    double unit, const float* __restrict__ gw, const double* __restrict__ wph, const int32_t* __restrict__ iq_kk,
+    double unit, double inv_unit, double qm, double u_hi, const float* __restrict__ gw, const double* __restrict__ wph,
+    const int32_t* __restrict__ iq_kk,
     const int32_t* __restrict__ iks_i, const int32_t* __restrict__ iks_f, long nk_i, const double* __restrict__ eps_f,
     const int32_t* __restrict__ f_to_i, int nm, long nvf, long per, int nsplit, double w_ac, const int* __restrict__ slots,
     const TParams* __restrict__ tp, double* __restrict__ part) {
   extern __shared__ __align__(16) uint32_t fd_cells[];  // kSmemTab: the cell table
-  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε as a float pair, ωq's fraction f and
-  // 1 - f}, {the column, ωq's whole number}
+  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε' of the absorption and of the emission
+  // as pairs}, {the column, ωq's whole number, its fraction f and 1 - f (float bits)}
   __shared__ float4 s_a[kFdTile], s_e[kFdTile];
-  __shared__ int2 s_c[kFdTile];
+  __shared__ int4 s_c[kFdTile];
   if constexpr (kSmemTab)
     for (int k = threadIdx.x; k < ntab; k += kFdTile) fd_cells[k] = tab_g[k];
   const uint32_t* tab = kSmemTab ? fd_cells : tab_g;
@@ -521,7 +526,7 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
   const float4* rec = rec_all + ncell * a;
   const float* dim = dim_all + ncell * a;
   const float2 mu = split_df(tq.mu);
-  float p[NPT], q[NPT];
+  float p[NPT], qe[NPT];
   int off[NPT];
 #pragma unroll
   for (int n = 0; n < NPT; ++n) {
@@ -530,16 +535,17 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     const float wm = (wn.x - mu.x) + (wn.y - mu.y);
     const float Ew = exp_comp(-fabsf(wm), T);  // E, or 1/E above μ
     p[n] = wm <= 0.f ? 1.f : Ew;
-    q[n] = wm <= 0.f ? Ew : 1.f;
+    qe[n] = wm <= 0.f ? Ew : 1.f;
     off[n] = offs[iw] + pad;
   }
   const int ki = iks_i[i];
+  const float uf = float(u_hi);
   auto side = [&](int b, float frac, float2 e, int col, float o, float g, float& run) {
     const uint32_t t = tab[b];  // the cell, and b's distance from its lower node + 32768
-    const float dx = (__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7610)) - 8421376.f) + frac;
+    const float n = __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7610)) - 8421376.f, dx = n + frac;
     const int at = col + int(t >> 16);
     const float4 r = rec[at];
-    const float zr = (r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
+    const float zr = fmaf(n, uf, r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
     const float si = fmaf(dx, dim[at], r.w);
     const float d = fmaf(zr, zr, si * si) * o;
     run = fmaf(g * si, rcp_f(d), run);
@@ -552,19 +558,20 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     const long vf = t0 + threadIdx.x;
     __syncthreads();  // the previous tile's readers are done (and, first, the table is staged)
     // below ω_acoustic no term: zero coupling, and ε = -1e25, so that |z|² overflows and the reciprocal is 0
-    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, 0.f, 1.f);
-    int2 sc = make_int2(0, 0);
+    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, -1e25f, 0.f);
+    int4 sc = make_int4(0, 0, 0, 0);
     if (vf < t_end) {
       const int nu = int(vf % nm);
       const long f = vf / nm;
       const double wq = wph[nu + long(nm) * iq_kk[ki + nk_i * long(iks_f[f])]];
       if (!(wq < w_ac)) {
-        const float2 ep = split_df(eps_f[f]);
         const float wp = float(wq), n = occ_boson_f(wp, T), g = gw[vf + nvf * i];
-        const double wu = wq / unit, wb = fmin(floor(wu), double(pad - 1));
+        // (the fraction exactly, whichever side of a whole number the product rounds to)
+        const double wb = fmin(floor(wq * inv_unit), double(pad - 1)), fr = fma(-wb, unit, wq) * inv_unit, ef = eps_f[f];
+        const float2 ea = split_q(fma(-fr, u_hi, ef), qm), ee = split_q(fma(fr - 1.0, u_hi, ef), qm);
         sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp, T), exp_comp(-wp, T));
-        se = make_float4(ep.x, ep.y, float(wu - wb), float(1.0 - (wu - wb)));
-        sc = make_int2((nw + 1) * f_to_i[f], int(wb));
+        se = make_float4(ea.x, ea.y, ee.x, ee.y);
+        sc = make_int4((nw + 1) * f_to_i[f], int(wb), __float_as_int(float(fr)), __float_as_int(float(1.0 - fr)));
       }
     }
     s_a[threadIdx.x] = sa;
@@ -583,13 +590,12 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
         const int k1 = min(nt, k0 + kFdRun);
 #pragma unroll 2
         for (int k = k0; k < k1; ++k) {
-          const float4 A = s_a[k], Q = s_e[k];
-          const int2 C = s_c[k];
-          const float2 e = make_float2(Q.x, Q.y);
+          const float4 A = s_a[k], E = s_e[k];
+          const int4 C = s_c[k];
 #pragma unroll
           for (int n = 0; n < decltype(nodes)::value; ++n) {
-            side(off[n] + C.y, Q.z, e, C.x, fmaf(q[n], A.z, p[n]), A.x, run0[n]);
-            side(off[n] - C.y - 1, Q.w, e, C.x, fmaf(q[n], A.w, p[n]), A.y, run1[n]);
+            side(off[n] + C.y, __int_as_float(C.z), make_float2(E.x, E.y), C.x, fmaf(qe[n], A.z, p[n]), A.x, run0[n]);
+            side(off[n] - C.y - 1, __int_as_float(C.w), make_float2(E.z, E.w), C.x, fmaf(qe[n], A.w, p[n]), A.y, run1[n]);
           }
         }
 #pragma unroll
@@ -604,7 +610,7 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
 #pragma unroll
   for (int n = 0; n < NPT; ++n) {
     const int iw = iw0 + kFdTile * n;
-    if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc[n] * (double(p[n]) + double(q[n]));
+    if (iw < nw) part[iw + long(nw) * i + slab * blockIdx.z] = acc[n] * (double(p[n]) + double(qe[n]));
   }
 }
 
@@ -899,6 +905,7 @@ void tc_setup(Scgd0Plan* P) {
   // Σ within four times that stay below the 2^24 that FP32 adds exactly
   P->re_q = std::ldexp(1.0, std::ilogb(std::max(std::fabs(P->ws.nodes.front()), std::fabs(P->ws.nodes.back()))) + 1 - 20);
   P->re_qm = float(1.5 * 0x1p23 * P->re_q);
+  P->re_qmd = 1.5 * 0x1p52 * P->re_q;
   if (nw > (1l << 30) || ni > (1l << 30) || nk > (1l << 30)) fail(EPSP_EINVAL, "sizes beyond the 32-bit tile grid");
   T->epair.alloc(ctx, size_t(ni));
   split_df_kernel<<<div_up(size_t(ni), 256), 256, 0, s>>>(P->d_eps_i.p, ni, T->epair.p);
@@ -964,9 +971,9 @@ void tc_setup(Scgd0Plan* P) {
   T->rec.alloc(ctx, size_t((nw + 1) * ni));
   T->dim.alloc(ctx, size_t((nw + 1) * ni));
   T->modes.alloc(ctx, size_t(P->nm));
-  split_q_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_t.p, 2 * nwm, P->re_q, T->tf.p);
+  split_q_kernel<<<div_up(size_t(2 * nwm), 256), 256, 0, s>>>(P->d_cell_t.p, 2 * nwm, P->re_qmd, T->tf.p);
   EPSP_LAUNCHED(ctx);
-  split_q_kernel<<<div_up(size_t(P->nc), 256), 256, 0, s>>>(P->d_epsc.p, P->nc, P->re_q, T->ef.p);
+  split_q_kernel<<<div_up(size_t(P->nc), 256), 256, 0, s>>>(P->d_epsc.p, P->nc, P->re_qmd, T->ef.p);
   EPSP_LAUNCHED(ctx);
   T->opK = operand(T->Kt, nw, nk, T->Kp, kTcBM);
   T->opG = operand(T->G, ni, nk, T->Kp, T->bn1);
@@ -1009,8 +1016,9 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
     const long slab = nw * ni, ncell = (nw + 1) * ni, nvf = P->nm * P->nf;
     ensure(T->fdrec, ctx, size_t(ncell * nA));
     ensure(T->fddim, ctx, size_t(ncell * nA));
+    const double u_hi = std::rint(P->fd_unit / P->re_q) * P->re_q;
     fd_cell_kernel<<<dim3(div_up(size_t(ncell), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
-        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, P->fd_unit, T->fdrec.p, T->fddim.p);
+        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, P->fd_unit, float(P->fd_unit - u_hi), P->re_qmd, T->fdrec.p, T->fddim.p);
     EPSP_LAUNCHED(ctx);
     const size_t tab = sizeof(uint32_t) * P->d_fdtab.n;
     const int nsplit = fd_splits(P, nA), npt = fd_nodes(P);
@@ -1020,8 +1028,7 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
     auto go = [&](auto kern, size_t bytes) {
       EPSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
       kern<<<grid, kFdTile, bytes, ctx->stream>>>(int(nw), slab, T->fdrec.p, T->fddim.p, P->d_wtab.p, P->d_fdoff.p,
-                                                  P->d_fdtab.p, int(P->d_fdtab.n), P->fd_pad, P->fd_unit, P->d_gwf.p,
-                                                  P->d_wph.p, P->d_iq.p, P->d_iksi.p, P->d_iksf.p, P->nk_i, P->d_epsf.p,
+                                                  P->d_fdtab.p, int(P->d_fdtab.n), P->fd_pad, P->fd_unit, 1.0 / P->fd_unit, P->re_qmd, u_hi, P->d_gwf.p, P->d_wph.p, P->d_iq.p, P->d_iksi.p, P->d_iksf.p, P->nk_i, P->d_epsf.p,
                                                   P->d_fti.p, int(P->nm), nvf, per, nsplit, P->w_ac, d_slots, d_tp,
                                                   T->fdpart.p);
     };

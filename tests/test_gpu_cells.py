@@ -1,5 +1,6 @@
-"""The kernel tensor of the tensor-core path (csrc/scgd0_tc.cu) where Σ(ω ± ω_ν) lies far inside wide cells of the grid and
-a pole lies within its width of the point: Re z = (x - ε) - Re Σ(x) has to keep the distance to the pole.
+"""The Fan-Migdal sums of the tensor-core path (csrc/scgd0_tc.cu: the kernel tensor, and term by term for dispersive modes)
+where Σ(ω ± ω_ν) lies far inside wide cells of the grid and a pole lies within its width of the point: Re z =
+(x - ε) - Re Σ(x) has to keep the distance to the pole.
 
 Tolerance: Re z comes from float pairs but for the step along the cell times Σ's slope, rounded to 2^-25 of 0.25 x 0.01 eV:
 7e-11 eV, which against the width of 2e-4 eV moves an element by 4e-7 at most; half a dozen FP32 roundings an element and the
@@ -14,23 +15,37 @@ from epspectral_gb300 import FrequencyGrid
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("ni,nf,wq", [(31, 31, 0.13), (32, 64, 0.2371), (5, 96, 0.0613)])
-def test_sharp_poles_in_wide_cells_match_oracle(oracle, ni, nf, wq):
-    from epspectral_gb300 import api
+def _setup_with_poles(ni, nf, wq, off, unit, dispersive):
+    """Inner state f's pole lies within its width of ω_j + ω_ν (j = f mod nω), where it takes Σ of its representative."""
     from test_gpu_fp64_products import _setup
-    nw, eta = 33, 2e-4
-    g = FrequencyGrid(-4.0, 0.25, np.arange(nw))
-    w = g.nodes()
-    s = dict(_setup(nw, ni, 1, nf), omegas=g, omegas_spectral=g, omega_ph=np.full((1, 2), wq, order="F"))
+    eta, g = 2e-4, FrequencyGrid(-4.0, unit, off)
+    w, nw = g.nodes(), len(off)
+    wph = np.full((1, 2), wq, order="F")
+    if dispersive:
+        wph[0, 1] = 0.9 * wq  # (every pair reads the first)
+    s = dict(_setup(nw, ni, 1, nf), omegas=g, omegas_spectral=g, omega_ph=wph)
     s["g2"] = np.asfortranarray(1.0 + np.abs(R.pseudorandom(1, ni, nf, seed=9)))
     S = np.empty((nw, ni), dtype=np.complex128, order="F")
     S.real = 0.1 * R.pseudorandom(ni, seed=7)[None, :] + 0.01 * w[:, None]
     S.imag = -eta
-    # inner state f's pole: within its width of ω_j + ω_ν (j = f mod nω), where it takes Σ of its representative
     j, rep = np.arange(nf) % nw, s["f_to_i"]
     s["eps_f"] = w[j] + wq - (S.real[j, rep] + 0.01 * wq) + 2 * eta * R.pseudorandom(nf, seed=11)
-    ref = oracle.imsigma(s, S, 0.07, 0.03, np.zeros((nw, ni)), omega_acoustic=1e-3)
+    return s, S
+
+
+UNIFORM = (np.arange(33), 0.25)
+GRADED = (np.concatenate([np.arange(0, 65, 5), np.arange(65, 95), np.arange(95, 161, 5)]), 0.05)
+
+
+@pytest.mark.parametrize("dispersive", [False, True])
+@pytest.mark.parametrize("off,unit", [UNIFORM, GRADED])
+@pytest.mark.parametrize("ni,nf,wq", [(31, 31, 0.13), (32, 64, 0.2371), (5, 96, 0.0613)])
+def test_sharp_poles_in_wide_cells_match_oracle(oracle, ni, nf, wq, off, unit, dispersive):
+    from epspectral_gb300 import api
+    s, S = _setup_with_poles(ni, nf, wq, off, unit, dispersive)
+    zero = np.zeros(S.shape)
+    ref = oracle.imsigma(s, S, 0.07, 0.03, zero, omega_acoustic=1e-3)
     plan = api.Scgd0Plan(s, path="gemm_bf16", omega_acoustic=1e-3)
-    got = plan.imsigma(S, 0.07, 0.03, np.zeros((nw, ni)))
+    got = plan.imsigma(S, 0.07, 0.03, zero)
     plan.close()
     assert np.linalg.norm(got - ref) <= 1e-6 * np.linalg.norm(ref)

@@ -1460,13 +1460,24 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
     if (!(occ->Tlist[iT] >= 0)) fail(EPSP_EINVAL, "Temperature must be positive");
   const long nw = P->nw, ni = P->ni, nwa = P->nwa;
   const long slab = nw * ni;
+  if (sigma_init)
+    for (long k = 0; k < 2 * slab * nT; ++k)
+      if (!std::isfinite(sigma_init[k])) fail(EPSP_EINVAL, "Sigma_init must be finite");
+  // From here the plan's Σ is this run's: none until the run has succeeded. A run that fails waits for what it has
+  // launched (an iteration may be in flight behind the one that failed), so that nothing writes after the call.
+  P->sigma_nT = 0;
+  struct Drain {
+    cudaStream_t s;
+    bool on = true;
+    ~Drain() {
+      if (on) cudaStreamSynchronize(s);
+    }
+  } drain{s};
   DBuf<double2>& S = P->w_S;
   DBuf<double2>& Snew = P->w_Snew;
   if (ensure(S, ctx, size_t(slab * nT))) ++P->w_gen;
   if (ensure(Snew, ctx, size_t(slab * nT))) ++P->w_gen;
   if (sigma_init) {
-    for (long k = 0; k < 2 * slab * nT; ++k)
-      if (!std::isfinite(sigma_init[k])) fail(EPSP_EINVAL, "Sigma_init must be finite");
     long pu = prof_begin(ctx, "scgd0_io");
     S.upload(reinterpret_cast<const double2*>(sigma_init), size_t(slab * nT), s);
     prof_end(ctx, pu);
@@ -1774,9 +1785,10 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
   hist->niter = niter;
   long pd = prof_begin(ctx, "scgd0_io");
   if (sigma_out) S.download(reinterpret_cast<double2*>(sigma_out), size_t(slab * nT), s);
-  P->sigma_nT = nT;
   prof_end(ctx, pd);
   EPSP_CUDA(cudaStreamSynchronize(s));
+  drain.on = false;
+  P->sigma_nT = nT;
   for (int64_t iT = 0; iT < nT; ++iT) {
     mu_out[iT] = mu[size_t(iT)];
     converged[iT] = active[size_t(iT)] ? 0 : 1;

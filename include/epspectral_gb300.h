@@ -228,7 +228,7 @@ epsp_status epsp_scgd0_run(epsp_scgd0_plan* plan, const epsp_occ* occ, const dou
  * like sigma_out (nT of that run, may be NULL), valid until the next run or the plan's destruction
  * (no counterpart in the reference). epsp_scgd0_run takes sigma_out = NULL to leave Σ there only;
  * epsp_ladder_run and epsp_ladder_run_batched accept this pointer as their sigma. EPSP_EINVAL before
- * the first run. */
+ * the first run and after one that failed once it had begun. */
 epsp_status epsp_scgd0_sigma_device(const epsp_scgd0_plan* plan, const double** sigma_dev, int64_t* nT);
 
 /* One Fan-Migdal sum at one temperature: imsigma [nω, ni] += Σ_{νf} term, with sigma_in [nω, ni]

@@ -162,8 +162,14 @@ inline void prof_end(Ctx* c, long idx) {
 // that runs.) A kernel launched plainly passes the wait at once.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class... P, class... A>
-inline void launch_after(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+template <class T>
+struct Exactly {  // (not deduced from: the kernel alone says what its parameters are)
+  using type = T;
+};
+// The arguments convert to the kernel's parameters as in a call (no pointer to another type, no lost const).
+template <class... P>
+inline void launch_after(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                         typename Exactly<P>::type... args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
@@ -174,7 +180,7 @@ inline void launch_after(cudaStream_t s, void (*kern)(P...), dim3 grid, dim3 blo
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  EPSP_CUDA(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+  EPSP_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 #endif
 

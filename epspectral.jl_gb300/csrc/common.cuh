@@ -5,9 +5,11 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 #include <cmath>
@@ -83,6 +85,32 @@ struct G2Kept {
   ~G2Kept() { release(); }
 };
 
+// Device memory that its owner can do without. What is entered in a context's list is asked for it when an allocation of
+// that context finds no room.
+struct Spare {
+  virtual bool give_back() = 0;  // frees it; false where there is nothing to free or it is in use
+
+ protected:
+  ~Spare() = default;
+};
+using Spares = std::vector<Spare*>;
+// Keeps a Spare in the list of the context that it first gets (the list outlives the context).
+struct SpareEntry {
+  std::shared_ptr<Spares> list;
+  Spare* me = nullptr;
+  void enter(const std::shared_ptr<Spares>& l, Spare* s) {
+    if (list) return;
+    list = l;
+    list->push_back(me = s);
+  }
+  SpareEntry() = default;
+  SpareEntry(const SpareEntry&) = delete;
+  SpareEntry& operator=(const SpareEntry&) = delete;
+  ~SpareEntry() {
+    if (list) list->erase(std::find(list->begin(), list->end(), me));
+  }
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -93,8 +121,11 @@ struct Ctx {
   std::string prof_name;
   std::vector<cudaEvent_t> prof_events;  // pairs (start, stop)
   size_t prof_used = 0;
-  // Host-side test hook: the next allocation of at least `fail_alloc_bytes` fails (0 = off).
+  std::shared_ptr<Spares> spares = std::make_shared<Spares>();
+  // Host-side test hook: the next allocation of at least `fail_alloc_bytes` finds no room (0 = off).
   size_t fail_alloc_bytes = 0;
+  // Test hook: the size of the FP64 products' work buffers (0 = the default; below 1 MiB: as where none fits).
+  size_t product_bytes = 0;
   // Test hook of the one-CTA tensor-core GEMM: the producer skips K block `stall_kb` of every tile
   // (-1 = off) and the pipeline waits give up after `stall_wait_limit` tries (0 = the default).
   int stall_kb = -1;
@@ -217,12 +248,17 @@ struct DBuf {
     n = count;
     if (count == 0) return;
     size_t bytes = count * sizeof(T);
-    if (c && c->fail_alloc_bytes && bytes >= c->fail_alloc_bytes) {
-      c->fail_alloc_bytes = 0;
-      fail(EPSP_ENOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed (test hook)");
-    }
+    const bool hook = c && c->fail_alloc_bytes && bytes >= c->fail_alloc_bytes;
+    if (hook) c->fail_alloc_bytes = 0;
     const auto t0 = std::chrono::steady_clock::now();
-    cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = hook ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && c && !c->spares->empty()) {
+      (void)cudaGetLastError();
+      cudaStreamSynchronize(c->stream);  // (what is given back may be in use there)
+      bool any = false;
+      for (Spare* s : *c->spares) any |= s->give_back();
+      if (any) e = cudaMalloc(&p, bytes);
+    }
     if (c) {
       c->alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
       ++c->alloc_calls;
@@ -230,7 +266,8 @@ struct DBuf {
     if (e != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
-      fail(EPSP_ENOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
+      fail(EPSP_ENOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e) +
+                            (hook ? " (test hook)" : ""));
     }
   }
   void upload(const T* h, size_t count, cudaStream_t s) {

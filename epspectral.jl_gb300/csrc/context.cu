@@ -176,10 +176,18 @@ epsp_status epsp_timer_end(epsp_ctx* c, double* ms) {
 }
 
 /* Test hook (not in the reference): the next device allocation of at least `bytes` bytes made
- * through this context fails with EPSP_ENOMEM, as a device without room would. 0 switches it off. */
+ * through this context finds no room, as on a full device. 0 switches it off. */
 epsp_status epsp_test_fail_alloc(epsp_ctx* c, uint64_t bytes) {
   if (!c) return EPSP_EINVAL;
   c->c.fail_alloc_bytes = size_t(bytes);
+  return EPSP_OK;
+}
+
+/* Test hook (not in the reference): the FP64 products (csrc/oz_gemm.cuh) run in panels whose work buffers hold `bytes`
+ * bytes each, of 128 rows or 64 columns at least (below 1 MiB: as where none fits the device); 0 restores the default. */
+epsp_status epsp_test_product_panels(epsp_ctx* c, uint64_t bytes) {
+  if (!c) return EPSP_EINVAL;
+  c->c.product_bytes = size_t(bytes);
   return EPSP_OK;
 }
 

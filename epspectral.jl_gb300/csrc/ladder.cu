@@ -26,6 +26,7 @@
 #include "tc_gemm.cuh"
 
 #include <algorithm>
+#include <deque>
 #include <chrono>
 #include <type_traits>
 #include <complex>
@@ -79,8 +80,8 @@ struct LadderPlan {
   long Ktot = 0;
   // FP64 paths: the products' work buffers, and the digit planes of KK, G̃ and (per chunk, as B̃) B̃
   OzWork oz;
-  OzPlanes ozKK, ozGt;
-  std::vector<OzPlanes> ozBt;
+  OzKept ozKK, ozGt;
+  std::deque<OzKept> ozBt;
   double Bt_T = std::numeric_limits<double>::quiet_NaN();  // temperature B̃ was built for
   // GEMM paths: rows (j, q, c0, ri) with j padded to nwp (a multiple of 32), K = (ν, b, i') with ν
   // padded to nmp (a multiple of 16)
@@ -1944,7 +1945,7 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
       P->d_xtab = to_device(ctx, x);
       P->d_Af.alloc(ctx, size_t(M * P->Kx));
       P->d_Af.zero(s);  // rows j >= nω and the columns of padding modes stay zero
-      oz_split(ctx, P->d_Gt.p, P->Kx, N, P->Kx, true, oz_tile_n(N), P->ozGt);
+      P->ozGt.keep(ctx, P->d_Gt.p, P->Kx, N, P->Kx, true, oz_tile_n(N));
       EPSP_CUDA(cudaStreamSynchronize(s));  // x is a local
     } else {
       plog.mark("g2 streamed, G~ built");
@@ -2053,7 +2054,7 @@ LadderPlan* ladder_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts
   } else {
     P->d_Y.alloc(ctx, size_t(nw * 48 * ni));
     P->d_KY.alloc(ctx, size_t(nw * 48 * ni));
-    oz_split(ctx, P->d_KK.p, nw, nw, nw, false, kOzBoxM, P->ozKK);
+    P->ozKK.keep(ctx, P->d_KK.p, nw, nw, nw, false, kOzBoxM);
     EPSP_CUDA(cudaStreamSynchronize(s));
     P->d_Gm.alloc(ctx, size_t(nw * 4 * ni));
     P->d_Gp.alloc(ctx, size_t(nw * 4 * ni));
@@ -2123,8 +2124,8 @@ static void build_Bt(LadderPlan* P, double T) {
     star_sum_kernel<<<div_up(size_t(total), 256), 256, 0, s>>>(P->d_B.p, P->d_R.p, P->d_by_star.p, P->d_star_ptr.p, c.i0, nip,
                                                                c.f0, nfc, int(ns), int(ni), P->Ktot, c.k_off, P->d_Bt.p);
     EPSP_LAUNCHED(ctx);
-    oz_split(ctx, P->d_Bt.p + c.k_off, P->Ktot, 6 * ni, ns * 3 * nip, true, oz_tile_n(6 * ni),
-             P->ozBt[size_t(&c - P->chunks.data())]);
+    P->ozBt[size_t(&c - P->chunks.data())].keep(ctx, P->d_Bt.p + c.k_off, P->Ktot, 6 * ni, ns * 3 * nip, true,
+                                                oz_tile_n(6 * ni));
   }
   P->Bt_T = T;
 }

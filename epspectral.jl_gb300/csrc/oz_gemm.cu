@@ -425,6 +425,19 @@ __global__ void __launch_bounds__(256) oz_sum_kernel(const int* __restrict__ sum
   *c = beta == 0 ? val : val + beta * *c;
 }
 
+// The same as FP64 sums, for a device without room for the smallest panel's work buffers.
+__global__ void __launch_bounds__(256) oz_plain_kernel(long M, long N, long K, const double* __restrict__ A, long lda,
+                                                       const double* __restrict__ B, long ldb, double beta,
+                                                       double* __restrict__ C, long ldc) {
+  pdl_wait();
+  const long idx = long(blockIdx.x) * 256 + threadIdx.x, m = idx % M, n = idx / M;
+  if (n >= N) return;
+  double val = 0;
+  for (long k = 0; k < K; ++k) val = fma(A[m + lda * k], B[k + ldb * n], val);
+  double* c = C + m + ldc * n;
+  *c = beta == 0 ? val : val + beta * *c;
+}
+
 // ---- host ----
 
 int oz_tile_n(long N) {
@@ -518,8 +531,6 @@ static void gemm_panel(Ctx* ctx, OzWork& W, const OzPlanes& A, long m0, long M, 
   }
   if (long(sh.nM) * sh.nN * sh.nseg * sh.per_seg > (1l << 30)) fail(EPSP_EINVAL, "sizes beyond the 32-bit tile grid");
   const size_t n = size_t(sh.nseg) * kOzOrders * size_t(sh.M) * size_t(sh.N);
-  ensure(W.sums, ctx, n);
-  if (ensure(W.err, ctx, 1)) W.err.zero(s);
   if (shared) EPSP_CUDA(cudaMemsetAsync(W.sums.p, 0, n * sizeof(int), s));
   switch (B.box) {
     case 256: launch_mma<256>(ctx, A, B, sh, W.sums.p, W.err.p); break;
@@ -532,22 +543,103 @@ static void gemm_panel(Ctx* ctx, OzWork& W, const OzPlanes& A, long m0, long M, 
   EPSP_LAUNCHED(ctx);
 }
 
-void oz_gemm(Ctx* ctx, OzWork& W, long M, long N, long K, const double* A, long lda, const OzPlanes* pA, const double* B,
-             long ldb, const OzPlanes* pB, double beta, double* C, long ldc) {
-  if (M <= 0 || N <= 0) return;
-  if (!pB) {
-    oz_split(ctx, B, ldb, N, K, true, oz_tile_n(N), W.b);
-    pB = &W.b;
+bool OzKept::give_back() {
+  if (!on || busy) return false;
+  p.release();
+  on = false;
+  return true;
+}
+
+void OzKept::keep(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_major, int box) {
+  entry.enter(ctx->spares, this);
+  const size_t values = size_t(kOzDigits) * size_t(rows) * size_t((K + 63) / 64 * 64);
+  if (!(p.q.p && p.q.n >= values) && 2 * values > (size_t(64) << 20)) {  // (small ones without asking)
+    size_t room = 0, all = 0;
+    EPSP_CUDA(cudaMemGetInfo(&room, &all));
+    if (2 * values > room / 4) {
+      give_back();
+      return;
+    }
   }
-  // panels of rows: at most 4 GiB of integer sums, and of planes for an A that is split here
+  busy = true;
+  try {
+    oz_split(ctx, S, ld, rows, K, k_major, box, p);
+    on = true;
+  } catch (const Error& e) {
+    on = false;
+    p.release();
+    if (e.code != EPSP_ENOMEM) {
+      busy = false;
+      throw;
+    }
+  }
+  busy = false;
+}
+
+bool OzWork::give_back() {
+  if (busy || !(a.q.p || b.q.p || sums.p)) return false;
+  a.release();
+  b.release();
+  sums.release();
+  return true;
+}
+
+static void reserve(Ctx* ctx, OzPlanes& P, long rows, long Kp) {
+  bool grown = ensure(P.q, ctx, size_t(kOzDigits * rows * Kp));
+  grown |= ensure(P.mx, ctx, size_t(rows));
+  if (grown) P.rows = 0;  // the map's address is no longer the buffer's
+}
+
+void oz_gemm(Ctx* ctx, OzWork& W, long M, long N, long K, const double* A, long lda, const OzKept* kA, const double* B,
+             long ldb, const OzKept* kB, double beta, double* C, long ldc) {
+  if (M <= 0 || N <= 0) return;
+  W.entry.enter(ctx->spares, &W);
+  struct InUse {
+    OzWork& w;
+    ~InUse() { w.busy = false; }
+  } use{W};
+  W.busy = true;
+  if (ensure(W.err, ctx, 1)) W.err.zero(ctx->stream);
   const long Kp = (K + 63) / 64 * 64, nseg = Kp / (kOzSegChunks * kOzChunk) + 1;
-  long panel = (4l << 30) / (4 * kOzOrders * nseg * N);
-  if (!pA) panel = std::min(panel, (4l << 30) / (2 * kOzDigits * Kp));
-  panel = std::max<long>(kOzBoxM, panel / kOzBoxM * kOzBoxM);
-  for (long m0 = 0; m0 < M; m0 += panel) {
-    const long m = std::min(panel, M - m0);
+  long room = long(ctx->product_bytes ? ctx->product_bytes : size_t(4) << 30);  // of each buffer
+  long pm = 0, pn = 0;
+  const OzPlanes *pA = nullptr, *pB = nullptr;
+  // the panels: every buffer is there before the first is used, since a product may add to C
+  for (bool ready = false; !ready;) {
+    if (room < (1l << 20)) {
+      launch_after(ctx->stream, oz_plain_kernel, div_up(size_t(M) * size_t(N), 256), 256, 0, M, N, K, A, lda, B, ldb, beta, C, ldc);
+      EPSP_LAUNCHED(ctx);
+      return;
+    }
+    auto most = [&](long all, long tile, long bytes) { return std::min(all, std::max(tile, room / bytes / tile * tile)); };
+    pA = kA ? kA->planes() : nullptr;
+    pB = kB ? kB->planes() : nullptr;
+    pn = pB ? N : most(N, 64, 2 * kOzDigits * Kp);
+    pm = most(M, kOzBoxM, 4 * kOzOrders * nseg * pn);
+    if (!pA) pm = std::min(pm, most(M, kOzBoxM, 2 * kOzDigits * Kp));
+    try {
+      if (!pA) reserve(ctx, W.a, pm, Kp);
+      if (!pB) reserve(ctx, W.b, pn, Kp);
+      ensure(W.sums, ctx, size_t(nseg * kOzOrders) * size_t(pm) * size_t(pn));
+      // (what an allocation took may have been these operands' planes)
+      ready = pA == (kA ? kA->planes() : nullptr) && pB == (kB ? kB->planes() : nullptr);
+    } catch (const Error& e) {
+      if (e.code != EPSP_ENOMEM) throw;
+      W.a.release();
+      W.b.release();
+      W.sums.release();
+      room /= 4;
+    }
+  }
+  for (long m0 = 0; m0 < M; m0 += pm) {
+    const long m = std::min(pm, M - m0);
     if (!pA) oz_split(ctx, A + m0, lda, m, K, false, kOzBoxM, W.a);
-    gemm_panel(ctx, W, pA ? *pA : W.a, pA ? m0 : 0, m, *pB, A + m0, lda, B, ldb, beta, C + m0, ldc);
+    for (long n0 = 0; n0 < N; n0 += pn) {
+      const long n = std::min(pn, N - n0);
+      if (!pB && (m0 == 0 || pn < N)) oz_split(ctx, B + ldb * n0, ldb, n, K, true, oz_tile_n(n), W.b);
+      gemm_panel(ctx, W, pA ? *pA : W.a, pA ? m0 : 0, m, pB ? *pB : W.b, A + m0, lda, B + ldb * n0, ldb, beta,
+                 C + m0 + ldc * n0, ldc);
+    }
   }
 }
 

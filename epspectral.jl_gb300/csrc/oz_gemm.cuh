@@ -45,14 +45,36 @@ struct OzPlanes {
   long rows = 0, K = 0, Kp = 0;
   int box = 0;  // rows of the tensor map's box
   CUtensorMap map;
+  void release() {
+    q.release();
+    mx.release();
+    rows = K = Kp = 0;
+  }
 };
 
-// Work buffers of a plan's products: the planes of the operands that change, the integer sums, and
-// the flag a bounded wait sets.
-struct OzWork {
+// The planes of an operand that does not change, split once and kept beside it (16 bytes a value, twice the operand)
+// while there is room: not where they would take more than a quarter of the free memory (asked from 64 MiB on), and
+// given back to an allocation that finds none. The products split the operand themselves where they are not kept (the same results).
+class OzKept final : Spare {
+  OzPlanes p;
+  bool on = false, busy = false;
+  SpareEntry entry;
+  bool give_back() override;
+
+ public:
+  void keep(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_major, int box);
+  const OzPlanes* planes() const { return on ? &p : nullptr; }
+};
+
+// Work buffers of a plan's products: the planes of the operands that are split for one product, the integer sums, and
+// the flag a bounded wait sets. Given back, but for the flag, to an allocation that finds no room.
+struct OzWork final : Spare {
   OzPlanes a, b;
   DBuf<int> sums;
   DBuf<int> err;
+  bool busy = false;
+  SpareEntry entry;
+  bool give_back() override;
 };
 
 // The column tile for N columns: 64, 128, 192 or 256.
@@ -62,11 +84,13 @@ int oz_tile_n(long N);
 // (k_major) or S[r + ld k]. P's buffers are kept and grown as needed.
 void oz_split(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_major, int box, OzPlanes& P);
 
-// C [M, N] = A B + beta C with A[m + lda k], B[k + ldb n]. An operand that does not change is split once by the
-// caller and given as planes too (pA with boxes of kOzBoxM rows, pB of oz_tile_n(N)); the others are split
-// here, into W's buffers. Runs over panels of rows, so that the work buffers stay below about 8 GiB.
-void oz_gemm(Ctx* ctx, OzWork& W, long M, long N, long K, const double* A, long lda, const OzPlanes* pA, const double* B,
-             long ldb, const OzPlanes* pB, double beta, double* C, long ldc);
+// C [M, N] = A B + beta C with A[m + lda k], B[k + ldb n]. An operand that does not change may be kept by the caller
+// (kA with boxes of kOzBoxM rows, kB of oz_tile_n(N)); the others are split here, into W's buffers. Runs over
+// panels of rows and, where B is split here, of columns, so that the planes and the sums hold 4 GiB each at most (of one
+// tile at least), less where the device has no room, and by FP64 sums where it has none at all. Panels do
+// not change an element: each is its own exact sum.
+void oz_gemm(Ctx* ctx, OzWork& W, long M, long N, long K, const double* A, long lda, const OzKept* kA, const double* B,
+             long ldb, const OzKept* kB, double beta, double* C, long ldc);
 
 // Fails with EPSP_EDEVICE_TIMEOUT if a bounded wait of a product ran out (synchronises, clears the flag).
 void oz_check(Ctx* ctx, OzWork& W);

@@ -1335,7 +1335,7 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
     P->d_Fe.alloc(ctx, size_t(P->nw * nm));
     if (P->path == EPSP_PATH_GEMM_FP64) {
       P->d_Kt.alloc(ctx, size_t(P->nw * nm * P->nc));
-      oz_split(ctx, P->d_G.p, nm * P->nc, ni, nm * P->nc, true, oz_tile_n(ni), P->ozG);
+      P->ozG.keep(ctx, P->d_G.p, nm * P->nc, ni, nm * P->nc, true, oz_tile_n(ni));
     } else {
       tc_setup(P);
     }
@@ -1344,7 +1344,7 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
     fail(EPSP_EINVAL, "unknown path");
   }
   if (P->path != EPSP_PATH_GEMM_BF16) {
-    oz_split(ctx, P->d_KK.p, P->nw, P->nw, P->nw, false, kOzBoxM, P->ozKK);
+    P->ozKK.keep(ctx, P->d_KK.p, P->nw, P->nw, P->nw, false, kOzBoxM);
     EPSP_CUDA(cudaStreamSynchronize(s));
   }
   plog.mark("cells, tensor-core operands");

@@ -56,7 +56,7 @@ struct Scgd0Plan {
   bool fm_fast = false;
   // FP64 paths: the products' work buffers, and the digit planes of the operands that do not change
   OzWork oz;
-  OzPlanes ozKK, ozG;
+  OzKept ozKK, ozG;
   // GEMM paths
   bool star_reduced = false;
   long nc = 0;

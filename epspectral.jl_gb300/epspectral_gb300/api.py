@@ -60,6 +60,7 @@ def lib():
         "epsp_profile_kernel": (C.c_int, [vp, C.c_char_p]),
         "epsp_profile_read": (C.c_int, [vp, P(d), P(i64)]),
         "epsp_test_fail_alloc": (C.c_int, [vp, C.c_uint64]),
+        "epsp_test_product_panels": (C.c_int, [vp, C.c_uint64]),
         "epsp_test_gemm_stall": (C.c_int, [vp, C.c_int32, C.c_uint32]),
         "epsp_test_g2_host_gather": (C.c_int, [vp, C.c_int32]),
         "epsp_host_register": (C.c_int, [vp, vp, C.c_uint64]),
@@ -151,8 +152,14 @@ class Context:
         return ms.value
 
     def fail_next_alloc(self, nbytes: int):
-        """Test hook: the next device allocation of at least nbytes fails with ENOMEM."""
+        """Test hook: the next device allocation of at least nbytes finds no room (ENOMEM, unless the context's plans
+        have memory to give back)."""
         self.check(lib().epsp_test_fail_alloc(self.handle, int(nbytes)))
+
+    def product_panels(self, nbytes: int = 0):
+        """Test hook: the FP64 products' work buffers hold nbytes each (below 1 MiB: as where none fits the device);
+        product_panels() restores the default."""
+        self.check(lib().epsp_test_product_panels(self.handle, int(nbytes)))
 
     def keep_g2(self, on: bool):
         """Keep the last g2 a plan set-up streamed on the device, for a later set-up of the same array

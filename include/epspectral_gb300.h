@@ -177,8 +177,13 @@ int64_t epsp_kernel_launches(const epsp_ctx* ctx);
  *    (address, size, element type) in the same order reads it instead of streaming g2 again (an
  *    scGD0 plan and a ladder plan of one model). The caller must not change the array in between;
  *    on = 0 (the default) switches it off and frees the copy;
- *  - epsp_test_fail_alloc makes the next device allocation of at least `bytes` bytes fail with
- *    EPSP_ENOMEM (0 switches it off), to test the error path without exhausting a device;
+ *  - epsp_test_fail_alloc makes the next device allocation of at least `bytes` bytes find no room (0
+ *    switches it off), to test without exhausting a device: EPSP_ENOMEM, unless the context's plans
+ *    have memory to give back (the FP64 paths' digit planes and work buffers), after which it is tried
+ *    again;
+ *  - epsp_test_product_panels makes the FP64 paths' products run in panels whose work buffers hold
+ *    `bytes` bytes each (128 rows or 64 columns at least; below 1 MiB as plain FP64 sums, as where no
+ *    work buffer fits the device; 0, the default: 4 GiB, less where the device has no room);
  *  - epsp_test_gemm_stall makes the one-CTA tensor-core GEMM kernel's producer skip K block
  *    `skip_kblock` of every tile (-1 switches it off) and that kernel's pipeline waits give up after
  *    `wait_limit` tries (0: the default, about 2^26), so that a call returns EPSP_EDEVICE_TIMEOUT
@@ -205,6 +210,7 @@ epsp_status epsp_ctx_keep_g2(epsp_ctx* ctx, int32_t on);
 epsp_status epsp_host_register(epsp_ctx* ctx, void* ptr, uint64_t bytes);
 epsp_status epsp_host_unregister(epsp_ctx* ctx, void* ptr);
 epsp_status epsp_test_fail_alloc(epsp_ctx* ctx, uint64_t bytes);
+epsp_status epsp_test_product_panels(epsp_ctx* ctx, uint64_t bytes);
 epsp_status epsp_test_gemm_stall(epsp_ctx* ctx, int32_t skip_kblock, uint32_t wait_limit);
 epsp_status epsp_test_g2_host_gather(epsp_ctx* ctx, int32_t on);
 

@@ -584,14 +584,15 @@ __global__ void coupling_rot_chunk_kernel(const T* __restrict__ g2c, const doubl
 //   q = 5    : (1 + n_ν) X+ + n_ν X- of c12 = 12
 // Thread (j, c0, k) forms all twelve rows: 72 FP64 operations, which bound the kernel (six an element; one
 // thread per element took about 18 and eight 16-byte loads: 647 us for 7680 x 2880, here 240). Rows j >= nω
-// and the columns of padding modes stay zero from the set-up. Grid (nω / 128, 3 ni, 2 nm).
+// and the columns of padding modes stay zero from the set-up. Grid (nω / 128 x 2 nm, 3 ni), (ν, c0) fastest.
 __global__ void __launch_bounds__(128) xgen_f64_kernel(const double2* __restrict__ J, const double4* __restrict__ xtab,
                                                        const double* __restrict__ nnu, int nw, int nwp, int nm, int nmp,
                                                        double* __restrict__ A) {
   pdl_wait();
-  const int j = blockIdx.x * 128 + threadIdx.x;
+  const unsigned z = blockIdx.x % (2u * unsigned(nm));
+  const int j = int(blockIdx.x / (2u * unsigned(nm))) * 128 + int(threadIdx.x);
   if (j >= nw) return;
-  const int b = blockIdx.y % 3, nu = blockIdx.z / 2, c0 = blockIdx.z % 2;
+  const int b = blockIdx.y % 3, nu = int(z / 2), c0 = int(z % 2);
   const long ip = blockIdx.y / 3;
   const double n = nnu[nu];
   const double4 t[2] = {xtab[(2l * nu) * nwp + j], xtab[(2l * nu + 1) * nwp + j]};
@@ -2187,7 +2188,7 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   set_mode_occupations(P, T);
   const long nwp = P->nwp, M = 24 * nwp, N = 3 * ni;
   long px = prof_begin(ctx, "xgen");
-  launch_after(s, xgen_f64_kernel, dim3(div_up(size_t(nw), 128), unsigned(3 * ni), unsigned(2 * P->nm)), 128, 0, 
+  launch_after(s, xgen_f64_kernel, dim3(div_up(size_t(nw), 128) * unsigned(2 * P->nm), unsigned(3 * ni)), 128, 0,
       J, P->d_xtab.p, P->d_nnu.p, int(nw), int(nwp), int(P->nm), int(P->nmp), P->d_Af.p);
   EPSP_LAUNCHED(ctx);
   prof_end(ctx, px);

@@ -31,6 +31,7 @@ inline void cuda_check(cudaError_t e, const char* what, const char* file, int li
   if (e != cudaSuccess) {
     char buf[512];
     std::snprintf(buf, sizeof buf, "%s failed at %s:%d: %s", what, file, line, cudaGetErrorString(e));
+    (void)cudaGetLastError();  // reported here: the next launch's check must not find it again
     fail(e == cudaErrorMemoryAllocation ? EPSP_ENOMEM : EPSP_ECUDA, buf);
   }
 }

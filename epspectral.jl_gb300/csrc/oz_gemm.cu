@@ -103,28 +103,28 @@ __global__ void __launch_bounds__(256) oz_split_m_kernel(const double* __restric
                                                          const uint32_t* __restrict__ mx, __nv_bfloat16* __restrict__ q) {
   pdl_wait();
   __shared__ unsigned long long tile[64][65];  // [k][r]
-  const long r0 = long(blockIdx.x) * 64;
-  const int tx = threadIdx.x % 64, ty = threadIdx.x / 64;
-  const long r = r0 + tx;
-  const uint32_t h = r < rows ? mx[r] : 0u;
-  const bool on = r < rows && oz_finite(h);
-  const int e = oz_exp(h);
-  for (long k0 = long(blockIdx.y) * 64; k0 < Kp; k0 += long(gridDim.y) * 64) {
+  const long r0 = long(blockIdx.x) * 64, k0 = (long(blockIdx.z) * gridDim.y + blockIdx.y) * 64;
+  if (k0 >= Kp) return;
+  {
+    const int tx = threadIdx.x % 64, ty = threadIdx.x / 64;
+    const long r = r0 + tx;
+    const uint32_t h = r < rows ? mx[r] : 0u;
+    const bool on = r < rows && oz_finite(h);
+    const int e = oz_exp(h);
 #pragma unroll 4
     for (int j = ty; j < 64; j += 4) {
       const long k = k0 + j;
       tile[j][tx] = oz_fixed(on && k < K ? S[r + ld * k] : 0.0, e);
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 512; t += 256) {  // 8 lanes write one row's 64 values
-      const int rl = t / 8, kg = t % 8;
-      if (r0 + rl >= rows || k0 + 8 * kg >= Kp) continue;
-      unsigned long long u[8];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 512; t += 256) {  // 8 lanes write one row's 64 values
+    const int rl = t / 8, kg = t % 8;
+    if (r0 + rl >= rows || k0 + 8 * kg >= Kp) continue;
+    unsigned long long u[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = tile[8 * kg + j][rl];
-      oz_store(u, rows, r0 + rl, Kp, k0 + 8 * kg, q);
-    }
-    __syncthreads();
+    for (int j = 0; j < 8; ++j) u[j] = tile[8 * kg + j][rl];
+    oz_store(u, rows, r0 + rl, Kp, k0 + 8 * kg, q);
   }
 }
 
@@ -481,7 +481,7 @@ void oz_split(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_majo
   const long kper = std::max<long>(std::min<long>(512, std::max<long>(16, (K + kb - 1) / kb)), (K + kMaxY - 1) / kMaxY);
   launch_after(s, oz_max_m_kernel, dim3(unsigned(nb), div_up(size_t(K), size_t(kper))), 256, 0, S, ld, rows, K, kper, P.mx.p);
   EPSP_LAUNCHED(ctx);
-  launch_after(s, oz_split_m_kernel, dim3(div_up(size_t(rows), 64), unsigned(std::min(Kp / 64, kMaxY))), 256, 0, S, ld, rows, K, Kp, P.mx.p, P.q.p);
+  launch_after(s, oz_split_m_kernel, dim3(div_up(size_t(rows), 64), unsigned(std::min(Kp / 64, kMaxY)), div_up(size_t(Kp / 64), size_t(kMaxY))), 256, 0, S, ld, rows, K, Kp, P.mx.p, P.q.p);
   EPSP_LAUNCHED(ctx);
 }
 

@@ -127,7 +127,7 @@ struct Ctx {
   size_t fail_alloc_bytes = 0;
   // Test hook: the size of the FP64 products' work buffers (0 = the default; below 1 MiB: as where none fits).
   size_t product_bytes = 0;
-  // Test hook of the one-CTA tensor-core GEMM: the producer skips K block `stall_kb` of every tile
+  // Test hook of the one-CTA tensor-core GEMM and of the digit products: the producer skips K block `stall_kb` of every tile
   // (-1 = off) and the pipeline waits give up after `stall_wait_limit` tries (0 = the default).
   int stall_kb = -1;
   unsigned stall_wait_limit = 0;

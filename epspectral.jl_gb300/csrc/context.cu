@@ -203,8 +203,8 @@ epsp_status epsp_ctx_keep_g2(epsp_ctx* c, int32_t on) {
   return EPSP_OK;
 }
 
-/* Test hook (not in the reference): the one-CTA tensor-core GEMM kernel's producer skips K block
- * `skip_kblock` of every tile (-1 switches it off), and that kernel's pipeline waits give up after
+/* Test hook (not in the reference): the one-CTA tensor-core GEMM kernel's and the FP64 digit products'
+ * producer skips K block `skip_kblock` of every tile (-1 switches it off), and their pipeline waits give up after
  * `wait_limit` tries (0 restores the default), so a call returns EPSP_EDEVICE_TIMEOUT from a wait
  * that runs out on the device rather than from a fault. */
 epsp_status epsp_test_gemm_stall(epsp_ctx* c, int32_t skip_kblock, uint32_t wait_limit) {

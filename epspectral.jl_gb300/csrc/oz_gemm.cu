@@ -160,12 +160,15 @@ struct OzSmem {
 // Bound: at BN = 256 shared memory (12 KB of operand reads and 12 KB of fills per 128 x 256 x 16 product,
 // of 128 B a cycle: 0.72 of the tensor rate); the tile narrows with N so that no more than a quarter
 // of it is padding, and `run` shortens until every SM has several items.
-template <int BN>
+// HOOK: the test hook's kernel, whose producer leaves out K block stall_kb and whose waits give up after hook_limit tries
+// (with both as arguments of the one kernel it took 3 % longer: 7680 x 180 x 2880 541 -> 556 us).
+template <int BN, bool HOOK>
 __global__ void __launch_bounds__(320, 1)
     oz_mma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const OzShape sh,
-                  int* __restrict__ sums, int* __restrict__ err) {
+                  int* __restrict__ sums, int* __restrict__ err, int stall_kb, unsigned hook_limit) {
   using L = OzSmem<BN>;
   constexpr int STAGES = L::kStages;
+  const unsigned wait_limit = HOOK ? hook_limit : kWaitLimit;
   constexpr int kCols = BN / 2;  // columns of one epilogue warp
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(320, 1)
       for (int c = o.c0; c < o.c1 && !stop; ++c, chunk_next(o, ch)) {
         for (int kb = ch.b0; kb < ch.b1; ++kb) {
           const int st = g % STAGES;
-          if (g >= STAGES && !mbar_wait(empty0 + 8 * st, ((g / STAGES) & 1) ^ 1)) {
+          if (g >= STAGES && !mbar_wait(empty0 + 8 * st, ((g / STAGES) & 1) ^ 1, wait_limit)) {
             atomicExch(&s_abort, 1);
             stop = true;
             break;
@@ -268,6 +271,10 @@ __global__ void __launch_bounds__(320, 1)
           if (aborted()) {
             stop = true;
             break;
+          }
+          if (HOOK && kb == stall_kb) {  // the issuer's wait for this block runs out
+            ++g;
+            continue;
           }
           const uint32_t dst = smem_u32(smem + st * L::kStage), fb = full0 + 8 * st;
           mbar_expect_tx(fb, L::kStage);
@@ -278,8 +285,8 @@ __global__ void __launch_bounds__(320, 1)
         }
       }
     }
-    if (aborted())  // wait (bounded) for the copies issued into stages not yet consumed
-      for (int k = max(0, g - STAGES); k < g; ++k) mbar_wait(full0 + 8 * (k % STAGES), (k / STAGES) & 1);
+    // wait (bounded) for the last copies, so that none is in flight when the block leaves, whichever warp gave up and when
+    for (int k = max(0, g - STAGES); k < g; ++k) mbar_wait(full0 + 8 * (k % STAGES), (k / STAGES) & 1, wait_limit);
   } else if (warp == 1 && lane == 0) {
     constexpr uint32_t idesc = idesc_f32acc<false>(BN);
     const uint64_t desc0 = sw128_desc(smem_u32(smem));
@@ -292,7 +299,7 @@ __global__ void __launch_bounds__(320, 1)
       for (int c = o.c0; c < o.c1 && !stop; ++c, ++t, chunk_next(o, ch)) {
         const int b = t & 1;
         const uint32_t acc = tmem + uint32_t(b * BN);
-        if (t >= 2 && !mbar_wait(acce0 + 8 * b, ((t >> 1) & 1) ^ 1)) {
+        if (t >= 2 && !mbar_wait_issuer(acce0 + 8 * b, ((t >> 1) & 1) ^ 1, &s_abort)) {
           atomicExch(&s_abort, 1);
           stop = true;
           break;
@@ -331,8 +338,9 @@ __global__ void __launch_bounds__(320, 1)
       Chunk ch = chunk_first(o);
       for (int c = o.c0; c < o.c1; ++c, ++t, chunk_next(o, ch)) {
         const int b = t & 1;
-        if (!mbar_wait(accf0 + 8 * b, (t >> 1) & 1)) atomicExch(&s_abort, 1);
-        if (aborted()) {
+        const bool got = mbar_wait(accf0 + 8 * b, (t >> 1) & 1, wait_limit);
+        if (!got) atomicExch(&s_abort, 1);
+        if (!__all_sync(0xffffffffu, got && !aborted())) {  // (the warp as one: the tensor memory loads are collective)
           stop = true;
           break;
         }
@@ -488,9 +496,12 @@ void oz_split(Ctx* ctx, const double* S, long ld, long rows, long K, bool k_majo
 template <int BN>
 static void launch_mma(Ctx* ctx, const OzPlanes& A, const OzPlanes& B, const OzShape& sh, int* sums, int* err) {
   using L = OzSmem<BN>;
-  EPSP_CUDA(cudaFuncSetAttribute(oz_mma_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
+  const bool hook = ctx->stall_kb >= 0 || ctx->stall_wait_limit;
+  auto* kern = hook ? oz_mma_kernel<BN, true> : oz_mma_kernel<BN, false>;
+  EPSP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
   const int items = sh.nM * sh.nN * sh.nseg * sh.per_seg;
-  launch_after(ctx->stream, oz_mma_kernel<BN>, std::min(items, ctx->sm_count), 320, L::kBytes, A.map, B.map, sh, sums, err);
+  launch_after(ctx->stream, kern, std::min(items, ctx->sm_count), 320, L::kBytes, A.map, B.map, sh, sums, err, ctx->stall_kb,
+               ctx->stall_wait_limit ? ctx->stall_wait_limit : kWaitLimit);
   EPSP_LAUNCHED(ctx);
 }
 

@@ -168,8 +168,8 @@ class Context:
         self.check(lib().epsp_ctx_keep_g2(self.handle, 1 if on else 0))
 
     def stall_gemm(self, skip_kblock: int = -1, wait_limit: int = 0):
-        """Test hook: the one-CTA tensor-core GEMM skips K block skip_kblock of every tile and gives
-        up its pipeline waits after wait_limit tries (EDEVICE_TIMEOUT); stall_gemm() switches it off."""
+        """Test hook: the one-CTA tensor-core GEMM and the FP64 products skip K block skip_kblock of every tile and give
+        up their pipeline waits after wait_limit tries (EDEVICE_TIMEOUT); stall_gemm() switches it off."""
         self.check(lib().epsp_test_gemm_stall(self.handle, int(skip_kblock), int(wait_limit)))
 
     def host_register(self, a: np.ndarray):

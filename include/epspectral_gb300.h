@@ -184,9 +184,9 @@ int64_t epsp_kernel_launches(const epsp_ctx* ctx);
  *  - epsp_test_product_panels makes the FP64 paths' products run in panels whose work buffers hold
  *    `bytes` bytes each (128 rows or 64 columns at least; below 1 MiB as plain FP64 sums, as where no
  *    work buffer fits the device; 0, the default: 4 GiB, less where the device has no room);
- *  - epsp_test_gemm_stall makes the one-CTA tensor-core GEMM kernel's producer skip K block
- *    `skip_kblock` of every tile (-1 switches it off) and that kernel's pipeline waits give up after
- *    `wait_limit` tries (0: the default, about 2^26), so that a call returns EPSP_EDEVICE_TIMEOUT
+ *  - epsp_test_gemm_stall makes the one-CTA tensor-core GEMM kernel's and the FP64 digit products'
+ *    producer skip K block `skip_kblock` of every tile (-1 switches it off) and their pipeline waits give
+ *    up after `wait_limit` tries (0: the default, about 2^26), so that a call returns EPSP_EDEVICE_TIMEOUT
  *    from a bounded device wait (the kernel frees its tensor memory and returns; the context and
  *    the plan stay usable);
  *  - epsp_test_g2_host_gather(ctx, 1) makes the set-ups' g2 stream gather g2 on the host into

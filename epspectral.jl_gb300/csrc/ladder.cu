@@ -1280,20 +1280,13 @@ __global__ void __launch_bounds__(256) combine_kernel(const __grid_constant__ Co
   }
 }
 
-// Y[r] = a X[r] + b Y[r]: complex a, b from the host (a_dev, b_dev null) or per right-hand side
-// from device memory.
+// Y = a X + b Y, complex a and b from the host.
 template <class V>
-__global__ void axpby_kernel(double2 a, const double2* __restrict__ a_dev, const V* __restrict__ X, double2 b,
-                             const double2* __restrict__ b_dev, V* __restrict__ Y, long n, const int* __restrict__ rmap) {
+__global__ void axpby_kernel(double2 a, const V* __restrict__ X, double2 b, V* __restrict__ Y, long n) {
   pdl_wait();
   using R = typename VecOf<V>::R;
   __shared__ R c[4];
-  const long r = slot_rhs<V>(rmap);
-  if (threadIdx.x == 0) {  // (rounded once a block, as in combine_kernel)
-    if (a_dev) a = a_dev[r];
-    if (b_dev) b = b_dev[r];
-    c[0] = R(a.x), c[1] = R(a.y), c[2] = R(b.x), c[3] = R(b.y);
-  }
+  if (threadIdx.x == 0) c[0] = R(a.x), c[1] = R(a.y), c[2] = R(b.x), c[3] = R(b.y);  // (once a block, as in combine_kernel)
   __syncthreads();
   const R ax = c[0], ay = c[1], bx = c[2], by = c[3];
   const long k0 = long(blockIdx.x) * (256 * kVecPer) + threadIdx.x;
@@ -1301,14 +1294,14 @@ __global__ void axpby_kernel(double2 a, const double2* __restrict__ a_dev, const
 #pragma unroll
   for (int e = 0; e < kVecPer; ++e)
     if (k0 + 256 * e < n) {
-      xv[e] = X[n * r + k0 + 256 * e];
-      yv[e] = Y[n * r + k0 + 256 * e];
+      xv[e] = X[k0 + 256 * e];
+      yv[e] = Y[k0 + 256 * e];
     }
 #pragma unroll
   for (int e = 0; e < kVecPer; ++e)
     if (k0 + 256 * e < n)
-      Y[n * r + k0 + 256 * e] = VecOf<V>::make(ax * xv[e].x - ay * xv[e].y + bx * yv[e].x - by * yv[e].y,
-                                               ax * xv[e].y + ay * xv[e].x + bx * yv[e].y + by * yv[e].x);
+      Y[k0 + 256 * e] = VecOf<V>::make(ax * xv[e].x - ay * xv[e].y + bx * yv[e].x - by * yv[e].y,
+                                       ax * xv[e].y + ay * xv[e].x + bx * yv[e].y + by * yv[e].x);
 }
 
 // Y[r] = a X[r] (Y is not read); a from the host or per right-hand side from device memory.
@@ -1334,59 +1327,6 @@ __global__ void scale_kernel(double2 a, const double2* __restrict__ a_dev, const
   for (int e = 0; e < kVecPer; ++e)
     if (k0 + 256 * e < n)
       Y[n * r + k0 + 256 * e] = VecOf<V>::make(ax * xv[e].x - ay * xv[e].y, ax * xv[e].y + ay * xv[e].x);
-}
-
-// q -= h v (h from device memory) and the block partials of |q|^2 of the result, in the order of
-// dot_partial_kernel (the norm of what the projection leaves, in the same pass). Single vectors.
-template <class V>
-__global__ void __launch_bounds__(256) axpy_norm_kernel(V* __restrict__ q, const V* __restrict__ v,
-                                                        const double2* __restrict__ h, long n, double2* __restrict__ part) {
-  using R = typename VecOf<V>::R;
-  __shared__ double sr[256];
-  const double2 hd = *h;
-  const R hx = R(hd.x), hy = R(hd.y);
-  double ar = 0;
-  if constexpr (std::is_same_v<V, double2>) {
-    for (long k = long(blockIdx.x) * 256 + threadIdx.x; k < n; k += long(gridDim.x) * 256) {
-      const V x = v[k];
-      V a = q[k];
-      a = VecOf<V>::make(a.x - (hx * x.x - hy * x.y), a.y - (hx * x.y + hy * x.x));
-      q[k] = a;
-      ar += a.x * a.x + a.y * a.y;
-    }
-  } else {
-    // runs of kRun strided elements, their loads issued together
-    const long stride = long(gridDim.x) * 256;
-    for (long k0 = long(blockIdx.x) * 256 + threadIdx.x; k0 < n; k0 += stride * kRun) {
-      V xs[kRun], as[kRun];
-#pragma unroll
-      for (int t = 0; t < kRun; ++t) {
-        const long k = k0 + stride * t;
-        if (k < n) {
-          xs[t] = v[k];
-          as[t] = q[k];
-        }
-      }
-      float fr = 0.f;
-#pragma unroll
-      for (int t = 0; t < kRun; ++t) {
-        const long k = k0 + stride * t;
-        if (k < n) {
-          const V a = VecOf<V>::make(as[t].x - (hx * xs[t].x - hy * xs[t].y), as[t].y - (hx * xs[t].y + hy * xs[t].x));
-          q[k] = a;
-          fr += a.x * a.x + a.y * a.y;
-        }
-      }
-      ar += fr;
-    }
-  }
-  sr[threadIdx.x] = ar;
-  __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sr[threadIdx.x] += sr[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = make_double2(sr[0], 0.0);
 }
 
 // Complex FP64 scalar arithmetic of the device Givens step (the operations of std::complex<double>
@@ -1605,15 +1545,13 @@ __global__ void gmres_givens_kernel(const double2* __restrict__ h1, const double
   inv_out->y = 0;
 }
 
-// O[r] = X[r] - Y[r] resp. X[r] + Y[r].
+// O = X - Y resp. X + Y.
 template <class V>
-__global__ void sub_kernel(const V* __restrict__ X, const V* __restrict__ Y, V* __restrict__ O, long n,
-                           const int* __restrict__ rmap) {
+__global__ void sub_kernel(const V* __restrict__ X, const V* __restrict__ Y, V* __restrict__ O, long n) {
   long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const long r = slot_rhs<V>(rmap);
-  const V x = X[n * r + k], y = Y[n * r + k];
-  O[n * r + k] = VecOf<V>::make(x.x - y.x, x.y - y.y);
+  const V x = X[k], y = Y[k];
+  O[k] = VecOf<V>::make(x.x - y.x, x.y - y.y);
 }
 
 template <class V>
@@ -2199,7 +2137,7 @@ static void apply_L(LadderPlan* P, const double2* J, double2* LJ, const double2*
   launch_after(s, y_gemm_kernel, div_up(size_t(ny), 256), 256, 0, P->d_D.p, int(nw), int(nwp), N, P->d_Y.p);
   EPSP_LAUNCHED(ctx);
   oz_gemm(ctx, P->oz, nw, 8 * N, nw, P->d_KK.p, nw, &P->ozKK, P->d_Y.p, nw, nullptr, 0.0, P->d_KY.p, nw);
-  launch_after(s, finish_gemm_kernel<double>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, 
+  launch_after(s, finish_gemm_kernel<double>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0,
       P->d_D.p, M, 1, 0, P->d_KY.p, 1, 0, P->d_Gm.p, P->d_Gp.p, nullptr, int(nw), int(nwp), int(ni), LJ, X);
   EPSP_LAUNCHED(ctx);
 }
@@ -2245,7 +2183,7 @@ static void apply_L(LadderPlan* P, const float2* J, float2* LJ, const float2* X 
   int sp2 = tc_gemm_launch(ctx, P->opKK, P->opY, int(nw), int(8 * N), int(nw), P->d_part2.p, nw, nw * 8 * N, 16, P->d_err.p,
                            "tc_ladder_kk");
   pl = prof_begin(ctx, "lfinish");
-  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0, 
+  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), 1), 256, 0,
       P->d_Dz.p, M, 1, 0, P->d_part2.p, sp2, nw * 8 * N, P->d_Gmf.p, P->d_Gpf.p, nullptr, int(nw), int(nwp), int(ni), LJ,
       X);
   EPSP_LAUNCHED(ctx);
@@ -2411,7 +2349,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
       auto op = [&](const V* x, V* y) {  // y = x - L(x)
         if (P->path == EPSP_PATH_DIRECT_FP64) {
           apply_L(P, x, LJ.p);
-          sub_kernel<V><<<eb, 256, 0, s>>>(x, LJ.p, y, n, nullptr);
+          sub_kernel<V><<<eb, 256, 0, s>>>(x, LJ.p, y, n);
           EPSP_LAUNCHED(ctx);
         } else {
           apply_L(P, x, y, x);  // the last pass of the operator forms x - L(x)
@@ -2438,7 +2376,7 @@ static void ladder_run_t(LadderPlan* P, const double* sigma, const double* mu, c
         if (warm) {          // r0 = b - A x0
           if (!needJ) cond_launch(P, J.p, Ybuf.p + ny);  // slot 1: σ(x0)
           op(J.p, W.p);
-          launch_after(s, axpby_kernel<V>, vb, 256, 0, make_double2(1, 0), nullptr, J0.p, make_double2(-1, 0), nullptr, W.p, n, nullptr);
+          launch_after(s, axpby_kernel<V>, vb, 256, 0, make_double2(1, 0), J0.p, make_double2(-1, 0), W.p, n);
           EPSP_LAUNCHED(ctx);
           dot_dev(P, W.p, W.p, n, part, Hdev.p + hB2);
           r0 = W.p;
@@ -2753,13 +2691,13 @@ static void apply_one_minus_L_batch(LadderPlan* P, LadderBatch& B, const float2*
                  reinterpret_cast<const int2*>(P->d_zwin.p), B.nnu.p, B.rmap.p, int(nw), int(nwp), int(P->nm), B.D.p, Mt,
                  P->d_err.p);
   EPSP_LAUNCHED(ctx);
-  launch_after(s, y_split_kernel, dim3(div_up(size_t(P->Kp2), 256), unsigned(N), unsigned(nA)), 256, 0, 
+  launch_after(s, y_split_kernel, dim3(div_up(size_t(P->Kp2), 256), unsigned(N), unsigned(nA)), 256, 0,
       B.D.p, Mt, 1, 0, int(nw), int(nwp), N, P->Kp2, B.Yh.p, B.Yl.p);
   EPSP_LAUNCHED(ctx);
   const long N2 = 8 * N * nA;
   int sp2 = tc_gemm_launch(ctx, P->opKK, B.opY, int(nw), int(N2), int(nw), B.part2.p, nw, nw * N2, 16, P->d_err.p,
                            "tc_ladder_kk");
-  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(nA)), 256, 0, 
+  launch_after(s, finish_gemm_kernel<float>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(nA)), 256, 0,
       B.D.p, Mt, 1, 0, B.part2.p, sp2, nw * N2, B.Gm.p, B.Gp.p, B.rmap.p, int(nw), int(nwp), int(ni), W, X);
   EPSP_LAUNCHED(ctx);
 }
@@ -2877,10 +2815,10 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
     B.tp.upload(tp.data(), tp.size(), s);
     B.nnu.upload(nnu.data(), nnu.size(), s);
     B.pp.upload(pp.data(), pp.size(), s);
-    launch_after(s, propagators_batch_kernel, dim3(div_up(size_t(nw), 128), unsigned(ni), unsigned(nP)), 128, 0, 
+    launch_after(s, propagators_batch_kernel, dim3(div_up(size_t(nw), 128), unsigned(ni), unsigned(nP)), 128, 0,
         S_all.p, P->d_ws.p, int(nw), B.jm.p, B.tm.p, B.jp.p, B.tp.p, P->d_eps_i.p, B.pp.p, B.Gm.p, B.Gp.p, int(ni));
     EPSP_LAUNCHED(ctx);
-    launch_after(s, attach_bare_kernel<float2>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(4 * nP)), 256, 0, 
+    launch_after(s, attach_bare_kernel<float2>, dim3(div_up(size_t(nw), 256), unsigned(6 * ni), unsigned(4 * nP)), 256, 0,
         B.Gm.p, B.Gp.p, P->d_v.p, int(nw), int(ni), B.J0.p);
     EPSP_LAUNCHED(ctx);
     conductivity_batch(P, B, B.J0.p, nP, pp, sb, idx);
@@ -2925,7 +2863,7 @@ void ladder_run_batched(LadderPlan* P, const double* sigma, const double* mu, co
       apply_one_minus_L_batch(P, B, B.V[size_t(k - 1)].p, nA, B.W.p);
       dot_batch(B.V[0].p, B.W.p, nA, B.H.p);
       for (int i = 0; i < k; ++i) {  // modified Gram-Schmidt; the last pass takes the norm
-        launch_after(s, axpy_dot_kernel<float2>, dim3(kDotBlocksB, unsigned(nA)), 256, 0, 
+        launch_after(s, axpy_dot_kernel<float2>, dim3(kDotBlocksB, unsigned(nA)), 256, 0,
             B.W.p, B.V[size_t(i)].p, B.H.p + long(i) * R, i + 1 < k ? B.V[size_t(i + 1)].p : nullptr, n, B.rmap.p, B.dpart.p);
         EPSP_LAUNCHED(ctx);
         launch_after(s, dot_final_kernel, unsigned(nA), 256, 0, B.dpart.p, kDotBlocksB, B.rmap.p, B.H.p + long(i + 1) * R);

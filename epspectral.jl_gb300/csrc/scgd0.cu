@@ -446,12 +446,6 @@ __global__ void __launch_bounds__(256) err_copy_kernel(const double2* __restrict
   err_copy(k < n ? Snew_all[t * n + k] : make_double2(0.0, 0.0), k < n, S_all + t * n + k, errbits_all + t);
 }
 
-__global__ void assemble_f32_kernel(const float* __restrict__ re, const float* __restrict__ im, double2* __restrict__ out,
-                                    long n) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k < n) out[k] = make_double2(double(re[k]), double(im[k]));
-}
-
 // Average over degenerate multiplets (src/scgd0.jl:293-301): thread per (ω, multiplet), the sum
 // over members in order divided by the count.
 __global__ void multiplet_kernel(double2* __restrict__ Sall, int nw, long slab, const int* __restrict__ slots,
@@ -1352,9 +1346,6 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
   P->d_Sin.alloc(ctx, size_t(P->nw * ni));
   P->d_ImS.alloc(ctx, size_t(P->nw * ni));
   P->d_ReS.alloc(ctx, size_t(P->nw * ni));
-  P->d_A.alloc(ctx, size_t(P->nwa * ni));
-  P->d_colsum.alloc(ctx, size_t(ni));
-  P->d_D.alloc(ctx, size_t(P->nwa));
   plog.mark("iteration buffers");
   return guard.release();
 }
@@ -1391,7 +1382,7 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
         const long per = std::max<long>(8, (len + want - 1) / want);
         const int splits = int((len + per - 1) / per);
         ensure(P->w_fmpart, ctx, size_t(nw * ni * splits));
-        launch_after(s, fm_direct_fast_kernel, dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0, 
+        launch_after(s, fm_direct_fast_kernel, dim3(tiles.x, tiles.y, unsigned(splits)), 32 * wpb, 0,
             P->d_ws.p, int(nw), P->d_wkey.p, P->d_jtab.p, int(P->d_jtab.n), float(P->ct.x0), float(P->ct.inv_h),
             P->fm_guard, P->w_fmtab.p, P->d_g2t.p, P->d_wqt.p, nvf, P->d_eps_f.p, P->d_w_f.p, P->d_f_to_i.p, int(nm),
             nm * f0, nm * f1, per, mu, T, 1.0 / T, P->w_ac, P->w_fmpart.p);
@@ -1421,7 +1412,7 @@ void scgd0_imsigma(Scgd0Plan* P, const double2* d_Sin, double mu, double T, doub
     ensure(P->w_fmtab, ctx, size_t((nw + 1) * ni));
     launch_after(s, fm_cell_kernel, div_up(size_t((nw + 1) * ni), 128), 128, 0, P->d_ws.p, int(nw), d_Sin, ni, P->w_fmtab.p);
     EPSP_LAUNCHED(ctx);
-    launch_after(s, kbuild_f64_kernel, dim3(div_up(size_t(nw), 128), unsigned(nk)), 128, 0, 
+    launch_after(s, kbuild_f64_kernel, dim3(div_up(size_t(nw), 128), unsigned(nk)), 128, 0,
         int(nw), P->w_fmtab.p, P->d_cell_j.p, P->d_cell_t.p, P->d_wnu.p, int(nm), P->d_epsc.p, P->d_colc.p, P->d_Fa.p,
         P->d_Fe.p, P->w_ac, P->d_Kt.p);
     EPSP_LAUNCHED(ctx);
@@ -1638,7 +1629,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
         }
       }
       if (P->nmult > 0 && !f32_spec) {
-        launch_after(s, multiplet_kernel, dim3(div_up(size_t(nw * P->nmult), 256), unsigned(nA)), 256, 0, 
+        launch_after(s, multiplet_kernel, dim3(div_up(size_t(nw * P->nmult), 256), unsigned(nA)), 256, 0,
             Snew.p, int(nw), slab, d_slots.p, P->d_mptr.p, P->d_midx.p, P->nmult);
         EPSP_LAUNCHED(ctx);
       }
@@ -1653,7 +1644,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
                      D_b.p, d_minA, mu_in, tc_err_ptr(P), d_tcerr, d_err, ctl);
         EPSP_LAUNCHED(ctx);
       } else {
-        launch_after(s, spectral_A_kernel, dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0, 
+        launch_after(s, spectral_A_kernel, dim3(div_up(size_t(nwa), 256), unsigned(ni), unsigned(nA)), 256, 0,
             Snew.p, int(nw), slab, d_slots.p, P->d_wsa.p, int(nwa), P->d_jsp.p, P->d_tsp.p, P->d_eps_i.p, A_b.p, int(ni));
         EPSP_LAUNCHED(ctx);
         launch_after(s, spectral_colsum_kernel, dim3(unsigned(ni), unsigned(nA)), 256, 0, A_b.p, int(nwa), int(ni), P->d_Wa.p,
@@ -1662,7 +1653,7 @@ void scgd0_run(Scgd0Plan* P, const epsp_occ* occ, const double* eta_min, double 
         launch_after(s, min_kernel, unsigned(nA), 256, 0, colsum_b.p, int(ni), d_slots.p, d_minA);
         EPSP_LAUNCHED(ctx);
         if (!fix_mu) {
-          launch_after(s, spectral_D_kernel, dim3(unsigned(spec_nab), unsigned(nA)), 256, 0, 
+          launch_after(s, spectral_D_kernel, dim3(unsigned(spec_nab), unsigned(nA)), 256, 0,
               A_b.p, int(nwa), int(ni), P->d_w_i.p, P->d_Wa.p, P->d_wsa.p, d_slots.p, D_b.p, mu_in);
           EPSP_LAUNCHED(ctx);
         }

@@ -92,7 +92,7 @@ struct Scgd0Plan {
   std::unique_ptr<Tc, void (*)(Tc*)> tc{nullptr, [](Tc*) {}};
   // iteration buffers
   DBuf<double2> d_Sin;
-  DBuf<double> d_ImS, d_ReS, d_A, d_colsum, d_D;
+  DBuf<double> d_ImS, d_ReS;
   // work buffers of scgd0_run, kept across runs (grown when a run needs more temperatures)
   DBuf<double2> w_S, w_Snew, w_Sin;
   int64_t sigma_nT = 0;  // temperatures of the last run's Σ in w_S (0: no run yet)
@@ -132,7 +132,6 @@ void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS);
 void tc_imsigma_disp(Scgd0Plan* P, const double2* d_Sin, double mu, double T, double* d_ImS);
 // The g2 upload of the term-by-term sums: g2 [nm, ni, nf] of any dtype to [nm nf, ni] FP64 (scgd0.cu).
 void upload_g2_permuted(Ctx* ctx, const epsp_model* m, DBuf<double>& g2t);
-void tc_kk_assemble(Scgd0Plan* P, double2* d_Snew);
 // Buffers and tensor maps for up to nT temperatures in one iteration.
 void tc_reserve(Scgd0Plan* P, long nT);
 // The temperatures tc_reserve's buffers hold now.
@@ -149,8 +148,6 @@ void tc_iterate(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, d
 // slots[0 .. nA) from Σ itself (afterwards each iteration leaves it for the next).
 void tc_start(Scgd0Plan* P, long nT, const TParams* d_tp);
 void tc_take_sigma(Scgd0Plan* P, int nA, const int* d_slots, const TParams* d_tp, const double2* d_S_all);
-// Fails with EPSP_EDEVICE_TIMEOUT if a tensor-core GEMM's bounded wait ran out (synchronises).
-void tc_check(Scgd0Plan* P);
 // The device flag the tensor-core GEMMs set when a bounded wait runs out.
 int* tc_err_ptr(Scgd0Plan* P);
 

@@ -297,20 +297,6 @@ static size_t kbuild_smem_bytes(long nm) { return size_t(kKbCols * nm * (kKbW + 
 // finalize_fm_batch_kernel writes them; else ImΣ added into add_out [nω, ni] (slot 0).
 constexpr int kFdTile = 256;
 
-__device__ __forceinline__ float2 pair_add(float2 a, float2 b) {  // a + b as a float pair
-  float e;
-  const float s = two_sum(a.x, b.x, e);
-  e += a.y + b.y;
-  const float h = s + e;
-  return make_float2(h, e - (h - s));
-}
-__device__ __forceinline__ bool pair_le(float2 a, float2 b) {  // a <= b for float pairs (normalised)
-  return a.x < b.x || (a.x == b.x && a.y <= b.y);
-}
-__device__ __forceinline__ float occ_fermion_f(float e, float T) {  // occ_fermion, src/utils.jl:14-22
-  if (T > 1.4901161193847656e-08f) return 1.f / (__expf(e / T) + 1.f);
-  return e > 0.f ? 0.f : (e < 0.f ? 1.f : 0.5f);
-}
 __device__ __forceinline__ float occ_boson_f(float e, float T) {  // occ_boson, src/utils.jl:24-38
   if (T > 1.4901161193847656e-08f) return e == 0.f ? -0.5f : 1.f / expm1f(e / T);
   return e > 0.f ? 0.f : (e == 0.f ? -0.5f : -1.f);
@@ -673,16 +659,6 @@ __global__ void finalize_add_kernel(const float* __restrict__ part, long n, int 
   float s = 0.f;
   for (int p = 0; p < splits; ++p) s += part[k + stride * p];
   out[k] += double(s);
-}
-
-// Σ_new = Σ_s part[s] + i ImΣ.
-__global__ void finalize_assemble_kernel(const float* __restrict__ part, long n, int splits, long stride,
-                                         const double* __restrict__ im, double2* __restrict__ out) {
-  long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  float s = 0.f;
-  for (int p = 0; p < splits; ++p) s += part[k + stride * p];
-  out[k] = make_double2(double(s), im[k]);
 }
 
 // exp(ω_ν/T) and n(ω_ν) of every temperature and mode of a run (the quotient's rounding put back); 0 where the
@@ -1206,20 +1182,6 @@ void tc_imsigma(Scgd0Plan* P, const double2* d_Sin, double* d_ImS) {
   check_err(P);
 }
 
-void tc_kk_assemble(Scgd0Plan* P, double2* d_Snew) {
-  Ctx* ctx = P->ctx;
-  cudaStream_t s = ctx->stream;
-  auto* T = P->tc.get();
-  const long nw = P->nw, ni = P->ni, slab = nw * ni;
-  split3_rows_kernel<<<div_up(size_t(ni * T->Kp2), 256), 256, 0, s>>>(P->d_ImS.p, nw, ni, nw, T->Kp2, false, T->Im[0].p,
-                                                                      T->Im[1].p, T->Im[2].p);
-  EPSP_LAUNCHED(ctx);
-  int sp = tc_gemm_launch(ctx, T->opKK, T->opIm, int(nw), int(ni), int(nw), T->part.p, nw, slab,
-                          max_splits_for(nw, kKbCapKK), T->err.p, "tc_kk", kKbCapKK);
-  finalize_assemble_kernel<<<div_up(size_t(slab), 256), 256, 0, s>>>(T->part.p, slab, sp, slab, P->d_ImS.p, d_Snew);
-  EPSP_LAUNCHED(ctx);
-}
-
 void tc_reserve(Scgd0Plan* P, long nT) {
   auto* T = P->tc.get();
   if (nT <= T->capT && T->ImS_b.p) return;
@@ -1254,7 +1216,6 @@ void tc_reserve(Scgd0Plan* P, long nT) {
   T->capT = nT;
 }
 
-void tc_check(Scgd0Plan* P) { check_err(P); }
 
 int* tc_err_ptr(Scgd0Plan* P) { return P->tc->err.p; }
 

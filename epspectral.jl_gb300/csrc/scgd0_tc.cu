@@ -454,9 +454,11 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
 // Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
-// search for the nearest node and a record for either side of it, 2.46 now (2.30 with (b + f) u as one FP32 number): 7.7
-// wavefronts a side and warp keep the L1 data pipe 85 % busy (4.7 of them the records, 20 bytes a lane), the issue slots
-// 71 % in that form.
+// search for the nearest node and a record for either side of it, 2.41 now (2.31 with (b + f) u as one FP32 number, whose
+// 7.7 wavefronts a side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue
+// slots 71 %). Four blocks an SM and one pair at a time for two nodes a thread, three and two for one (us at 501 nodes x
+// 105 states, 417 x 60 and, for one node, 200 x 105, 209 x 30): 2412, 867 and 1318, 261; four and two 2458, 921 and -, 293;
+// three and one 2491, 840; two and four -, - and 1373, 242.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
 // modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
@@ -488,7 +490,7 @@ __global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __r
 }
 
 template <int NPT, bool kSmemTab>
-__global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
+__global__ void __launch_bounds__(kFdTile, NPT == 1 ? 3 : 4) fm_disp_fast_kernel(
     int nw, long slab, const float4* __restrict__ rec_all, const float* __restrict__ dim_all,
     const float4* __restrict__ wtab_g, const int32_t* __restrict__ offs, const uint32_t* __restrict__ tab_g, int ntab, int pad,
     double unit, double inv_unit, double qm, double u_hi, const float* __restrict__ gw, const double* __restrict__ wph,
@@ -568,13 +570,14 @@ __global__ void __launch_bounds__(kFdTile, 4) fm_disp_fast_kernel(
     // (a warp past the last node, or whose second nodes are, does that part of the work no more than it must)
     if (iw0 - int(threadIdx.x % 32) >= nw) continue;
     const bool both = NPT == 1 || iw0 - int(threadIdx.x % 32) + kFdTile < nw;
+    constexpr int kUnroll = NPT == 1 ? 2 : 1;
     auto terms = [&](auto nodes) {
       for (int k0 = 0; k0 < nt; k0 += kFdRun) {
         float run0[NPT], run1[NPT];
 #pragma unroll
         for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
         const int k1 = min(nt, k0 + kFdRun);
-#pragma unroll 2
+#pragma unroll kUnroll
         for (int k = k0; k < k1; ++k) {
           const float4 A = s_a[k], E = s_e[k];
           const int4 C = s_c[k];

@@ -1078,8 +1078,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 5 : 1) finish_gemm_kerne
 // Batched over blockIdx.y: slot z works on the vectors of right-hand side r = rmap[z] (r = z without
 // rmap), stored n apart.
 
-// Three blocks an SM: a block's tree of FP64 sums takes as long as eight elements a thread (1024 blocks: the ladder
-// of 105 states x 625 nodes 1.78 ms, 456: 1.70, 304: 1.71 but a step of 495 x 1251 4.95 instead of 4.88).
+// Blocks of a dot product: a number, and not a multiple of the chip's SMs, since the blocks' partials make the order of the
+// sum and with it the bits of the result. About three for each of GB300's 152 SMs: a block's tree of FP64 sums takes as
+// long as eight elements a thread (1024 blocks: the ladder of 105 states x 625 nodes 1.78 ms, 456: 1.70, 304: 1.71 but a step of
+// 495 x 1251 4.95 instead of 4.88).
 constexpr int kDotBlocks = 456;
 // maxpy_kernel's blocks (one tree each): more from 16 elements a thread on, where its loads and stores in flight bound it
 // (n = 1.5e7: 1024 blocks 72 us, 456 108).
@@ -2614,7 +2616,7 @@ __global__ void propagators_batch_kernel(const double2* __restrict__ S_all, cons
 }
 
 // The batched BLAS-1 are the kernels above with blockIdx.y over the slots and rmap.
-constexpr int kDotBlocksB = 128;  // a right-hand side (256: the map of 16 4.48 ms, 128: 4.43)
+constexpr int kDotBlocksB = 128;  // of one right-hand side, of which there are several (256: the map of 16 4.48 ms, 128: 4.43)
 
 // Buffers of a batch of right-hand sides (capacity cap), tensor maps over them.
 struct LadderBatch {

@@ -157,9 +157,10 @@ struct OzSmem {
 // chunk runs and added into registers (adding 1.5 2^23 puts the integer into the mantissa, so a sum
 // costs one FP32 and one integer addition); after an item's last chunk the registers go to
 // sums[(seg, d)][n][m] by integer atomics (exact in any order), or by a store where the order is one item.
-// Bound: at BN = 256 shared memory (12 KB of operand reads and 12 KB of fills per 128 x 256 x 16 product,
-// of 128 B a cycle: 0.72 of the tensor rate); the tile narrows with N so that no more than a quarter
-// of it is padding, and `run` shortens until every SM has several items.
+// Bound: shared memory (at BN = 256, 12 KB of operand reads and 12 KB of fills per 128 x 256 x 16 product, of 128 B a
+// cycle: 0.72 of the tensor rate) and the issuing thread. The tile's width takes the fewest shared-memory cycles for
+// N, its padding included (oz_tile_n: half of a 128-wide tile is padding at N = 65, most of a 64-wide one below 32), and
+// `run` the shortest estimated time over the SMs (gemm_panel; a small product has fewer items than SMs).
 // HOOK: the test hook's kernel, whose producer leaves out K block stall_kb and whose waits give up after hook_limit tries
 // (with both as arguments of the one kernel it took 3 % longer: 7680 x 180 x 2880 541 -> 556 us).
 template <int BN, bool HOOK>
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(256) oz_plain_kernel(long M, long N, long K, c
 // ---- host ----
 
 int oz_tile_n(long N) {
-  // cycles of one product of the tile's width: the tensor rate (0.53 a column) or, wider, shared memory
+  // shared-memory cycles of one 16-term step of all tiles: A's 128 rows and the tile's columns, padding included
   int best = 64;
   long cost = -1;
   for (int bn : {256, 192, 128, 64}) {

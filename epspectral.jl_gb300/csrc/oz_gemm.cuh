@@ -3,7 +3,7 @@
 //
 //   C[M, N] = op(A)[M, K] B[K, N] + beta C, column-major, FP64 in and out.
 //
-// GB300 has 1.25 TFLOP/s of FP64 and about 2400 of BF16, so the product is formed from exact integer
+// GB300 has 1.25 TFLOP/s of FP64 and 1950 of BF16 (measured), so the product is formed from exact integer
 // products (the error-free splitting of Ozaki, Ogita, Oishi and Rump, 2012, on integers): each row
 // of A and each column of B is scaled by a power of two of its own (its largest magnitude < 2^e) and
 // rounded to 62-bit fixed point, written as eight balanced base-256 digits q_0..q_7 (|q| <= 128, exact
@@ -13,8 +13,12 @@
 // products; order 9 starts at 2^-68 of the two largest magnitudes), summed as one 128-bit integer and
 // rounded to FP64 once. So the result is reproducible bit for bit in any order of summation, and
 //   |error| <= 2^-53 |C_mn| + K 2^-60 max_k |A_mk| max_k |B_kn|,
-// the rounding of the inputs (2^-63 each) and the dropped orders. Rows or columns that hold an infinity
-// or a NaN are summed in FP64 directly, as IEEE arithmetic gives them.
+// the rounding of the inputs (2^-63 each) and the dropped orders. An operand's value that lies 2^-9 or more below the
+// largest of its row (A) or column (B) thus keeps fewer bits than FP64's 53, and one 2^-63 below none: an element of C far
+// below the products of those maxima is as accurate as the second term says. In the library's products, whose elements
+// spread over six decades, each element was closer to the exact sum than FP64 sums are (1e-16 against 3e-15 at worst, 15
+// modes x 30 states, widths of 1 and 10 meV). Rows or columns that hold an infinity or a NaN are summed in FP64
+// directly, as IEEE arithmetic gives them.
 //
 // A 64 x 64-tile FP64 SIMT kernel stood here before (1.2 TFLOP/s at large sizes, one block per tile).
 // Kernel time on one GB300, split of the changing operand and sum of the orders included:

@@ -393,7 +393,6 @@ __global__ void coupling_sum_chunk_kernel(const T* __restrict__ g2c, int nm, int
   }
 }
 
-// Σ_new = ReΣ + i ImΣ (src/scgd0.jl:290-291).
 // max of |a - S[k]| over the block's elements into *errbits, and S[k] ← a (src/scgd0.jl:326-328). The maximum of
 // non-negative doubles is taken on their bit patterns, which order the same way; NaN wins, as in Julia's maximum. It is
 // taken of the squares, and one root a block: a hypot an element, which a block falls back to where a square leaves the
@@ -423,7 +422,7 @@ __device__ __forceinline__ void err_copy(double2 a, bool on, double2* S, unsigne
   }
 }
 
-// Σ_new = re + i im of one temperature; with S, which then is its Σ, also max |Σ_new - Σ| and Σ ← Σ_new. Hands the
+// Σ_new = re + i im (src/scgd0.jl:290-291) of one temperature; with S, which then is its Σ, also max |Σ_new - Σ| and Σ ← Σ_new. Hands the
 // products' error flag on to the host's copy. 256 threads.
 __global__ void __launch_bounds__(256) assemble_kernel(const double* __restrict__ re, const double* __restrict__ im,
                                                        double2* __restrict__ out, long n, double2* __restrict__ S,
@@ -540,12 +539,11 @@ __global__ void __launch_bounds__(256) spectral_colsum_kernel(const double* __re
 // With ωa = ω_j + d_a (j = j_sp(a), t = t_sp(a)), the denominator's real part is
 //   ωa - ε_i - [(1 - t) ReΣ_j + t ReΣ_{j+1}] = d_a - v_j - t δ_j,
 //   v_j = ε_i - ω_j + ReΣ_j,  δ_j = ReΣ_{j+1} - ReΣ_j,
-// where v_j and δ_j are formed in FP64 once per grid node (nω ni, not nωa ni) and rounded to FP32.
-// Near a pole all three terms are of the size of the grid spacing, so the FP32 difference keeps an
+// where v_j and δ_j are formed on float pairs once per grid node (nω ni, not nωa ni) and rounded to FP32
+// (P[i][j] = (v_j, δ_j, ImΣ_j, ImΣ_{j+1}), by kk_epilogue_kernel). Near a pole all three terms are of the size of the grid spacing, so the FP32 difference keeps an
 // absolute error ~1e-7 h (~1e-10 eV). (Interpolating Σ in FP32 and subtracting it from ωa - ε_i
 // instead leaves ~1e-8 eV, which near a pole puts ~1e-5 into A and, through μ, a floor of ~1e-7 eV
 // under the iteration's convergence.)
-// (The terms P[i][j] = (v_j, δ_j, ImΣ_j, ImΣ_{j+1}) come from kk_epilogue_kernel.)
 // A[a, i] = -Im(1/(d_a - v_j - t δ_j + i((1-t) ImΣ_j + t ImΣ_{j+1})))/π, never stored: a block of
 // 64 nodes a and one chunk of 32 states accumulates Σ_i A w_i per node (Dpart[slot][chunk][a]) and
 // Σ_a A Wa per state (Cpart[slot][i][a-block], summed over the block's warps in warp order), both in

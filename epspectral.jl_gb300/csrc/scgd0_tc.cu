@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // search for the nearest node and a record for either side of it, 2.41 now (2.31 with (b + f) u as one FP32 number, whose
 // 7.7 wavefronts a side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue
 // slots 71 %). Four blocks an SM and one pair at a time for two nodes a thread, three and two for one (us at 501 nodes x
-// 105 states, 417 x 60 and, for one node, 200 x 105, 209 x 30): 2412, 867 and 1318, 261; four and two 2458, 921 and -, 293;
+// 105 states, 416 x 60 and, for one node, 201 x 105, 208 x 30): 2412, 867 and 1318, 261; four and two 2458, 921 and -, 293;
 // three and one 2491, 840; two and four -, - and 1373, 242.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
@@ -894,7 +894,7 @@ void tc_setup(Scgd0Plan* P) {
     fd_node_table_kernel<<<div_up(size_t(nw), 256), 256, 0, s>>>(P->d_ws.p, int(nw), P->d_wtab.p);
     EPSP_LAUNCHED(ctx);
   }
-  if (P->disp) {  // the Kramers-Kronig map's operands only: the Fan-Migdal sum is fm_disp_f32_kernel
+  if (P->disp) {  // the Kramers-Kronig map's operands only: the Fan-Migdal sum goes term by term (launch_fm_disp)
     for (int p = 0; p < kNs; ++p) {
       T->KK[p].alloc(ctx, size_t(nw * T->Kp2));
       T->Im[p].alloc(ctx, size_t(ni * T->Kp2));

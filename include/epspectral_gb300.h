@@ -57,8 +57,10 @@ enum { EPSP_METAL = 0, EPSP_SEMICONDUCTOR = 1 };
  *                dispersion. This is the parity path.
  *  GEMM_FP64   : dispersionless modes only: the Fan-Migdal sum recast as a kernel tensor times a
  *                coupling matrix, the ladder's shift sums regrouped per mode; FP64 arithmetic.
- *                (The products of both FP64 paths are exact integer products of eight digits a
- *                value on the tensor cores, rounded to FP64 once.)
+ *                (The products of both FP64 paths: values as 62-bit fixed point under the largest
+ *                of their row or column, in eight digits whose products of the nine leading orders
+ *                are summed exactly on the tensor cores and rounded to FP64 once. Error: 2^-53 of the
+ *                element and K 2^-60 of the largest of its row times the largest of its column.)
  *  GEMM_BF16X3 : as GEMM_FP64, with the contractions on the tcgen05 tensor cores in BF16 hi/lo
  *                split precision (three products, FP32 accumulation); the chemical-potential
  *                bisection, the carrier integral and the GMRES orthogonalisation stay FP64.

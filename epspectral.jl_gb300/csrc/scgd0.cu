@@ -1300,7 +1300,11 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
     {
       const auto& w = P->ws.nodes;
       const long n = P->nw;
-      // (cell tables: cell j is entry j + 1, entry 0 the flat part below the grid)
+      // (cell tables: cell j is entry j + 1, entry 0 the flat part below the grid.) FP32 records: a point that misses a
+      // node from below by rounding alone, as where the modes are multiples of the grid's step, is taken from that node;
+      // as the far end of the cell below it would carry 2^-24 of the values at that cell's start, which may be large
+      // against those at the node.
+      const double snap = P->path == EPSP_PATH_GEMM_BF16 ? 0x1p-44 * std::max(std::fabs(w.front()), std::fabs(w.back())) : 0.0;
       std::vector<int32_t> cj(size_t(2 * n * nm));
       std::vector<double> cdx(cj.size());
       for (long side = 0; side < 2; ++side)
@@ -1315,6 +1319,7 @@ Scgd0Plan* scgd0_setup(Ctx* ctx, const epsp_model* m, const epsp_options* opts) 
             } else {
               const int32_t c = ct.jtab[size_t(int64_t((x - ct.x0) * ct.inv_h))];
               e = c + (w[size_t(c)] <= x ? 1 : 0);
+              if (w[size_t(e)] - x <= snap) ++e;
             }
             const size_t k = size_t(iw + n * (nu + nm * side));
             cj[k] = e;

@@ -445,7 +445,9 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 //    ε (ε' = ε - f u_hi, a pair a side), so Re z = ((U_hi - ε'_hi) + b u_hi) + ((U_lo - ε'_lo) + (b + f) (u_lo - u ReΣ')).
 //    High parts are multiples of one quantum (split_q): the first bracket is exact, and Re z keeps its distance to a
 //    pole anywhere in a wide cell (as (b + f) times u (1 - ReΣ') in FP32, terms near poles 0.2 meV wide were off by
-//    1e-5 in cells of 0.25 eV). The cells below and above the grid have slopes 0 (fd_cell_kernel).
+//    1e-5 in cells of 0.25 eV). The cells below and above the grid have slopes 0 (fd_cell_kernel). Where ωq is a whole
+//    number to rounding, x is that node on both sides (not the far end of the cell below, 2^-24 of whose start's ImΣ may
+//    be large against the node's).
 //  * n + f(x_a - μ) = (1 + n)(1 + E)/(1 + E e) and n + 1 - f(x_e - μ) = n (1 + E)/(1 + E/e), E = exp((ω - μ)/T),
 //    e = exp(ωq/T): one FMA a side, the bracket's reciprocal shared with 1/|z|², and 1 + E outside the sum
 //    (both sides over E above μ, so that every factor stays below e^40).
@@ -454,11 +456,11 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
 // Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
-// search for the nearest node and a record for either side of it, 2.41 now (2.31 with (b + f) u as one FP32 number, whose
+// search for the nearest node and a record for either side of it, 2.49 now (2.31 with (b + f) u as one FP32 number, whose
 // 7.7 wavefronts a side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue
-// slots 71 %). Four blocks an SM and one pair at a time for two nodes a thread, three and two for one (us at 501 nodes x
-// 105 states, 416 x 60 and, for one node, 201 x 105, 208 x 30): 2412, 867 and 1318, 261; four and two 2458, 921 and -, 293;
-// three and one 2491, 840; two and four -, - and 1373, 242.
+// slots 71 %). Three blocks an SM and two pairs in flight (us at 501 nodes x 105 states, 416 x 60, 312 x 30 with two nodes
+// a thread, 201 x 105 and 208 x 30 with one): 2488, 859, 442, 1327, 261; four and one 2472, 920, -; four and two 2478, 939,
+// 517; four and four 2452, 905, 496; three and one 2519, 852, 443.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
 // modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
@@ -490,7 +492,7 @@ __global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __r
 }
 
 template <int NPT, bool kSmemTab>
-__global__ void __launch_bounds__(kFdTile, NPT == 1 ? 3 : 4) fm_disp_fast_kernel(
+__global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
     int nw, long slab, const float4* __restrict__ rec_all, const float* __restrict__ dim_all,
     const float4* __restrict__ wtab_g, const int32_t* __restrict__ offs, const uint32_t* __restrict__ tab_g, int ntab, int pad,
     double unit, double inv_unit, double qm, double u_hi, const float* __restrict__ gw, const double* __restrict__ wph,
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(kFdTile, NPT == 1 ? 3 : 4) fm_disp_fast_kernel
     const TParams* __restrict__ tp, double* __restrict__ part) {
   extern __shared__ __align__(16) uint32_t fd_cells[];  // kSmemTab: the cell table
   // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε' of the absorption and of the emission
-  // as pairs}, {the column, ωq's whole number, its fraction f and 1 - f (float bits)}
+  // as pairs}, {the column, ωq's whole numbers of the absorption and (<< 16) of the emission, what they leave (float bits)}
   __shared__ float4 s_a[kFdTile], s_e[kFdTile];
   __shared__ int4 s_c[kFdTile];
   if constexpr (kSmemTab)
@@ -554,12 +556,14 @@ __global__ void __launch_bounds__(kFdTile, NPT == 1 ? 3 : 4) fm_disp_fast_kernel
       const double wq = wph[nu + long(nm) * iq_kk[ki + nk_i * long(iks_f[f])]];
       if (!(wq < w_ac)) {
         const float wp = float(wq), n = occ_boson_f(wp, T), g = gw[vf + nvf * i];
-        // (the fraction exactly, whichever side of a whole number the product rounds to)
-        const double wb = fmin(floor(wq * inv_unit), double(pad - 1)), fr = fma(-wb, unit, wq) * inv_unit, ef = eps_f[f];
-        const float2 ea = split_q(fma(-fr, u_hi, ef), qm), ee = split_q(fma(fr - 1.0, u_hi, ef), qm);
+        // x = ω + ωq = b + wb and fr, ω - ωq = b - wb - up and fe, in units; fr within 2^-32 of a whole number is next to it
+        const double wb = fmin(floor(fma(wq, inv_unit, 0x1p-32)), double(pad - 1)), fr = fma(-wb, unit, wq) * inv_unit;
+        const int up = fr > 0x1p-32 ? 1 : 0;
+        const double fe = double(up) - fr, ef = eps_f[f];
+        const float2 ea = split_q(fma(-fr, u_hi, ef), qm), ee = split_q(fma(-fe, u_hi, ef), qm);
         sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp, T), exp_comp(-wp, T));
         se = make_float4(ea.x, ea.y, ee.x, ee.y);
-        sc = make_int4((nw + 1) * f_to_i[f], int(wb), __float_as_int(float(fr)), __float_as_int(float(1.0 - fr)));
+        sc = make_int4((nw + 1) * f_to_i[f], int(wb) | (int(wb) + up) << 16, __float_as_int(float(fr)), __float_as_int(float(fe)));
       }
     }
     s_a[threadIdx.x] = sa;
@@ -570,21 +574,21 @@ __global__ void __launch_bounds__(kFdTile, NPT == 1 ? 3 : 4) fm_disp_fast_kernel
     // (a warp past the last node, or whose second nodes are, does that part of the work no more than it must)
     if (iw0 - int(threadIdx.x % 32) >= nw) continue;
     const bool both = NPT == 1 || iw0 - int(threadIdx.x % 32) + kFdTile < nw;
-    constexpr int kUnroll = NPT == 1 ? 2 : 1;
     auto terms = [&](auto nodes) {
       for (int k0 = 0; k0 < nt; k0 += kFdRun) {
         float run0[NPT], run1[NPT];
 #pragma unroll
         for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
         const int k1 = min(nt, k0 + kFdRun);
-#pragma unroll kUnroll
+#pragma unroll 2
         for (int k = k0; k < k1; ++k) {
           const float4 A = s_a[k], E = s_e[k];
           const int4 C = s_c[k];
+          const int wa = C.y & 0xffff, we = C.y >> 16;
 #pragma unroll
           for (int n = 0; n < decltype(nodes)::value; ++n) {
-            side(off[n] + C.y, __int_as_float(C.z), make_float2(E.x, E.y), C.x, fmaf(qe[n], A.z, p[n]), A.x, run0[n]);
-            side(off[n] - C.y - 1, __int_as_float(C.w), make_float2(E.z, E.w), C.x, fmaf(qe[n], A.w, p[n]), A.y, run1[n]);
+            side(off[n] + wa, __int_as_float(C.z), make_float2(E.x, E.y), C.x, fmaf(qe[n], A.z, p[n]), A.x, run0[n]);
+            side(off[n] - we, __int_as_float(C.w), make_float2(E.z, E.w), C.x, fmaf(qe[n], A.w, p[n]), A.y, run1[n]);
           }
         }
 #pragma unroll
@@ -1098,7 +1102,7 @@ static void fd_table(Scgd0Plan* P) {
   div = std::max(1l, div);
   const double unit = g.unit * double(div), wq = P->wq_max / unit;
   if (!(wq < double(kFdMaxCell - 1)) || widest / div > kFdMaxCell || nw > 65534 || (nw + 1) * P->ni >= (1l << 31)) return;
-  const long pad = long(std::floor(std::max(0.0, wq))) + 1;  // the whole numbers are 0 .. pad - 1
+  const long pad = long(std::floor(std::max(0.0, wq))) + 2;  // the whole numbers are 0 .. pad - 1 (rounded up at most)
   const long range = (g.offsets[size_t(nw - 1)] - g.offsets[0]) / div, n = range + 2 * pad;
   if (n > kFdMaxTable) return;
   std::vector<int32_t> off(static_cast<size_t>(nw));

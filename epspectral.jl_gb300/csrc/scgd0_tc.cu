@@ -475,20 +475,22 @@ __device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v 
 }
 
 // Records [column][nω + 1] of slot blockIdx.y: cell 0 is below the grid, cell c from node c - 1 to node c, cell nω above.
+// Slopes in FP64 and rounded once: far inside a wide cell they are what is left of the error.
 __global__ void fd_cell_kernel(const float4* __restrict__ Sf_all, const int* __restrict__ slots,
-                               const float4* __restrict__ wtab, const double* __restrict__ ws, int nw, long slab, double unit,
-                               float u_lo, double qm, float4* __restrict__ rec, float* __restrict__ dim) {
+                               const double* __restrict__ ws, int nw, long slab, double unit, double u_hi, double qm,
+                               float4* __restrict__ rec, float* __restrict__ dim) {
   const long ncell = slab / nw * (nw + 1);
   const long k = long(blockIdx.x) * blockDim.x + threadIdx.x;
   if (k >= ncell) return;
-  const int c = int(k % (nw + 1)), j = max(c - 1, 0);
+  const int c = int(k % (nw + 1)), j = max(c - 1, 0), o = min(c, nw - 1);
   const float4* Sf = Sf_all + slab * slots[blockIdx.y] + k / (nw + 1) * nw;
-  const float4 s = Sf[j], o = Sf[min(c, nw - 1)];
-  const float2 u = split_q(ws[j] - (double(s.x) + double(s.y)), qm);
-  const float inv = c == 0 || c == nw ? 0.f : wtab[j].z;
-  const float dre = ((o.x - s.x) + (o.y - s.y)) * inv, di = (o.z - s.z) * inv;
-  rec[ncell * blockIdx.y + k] = make_float4(u.x, u.y, fmaf(-float(unit), dre, u_lo), s.z);
-  dim[ncell * blockIdx.y + k] = float(unit) * di;
+  const float4 s = Sf[j], t = Sf[o];
+  const double re = double(s.x) + double(s.y);
+  const float2 u = split_q(ws[j] - re, qm);
+  const double per = o > j ? unit / (ws[o] - ws[j]) : 0.0;  // (0 below and above the grid)
+  rec[ncell * blockIdx.y + k] =
+      make_float4(u.x, u.y, float((unit - u_hi) - per * ((double(t.x) + double(t.y)) - re)), s.z);
+  dim[ncell * blockIdx.y + k] = float(per * (double(t.z) - double(s.z)));
 }
 
 template <int NPT, bool kSmemTab>
@@ -1001,7 +1003,7 @@ static void launch_fm_disp(Scgd0Plan* P, int nA, const int* d_slots, const TPara
     ensure(T->fddim, ctx, size_t(ncell * nA));
     const double u_hi = std::rint(P->fd_unit / P->re_q) * P->re_q;
     fd_cell_kernel<<<dim3(div_up(size_t(ncell), 256), unsigned(nA)), 256, 0, ctx->stream>>>(
-        T->Sf.p, d_slots, P->d_wtab.p, P->d_ws.p, int(nw), slab, P->fd_unit, float(P->fd_unit - u_hi), P->re_qmd, T->fdrec.p, T->fddim.p);
+        T->Sf.p, d_slots, P->d_ws.p, int(nw), slab, P->fd_unit, u_hi, P->re_qmd, T->fdrec.p, T->fddim.p);
     EPSP_LAUNCHED(ctx);
     const size_t tab = sizeof(uint32_t) * P->d_fdtab.n;
     const int nsplit = fd_splits(P, nA), npt = fd_nodes(P);

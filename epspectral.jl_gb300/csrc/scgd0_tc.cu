@@ -456,11 +456,11 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
 // Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
-// search for the nearest node and a record for either side of it, 2.49 now (2.31 with (b + f) u as one FP32 number, whose
+// search for the nearest node and a record for either side of it, 2.48 now (2.31 with (b + f) u as one FP32 number, whose
 // 7.7 wavefronts a side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue
-// slots 71 %). Three blocks an SM and two pairs in flight (us at 501 nodes x 105 states, 416 x 60, 312 x 30 with two nodes
-// a thread, 201 x 105 and 208 x 30 with one): 2488, 859, 442, 1327, 261; four and one 2472, 920, -; four and two 2478, 939,
-// 517; four and four 2452, 905, 496; three and one 2519, 852, 443.
+// slots 71 %). Three blocks an SM and two pairs in flight (us at 501 nodes x 105 states, 416 x 60 x 2 temperatures, 312 x
+// 30 with two nodes a thread, 201 x 105 and 208 x 30 with one): 2475, 583, 164, 1270, 103, and 241 ms at 1251 x 495; four
+// and one 2429, 613, 191, 1252, 125, and 252 ms.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
 // modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
@@ -980,13 +980,14 @@ static void check_err(Scgd0Plan* P) {
 // 32.1; the second node's work is skipped by the warps that have none).
 static int fd_nodes(const Scgd0Plan* P) { return P->nw > kFdTile ? 2 : 1; }
 
-// Splits of the (ν, f) range for nA slots: about 40 blocks a multiprocessor (four are resident, so the last wave is a
-// tenth of the time), eight tiles of pairs a split at least (a block's tables and tail).
+// Splits of the (ν, f) range for nA slots: about 40 blocks a multiprocessor (three are resident, so the last wave is a
+// small part of the time), two tiles of pairs a split at least (a block's tables and tail; with eight, which left SMs
+// idle, 416 nodes x 60 states x 2 temperatures took 859 us, now 583, 208 x 30 262, now 103, 501 x 105 2486, now 2475).
 static int fd_splits(const Scgd0Plan* P, long nA) {
   const long tiles = div_up(size_t(P->nm * P->nf), kFdTile);
   const long blocks = long(div_up(size_t(P->nw), size_t(kFdTile * fd_nodes(P)))) * P->ni * nA;
   const long want = std::max<long>(1, (40l * P->ctx->sm_count + blocks - 1) / blocks);
-  const long n = std::min(want, std::max<long>(1, tiles / 8));
+  const long n = std::min(want, std::max<long>(1, tiles / 2));
   return int(div_up(size_t(tiles), div_up(size_t(tiles), size_t(n))));  // no empty split
 }
 

@@ -456,11 +456,12 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
 // last of the waves of resident blocks weighs little (partials summed in order by fd_finish_kernel); at 501 nodes and
 // 105 states the unsplit grid of 210 blocks left a third of the SMs half empty.
 // Measured: 1.2e9 terms (501 nodes, 105 states, 15 modes, 1536 inner states) 13.0 ms by the kernel above, 3.25 with a
-// search for the nearest node and a record for either side of it, 2.48 now (2.31 with (b + f) u as one FP32 number, whose
-// 7.7 wavefronts a side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue
-// slots 71 %). Three blocks an SM and two pairs in flight (us at 501 nodes x 105 states, 416 x 60 x 2 temperatures, 312 x
-// 30 with two nodes a thread, 201 x 105 and 208 x 30 with one): 2475, 583, 164, 1270, 103, and 241 ms at 1251 x 495; four
-// and one 2429, 613, 191, 1252, 125, and 252 ms.
+// search for the nearest node and a record for either side of it, 2.31 with (b + f) u as one FP32 number (7.7 wavefronts a
+// side and warp, 4.7 of them the records' 20 bytes a lane, kept the L1 data pipe 90 % busy and the issue slots 71 %), 2.48
+// with it exact, 2.32 now, a term's two sides in one instruction where their operands lie side by side. Three blocks an SM
+// and two pairs in flight (us there, at 416 nodes x 60 states x 2 temperatures, 312 x 30 with two nodes a thread, 201 x
+// 105 and 208 x 30 with one): 2320, 551, 148, 1237, 103, and 230 ms at 1251 x 495; four and two 2286, 575, 162, 1223, 99, and
+// 245 ms; three and one 2355, 557, 163, 1228, 119; two and four 2401, 559, 136, 1363, 92.
 constexpr float kFdMaxArg = 40.f;
 // Terms of an FP32 run (added into FP64). Error of one sum against the FP64 kernel, relative (30 states x 251 nodes x 6
 // modes, 105 x 501 x 15): 7.6e-8, 2.7e-8 with runs of a tile's 256, 3.9e-8, 1.5e-8 with 64, 3.4e-8, 1.4e-8 with 32; the
@@ -468,6 +469,34 @@ constexpr float kFdMaxArg = 40.f;
 constexpr int kFdRun = 64;
 constexpr long kFdMaxTable = 1l << 24;  // entries; those that fit 96 KB are kept in shared memory
 constexpr long kFdMaxCell = 32767;      // grid units of a cell or ωq: distances are 16 bits
+
+// Two FP32 values in a register pair, and operations on both (each rounded as alone).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pk(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 upk(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 
 __device__ __forceinline__ float exp_comp(float v, float T) {  // exp(v / T), v / T's rounding put back
   const float a = v / T, E = expf(a);
@@ -503,7 +532,7 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
     const int32_t* __restrict__ f_to_i, int nm, long nvf, long per, int nsplit, double w_ac, const int* __restrict__ slots,
     const TParams* __restrict__ tp, double* __restrict__ part) {
   extern __shared__ __align__(16) uint32_t fd_cells[];  // kSmemTab: the cell table
-  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {ε' of the absorption and of the emission
+  // the staged (ν, f) pairs: {w_f g2 (1 + n), w_f g2 n, exp(ωq/T), exp(-ωq/T)}, {-ε' of the absorption and of the emission
   // as pairs}, {the column, ωq's whole numbers of the absorption and (<< 16) of the emission, what they leave (float bits)}
   __shared__ float4 s_a[kFdTile], s_e[kFdTile];
   __shared__ int4 s_c[kFdTile];
@@ -532,15 +561,21 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
   }
   const int ki = iks_i[i];
   const float uf = float(u_hi);
-  auto side = [&](int b, float frac, float2 e, int col, float o, float g, float& run) {
-    const uint32_t t = tab[b];  // the cell, and b's distance from its lower node + 32768
-    const float n = __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7610)) - 8421376.f, dx = n + frac;
-    const int at = col + int(t >> 16);
-    const float4 r = rec[at];
-    const float zr = fmaf(n, uf, r.x - e.x) + fmaf(dx, r.z, r.y - e.y);
-    const float si = fmaf(dx, dim[at], r.w);
-    const float d = fmaf(zr, zr, si * si) * o;
-    run = fmaf(g * si, rcp_f(d), run);
+  // both sides of a term at one node, two FP32 operations an instruction: the record's differences, then (absorption,
+  // emission) side by side
+  const F2 magic = pk(-8421376.f, -8421376.f);
+  auto sides = [&](int ba, int be, F2 frac, F2 ea, F2 ee, int col, F2 o, F2 g, F2& run) {
+    const uint32_t ta = tab[ba], te = tab[be];  // the cell, and b's distance from its lower node + 32768
+    const F2 n = add2(pk(__uint_as_float(__byte_perm(ta, 0x4B000000u, 0x7610)), __uint_as_float(__byte_perm(te, 0x4B000000u, 0x7610))), magic);
+    const F2 dx = add2(n, frac);
+    const int aa = col + int(ta >> 16), ae = col + int(te >> 16);
+    const float4 ra = rec[aa], re = rec[ae];
+    const F2 ua = add2(pk(ra.x, ra.y), ea), ue = add2(pk(re.x, re.y), ee);
+    const float2 nn = upk(n), dd = upk(dx), va = upk(ua), ve = upk(ue);
+    const F2 zr = pk(fmaf(nn.x, uf, va.x) + fmaf(dd.x, ra.z, va.y), fmaf(nn.y, uf, ve.x) + fmaf(dd.y, re.z, ve.y));
+    const F2 si = pk(fmaf(dd.x, dim[aa], ra.w), fmaf(dd.y, dim[ae], re.w));
+    const float2 d = upk(mul2(fma2(zr, zr, mul2(si, si)), o));
+    run = fma2(mul2(g, si), pk(rcp_f(d.x), rcp_f(d.y)), run);
   };
   double acc[NPT];
 #pragma unroll
@@ -550,7 +585,7 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
     const long vf = t0 + threadIdx.x;
     __syncthreads();  // the previous tile's readers are done (and, first, the table is staged)
     // below ω_acoustic no term: zero coupling, and ε = -1e25, so that |z|² overflows and the reciprocal is 0
-    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(-1e25f, 0.f, -1e25f, 0.f);
+    float4 sa = make_float4(0.f, 0.f, 1.f, 1.f), se = make_float4(1e25f, 0.f, 1e25f, 0.f);
     int4 sc = make_int4(0, 0, 0, 0);
     if (vf < t_end) {
       const int nu = int(vf % nm);
@@ -564,7 +599,7 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
         const double fe = double(up) - fr, ef = eps_f[f];
         const float2 ea = split_q(fma(-fr, u_hi, ef), qm), ee = split_q(fma(-fe, u_hi, ef), qm);
         sa = make_float4(g * (n + 1.f), g * n, exp_comp(wp, T), exp_comp(-wp, T));
-        se = make_float4(ea.x, ea.y, ee.x, ee.y);
+        se = make_float4(-ea.x, -ea.y, -ee.x, -ee.y);
         sc = make_int4((nw + 1) * f_to_i[f], int(wb) | (int(wb) + up) << 16, __float_as_int(float(fr)), __float_as_int(float(fe)));
       }
     }
@@ -578,9 +613,9 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
     const bool both = NPT == 1 || iw0 - int(threadIdx.x % 32) + kFdTile < nw;
     auto terms = [&](auto nodes) {
       for (int k0 = 0; k0 < nt; k0 += kFdRun) {
-        float run0[NPT], run1[NPT];
+        F2 run[NPT];
 #pragma unroll
-        for (int n = 0; n < NPT; ++n) run0[n] = run1[n] = 0.f;
+        for (int n = 0; n < NPT; ++n) run[n] = pk(0.f, 0.f);
         const int k1 = min(nt, k0 + kFdRun);
 #pragma unroll 2
         for (int k = k0; k < k1; ++k) {
@@ -589,12 +624,12 @@ __global__ void __launch_bounds__(kFdTile, 3) fm_disp_fast_kernel(
           const int wa = C.y & 0xffff, we = C.y >> 16;
 #pragma unroll
           for (int n = 0; n < decltype(nodes)::value; ++n) {
-            side(off[n] + wa, __int_as_float(C.z), make_float2(E.x, E.y), C.x, fmaf(qe[n], A.z, p[n]), A.x, run0[n]);
-            side(off[n] - we, __int_as_float(C.w), make_float2(E.z, E.w), C.x, fmaf(qe[n], A.w, p[n]), A.y, run1[n]);
+            sides(off[n] + wa, off[n] - we, pk(__int_as_float(C.z), __int_as_float(C.w)), pk(E.x, E.y), pk(E.z, E.w), C.x,
+                  fma2(pk(qe[n], qe[n]), pk(A.z, A.w), pk(p[n], p[n])), pk(A.x, A.y), run[n]);
           }
         }
 #pragma unroll
-        for (int n = 0; n < decltype(nodes)::value; ++n) acc[n] += double(run0[n]) + double(run1[n]);
+        for (int n = 0; n < decltype(nodes)::value; ++n) acc[n] += double(upk(run[n]).x) + double(upk(run[n]).y);
       }
     };
     if (both)
@@ -982,7 +1017,7 @@ static int fd_nodes(const Scgd0Plan* P) { return P->nw > kFdTile ? 2 : 1; }
 
 // Splits of the (ν, f) range for nA slots: about 40 blocks a multiprocessor (three are resident, so the last wave is a
 // small part of the time), two tiles of pairs a split at least (a block's tables and tail; with eight, which left SMs
-// idle, 416 nodes x 60 states x 2 temperatures took 859 us, now 583, 208 x 30 262, now 103, 501 x 105 2486, now 2475).
+// idle, 416 nodes x 60 states x 2 temperatures took 1.5 times as long, 208 x 30 2.5 times, 501 x 105 as long).
 static int fd_splits(const Scgd0Plan* P, long nA) {
   const long tiles = div_up(size_t(P->nm * P->nf), kFdTile);
   const long blocks = long(div_up(size_t(P->nw), size_t(kFdTile * fd_nodes(P)))) * P->ni * nA;

@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kFdTile) fm_disp_f32_kernel(
   }
 }
 
-// The same sum in about 50 instructions a term (the L1 data pipe bounds it; fm_disp_f32_kernel above takes about 180),
+// The same sum in about 47 instructions a term (the L1 data pipe bounds it; fm_disp_f32_kernel above takes about 180),
 // for temperatures above ωq / 40:
 //  * Frequencies in grid units u (the nodes are origin + offset u, whole offsets): x = ω ± ωq is a whole number b,
 //    ωq's being the same for all nodes, and a fraction that all nodes share. A table over b gives the cell that x is in
